@@ -610,6 +610,59 @@ def latent_kv_write(x, norm_weight, eps, inv_freq, interleaved, cache, page_tabl
           _stream())
 
 
+def latent_prefill_supported(dim, rot, value_dim, kv_rank, page_size) -> bool:
+    return bool(load().cpi_latent_prefill_supported(c_int(int(dim)), c_int(int(rot)), c_int(int(value_dim)), c_int(int(kv_rank)),
+                                                    c_int(int(page_size))))
+
+
+def latent_first_row(start, window) -> int:
+    """First position whose cached row the queries of a sequence that continue at `start` need: whole pages of 64."""
+    return max(0, start - window + 1) // 64 * 64 if window else 0
+
+
+def latent_key_rows(pages, out, page_table, batch, *, window=0):
+    """The cached rows that the step's queries can see, sequence after sequence, from pages [pages, 1, 64, row] into the
+    dense matrix out [R, row]: per sequence the positions latent_first_row(start, window) .. start + new - 1."""
+    _need_cuda(pages, out, page_table)
+    row = pages.shape[3]
+    assert pages.is_contiguous() and pages.shape[1:3] == (1, 64) and out.is_contiguous() and out.shape[1] == row
+    assert pages.dtype == out.dtype == torch.bfloat16
+    lengths = [st + n - latent_first_row(st, window) for st, n in zip(batch.starts, batch.n_new)]
+    assert out.shape[0] == sum(lengths)
+    _call("cpi_latent_key_rows", _p(pages), _p(out), c_int(row), _p(page_table), c_int(page_table.shape[1]), _p(batch.seq_slot),
+          _p(batch.seq_start), _p(batch.seq_new), c_int(batch.n_seqs), c_int(max(lengths)), c_int(int(window)), _stream())
+
+
+def latent_q_rows(q, inv_freq, interleaved, out, token_pos, *, n_heads, dim, rot, amplitude=1.0):
+    """out [T, heads * (dim + rot)] = q (float32) in bfloat16, the last `rot` elements of every head rotated by position."""
+    _need_cuda(q, inv_freq, out, token_pos)
+    _rowmajor(q, "latent_q_rows q")
+    T = q.shape[0]
+    assert q.dtype == torch.float32 and out.dtype == torch.bfloat16 and out.is_contiguous()
+    assert q.shape == out.shape == (T, n_heads * (dim + rot))
+    assert inv_freq is None or (inv_freq.dtype == torch.float32 and inv_freq.numel() == rot // 2)
+    _call("cpi_latent_q_rows", _p(q), c_long(q.stride(0)), _p(inv_freq), c_int(int(interleaved)), c_float(float(amplitude)), _p(out),
+          _p(token_pos), c_int(T), c_int(n_heads), c_int(dim), c_int(rot), _stream())
+
+
+def latent_prefill(q, kv, rows, out, batch, *, heads, out_heads, rank, scale, sink=None, window=0):
+    """Prompt attention with formed keys and values: the heads `heads` = (first, past the last) of q [T, out_heads * 192]
+    over kv [R, heads * 256] (a head's 128 key elements, then its 128 value elements) and the rotated key parts
+    rows[:, rank:] of rows [R, rank + 64] (`latent_key_rows`), into those heads of out [T, out_heads * 128]."""
+    h0, h1 = heads
+    _need_cuda(q, kv, rows, out, sink)
+    T, R = batch.n_tokens, rows.shape[0]
+    assert q.dtype == kv.dtype == rows.dtype == out.dtype == torch.bfloat16
+    assert q.is_contiguous() and kv.is_contiguous() and rows.is_contiguous() and out.is_contiguous()
+    assert q.shape == (T, out_heads * 192) and out.shape == (T, out_heads * 128)
+    assert kv.shape == (R, (h1 - h0) * 256) and rows.shape[1] == rank + 64
+    assert sink is None or (sink.dtype == torch.float32 and sink.numel() == out_heads)
+    _call("cpi_latent_prefill", _p(q), _p(kv), _p(rows), c_int(rank), _p(out), c_long(R), _p(batch.token_seq), _p(batch.token_pos),
+          _p(batch.seq_start), _p(batch.seq_new), _p(batch.tile_tok0), _p(batch.tile_rows), c_int(batch.n_q_tiles), c_int(T),
+          c_int(h1 - h0), c_int(out_heads), c_int(h0), c_int(int(window)), c_float(float(scale)), _p(sink),
+          _p(tc_error_flag(q.device)), _stream())
+
+
 def latent_q_split(q, inv_freq, interleaved, plain, full, offsets, rows, token_pos, *, n_heads, dim, rot, rank,
                    amplitude=1.0):
     """From float32 rows q [T, heads * (dim + rot)]: a head's first `dim` elements go to plain[head * T + t] (rows laid

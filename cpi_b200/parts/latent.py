@@ -38,6 +38,12 @@ from .base import Mixer, RotaryEncoding, build_part, register_mixer
 from .linear import MODE_ADD, MODE_STORE, project
 
 
+# set to False to run every prompt over the cached rows themselves (tests compare the two forms)
+use_formed_keys = True
+# bytes of keys and values formed at a time; a step with more forms and attends a few heads after another
+FORMED_BYTES = 1 << 29
+
+
 def use_tensor_core_kernels() -> bool:
     """The switch of the attention part: off, every attention runs through the general kernel."""
     return _attention.use_tensor_core_kernels
@@ -80,7 +86,7 @@ class LatentAttentionMixer(Mixer):
         self.tn = {k: prefix + v for k, v in tn.items()}
         self.ws = workspace
         self.w_down = self.w_uq = self.w_ukT = self.w_uv = self.w_o = None
-        self.w_qnorm = self.w_cnorm = self.sink = self.rotary = None
+        self.w_qnorm = self.w_cnorm = self.sink = self.rotary = self.w_kv = None
 
     def requirements(self):
         t, H = self.tn, self.hidden
@@ -107,6 +113,10 @@ class LatentAttentionMixer(Mixer):
         uk = source.get(t["uk"], device).view(self.nh, self.d, self.kv_rank)
         self.w_ukT = uk.transpose(1, 2).contiguous()                                   # [heads, kv_rank, dim]
         self.w_uv = source.get(t["uv"], device).view(self.nh, self.dv, self.kv_rank).contiguous()
+        if uk.is_cuda and uk.dtype == self.w_uv.dtype == torch.bfloat16 \
+                and K.latent_prefill_supported(self.d, self.r, self.dv, self.kv_rank, 64):
+            # for prompts whose keys and values are formed: head after head its rows of W_uk, then of W_uv
+            self.w_kv = torch.cat([uk, self.w_uv], dim=1).view(self.nh * (self.d + self.dv), self.kv_rank).contiguous()
         self.w_o = source.get(t["o"], device).contiguous()
         self.w_qnorm = f32("dq_norm")
         if self.has_kv:
@@ -128,7 +138,7 @@ class LatentAttentionMixer(Mixer):
 
     def forward(self, h, residual, batch, cache, add=True):
         T, f32, dt = h.shape[0], torch.float32, h.dtype
-        H, D, R, rank, row = self.nh, self.d, self.r, self.kv_rank, self.row
+        H, D, R, rank = self.nh, self.d, self.r, self.kv_rank
         pages, table, page_size = cache.stream("latent")
         inv_freq = None if self.rotary is None else self.rotary.inv_freq
         inter = self.rotary is not None and self.rotary.interleaved
@@ -147,6 +157,60 @@ class LatentAttentionMixer(Mixer):
         q = self.ws.get("latent_q", (T, H * (D + R)), f32)
         with phase("qkv"):
             project(cq, self.w_uq, q)
+        out = self.ws.get("latent_values", (T, H * self.dv), dt)
+        if self._forms_keys(batch, dt, page_size):
+            self._attend_formed(q, out, pages, table, batch, inv_freq, inter, amp)
+        else:
+            self._attend_latent(q, out, pages, table, page_size, batch, inv_freq, inter, amp)
+        if self.gate_rows:
+            with phase("head_post"):
+                K.head_turn(out, out, batch.token_pos, n_heads=H, value_dim=self.dv, gate=gate)
+        with phase("wo"):
+            project(out, self.w_o, residual, MODE_ADD if add else MODE_STORE)
+
+    # ---- keys and values formed for the step
+    def _forms_keys(self, batch, dt, page_size) -> bool:
+        """Whether a step forms the heads' keys and values: prompts in bfloat16 with heads of the kernel's sizes.
+
+        Forming costs time with the rows of all sequences together (0.7 ns a row and head at a latent rank of 512);
+        the other form takes a sequence's keys one tile after another in one block, 0.1 us a key, however few its queries
+        are, and with many queries it does 3.4 times the arithmetic.  So forming loses only where few queries meet a key
+        AND many sequences share the launch.  Measured with 16 heads (formed / not): one prompt of 2,048 tokens 180 / 723
+        us, of 4,096 309 / 2,188; 2 tokens behind 2,000 positions 95 / 233; 8 prompts of 20 tokens 82 / 93; but 16 sequences
+        of 2 tokens behind 1,000 positions 221 / 153, and the line lies between the last two."""
+        if (self.w_kv is None or not use_formed_keys or not use_tensor_core_kernels() or dt != torch.bfloat16 or batch.is_decode
+                or not batch.n_q_tiles or not K.latent_prefill_supported(self.d, self.r, self.dv, self.kv_rank, page_size)):
+            return False
+        rows = pairs = longest = 0
+        for start, n in zip(batch.starts, batch.n_new):
+            keys = start + n - K.latent_first_row(start, self.window)
+            rows, longest = rows + keys, max(longest, keys)
+            pairs += n * min(start + (n + 1) // 2, self.window or start + n)
+        return pairs >= 32 * rows or rows * self.nh <= 128 * longest
+
+    def _attend_formed(self, q, out, pages, table, batch, inv_freq, inter, amp):
+        H, D, R, rank, bf16 = self.nh, self.d, self.r, self.kv_rank, torch.bfloat16
+        n_rows = sum(start + n - K.latent_first_row(start, self.window) for start, n in zip(batch.starts, batch.n_new))
+        rows = self.ws.get("latent_key_rows", (n_rows, self.row), bf16)
+        heads = self.ws.get("latent_q_heads", (batch.n_tokens, H * (D + R)), bf16)
+        with phase("kv_store"):
+            K.latent_key_rows(pages, rows, table, batch, window=self.window)
+            K.latent_q_rows(q, inv_freq, inter, heads, batch.token_pos, n_heads=H, dim=D, rot=R, amplitude=amp)
+        per = D + self.dv
+        group = max(1, min(H, FORMED_BYTES // (2 * n_rows * per)))
+        for h0 in range(0, H, group):
+            h1 = min(H, h0 + group)
+            kv = self.ws.get("latent_formed", (n_rows, (h1 - h0) * per), bf16)
+            with phase("qkv"):
+                project(rows[:, :rank], self.w_kv[h0 * per:h1 * per], kv)
+            with phase("latent_attention"):
+                K.latent_prefill(heads, kv, rows, out, batch, heads=(h0, h1), out_heads=H, rank=rank, scale=self.scale,
+                                 sink=self.sink, window=self.window)
+
+    # ---- attention over the cached rows themselves
+    def _attend_latent(self, q, out, pages, table, page_size, batch, inv_freq, inter, amp):
+        T, dt = q.shape[0], out.dtype
+        H, D, R, rank, row = self.nh, self.d, self.r, self.kv_rank, self.row
         plain = self.ws.get("latent_q_plain", (H * T, D), dt)               # head-major rows
         full = self.ws.get("latent_q_full", (T, H * row), dt)
         offsets = self.ws.get("latent_offsets", (H + 1,), torch.int32)
@@ -158,7 +222,6 @@ class LatentAttentionMixer(Mixer):
             project(plain, self.w_ukT, full.view(T * H, row)[:, :rank], MODE_STORE, out_rows=rows, group_offsets=offsets,
                     n_groups=H, rows_per_group_hint=T)
         lat = self.ws.get("latent_att_heads", (H * T, rank), dt)            # head-major, the latent part only
-        out = self.ws.get("latent_values", (T, H * self.dv), dt)
         if use_tensor_core_kernels() and dt == torch.bfloat16 and K.latent_attention_supported(row, rank):
             with phase("latent_attention"):
                 if batch.is_decode:
@@ -185,8 +248,3 @@ class LatentAttentionMixer(Mixer):
         with phase("wo"):
             project(lat, self.w_uv, out.view(T * H, self.dv), MODE_STORE, out_rows=rows, group_offsets=offsets,
                     n_groups=H, rows_per_group_hint=T)
-        if self.gate_rows:
-            with phase("head_post"):
-                K.head_turn(out, out, batch.token_pos, n_heads=H, value_dim=self.dv, gate=gate)
-        with phase("wo"):
-            project(out, self.w_o, residual, MODE_ADD if add else MODE_STORE)
