@@ -817,6 +817,43 @@ def linear_scan(k, q, v, state, out, batch, *, n_heads, heads_per_group, n_rows,
     launch_count += 2 if run_len else 0
 
 
+def linear_chunks_supported(n_rows, n_cols) -> bool:
+    return bool(load().cpi_linear_chunks_supported(c_int(int(n_rows)), c_int(int(n_cols))))
+
+
+def linear_chunks_scratch(n_heads, heads_per_group, n_rows, n_cols, *, z=None, beta=None) -> int:
+    """Floats of scratch that `linear_chunks` needs per chunk of 64 tokens."""
+    fn = load().cpi_linear_chunks_scratch
+    fn.restype = c_long
+    return int(fn(c_int(0 if z is None else 1 if beta is None else 2), c_int(n_heads), c_int(n_heads // heads_per_group),
+                  c_int(n_rows), c_int(n_cols)))
+
+
+def linear_chunks(k, q, v, state, out, batch, *, n_heads, heads_per_group, n_rows, n_cols, scratch, z=None, z_bias=None, tau=1.0,
+                  decay_kind=0, dt=None, dt_bias=None, a_log=None, skip=None, q_scale=1.0, beta=None):
+    """`linear_scan` over prompts, in chunks of 64 tokens worked on side by side (see recurrent_chunks.cu): with `z` the
+    row decays before their transform, or with `dt` the raw step sizes; `beta`: the delta rule.  `scratch`: float32, a
+    multiple of `linear_chunks_scratch` elements; the step runs in segments of as many chunks as that holds."""
+    global launch_count
+    small = [t for t in (z_bias, dt_bias, a_log, skip) if t is not None]
+    _need_cuda(k, q, v, state, out, z, dt, beta, scratch, *small)
+    for t in (k, q, v, out, z, dt, beta):
+        assert t is None or (t.dtype == torch.float32 and t.dim() == 2 and t.stride(1) == 1)
+    assert state.dtype == torch.float32 and state.is_contiguous() and tuple(state.shape[1:]) == (n_heads, n_rows, n_cols)
+    sd = small[0].dtype if small else torch.float32
+    assert all(t.dtype == sd and t.is_contiguous() for t in small)
+    total = sum(-(-n // 64) for n in batch.n_new)
+    seg = min(total, scratch.numel() // linear_chunks_scratch(n_heads, heads_per_group, n_rows, n_cols, z=z, beta=beta))
+    assert scratch.dtype == torch.float32 and scratch.is_contiguous() and seg > 0
+    _call("cpi_linear_chunks", _p(k), c_long(k.stride(0)), _p(q), c_long(q.stride(0)), _p(v), c_long(v.stride(0)),
+          _p(z), c_long(0 if z is None else z.stride(0)), _p(z_bias), c_float(1.0 / float(tau)), c_int(int(decay_kind)),
+          _p(dt), c_long(0 if dt is None else dt.stride(0)), _p(dt_bias), _p(a_log),
+          _p(skip), c_int(dtype_code(sd)), _p(beta), c_long(0 if beta is None else beta.stride(0)), c_float(q_scale), _p(state),
+          _p(out), c_long(out.stride(0)), _p(batch.seq_slot), _p(batch.seq_tok0), _p(batch.seq_new), c_int(batch.n_seqs),
+          c_int(total), c_int(n_heads), c_int(heads_per_group), c_int(n_rows), c_int(n_cols), _p(scratch), c_int(seg), _stream())
+    launch_count += 4 * -(-total // seg) - 1
+
+
 def silu_rows(x, out=None):
     """out = silu(x) over float32 rows (a column slice allowed); out float32 or bfloat16, by default x itself."""
     out = x if out is None else out

@@ -31,7 +31,7 @@
 //
 // A sequence's tokens are visited in order by one block per (sequence, head, slice of columns) with the same
 // arithmetic whether they come in one step or one at a time, so results do not depend on how a prompt is cut.
-#include "common.cuh"
+#include "decay.cuh"
 
 namespace cpi {
 
@@ -119,16 +119,6 @@ struct ScanParams {
 };
 
 enum ScanDecay : int { kStepDecay = 0, kRowDecay = 1, kConstDecay = 2, kConstDecayRuns = 3 };      // the last: what a run adds, no outputs
-
-__device__ __forceinline__ float softplus_f(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
-__device__ __forceinline__ float log_sigmoid_f(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
-// a = sigmoid(z + b)^(1 / tau); one function for the kernel that prepares a prompt's decays and for the recurrence
-// that computes a decoded token's own, so that both give the same bits
-// (kind 1: a = exp(-rate * softplus(z + b)), rate = exp(A_log) of the row's head)
-__device__ __forceinline__ float row_decay_f(float z, float b, float inv_tau, int kind = 0, float rate = 0.f) {
-  if (kind == 1) return expf(-rate * softplus_f(z + b));
-  return expf(log_sigmoid_f(z + b) * inv_tau);
-}
 
 struct RowDecayParams {
   float* z; long z_stride; const void* bias; int bias_dtype; float inv_tau; int n;

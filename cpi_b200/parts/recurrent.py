@@ -37,8 +37,16 @@ from .linear import MODE_ADD, MODE_STORE, project
 
 # steps whose longest portion has more tokens than this prepare the row decays with a kernel of their own
 DECAY_PREPASS_FROM = 16
-# set to False to run every recurrence with constant decays token by token (tests compare the two)
+# set to False to run every recurrence token by token (tests compare the two)
 use_chunked_kernel = True
+# A bfloat16 prompt's recurrence runs in chunks when its longest portion has this many tokens: the scan's time goes with the
+# longest portion, the chunks' with all tokens.  Mixers of width 2,048, chunks / scan in us, a prompt of 200, of 130, 8 of 200
+# and 32 of 100 tokens: gated linear attention (8 heads, 128 x 256) 113 / 124, 98 / 92, 213 / 322, 402 / 681; state space (64
+# heads, 128 x 64) 121 / 172, 104 / 114, 406 / 536, 818 / 1,048; delta rule (8 heads, 128 x 256) 134 / 128, 117 / 95, 357 / 414,
+# 709 / 789, a prompt of 500 178 / 231.
+CHUNKS_FROM, DELTA_CHUNKS_FROM = 192, 256
+# bytes of scratch for a step's chunks; a longer step runs in segments (a segment's states stay in the L2 between its passes)
+CHUNK_BYTES = 96 << 20
 # a recurrence with constant decays is cut into runs of at least this many tokens, until its blocks fill the GPU this often
 RUN_TOKENS = 64
 RUN_BLOCKS_PER_SM = 4
@@ -48,6 +56,30 @@ MAX_STATE_ROWS = 1024             # rows of a head's state that the recurrence's
 def _cat_rows(tensors):
     dt = torch.float32 if any(t.dtype == torch.float32 for t in tensors) else torch.bfloat16
     return torch.cat([t.to(dt) for t in tensors], dim=0).contiguous()
+
+
+def recurrence(ws, dtype, k, q, v, state, out, batch, *, n_heads, heads_per_group, n_rows, n_cols, z=None, z_bias=None, tau=1.0,
+               decay_kind=0, a_log=None, **kw):
+    """The recurrence of a step with data-dependent decays (`K.linear_scan`).  A long bfloat16 prompt's runs in chunks side
+    by side.  In float32 every token is visited in order, so that results do not depend on how a prompt is cut; a step of
+    many tokens prepares its row decays once per element instead of once per block of columns, a decode step leaves them
+    to the recurrence (one launch less), which computes the same expression."""
+    kw.update(n_heads=n_heads, heads_per_group=heads_per_group, n_rows=n_rows, n_cols=n_cols, z=z, a_log=a_log)
+    least = CHUNKS_FROM if kw.get("beta") is None else DELTA_CHUNKS_FROM
+    if (use_chunked_kernel and dtype == torch.bfloat16 and batch.max_new >= least and K.linear_chunks_supported(n_rows, n_cols)
+            and all(t is None or (t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0) for t in (k, q, v, z, out))):
+        per = K.linear_chunks_scratch(n_heads, heads_per_group, n_rows, n_cols, z=z, beta=kw.get("beta"))
+        total = sum(-(-n // 64) for n in batch.n_new)
+        chunks = -(-total // -(-total // max(1, CHUNK_BYTES // (4 * per))))            # segments of about the same length
+        scratch = ws.get("recurrence_chunks", (chunks * per,), torch.float32)
+        K.linear_chunks(k, q, v, state, out, batch, scratch=scratch, z_bias=z_bias, tau=tau, decay_kind=decay_kind, **kw)
+        return
+    if z is not None:
+        ready = batch.max_new > DECAY_PREPASS_FROM
+        if ready:
+            K.row_decay(z, z_bias, tau, kind=decay_kind, a_log=a_log, rows_per_head=n_rows)
+        kw.update(z_bias=z_bias, tau=tau, decay_ready=ready, decay_kind=decay_kind)
+    K.linear_scan(k, q, v, state, out, batch, **kw)
 
 
 @register_mixer("mamba2")
@@ -111,10 +143,9 @@ class Mamba2Mixer(Mixer):
                           batch, silu=True)
         y = self.ws.get("mamba_y", (T, inner), f32)
         with phase("scan"):
-            K.linear_scan(xbc[:, inner:inner + gn], xbc[:, inner + gn:], xbc[:, :inner], cache.state("ssm"), y, batch,
-                          n_heads=self.nh, heads_per_group=self.nh // self.groups, n_rows=self.n, n_cols=self.dv,
-                          dt=proj[:, inner + self.channels:], dt_bias=self.dt_bias, a_log=self.a_log,
-                          skip=self.d_skip)
+            recurrence(self.ws, h.dtype, xbc[:, inner:inner + gn], xbc[:, inner + gn:], xbc[:, :inner], cache.state("ssm"), y, batch,
+                       n_heads=self.nh, heads_per_group=self.nh // self.groups, n_rows=self.n, n_cols=self.dv,
+                       dt=proj[:, inner + self.channels:], dt_bias=self.dt_bias, a_log=self.a_log, skip=self.d_skip)
         with phase("gated_norm"):
             g = self.ws.get("mamba_gated", (T, inner), h.dtype)
             K.gated_norm(y, proj[:, :inner], self.w_norm, g, parts=self.norm_groups, gate_first=True, eps=self.eps)
@@ -175,15 +206,9 @@ class GLAMixer(Mixer):
             project(low, self.w_a2, z)
         o = self.ws.get("gla_o", (T, nv), f32)
         with phase("scan"):
-            # a step of many tokens prepares its decays once per element; a decode step leaves them to the
-            # recurrence (one launch less), which computes the same expression
-            ready = batch.max_new > DECAY_PREPASS_FROM
-            if ready:
-                K.row_decay(z, self.b_a2, self.tau)
-            K.linear_scan(proj[:, nk:2 * nk], proj[:, :nk], proj[:, 2 * nk:2 * nk + nv], cache.state("s"), o, batch,
-                          n_heads=self.nh, heads_per_group=1, n_rows=self.dk, n_cols=self.dv, z=z,
-                          z_bias=None if ready else self.b_a2, tau=self.tau, q_scale=self.dk ** -0.5,
-                          decay_ready=ready)
+            recurrence(self.ws, h.dtype, proj[:, nk:2 * nk], proj[:, :nk], proj[:, 2 * nk:2 * nk + nv], cache.state("s"), o, batch,
+                       n_heads=self.nh, heads_per_group=1, n_rows=self.dk, n_cols=self.dv, z=z, z_bias=self.b_a2, tau=self.tau,
+                       q_scale=self.dk ** -0.5)
         with phase("gated_norm"):
             g = self.ws.get("gla_gated", (T, nv), h.dtype)
             K.gated_norm(o, proj[:, 2 * nk + nv:], self.w_norm, g, parts=self.nh, gate_first=False, eps=self.eps)
@@ -276,13 +301,9 @@ class GatedDeltaMixer(Mixer):
             K.head_unit(qkv[:, :2 * nqk], heads=2 * self.nkv, dim=self.dk, eps=self.unit_eps)
         o = self.ws.get("gdr_o", (T, nv), f32)
         with phase("scan"):
-            ready = batch.max_new > DECAY_PREPASS_FROM
-            if ready:
-                K.row_decay(z, self.dt_bias, 1.0, kind=1, a_log=self.a_log, rows_per_head=self.dk)
-            K.linear_scan(qkv[:, nqk:2 * nqk], qkv[:, :nqk], qkv[:, 2 * nqk:], cache.state("s"), o, batch,
-                          n_heads=self.nh, heads_per_group=self.nh // self.nkv, n_rows=self.dk, n_cols=self.dv, z=z,
-                          z_bias=self.dt_bias, a_log=self.a_log, decay_kind=1, decay_ready=ready,
-                          q_scale=self.dk ** -0.5, beta=proj[:, o_b:o_a])
+            recurrence(self.ws, h.dtype, qkv[:, nqk:2 * nqk], qkv[:, :nqk], qkv[:, 2 * nqk:], cache.state("s"), o, batch,
+                       n_heads=self.nh, heads_per_group=self.nh // self.nkv, n_rows=self.dk, n_cols=self.dv, z=z,
+                       z_bias=self.dt_bias, a_log=self.a_log, decay_kind=1, q_scale=self.dk ** -0.5, beta=proj[:, o_b:o_a])
         with phase("gated_norm"):
             g = self.ws.get("gdr_gated", (T, nv), h.dtype)
             K.gated_norm(o, gate, self.w_norm, g, parts=self.nh, gate_first=False, eps=self.eps, gate_act="sigmoid")

@@ -1,0 +1,118 @@
+"""The recurrences in chunks against a token-by-token scan in 64 bits, and against the float32 scan's own error."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _plain(a, k, q, v, S, beta=None):
+    """S <- diag(a) S; S += k u^T with u = v, or beta (v - S^T k); o = S^T q.  a, k, q [T, H, N], v [T, H, Dv], S [H, N, Dv]."""
+    S, o = S.clone(), torch.empty_like(v)
+    for t in range(v.shape[0]):
+        S *= a[t][:, :, None]
+        u = v[t] if beta is None else beta[t][:, None] * (v[t] - torch.einsum("hnv,hn->hv", S, k[t]))
+        S += k[t][:, :, None] * u[:, None, :]
+        o[t] = torch.einsum("hnv,hn->hv", S, q[t])
+    return o, S
+
+
+def _batch(new, slots):
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    tok0 = [sum(new[:i]) for i in range(len(new))]
+    return SimpleNamespace(n_seqs=len(new), n_new=new, max_new=max(new), seq_slot=i32(slots), seq_tok0=i32(tok0), seq_new=i32(new))
+
+
+# edges of a chunk of 64 (one token less and more, one token), unequal sequences, segments shorter than the step, heads that
+# share q and k, decays from none to all, both sizes of a state's rows and one to four tiles of columns
+@pytest.mark.parametrize("kind", ["rows", "step", "delta"])
+@pytest.mark.parametrize("new,seg,rows,cols,decays", [
+    ([64], 1, 64, 64, "slow"), ([65], 2, 128, 64, "fast"), ([63, 1, 130], 3, 64, 128, "slow"), ([300], 2, 128, 256, "mixed"),
+    ([127, 128, 129], 1, 128, 128, "mixed"), ([1], 1, 64, 64, "none"), ([513, 70], 20, 64, 192, "fast"),
+    ([2] * 40 + [200, 3], 5, 64, 64, "mixed")])
+def test_chunks_equal_the_scan(kind, new, seg, rows, cols, decays):
+    from cpi_b200.csrc import lib as K
+    g = torch.Generator(device=DEV).manual_seed(5)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    rand = lambda *s: torch.rand(*s, generator=g, device=DEV)
+    T, H, hpg, B = sum(new), 4, 2, len(new)
+    G = H // hpg
+    k, q, v = randn(T, G * rows), randn(T, G * rows), randn(T, H * cols + 4)[:, :H * cols]
+    if kind == "delta":                                      # unit keys, as the mixer's are
+        k = torch.nn.functional.normalize(k.view(T, G, rows), dim=-1).view(T, G * rows)
+    skip = None
+    if kind == "step":
+        raw, bias, a_log, skip = randn(T, H), randn(H), randn(H), randn(H)
+        a_log += {"slow": -4.0, "fast": 2.0, "mixed": 0.0, "none": -40.0}[decays]
+        kw = dict(dt=raw, dt_bias=bias, a_log=a_log, skip=skip)
+        dt = torch.nn.functional.softplus(raw.double() + bias.double())
+        a = torch.exp(-torch.exp(a_log.double()) * dt)[:, :, None].expand(T, H, rows)
+    else:
+        # z such that sigmoid(z + bias)^(1 / tau) covers the decays; -inf and inf give 0 and 1
+        a = {"slow": 0.9 + 0.1 * rand(T, H, rows), "fast": rand(T, H, rows) ** 4, "none": torch.ones(T, H, rows, device=DEV),
+             "mixed": (rand(T, H, rows) * 1.5).clamp(max=1.0) * (rand(T, H, rows) > 0.02)}[decays]
+        kw = dict(z=torch.logit(a.double() ** 2).float().view(T, H * rows), z_bias=randn(H * rows), tau=2.0)
+        zd = (kw["z"].double() + kw["z_bias"].double()).view(T, H, rows)
+        a = torch.sigmoid(zd) ** 0.5
+        if kind == "delta":                                  # its decays: exp(-rate softplus(z + bias))
+            kw.update(beta=randn(T, H), decay_kind=1, a_log=randn(H), z=kw["z"].clamp(min=-30.0))
+            zd = (kw["z"].double() + kw["z_bias"].double()).view(T, H, rows)
+            a = torch.exp(-torch.exp(kw["a_log"].double())[:, None] * torch.nn.functional.softplus(zd))
+    slots = [B - i for i in range(B)]                        # another order, slot 0 unused
+    state = randn(B + 1, H, rows, cols)
+    batch, q_scale = _batch(new, slots), 0.25
+    per = K.linear_chunks_scratch(H, hpg, rows, cols, z=kw.get("z"), beta=kw.get("beta"))
+    scratch = torch.full((seg * per,), float("nan"), device=DEV)             # nothing is read that was not written
+    S, out = state.clone(), torch.full((T, H * cols), float("nan"), device=DEV)
+    size = dict(n_heads=H, heads_per_group=hpg, n_rows=rows, n_cols=cols)
+    K.linear_chunks(k, q, v, S, out, batch, scratch=scratch, q_scale=q_scale, **size, **kw)
+    S2, out2 = state.clone(), torch.empty_like(out)
+    K.linear_scan(k, q, v, S2, out2, batch, q_scale=q_scale, **size, **kw)
+    assert torch.equal(S[0], state[0])
+    kd, qd = (x.double().view(T, G, rows).repeat_interleave(hpg, 1) for x in (k, q))
+    vd, t0 = v.double().reshape(T, H, cols), 0
+    for n, slot in zip(new, slots):
+        sl = slice(t0, t0 + n)
+        vv = vd[sl] * (dt[sl][:, :, None] if kind == "step" else 1.0)
+        beta = torch.sigmoid(kw["beta"].double()[sl]) if kind == "delta" else None
+        o, ref = _plain(a.double()[sl], kd[sl], qd[sl] * q_scale, vv, state[slot].double(), beta)
+        if skip is not None:
+            o = o + skip.double()[:, None] * vd[sl]
+        err = lambda x, y: float((x.double() - y).norm() / y.norm())
+        # the scan's own error, and 2^-22 for sums of 64 terms taken in another order
+        assert err(out[sl].view(n, H, cols), o) <= 1.5 * err(out2[sl].view(n, H, cols), o) + 2.0 ** -22
+        assert err(S[slot], ref) <= 1.5 * err(S2[slot], ref) + 2.0 ** -22
+        t0 += n
+
+
+@pytest.mark.parametrize("kind", ["rows", "step", "delta"])
+def test_an_output_reads_nothing_of_later_tokens(kind):
+    """A NaN in a token's q, k, v and decay leaves the bits of every earlier token's output as they were."""
+    from cpi_b200.csrc import lib as K
+    g = torch.Generator(device=DEV).manual_seed(2)
+    T, H, rows, cols, at = 150, 2, 64, 64, 83
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    x = {n: randn(T, H * rows) * 0.2 for n in ("k", "q", "v")}
+    fixed = {}
+    if kind == "step":
+        x.update(dt=randn(T, H))
+        fixed = dict(dt_bias=randn(H), a_log=randn(H))
+    else:
+        x.update(z=torch.rand(T, H * rows, generator=g, device=DEV))
+        if kind == "delta":
+            x.update(beta=randn(T, H))
+    got = []
+    for broken in (False, True):
+        y = {n: t.clone() for n, t in x.items()}
+        if broken:
+            for t in y.values():
+                t[at] = float("nan")
+        per = K.linear_chunks_scratch(H, 1, rows, cols, z=y.get("z"), beta=y.get("beta"))
+        out = torch.zeros(T, H * cols, device=DEV)
+        K.linear_chunks(y.pop("k"), y.pop("q"), y.pop("v"), torch.zeros(1, H, rows, cols, device=DEV), out, _batch([T], [0]),
+                        scratch=torch.empty(3 * per, device=DEV), n_heads=H, heads_per_group=1, n_rows=rows,
+                        n_cols=cols, **y, **fixed)
+        got.append(out)
+    assert torch.equal(got[0][:at], got[1][:at]) and bool(got[1][at:].isnan().all())
