@@ -69,6 +69,8 @@ from .linear import MODE_ADD, MODE_STORE, project
 
 # set to False to run every attention through the general kernel (tests compare the two families)
 use_tensor_core_kernels = True
+# set to False to run every float32 attention query by query (tests compare the two)
+use_tile_kernel = True
 # set to False to prepare q, k and v with the separate general kernels (tests compare the two)
 use_fused_preparation = True
 
@@ -445,6 +447,16 @@ def attend(q, att, k_cache, v_cache, table, page_size, batch, *, n_heads, n_kv_h
                             n_kv_heads=nkv, head_dim=d, window_kind=wk, window_size=window_size,
                             scale=scale, sink=sink, keep_first=keep_first, softcap=softcap)
         return
+    if (use_tile_kernel and q.dtype == torch.float32 and not batch.is_decode and batch.n_q_tiles and d == dv and d in (64, 128)
+            and score_bias is None):
+        # a sliding window that reaches over every sequence so far is no window
+        everything = window_kind == "full" or (window_kind == "sliding"
+                                               and max(s + n for s, n in zip(batch.starts, batch.n_new)) <= window_size)
+        if everything or window_kind == "chunk":
+            K.attention_f32_tiles(q, att, k_cache, v_cache, table, page_size, batch, n_heads=nh, n_kv_heads=nkv, head_dim=d,
+                                  window_kind=K.WINDOW_FULL if everything else wk, window_size=window_size, scale=scale, sink=sink,
+                                  softcap=softcap)
+            return
     K.attention_general(q, att, k_cache, v_cache, table, page_size, batch.token_seq, batch.token_pos,
                         batch.seq_slot, n_heads=nh, n_kv_heads=nkv, head_dim=d, window_kind=wk,
                         window_size=window_size, scale=scale, score_bias=score_bias, sink=sink, value_dim=dv,
