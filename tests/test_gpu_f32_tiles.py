@@ -41,3 +41,33 @@ def test_attention_tiles_give_the_bits_of_the_general_kernel(starts, new, window
     K.attention_general(q, want, k, v, table, page, batch.token_seq, batch.token_pos, batch.seq_slot, **kw)
     K.attention_f32_tiles(q, got, k, v, table, page, batch, **kw)
     assert bool(want.isfinite().all()) and torch.equal(got, want)
+
+
+# both tile widths (64 and 128 weight rows), edges of both, K that is no multiple of 16 or 4, unaligned rows, groups of unequal
+# rows (one empty), a row gather and scatter, every mode and pair of types
+@pytest.mark.parametrize("M,N,K", [(64, 64, 16), (65, 129, 50), (200, 30, 7), (130, 4100, 64), (17, 1, 129), (700, 2056, 33)])
+@pytest.mark.parametrize("mode", [0, 1, 2, 3, 4, 5, 6])
+def test_products_of_many_rows_give_the_bits_of_the_kernel_for_few(M, N, K, mode):
+    from cpi_b200.csrc import lib as L
+    g = torch.Generator(device=DEV).manual_seed(M + mode)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    glu = mode in L.GATED_MODES
+    types = [(torch.float32, torch.float32, torch.float32), (torch.float32, torch.bfloat16, torch.float32),
+             (torch.bfloat16, torch.bfloat16, torch.bfloat16 if mode != 1 else torch.float32)]
+    for i, (ta, tw, to) in enumerate(types):
+        off = i % 2                                          # rows that do not start on 16 bytes
+        a = randn(M + 5, K + 4 * off + off).to(ta)[:, off:off + K]
+        groups = 3
+        w = (randn(groups, (2 if glu else 1) * N, K) * 0.1).to(tw)
+        rows = torch.randperm(M + 5, generator=g, device=DEV)[:M].int()
+        cut = M // 3
+        offsets = torch.tensor([0, cut, cut, M], dtype=torch.int32, device=DEV)
+        scale = randn(M)
+        for kw in (dict(), dict(a_rows=rows, group_offsets=offsets, n_groups=groups, row_scale=scale, out_rows=rows)):
+            ww = w if kw else w[0]
+            outs = []
+            for hint in (16, 64):
+                out = torch.linspace(-1, 1, (M + 5) * N, device=DEV).view(M + 5, N).to(to)
+                L.gemm_simt(a, ww, out, mode, m_rows=M, rows_per_group_hint=hint, gate_limit=0.7, **kw)
+                outs.append(out)
+            assert torch.equal(outs[0], outs[1]) and bool(outs[0].isfinite().all())
