@@ -557,8 +557,7 @@ __global__ void __launch_bounds__(F32_THREADS) attention_f32_tile_kernel(AttnPar
   float *kv = sm, *qs = kv + F32_K * LD, *ss = qs + F32_Q * LD, *al = ss + F32_K * LDS, *ls = al + F32_Q;
   int* nv = reinterpret_cast<int*>(ls + F32_Q);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait();                                                    // (no early launch of what follows: its waiting blocks slow this down)
   const int tile = blockIdx.x / subs, r0 = blockIdx.x % subs * F32_Q;
   const int rows = min(F32_Q, tile_rows[tile] - r0);
   if (rows <= 0) return;

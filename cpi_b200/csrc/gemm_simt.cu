@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(NT) gemm_simt_kernel(GemmParams p) {
 // its activation loads each take two cycles of the shared-memory pipe (32 distinct ones take eight).  The next 16 k come
 // through registers while 16 are multiplied.
 // Bound: the FP32 pipe with enough warps (one warp per scheduler issues packed instructions at half rate, three at 0.95 of it);
-// 509 x 2,048 -> 3,072 and 2,048 in float32: 984 -> 699 us together (the kernel above with 64 rows a tile before).
+// 509 x 2,048 -> 3,072 and 2,048 in float32: 984 -> 343 us together (the kernel above with 64 rows a tile before).
 template <typename T>
 __device__ __forceinline__ void load4(const T* p, bool live, bool vec, int k, int K, float (&v)[4]) {
   if (!live) { v[0] = v[1] = v[2] = v[3] = 0.f; return; }
@@ -187,7 +187,6 @@ __global__ void __launch_bounds__(TILE_THREADS) gemm_simt_tile_kernel(GemmParams
   constexpr int COLS = RT * 16, HALF = COLS / 2, OUT = GLU ? HALF : COLS;      // weight rows, their halves, output columns
   constexpr int LDM = TILE_ROWS + 4, LDC = COLS + 4, LA = TILE_ROWS * BK / 4 / TILE_THREADS, LW = COLS * BK / 4 / TILE_THREADS;
   __shared__ __align__(16) float As[2][BK][LDM], Ws[2][BK][LDC];
-  pdl_launch_dependents();
   pdl_wait();
   int m_begin = 0, m_end = p.M;
   const TW* w = reinterpret_cast<const TW*>(p.w);
@@ -275,6 +274,9 @@ __global__ void __launch_bounds__(TILE_THREADS) gemm_simt_tile_kernel(GemmParams
     if (more) stash(b ^ 1);
     __syncthreads();
   }
+  // (not earlier: blocks of the next kernel that wait beside the running ones slow them down, 343 us became 699 for the two
+  // products of the figure above)
+  pdl_launch_dependents();
 
   TO* out = reinterpret_cast<TO*>(p.out);
 #pragma unroll
