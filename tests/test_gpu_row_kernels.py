@@ -1,0 +1,52 @@
+"""Row kernels with more than one route: the vectorised convolution, the warp-sized gated norm, the choice and the lists of
+routed experts, and products whose features are no multiple of the two-SM kernel's tile."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rand(seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return lambda *s: torch.randn(*s, generator=g, device=DEV)
+
+
+# one and eight tokens a thread (by the number of blocks), sequence ends inside a thread's run, steps shorter than the taps
+@pytest.mark.parametrize("taps", [1, 2, 4, 8])
+@pytest.mark.parametrize("new,channels", [([1, 1, 1], 12), ([3, 2, 40], 516), ([309, 1, 9, 7], 4100)])
+def test_convolution_routes_give_the_same_bits(taps, new, channels):
+    from cpi_b200.csrc import lib as K
+    from cpi_b200.engine.batch import BatchStager
+    randn = _rand(taps)
+    T, B = sum(new), len(new)
+    stager = BatchStager(DEV)
+    batch = stager.stage(list(range(B)), [5] * B, [[0] * n for n in new], [[]] * B, torch.float32)
+    x, w, b, ib = randn(T, channels + 4), randn(channels, taps), randn(channels), randn(channels)
+    wide = torch.zeros(T, channels + 5, device=DEV)
+    wide[:, 1:] = x                                          # the same rows off their 16 bytes: the kernel without vectors
+    carry = randn(B, max(taps - 1, 0), channels)
+    outs = []
+    for rows in (x[:, 4:], wide[:, 5:]):
+        c, out = carry.clone(), torch.empty(T, channels, device=DEV)
+        K.causal_conv(rows, w, b, c, out, batch, silu=True, in_bias=ib)
+        outs.append((out, c))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("n", [4, 100, 128, 132, 256, 260, 512, 516, 1020, 1024])
+@pytest.mark.parametrize("first,act,shared", [(True, "silu", False), (False, "sigmoid", True), (False, "silu", False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_norm_of_every_width(n, first, act, shared, dtype):
+    from cpi_b200.csrc import lib as K
+    randn, T, parts = _rand(n), 7, 3
+    y, gate, w = randn(T, parts * n), randn(T, parts * n + 4)[:, 4:], randn(n if shared else parts * n)
+    out = torch.empty(T, parts * n, device=DEV, dtype=dtype)
+    K.gated_norm(y, gate, w, out, parts=parts, gate_first=first, eps=1e-5, gate_act=act)
+    g = torch.sigmoid(gate.double()) * (gate.double() if act == "silu" else 1.0)
+    v = (y.double() * g if first else y.double()).view(T, parts, n)
+    ref = (v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5)) * w.double().view(-1, n)
+    ref = ref.reshape(T, -1) * (1.0 if first else g)
+    # float32: the sum of n squares and a dozen operations; bfloat16: one rounding to 8 bits more
+    tol = 2.0 ** -19 if dtype == torch.float32 else 2.0 ** -8 * 1.01
+    assert bool(((out.double() - ref).abs() <= tol * ref.abs() + 2.0 ** -21 * ref.abs().max()).all())
