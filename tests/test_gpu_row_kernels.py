@@ -50,3 +50,43 @@ def test_gated_norm_of_every_width(n, first, act, shared, dtype):
     # float32: the sum of n squares and a dozen operations; bfloat16: one rounding to 8 bits more
     tol = 2.0 ** -19 if dtype == torch.float32 else 2.0 ** -8 * 1.01
     assert bool(((out.double() - ref).abs() <= tol * ref.abs() + 2.0 ** -21 * ref.abs().max()).all())
+
+
+@pytest.mark.parametrize("experts,top_k", [(1, 1), (16, 4), (33, 33), (256, 8), (40, 35)])
+@pytest.mark.parametrize("mode", [False, True, "softmax_chosen"])
+def test_choice_of_experts_with_ties_and_nan(experts, top_k, mode):
+    from cpi_b200.csrc import lib as K
+    T, randn = 70, _rand(experts)
+    logits = (randn(T, experts) * 2).round() / 2             # many ties
+    logits[3] = float("nan")
+    logits[4, ::2] = float("nan")
+    logits[5] = float("-inf")
+    logits[6, 0] = -0.0
+    idx, gate = torch.empty(T, top_k, dtype=torch.int32, device=DEV), torch.empty(T, top_k, device=DEV)
+    K.router_select(logits, idx, gate, top_k=top_k, sigmoid_gate=mode)
+    for t, row in enumerate(logits.tolist()):
+        order = sorted((e for e in range(experts) if row[e] == row[e]), key=lambda e: (-row[e], e))
+        order += [e for e in range(experts) if row[e] != row[e]]
+        assert idx[t].tolist() == order[:top_k]
+        chosen = torch.tensor([row[e] for e in order[:top_k]], dtype=torch.float64)
+        want = torch.ones(top_k, dtype=torch.float64) if mode is False else torch.sigmoid(chosen) if mode is True \
+            else torch.softmax(chosen, 0)
+        got = gate[t].double().cpu()
+        assert torch.equal(got.isnan(), want.isnan())
+        assert float((got - want).nan_to_num().abs().max()) <= 2.0 ** -20
+
+
+@pytest.mark.parametrize("T,top_k,experts", [(1, 1, 1), (700, 3, 20), (2048, 4, 16), (9000, 2, 256)])
+def test_expert_lists_are_stable(T, top_k, experts):
+    from cpi_b200.csrc import lib as K
+    g = torch.Generator(device=DEV).manual_seed(T)
+    idx = torch.randint(0, experts, (T, top_k), generator=g, device=DEV, dtype=torch.int32)
+    gate = torch.rand(T, top_k, generator=g, device=DEV)
+    i32 = lambda n: torch.empty(n, dtype=torch.int32, device=DEV)
+    offsets, token, slot, scale = i32(experts + 1), i32(T * top_k), i32(T * top_k), torch.empty(T * top_k, device=DEV)
+    K.moe_lists(idx, gate, offsets, token, scale, slot, n_tokens=T, top_k=top_k, n_experts=experts)
+    flat = idx.view(-1).long()
+    order = torch.sort(flat, stable=True).indices
+    assert torch.equal(token.long(), order // top_k) and torch.equal(scale, gate.view(-1)[order])
+    assert torch.equal(slot.long()[order], torch.arange(T * top_k, device=DEV))
+    assert offsets.tolist() == [0] + torch.bincount(flat, minlength=experts).cumsum(0).tolist()
