@@ -633,7 +633,10 @@ static int g_persistent = 1;
 extern "C" void cpi_gemm_tc_pair_persistent(int mode) { g_persistent = mode; }
 
 extern "C" int cpi_gemm_tc_pair_plan(int T, int N, int K, int swiglu, int n_groups) {
-  if (N % 256 != 0 || K % 8 != 0) return 0;
+  // Features that are no multiple of 256 leave part of the last pair's rows idle (their loads give zeros, their results are not
+  // stored): at most a fifth of the work from 1,024 on.  1,855 x 2,048 -> 10,304: 109 us on the
+  // single-CTA kernel, 85 here; 1,500 x 2,048 -> 3,144: 37, 24; 2,048 x 2,048 -> 1,344: 19, 17 (so 1,024 is near the line)
+  if ((N % 256 != 0 && (N < 1024 || n_groups > 0)) || K % 8 != 0) return 0;
   if (n_groups > 0) {
     // experts: one token tile per expert (its weights are then read once), sized for 1.5 x the mean rows
     if (n_groups > 256 || T < 64 * n_groups) return 0;
@@ -645,7 +648,7 @@ extern "C" int cpi_gemm_tc_pair_plan(int T, int N, int K, int swiglu, int n_grou
   const long sm_pairs = cpi::sm_count() / 2 > 0 ? cpi::sm_count() / 2 : 1;
   long best_cost = -1;
   int bn = 0;
-  const long pairs_x = N / 256;
+  const long pairs_x = (N + 255) / 256;
   const int w_rows = swiglu ? 256 : 128;
   for (int cand = 256; cand >= 160; cand -= 32) {
     const long pairs = pairs_x * ((T + cand - 1) / cand);
@@ -666,7 +669,7 @@ extern "C" int cpi_gemm_tc_pair(const void* x, long ldx, const void* w, void* ou
   const int gate_act = mode == 3 ? 1 : mode == 4 ? 2 : mode == 5 ? 3 : mode == 6 ? 4 : 0;
   if (mode == 3 || mode == 4) mode = 2;
   if (mode == 5 || mode == 6) mode = 0;
-  CPI_REQUIRE(N % 256 == 0 && K % 8 == 0 && ldx % 8 == 0, "gemm_tc_pair: N (%d) must be a multiple of 256, K (%d) and the row stride of 8", N, K);
+  CPI_REQUIRE((N % 256 == 0 || n_groups == 0) && K % 8 == 0 && ldx % 8 == 0, "gemm_tc_pair: K (%d) and the row stride must be multiples of 8, N (%d) in groups of 256", K, N);
   CPI_REQUIRE(bn >= 32 && bn <= 256 && bn % 32 == 0, "gemm_tc_pair: token tile %d (multiples of 32 up to 256)", bn);
   CPI_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0, "gemm_tc_pair: operands must be 16-byte aligned");
   CPI_REQUIRE(mode != tc2::kAdd || out_dtype == kF32, "gemm_tc_pair: ADD mode needs a float32 output");
@@ -677,18 +680,21 @@ extern "C" int cpi_gemm_tc_pair(const void* x, long ldx, const void* w, void* ou
   if (tc::get_map_3d_bf16(w, (uint64_t)K, (uint64_t)acc * N, (uint64_t)(n_groups > 0 ? n_groups : 1), tc2::BK, tc2::BM, &mw)) return 1;
   if (tc::get_map_2d_bf16(x, (uint64_t)K, (uint64_t)T, (uint64_t)ldx * 2, tc2::BK, 64, &mx)) return 1;
   tc2::Params p{out, ldo, out_rows, row_scale, group_offsets, n_groups, T, bn, N, (K + tc2::BK - 1) / tc2::BK, error_flag, gate_act, gate_limit};
-  dim3 grid(N / tc2::BM, (T + bn - 1) / bn + (n_groups > 0 ? (T < n_groups ? T : n_groups) : 0), 1);
+  const int n_pairs = (N + 255) / 256;
+  dim3 grid(2 * n_pairs, (T + bn - 1) / bn + (n_groups > 0 ? (T < n_groups ? T : n_groups) : 0), 1);
   CPI_REQUIRE(grid.y <= 65535, "gemm_tc_pair: too many token tiles (%u)", grid.y);
   const int cap = bn <= 128 ? 128 : 256;
   // (ADD: the persistent kernel wins where the mainloop is short against the epilogue; measured at 8,192 tokens
   // with the copy engine's add: K = 5120 314 against 321 us, K = 8192 513 against 495 us)
+  // (the persistent kernel stores whole 16-byte groups of a row only: rows that do not start on 16 bytes take the other one)
+  const bool rows16 = (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % (out_dtype == kF32 ? 4 : 8) == 0;
   const bool persistent = g_persistent == 2 || (g_persistent == 1 && (mode == tc2::kSwiglu ||
                                                 (mode == tc2::kAdd && T >= 4096 && K <= 6144)));
   const int n_slots = (T + bn - 1) / bn + (n_groups > 0 ? (T < n_groups ? T : n_groups) : 0);
   const bool persistent_groups = (g_persistent == 2 || (g_persistent == 1 && mode == tc2::kSwiglu)) && n_groups > 0 &&
                                  n_slots <= tc2::kMaxSlots;      // (measured: 2 % faster for SwiGLU, slower for STORE)
-  if ((n_groups == 0 ? persistent : persistent_groups) && cap == 256) {
-    const int n_pairs = N / 256, n_tok = n_slots;
+  if ((n_groups == 0 ? persistent : persistent_groups) && cap == 256 && rows16) {
+    const int n_tok = n_slots;
     if (mode == tc2::kStore && out_dtype == kBF16) return tc2::launch_persistent<256, tc2::kStore, __nv_bfloat16>(mw, mx, p, n_pairs, n_tok, stream);
     if (mode == tc2::kStore && out_dtype == kF32) return tc2::launch_persistent<256, tc2::kStore, float>(mw, mx, p, n_pairs, n_tok, stream);
     if (mode == tc2::kAdd) return tc2::launch_persistent<256, tc2::kAdd, float>(mw, mx, p, n_pairs, n_tok, stream);

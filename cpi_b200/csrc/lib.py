@@ -231,9 +231,10 @@ def gemm_pair_persistent(mode) -> None:
 
 
 def gemm_tc_pair(a, w, out, mode=MODE_STORE, *, m_rows=None, out_rows=None, row_scale=None, group_offsets=None,
-                 n_groups=0, rows_per_group_hint=None, gate_limit=0.0) -> bool:
+                 n_groups=0, rows_per_group_hint=None, gate_limit=0.0, any_features=False) -> bool:
     """The paired (two-SM) tcgen05 kernel for products with many tokens, dense or grouped (see
-    gemm_tc_pair.cu).  Returns False, having launched nothing, when the product is outside what it takes."""
+    gemm_tc_pair.cu).  Returns False, having launched nothing, when the product is outside what it takes.
+    `any_features`: a dense product may have any number of features from 1,024 on, not only multiples of 256."""
     grouped = group_offsets is not None
     if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16 or a.dim() != 2 or w.dim() != (3 if grouped else 2):
         return False
@@ -245,7 +246,7 @@ def gemm_tc_pair(a, w, out, mode=MODE_STORE, *, m_rows=None, out_rows=None, row_
     N = rows_w // 2 if mode in GATED_MODES else rows_w
     if w.shape[-1] != K or out.shape[1] != N or a.stride(0) % 8 or a.data_ptr() % 16 or w.data_ptr() % 16:
         return False
-    if grouped and w.shape[0] != n_groups:
+    if (grouped and w.shape[0] != n_groups) or (N % 256 and not any_features):
         return False
     if (mode in GATED_MODES and out.dtype != torch.bfloat16) or (mode == MODE_ADD and out.dtype != torch.float32):
         return False

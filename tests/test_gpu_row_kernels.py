@@ -90,3 +90,25 @@ def test_expert_lists_are_stable(T, top_k, experts):
     assert torch.equal(token.long(), order // top_k) and torch.equal(scale, gate.view(-1)[order])
     assert torch.equal(slot.long()[order], torch.arange(T * top_k, device=DEV))
     assert offsets.tolist() == [0] + torch.bincount(flat, minlength=experts).cumsum(0).tolist()
+
+
+# features past the last pair's first half, inside its second half, one more than a whole tile, odd (direct epilogue); a token
+# tile that ends early
+@pytest.mark.parametrize("N", [1025, 1100, 1344, 1480, 1536 + 8])
+@pytest.mark.parametrize("mode,out_dtype", [(0, torch.float32), (0, torch.bfloat16), (1, torch.float32), (2, torch.bfloat16), (5, torch.bfloat16)])
+def test_two_sm_products_of_any_number_of_features(N, mode, out_dtype):
+    from cpi_b200.csrc import lib as K
+    randn, T, Kd = _rand(N + mode), 700, 264
+    a, w = randn(T, Kd).bfloat16(), (randn((2 if mode == 2 else 1) * N, Kd) * 0.1).bfloat16()
+    out = randn(T, N + 8).to(out_dtype)
+    before = out.clone()
+    assert K.gemm_tc_pair(a, w, out[:, :N], mode, any_features=True)
+    acc = a.double() @ w.double().T
+    if mode == 2:
+        ref = torch.nn.functional.silu(acc[:, :N]) * acc[:, N:]
+    else:
+        ref = torch.relu(acc) ** 2 if mode == 5 else acc + (before[:, :N].double() if mode == 1 else 0.0)
+    # float32 sums of 264 products in the tensor cores' order, and the output's rounding
+    tol = 2.0 ** -16 if out_dtype == torch.float32 else 2.0 ** -8 * 1.02
+    assert bool(((out[:, :N].double() - ref).abs() <= tol * ref.abs() + 2.0 ** -14 * ref.abs().max() * 0.1).all())
+    assert torch.equal(out[:, N:], before[:, N:]) and int(K.tc_error_flag(DEV)) == 0
