@@ -174,7 +174,7 @@ class GLAMixer(Mixer):
         tn.update(p.get("tensor_names") or {})
         self.tn = {k: prefix + v for k, v in tn.items()}
         self.ws = workspace
-        self.w_qkvg = self.w_a1 = self.w_a2 = self.b_a2 = self.w_norm = self.w_o = None
+        self.w_in = self.w_a2 = self.b_a2 = self.w_norm = self.w_o = None
 
     def requirements(self):
         t, H, nk, nv = self.tn, self.hidden, self.nh * self.dk, self.nh * self.dv
@@ -184,8 +184,8 @@ class GLAMixer(Mixer):
 
     def load(self, source, device):
         t = self.tn
-        self.w_qkvg = _cat_rows([source.get(t[n], device) for n in ("q", "k", "v", "g")])
-        self.w_a1 = source.get(t["a1"], device).contiguous()
+        # the decays' first projection rides on the same product: [q | k | v | g | a1]
+        self.w_in = _cat_rows([source.get(t[n], device) for n in ("q", "k", "v", "g", "a1")])
         self.w_a2 = source.get(t["a2"], device).contiguous()
         self.b_a2 = source.get(t["a2_bias"], device).to(torch.float32).contiguous()
         self.w_norm = source.get(t["norm"], device).to(torch.float32).contiguous()
@@ -197,13 +197,12 @@ class GLAMixer(Mixer):
     def forward(self, h, residual, batch, cache, add=True):
         T, f32 = h.shape[0], torch.float32
         nk, nv = self.nh * self.dk, self.nh * self.dv
-        proj = self.ws.get("gla_proj", (T, 2 * nk + 2 * nv), f32)
-        low = self.ws.get("gla_low", (T, self.rank), h.dtype)
+        ng = 2 * nk + 2 * nv
+        proj = self.ws.get("gla_proj", (T, -(-(ng + self.rank) // 8) * 8), f32)[:, :ng + self.rank]      # rows on 16 bytes
         z = self.ws.get("gla_z", (T, nk), f32)
         with phase("qkv"):
-            project(h, self.w_qkvg, proj)
-            project(h, self.w_a1, low)
-            project(low, self.w_a2, z)
+            project(h, self.w_in, proj)
+            project(proj[:, ng:], self.w_a2, z)
         o = self.ws.get("gla_o", (T, nv), f32)
         with phase("scan"):
             recurrence(self.ws, h.dtype, proj[:, nk:2 * nk], proj[:, :nk], proj[:, 2 * nk:2 * nk + nv], cache.state("s"), o, batch,
@@ -211,7 +210,7 @@ class GLAMixer(Mixer):
                        q_scale=self.dk ** -0.5)
         with phase("gated_norm"):
             g = self.ws.get("gla_gated", (T, nv), h.dtype)
-            K.gated_norm(o, proj[:, 2 * nk + nv:], self.w_norm, g, parts=self.nh, gate_first=False, eps=self.eps)
+            K.gated_norm(o, proj[:, 2 * nk + nv:ng], self.w_norm, g, parts=self.nh, gate_first=False, eps=self.eps)
         with phase("wo"):
             project(g, self.w_o, residual, MODE_ADD if add else MODE_STORE)
 
