@@ -22,8 +22,15 @@
 // cannot reach the product (0 * NaN).  Formulas: src/engine/llama4_cpu_engine.cpp:195-250; the
 // reference's own prefill is a loop of single-token forwards (src/engine/llama4_cuda_engine.cu:571-580).
 //
+// Bound by the chain S -> softmax -> P V -> next S of each query tile (the tensor pipe is busy 40% of the time at 4,096 tokens)
+// and, on short prompts, by fetching its own code: with a branch for the soft cap at every score, position tests of four
+// instructions and the first tile's exponentials taken twice, 24 tokens of 16 heads took 17.6 us, 3,001 tokens of 40 heads 211
+// and 4,096 tokens 324 (530 TFLOP/s).  The cap compiled apart, a row's mask as one word per 32 columns and a small loop for the
+// first tile's maximum: 8.4, 138 and 226 us (760; 961 at 16,384 tokens).
+//
 // Every mbarrier wait is bounded; when one runs out the CTA sets *error_flag and leaves.
 #include "prefill_tc.cuh"
+#include <type_traits>
 
 namespace cpi {
 namespace pre {
@@ -47,8 +54,8 @@ struct Params {
 
 constexpr int kRingSlots = 5;           // key and value tiles in shared memory at a time
 
-template <int D>
-__global__ void __launch_bounds__(320) attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
+template <int D, bool CAPPED>
+__global__ void __launch_bounds__(kThreads) attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                 const __grid_constant__ CUtensorMap map_k,
                                                                 const __grid_constant__ CUtensorMap map_v, Params p) {
   constexpr int HALVES = D / 64;                       // 64-element (128-byte) column blocks of a row
@@ -68,7 +75,21 @@ __global__ void __launch_bounds__(320) attention_prefill_kernel(const __grid_con
   uint8_t* ring = q_s + 2 * Q_BYTES;                   // [NSLOT]
 
   pdl_launch_dependents();
+  if (tid == 0) {
+    mbar_init(&q_full, 1);
+    for (int s = 0; s < NSLOT; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&s_full[s], 1);
+      mbar_init(&p_full[s], 4); mbar_init(&o_done[s], 1);
+    }
+    abort_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
   pdl_wait();
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
   const int tile = blockIdx.y, head = blockIdx.x;       // heads are the fast axis: all heads of the longest tile start first
   const int kvh = head / (p.n_heads / p.n_kv_heads);
   const int tok0 = p.tile_tok0[tile], rows = p.tile_rows[tile];
@@ -96,20 +117,6 @@ __global__ void __launch_bounds__(320) attention_prefill_kernel(const __grid_con
   const int kt0 = 0, kt1 = has_b ? ke_x[1] : ke_x[0];                     // the union: every tile in it is met by A or B
   auto key_tile = [&](int kt) { return kt < n_kept ? kt : kt + gap; };
 
-  if (tid == 0) {
-    mbar_init(&q_full, 1);
-    for (int s = 0; s < NSLOT; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&s_full[s], 1);
-      mbar_init(&p_full[s], 4); mbar_init(&o_done[s], 1);
-    }
-    abort_s = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
@@ -243,8 +250,7 @@ __global__ void __launch_bounds__(320) attention_prefill_kernel(const __grid_con
     float m_ref = -1e30f, l_run = 0.f;                  // reference maximum of the exponentials; the row's sum
     // > 0: the maximum may be taken before scaling.  Under a soft cap c a raw score s first becomes tanh(s scale / c)
     // (monotonic too) and the factor is c log2(e)
-    const bool capped = p.cap_out > 0.f;
-    const float sc = capped ? p.cap_out : p.scale_log2, cap_in = p.cap_in;
+    const float sc = CAPPED ? p.cap_out : p.scale_log2, cap_in = p.cap_in;
     // the union's last key tile holds positions beyond the newest one: their value rows are zeroed by the group
     // whose P V on that tile is issued first (A if it meets the tile, otherwise B)
     const bool zero_duty = x == 0 ? (kt1 - 1 >= kb_x[0] && kt1 - 1 < ke_x[0]) : !(kt1 - 1 >= kb_x[0] && kt1 - 1 < ke_x[0]);
@@ -277,6 +283,24 @@ __global__ void __launch_bounds__(320) attention_prefill_kernel(const __grid_con
       // known to stand, because it goes over the S it came from.
       uint32_t w[BKV / 32][16];
       float mx, ls;
+      // The first tile has nothing to measure against: its maximum is taken alone, in a small loop (a CTA meets this code
+      // cold, and a short prompt waits for little else than for what it fetches of it).
+      if (j == 0) {
+        mx = -INFINITY;
+#pragma unroll 1
+        for (int c = 0; c < BKV; c += 32) {
+          float v[32], mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+          tmem_ld32(s_row + c, v);
+          const uint32_t in = visible(qp, lo, keep, key0 + c);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            if (CAPPED) v[e] = tanh_fast(v[e] * cap_in);
+            mx4[e & 3] = fmaxf(mx4[e & 3], (in >> e) & 1u ? v[e] : -INFINITY);
+          }
+          mx = fmaxf(mx, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])));
+        }
+        m_ref = fmaxf(mx * sc, m_ref);
+      }
       auto pass = [&](const float ref) {
         const float nref = -ref;
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, ls4[4] = {0.f, 0.f, 0.f, 0.f};
@@ -291,19 +315,18 @@ __global__ void __launch_bounds__(320) attention_prefill_kernel(const __grid_con
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
               float sv = __uint_as_float(raw[cc & 1][e]);
-              if (capped) sv = tanh_fast(sv * cap_in);
+              if (CAPPED) sv = tanh_fast(sv * cap_in);
               mx4[e & 3] = fmaxf(mx4[e & 3], sv);
               v[e] = exp2_fast(fmaf(sv, sc, nref));
             }
           } else {
+            const uint32_t in = visible(qp, lo, keep, key0 + cc * 32);
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
-              const int kp = key0 + cc * 32 + e;
-              const bool in = kp <= qp && (kp >= lo || kp < keep);
               float sv = __uint_as_float(raw[cc & 1][e]);
-              if (capped) sv = tanh_fast(sv * cap_in);
-              if (in) mx4[e & 3] = fmaxf(mx4[e & 3], sv);
-              v[e] = in ? exp2_fast(fmaf(sv, sc, nref)) : 0.f;
+              if (CAPPED) sv = tanh_fast(sv * cap_in);
+              mx4[e & 3] = fmaxf(mx4[e & 3], (in >> e) & 1u ? sv : -INFINITY);
+              v[e] = (in >> e) & 1u ? exp2_fast(fmaf(sv, sc, nref)) : 0.f;
             }
           }
           if (cc + 2 < BKV / 32) tmem_ld32_issue(s_row + (cc + 2) * 32, raw[cc & 1]);     // this buffer is consumed
@@ -317,24 +340,22 @@ __global__ void __launch_bounds__(320) attention_prefill_kernel(const __grid_con
         ls = (ls4[0] + ls4[1]) + (ls4[2] + ls4[3]);
       };
       // Optimistic: against the reference maximum the row already has.  Only if some row of the warp has
-      // outgrown its reference by more than the slack (always on its first tile) is the reference raised, O
+      // outgrown its reference by more than the slack (or is seen for the first time) is the reference raised, O
       // rescaled in tensor memory, and the pass repeated: S is still whole, nothing has been stored yet.
       pass(m_ref);
       const bool grow = mx > m_ref + (m_ref < -1e29f ? 0.f : kRescaleSlack);
       if (__any_sync(0xffffffffu, grow)) {
         const float m_new = grow ? mx : m_ref;
         const float f = exp2f(m_ref - m_new);
-        if (j > 0) {
-          // Every P V issued so far for this query tile has landed: the Q K^T whose S was waited for above was
-          // issued after the last of them, and its arrival covers everything issued before it.
+        // Every P V issued so far for this query tile has landed: the Q K^T whose S was waited for above was
+        // issued after the last of them, and its arrival covers everything issued before it.
 #pragma unroll 1
-          for (int c = 0; c < D; c += 32) {
-            float v[32];
-            tmem_ld32(o_row + c, v);
+        for (int c = 0; c < D; c += 32) {
+          float v[32];
+          tmem_ld32(o_row + c, v);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] *= f;
-            tmem_st32(o_row + c, v);
-          }
+          for (int e = 0; e < 32; ++e) v[e] *= f;
+          tmem_st32(o_row + c, v);
         }
         l_run *= f;
         m_ref = m_new;
@@ -423,14 +444,15 @@ extern "C" int cpi_attention_prefill(const void* q, void* out, const void* k_cac
   dim3 grid(n_heads, n_tiles);
   const int halves = head_dim / 64;
   const int smem = halves * 128 * 128 * (2 + pre::kRingSlots);     // Q of both tiles, the ring of K and V tiles
-  if (head_dim == 128) {
+  auto launch = [&](auto dim, auto capped) {             // (the soft cap is compiled apart, see above)
+    auto* kernel = pre::attention_prefill_kernel<dim.value, capped.value>;
     static bool set = false;
-    if (!set) { cudaFuncSetAttribute(pre::attention_prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); set = true; }
-    cpi::launch_pdl(pre::attention_prefill_kernel<128>, grid, 320, smem, stream, mq, mk, mv, p);
-  } else {
-    static bool set = false;
-    if (!set) { cudaFuncSetAttribute(pre::attention_prefill_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); set = true; }
-    cpi::launch_pdl(pre::attention_prefill_kernel<64>, grid, 320, smem, stream, mq, mk, mv, p);
-  }
+    if (!set) { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); set = true; }
+    cpi::launch_pdl(kernel, grid, pre::kThreads, smem, stream, mq, mk, mv, p);
+  };
+  auto launch_dim = [&](auto dim) {
+    if (p.cap_out > 0.f) launch(dim, std::true_type{}); else launch(dim, std::false_type{});
+  };
+  if (head_dim == 128) launch_dim(std::integral_constant<int, 128>{}); else launch_dim(std::integral_constant<int, 64>{});
   return check_launch("attention_prefill");
 }

@@ -62,7 +62,7 @@ struct Params {
   int* error_flag;
 };
 
-__global__ void __launch_bounds__(320) latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
+__global__ void __launch_bounds__(kThreads) latent_prefill_kernel(const __grid_constant__ CUtensorMap map_q,
                                                              const __grid_constant__ CUtensorMap map_k,
                                                              const __grid_constant__ CUtensorMap map_r,
                                                              const __grid_constant__ CUtensorMap map_v, Params p) {
@@ -254,6 +254,22 @@ __global__ void __launch_bounds__(320) latent_prefill_kernel(const __grid_consta
       const bool no_mask = key0 + BKV - 1 <= p0_x[x] && key0 >= lo_last;
       uint32_t w[BKV / 32][16];
       float mx, ls;
+      // (the first tile's maximum alone, then optimistic passes: see there)
+      if (j == 0) {
+        mx = -INFINITY;
+#pragma unroll 1
+        for (int c = 0; c < BKV; c += 32) {
+          float v[32], mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+          tmem_ld32(s_row + c, v);
+          const uint32_t in = visible(qp, lo, 0, key0 + c);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            mx4[e & 3] = fmaxf(mx4[e & 3], (in >> e) & 1u ? v[e] : -INFINITY);
+          }
+          mx = fmaxf(mx, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])));
+        }
+        m_ref = fmaxf(mx * sc, m_ref);
+      }
       auto pass = [&](const float ref) {
         const float nref = -ref;
         float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, ls4[4] = {0.f, 0.f, 0.f, 0.f};
@@ -267,18 +283,17 @@ __global__ void __launch_bounds__(320) latent_prefill_kernel(const __grid_consta
           if (no_mask) {
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
-              const float sv = __uint_as_float(raw[cc & 1][e]);
+              float sv = __uint_as_float(raw[cc & 1][e]);
               mx4[e & 3] = fmaxf(mx4[e & 3], sv);
               v[e] = exp2_fast(fmaf(sv, sc, nref));
             }
           } else {
+            const uint32_t in = visible(qp, lo, 0, key0 + cc * 32);
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
-              const int kp = key0 + cc * 32 + e;
-              const bool in = kp <= qp && kp >= lo;
-              const float sv = __uint_as_float(raw[cc & 1][e]);
-              if (in) mx4[e & 3] = fmaxf(mx4[e & 3], sv);
-              v[e] = in ? exp2_fast(fmaf(sv, sc, nref)) : 0.f;
+              float sv = __uint_as_float(raw[cc & 1][e]);
+              mx4[e & 3] = fmaxf(mx4[e & 3], (in >> e) & 1u ? sv : -INFINITY);
+              v[e] = (in >> e) & 1u ? exp2_fast(fmaf(sv, sc, nref)) : 0.f;
             }
           }
           if (cc + 2 < BKV / 32) tmem_ld32_issue(s_row + (cc + 2) * 32, raw[cc & 1]);     // this buffer is consumed
@@ -296,15 +311,15 @@ __global__ void __launch_bounds__(320) latent_prefill_kernel(const __grid_consta
       if (__any_sync(0xffffffffu, grow)) {
         const float m_new = grow ? mx : m_ref;
         const float f = exp2f(m_ref - m_new);
-        if (j > 0) {                                     // (every P V issued so far for this tile has landed, see there)
+        // Every P V issued so far for this query tile has landed: the Q K^T whose S was waited for above was
+        // issued after the last of them, and its arrival covers everything issued before it.
 #pragma unroll 1
-          for (int c = 0; c < DV; c += 32) {
-            float v[32];
-            tmem_ld32(o_row + c, v);
+        for (int c = 0; c < DV; c += 32) {
+          float v[32];
+          tmem_ld32(o_row + c, v);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] *= f;
-            tmem_st32(o_row + c, v);
-          }
+          for (int e = 0; e < 32; ++e) v[e] *= f;
+          tmem_st32(o_row + c, v);
         }
         l_run *= f;
         m_ref = m_new;
@@ -495,6 +510,6 @@ extern "C" int cpi_latent_prefill(const void* q, const void* kv, const void* row
     }
     set = true;
   }
-  cpi::launch_pdl(latent_prefill_kernel, dim3(n_heads, n_tiles), dim3(320), SMEM, stream, mq, mk, mr, mv, p);
+  cpi::launch_pdl(latent_prefill_kernel, dim3(n_heads, n_tiles), dim3(kThreads), SMEM, stream, mq, mk, mr, mv, p);
   return check_launch("latent_prefill");
 }

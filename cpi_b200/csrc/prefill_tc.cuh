@@ -17,6 +17,7 @@ constexpr uint32_t kSpinLimit = 1u << 24;
 // outgrown it by more than this many powers of two; the accumulated output then needs rescaling only
 // then (rarely after the first tiles), and intermediate values stay below 2^kRescaleSlack.
 constexpr float kRescaleSlack = 8.0f;
+constexpr int kThreads = 320;            // eight softmax warps, one that loads, one that issues the products
 constexpr int kTileRows = 2 * BQ;       // query rows a CTA takes: two tiles of 128
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
@@ -144,6 +145,11 @@ __device__ __forceinline__ int window_low(int kind, int size, int pos) {
   if (kind == 1) return (pos / size) * size;
   if (kind == 2) return max(0, pos - size + 1);
   return 0;
+}
+// bit e: a query at `pos` whose window begins at `lo`, the first `keep` positions always in it, sees key position key0 + e
+__device__ __forceinline__ uint32_t visible(int pos, int lo, int keep, int key0) {
+  auto below = [&](int n) { return n >= 32 ? 0xffffffffu : n <= 0 ? 0u : (1u << n) - 1u; };      // bits 0 .. n - 1
+  return below(pos + 1 - key0) & (~below(lo - key0) | below(keep - key0));
 }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
