@@ -6,6 +6,7 @@ cannot be built or loaded, `load()` raises, and every function below raises with
 from __future__ import annotations
 
 import ctypes
+import functools
 from ctypes import c_int, c_long, c_float, c_void_p
 
 import torch
@@ -69,7 +70,8 @@ def _p(t):
 
 
 def _stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    # (the current stream's handle alone: torch.cuda.current_stream() builds an object for it, 3 us of each launch's 18)
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _call(name, *args):
@@ -152,7 +154,7 @@ def device_error_flags(device) -> torch.Tensor:
     """int32[2] on the device that kernels write when something went wrong: word 0 is set to 1 by a tensor-core
     kernel whose bounded barrier wait ran out, word 1 to 1 + t by the embedding kernel when token t of a step
     was outside the vocabulary.  The engine reads and clears them."""
-    idx = torch.device(device).index or 0
+    idx = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
     if idx not in _errors:
         _errors[idx] = torch.zeros(2, dtype=torch.int32, device=device)
     return _errors[idx]
@@ -197,23 +199,28 @@ def gemm_tc(a, w, out, mode=MODE_STORE, *, n_out=None, m_rows=None, a_rows=None,
     T = m_rows if m_rows is not None else a.shape[0]
     if T > a.shape[0]:
         raise KernelError("gemm_tc: more logical rows than activation rows")
-    bn, splits, live_y = c_int(), c_int(), c_int()
-    load().cpi_gemm_tc_plan(c_int(T), c_int(N), c_int(K), c_int(n_groups if grouped else 0),
-                            c_int(int(mode in GATED_MODES)), ctypes.byref(bn), ctypes.byref(splits),
-                            ctypes.byref(live_y))
+    bn, splits = gemm_tc_plan(T, N, K, n_groups if grouped else 0, mode in GATED_MODES)
     _call("cpi_gemm_tc", _p(a), c_long(a.stride(0)), _p(w), _p(out), c_int(dtype_code(out.dtype)),
           c_long(out.stride(0)), _p(out_rows), _p(row_scale), _p(group_offsets), c_int(n_groups if grouped else 0),
-          c_int(T), c_int(N), c_int(K), c_int(mode), c_int(bn.value), c_int(splits.value),
+          c_int(T), c_int(N), c_int(K), c_int(mode), c_int(bn), c_int(splits),
           _p(tc_error_flag(a.device)), c_float(gate_limit), _stream())
     return True
 
 
-def gemm_tc_plan(T: int, N: int, K: int, n_groups: int = 0, swiglu: bool = False):
-    """(token rows per tile, k splits) that `gemm_tc` uses for a product of these sizes on this device."""
+@functools.lru_cache(maxsize=4096)
+def _plan(kind: str, device: int, T: int, N: int, K: int, n_groups: int, swiglu: bool):
+    """What the library plans for a product of these sizes on this device (a function of the sizes alone)."""
+    if kind == "pair":
+        return load().cpi_gemm_tc_pair_plan(c_int(T), c_int(N), c_int(K), c_int(int(swiglu)), c_int(n_groups))
     bn, splits, live_y = c_int(), c_int(), c_int()
     load().cpi_gemm_tc_plan(c_int(T), c_int(N), c_int(K), c_int(n_groups), c_int(int(swiglu)), ctypes.byref(bn),
                             ctypes.byref(splits), ctypes.byref(live_y))
     return bn.value, splits.value
+
+
+def gemm_tc_plan(T: int, N: int, K: int, n_groups: int = 0, swiglu: bool = False):
+    """(token rows per tile, k splits) that `gemm_tc` uses for a product of these sizes on this device."""
+    return _plan("single", torch._C._cuda_getDevice(), T, N, K, n_groups, bool(swiglu))
 
 
 def gemm_tc_wait_probe(spin_limit: int = 0, tx_extra: int = 0) -> None:
@@ -250,8 +257,7 @@ def gemm_tc_pair(a, w, out, mode=MODE_STORE, *, m_rows=None, out_rows=None, row_
         return False
     if (mode in GATED_MODES and out.dtype != torch.bfloat16) or (mode == MODE_ADD and out.dtype != torch.float32):
         return False
-    bn = load().cpi_gemm_tc_pair_plan(c_int(T), c_int(N), c_int(K), c_int(int(mode in GATED_MODES)),
-                                      c_int(n_groups if grouped else 0))
+    bn = _plan("pair", torch._C._cuda_getDevice(), T, N, K, n_groups if grouped else 0, mode in GATED_MODES)
     if bn <= 0:
         return False
     _need_cuda(a, w, out, out_rows, row_scale, group_offsets)

@@ -11,6 +11,7 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 
@@ -73,11 +74,12 @@ class BatchStager:
         for _ in range(self.RING):
             host = torch.empty(self._cap, dtype=torch.int32, pin_memory=pin)
             dev = torch.empty(self._cap, dtype=torch.int32, device=self.device)
-            self._ring.append([host, dev, None])
+            self._ring.append([host, dev, None, host.numpy()])
 
-    def stage(self, slots, starts, token_lists, wants, dtype, static_dev=None) -> StepBatch:
+    def stage(self, slots, starts, token_lists, wants, dtype, static_dev=None, views_of=None) -> StepBatch:
         """`static_dev`: an int32 device buffer to fill instead of the ring's (its address then stays the
-        same from step to step, which a captured CUDA graph needs)."""
+        same from step to step, which a captured CUDA graph needs).  `views_of`: a batch that `stage` made over that
+        buffer for a step of the same sizes; its arrays are filled again and it is returned, its host values unchanged."""
         B = len(slots)
         n_new = [len(t) for t in token_lists]
         T = sum(n_new)
@@ -95,29 +97,34 @@ class BatchStager:
         self._reserve(total)
         entry = self._ring[self._next]
         self._next = (self._next + 1) % self.RING
-        h, d, ev = entry
+        h, d, ev = entry[:3]
         if static_dev is not None:
             d = static_dev
         if ev is not None:
             ev.synchronize()
-        tokens, token_seq, token_pos, want_rows, tok0 = [], [], [], [], []
-        base = 0
-        for s, (toks, st, w) in enumerate(zip(token_lists, starts, wants)):
-            n = len(toks)
+        w = entry[3]                                  # the pinned buffer as a numpy array
+        tok0, base = [], 0
+        for n in n_new:
             tok0.append(base)
-            tokens += toks
-            token_seq += [s] * n
-            token_pos += range(st, st + n)
-            want_rows += [base + i for i in w]
             base += n
-        flat = (tokens + token_seq + token_pos + list(slots) + list(starts) + n_new + tok0 + want_rows
-                + [t[1] for t in tiles] + [t[2] for t in tiles])
-        h[:total] = torch.tensor(flat, dtype=torch.int32)
+        if max(n_new) == min(n_new) == 1:             # single tokens: a few numbers each, no query tiles
+            w[:total] = ([t[0] for t in token_lists] + list(range(B)) + list(starts) + list(slots) + list(starts) + n_new + tok0
+                         + [b + i for b, wt in zip(tok0, wants) for i in wt])
+        else:
+            for s, (toks, st, b, n) in enumerate(zip(token_lists, starts, tok0, n_new)):
+                w[b:b + n] = toks
+                w[T + b:T + b + n] = s
+                w[2 * T + b:2 * T + b + n] = np.arange(st, st + n, dtype=np.int32)
+            w[3 * T:total] = (list(slots) + list(starts) + n_new + tok0 + [b + i for b, wt in zip(tok0, wants) for i in wt]
+                              + [t[1] for t in tiles] + [t[2] for t in tiles])
         d[:total].copy_(h[:total], non_blocking=True)
         self.bytes_staged = total * 4
         if self.device.type == "cuda":
-            entry[2] = torch.cuda.Event()
-            entry[2].record()
+            if ev is None:
+                ev = entry[2] = torch.cuda.Event()
+            ev.record()
+        if views_of is not None:                      # the caller holds a batch of the same sizes in the same buffer
+            return views_of
         o = 0
 
         def take(n):

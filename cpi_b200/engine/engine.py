@@ -80,7 +80,7 @@ class Engine:
         # when a later step starts and whenever the caller has synchronised anyway (`check_device_errors`).
         self._err_dev = K.device_error_flags(self.device)
         self._err_host = torch.zeros(2, dtype=torch.int32, pin_memory=True)
-        self._err_event = None
+        self._err_event, self._err_copied = None, False
 
     # ---- construction ----------------------------------------------------------------------------
     @classmethod
@@ -129,9 +129,9 @@ class Engine:
             t = [int(x) for x in e.tokens]
             if not t:
                 raise ValueError(f"slot {e.slot}: a step entry without tokens")
-            for x in t:
-                if not 0 <= x < V:
-                    raise ValueError(f"slot {e.slot}: token id {x} is outside the vocabulary of {V}")
+            if min(t) < 0 or max(t) >= V:
+                x = next(x for x in t if not 0 <= x < V)
+                raise ValueError(f"slot {e.slot}: token id {x} is outside the vocabulary of {V}")
             w = [int(i) for i in e.want]
             for i in w:
                 if not 0 <= i < len(t):
@@ -195,9 +195,7 @@ class Engine:
             logits = self.model.run(batch, self.cache)
         self.cache.commit_step(slots, n_new)
         self.steps_run += 1
-        self._err_host.copy_(self._err_dev, non_blocking=True)
-        self._err_event = torch.cuda.Event()
-        self._err_event.record()
+        self._copy_error_flags()
         return logits
 
     def _run_decode_graph(self, slots, starts, toks, wants, device_tokens=None) -> torch.Tensor:
@@ -215,12 +213,12 @@ class Engine:
         if st is None:
             # first step of this kind: eager (it also sizes every workspace buffer and sets kernel attributes)
             dev = torch.empty(self.stager.words_needed(B, B, R), dtype=torch.int32, device=self.device)
-            self._graphs[key] = {"dev": dev, "graph": None, "logits": None, "gen": None, "kernels": 0}
+            self._graphs[key] = {"dev": dev, "graph": None, "logits": None, "gen": None, "kernels": 0, "batch": None}
             batch = self.stager.stage(slots, starts, toks, wants, self.dtype, static_dev=dev)
             if device_tokens is not None:
                 batch.tokens.copy_(device_tokens.view(-1))
             return self.model.run(batch, self.cache)
-        batch = self.stager.stage(slots, starts, toks, wants, self.dtype, static_dev=st["dev"])
+        batch = self.stager.stage(slots, starts, toks, wants, self.dtype, static_dev=st["dev"], views_of=st["batch"])
         if device_tokens is not None:
             batch.tokens.copy_(device_tokens.view(-1))          # after the staged copy, before the replay
         if st["graph"] is None:
@@ -230,7 +228,7 @@ class Engine:
             with torch.cuda.graph(g):
                 st["logits"] = self.model.run(batch, self.cache)
             st["kernels"] = K.kernel_launches() - before
-            st["graph"] = g
+            st["graph"], st["batch"] = g, batch
             st["gen"] = (self.ws.generation, K.scratch_generation)
         st["graph"].replay()
         self.graph_kernel_launches += st["kernels"]
@@ -258,12 +256,19 @@ class Engine:
         phases.install(self._phase_timer)
         return self._phase_timer
 
+    def _copy_error_flags(self) -> None:
+        self._err_host.copy_(self._err_dev, non_blocking=True)
+        if self._err_event is None:
+            self._err_event = torch.cuda.Event()
+        self._err_event.record()
+        self._err_copied = True
+
     def _raise_if_flagged(self, wait: bool) -> None:
         ev = self._err_event
-        if ev is None or (not wait and not ev.query()):
+        if not self._err_copied or (not wait and not ev.query()):
             return
         ev.synchronize()
-        self._err_event = None
+        self._err_copied = False
         gave_up, token = int(self._err_host[0]), int(self._err_host[1])
         if not (gave_up or token):
             return
@@ -278,7 +283,5 @@ class Engine:
         """Raises if a kernel flagged a bad input or gave up a wait since the last check.  Waits for the device:
         `generate`, `Model.step` and the command lines call it where they have the results on the host anyway;
         between such points every step looks at what the step before it left, without waiting."""
-        self._err_host.copy_(self._err_dev, non_blocking=True)
-        self._err_event = torch.cuda.Event()
-        self._err_event.record()
+        self._copy_error_flags()
         self._raise_if_flagged(wait=True)

@@ -8,6 +8,7 @@ class Workspace:
     def __init__(self, device):
         self.device = device
         self._buffers: dict = {}
+        self._views: dict = {}     # what `get` last returned for a name, type and shape (a view costs as much as a launch)
         self.generation = 0        # grows whenever a buffer is (re)allocated: captured graphs then hold stale addresses
         # A block may leave the write-back of its last sublayer to whoever touches the residual next (the next
         # block fuses it with its first read): (streams x, y, write weights, mixing matrix) or None.  Whoever
@@ -33,6 +34,9 @@ class Workspace:
             K.hc_step(p[0], y=p[1], write=p[2], mix=p[3])
 
     def get(self, name: str, shape, dtype: torch.dtype) -> torch.Tensor:
+        view = self._views.get((name, dtype, shape))
+        if view is not None:
+            return view
         n = 1
         for s in shape:
             n *= int(s)
@@ -45,5 +49,10 @@ class Workspace:
             buf = torch.empty(cap, dtype=dtype, device=self.device)
             self._buffers[key] = buf
             self.generation += 1
-        return buf[:n].view(*shape)
-
+            self._views.clear()               # (views of the buffer that this one replaces)
+        view = buf[:n].view(*shape)
+        if isinstance(shape, tuple):
+            if len(self._views) >= 1024:
+                self._views.clear()
+            self._views[(name, dtype, shape)] = view
+        return view
