@@ -74,7 +74,6 @@ __global__ void __launch_bounds__(kThreads) attention_prefill_kernel(const __gri
   uint8_t* q_s = smem_raw;                             // [2 query tiles]
   uint8_t* ring = q_s + 2 * Q_BYTES;                   // [NSLOT]
 
-  pdl_launch_dependents();
   if (tid == 0) {
     mbar_init(&q_full, 1);
     for (int s = 0; s < NSLOT; ++s) { mbar_init(&kv_full[s], 1); mbar_init(&kv_empty[s], 1); }
@@ -85,11 +84,15 @@ __global__ void __launch_bounds__(kThreads) attention_prefill_kernel(const __gri
     abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  pdl_wait();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  pdl_launch_dependents();                              // (not before the tensor memory is ours: see common.cuh)
+  pdl_wait();
   const int tile = blockIdx.y, head = blockIdx.x;       // heads are the fast axis: all heads of the longest tile start first
   const int kvh = head / (p.n_heads / p.n_kv_heads);
   const int tok0 = p.tile_tok0[tile], rows = p.tile_rows[tile];
@@ -116,10 +119,6 @@ __global__ void __launch_bounds__(kThreads) attention_prefill_kernel(const __gri
   const int ke_x[2] = {p1_x[0] / BKV + 1 - gap, has_b ? p1_x[1] / BKV + 1 - gap : 0};
   const int kt0 = 0, kt1 = has_b ? ke_x[1] : ke_x[0];                     // the union: every tile in it is met by A or B
   auto key_tile = [&](int kt) { return kt < n_kept ? kt : kt + gap; };
-
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
   const uint32_t tmem_s = tmem_base_s, tmem_o = tmem_base_s + 256;        // + 128 for tile B, both
   volatile int* abort_flag = &abort_s;
   bool ok = true;

@@ -65,12 +65,16 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
   return r;
 }
 
-// Programmatic dependent launch: a kernel launched with launch_pdl may start while the kernel before it
-// in the stream is still running.  Every such kernel calls pdl_launch_dependents() early (so that its
-// own successor may be scheduled) and pdl_wait() before it first reads or writes global memory that
-// another kernel of the stream produces or reads; pdl_wait() returns once the preceding kernel has
-// finished and its writes are visible.  What precedes the wait (barrier set-up, tensor-memory
-// allocation, loads of weights, which no kernel writes) overlaps the predecessor's tail.
+// Programmatic dependent launch: a kernel launched with launch_pdl may start while the kernel before it in the stream is
+// still running.  Every such kernel calls pdl_wait() before it first reads or writes global memory that another kernel of
+// the stream produces or reads; pdl_wait() returns once the preceding kernel has finished and its writes are visible.
+// pdl_launch_dependents() lets its own successor be scheduled; a kernel that does not call it does so by ending.  What
+// precedes the wait (barrier set-up, tensor-memory allocation, loads of weights, which no kernel writes) overlaps the
+// predecessor's tail.
+// A kernel that allocates tensor memory lets its successors start only when it has it.  Before, a successor's block that
+// fits the same SM could take the columns first and keep them until this kernel ends, which waits for those columns.  With
+// that order whoever holds columns belongs to a kernel that is wholly resident, has all it needs and waits for earlier
+// kernels only, so every allocation is served in the end.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

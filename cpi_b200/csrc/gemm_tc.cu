@@ -184,7 +184,6 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
 
-  pdl_launch_dependents();
   // ---- which tile ----
   // Groups with many tokens: the token tiles of one (weight tile, group) are neighbours in launch order,
   // so the second one finds the weight strip in the L2 that the first one pulled from DRAM.
@@ -235,6 +234,7 @@ __global__ void __launch_bounds__(128) gemm_tc_kernel(const __grid_constant__ CU
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
+  pdl_launch_dependents();                       // (not before the tensor memory is ours: see common.cuh)
   const uint32_t tmem_base = tmem_base_s;
   volatile int* abort_flag = &abort_s;
 

@@ -144,7 +144,6 @@ __global__ void __launch_bounds__(128) gemm_tc_pair_kernel(const __grid_constant
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t rank = cluster_rank();                          // 0: leader (issues the MMAs), 1: peer
-  pdl_launch_dependents();
 
   // ---- which tile (both CTAs of a pair share blockIdx.y, so they find the same one) ----
   int group = 0, t_begin = 0, t_end = p.T, tile_t = blockIdx.y;
@@ -205,6 +204,7 @@ __global__ void __launch_bounds__(128) gemm_tc_pair_kernel(const __grid_constant
   __syncthreads();
   cluster_sync();                                                // the peer's barriers exist before anyone signals them
   fence_after_sync();
+  pdl_launch_dependents();                                       // (not before the tensor memory is ours: see common.cuh)
   const uint32_t tmem_base = tmem_base_s;
   volatile int* abort_flag = &abort_s;
 
@@ -371,7 +371,6 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_persistent_kernel(const __gr
   uint8_t* ring = smem;
   uint8_t* epi = smem + (size_t)STAGES * STAGE_BYTES;
   const uint32_t rank = cluster_rank();
-  pdl_launch_dependents();
   const bool grouped = p.group_offsets != nullptr;
   if (grouped) {
     // the row lists come from the kernel before this one; one thread walks the groups and lists their tiles
@@ -433,6 +432,7 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_persistent_kernel(const __gr
   __syncthreads();
   cluster_sync();
   fence_after_sync();
+  pdl_launch_dependents();                                       // (not before the tensor memory is ours: see common.cuh)
   const uint32_t tmem_base = tmem_base_s;
   volatile int* abort_flag = &abort_s;
 

@@ -76,7 +76,6 @@ __global__ void __launch_bounds__(kThreads) latent_prefill_kernel(const __grid_c
   uint8_t* k_s = q_s + 2 * QB * BLOCK;                  // [NK]
   uint8_t* v_s = k_s + NK * BLOCK;                      // [NV]
 
-  pdl_launch_dependents();
   if (tid == 0) {
     mbar_init(&q_full, 1);
     for (int s = 0; s < NK; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); }
@@ -89,6 +88,10 @@ __global__ void __launch_bounds__(kThreads) latent_prefill_kernel(const __grid_c
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  pdl_launch_dependents();                              // (not before the tensor memory is ours: see common.cuh)
   pdl_wait();
   const int tile = blockIdx.y, head = blockIdx.x;       // heads are the fast axis: all heads of the longest tile start first
   const int tok0 = p.tile_tok0[tile], rows = p.tile_rows[tile];
@@ -106,9 +109,6 @@ __global__ void __launch_bounds__(kThreads) latent_prefill_kernel(const __grid_c
   const int kb_x[2] = {0, has_b ? (low(p0_x[1]) - key_first) / BKV : 0};
   const int ke_x[2] = {(p1_x[0] - key_first) / BKV + 1, has_b ? (p1_x[1] - key_first) / BKV + 1 : 0};
   const int kt1 = has_b ? ke_x[1] : ke_x[0];
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
   const uint32_t tmem_s = tmem_base_s, tmem_o = tmem_base_s + 256;        // + 128 for tile B, both
   volatile int* abort_flag = &abort_s;
   bool ok = true;

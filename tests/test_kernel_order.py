@@ -1,0 +1,41 @@
+"""An order that the kernels' sources have to keep, read from the sources: a kernel lets its successors start (programmatic
+dependent launch) only when it has its tensor memory.  A successor that started earlier on the same SM could take the
+columns and keep them until this kernel ends, which itself waits for them: neither would ever go on."""
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "cpi_b200", "csrc")
+ALLOCATES = re.compile(r"tcgen05\.alloc|\btmem_alloc\(")
+
+
+def _kernels():
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith(".cu"):
+            continue
+        text = re.sub(r"//[^\n]*|__launch_bounds__\([^)]*\)", "", open(os.path.join(CSRC, name)).read())
+        for m in re.finditer(r"__global__[^;{]*?(\w+)\s*\([^;{]*\)\s*\{", text):
+            depth, end = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[end], 0)
+                end += 1
+            yield f"{name}:{m.group(1)}", text[m.end():end]
+
+
+KERNELS = dict(_kernels())
+WITH_TENSOR_MEMORY = sorted(k for k, body in KERNELS.items() if ALLOCATES.search(body))
+
+
+def test_the_kernels_with_tensor_memory_are_found():
+    found = {k.split(":")[1] for k in WITH_TENSOR_MEMORY}
+    assert {"gemm_tc_kernel", "gemm_tc_pair_kernel", "gemm_tc_pair_persistent_kernel", "attention_prefill_kernel",
+            "latent_prefill_kernel"} <= found and len(KERNELS) > 60
+
+
+@pytest.mark.parametrize("name", WITH_TENSOR_MEMORY)
+def test_successors_start_after_the_tensor_memory_is_allocated(name):
+    body = KERNELS[name]
+    starts = [m.start() for m in re.finditer(r"pdl_launch_dependents\(\)", body)]
+    allocated = ALLOCATES.search(body).end()
+    assert all(s > allocated and "__syncthreads" in body[allocated:s] for s in starts)
