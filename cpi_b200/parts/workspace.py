@@ -34,6 +34,10 @@ class Workspace:
             K.hc_step(p[0], y=p[1], write=p[2], mix=p[3])
 
     def get(self, name: str, shape, dtype: torch.dtype) -> torch.Tensor:
+        """The buffer `name` of this type as a tensor of `shape` (any sequence of sizes), its contents whatever is there.
+        Callers that ask alike get the same tensor object, so its shape is not to be changed in place."""
+        if not isinstance(shape, tuple):
+            shape = tuple(shape)
         view = self._views.get((name, dtype, shape))
         if view is not None:
             return view
@@ -51,8 +55,7 @@ class Workspace:
             self.generation += 1
             self._views.clear()               # (views of the buffer that this one replaces)
         view = buf[:n].view(*shape)
-        if isinstance(shape, tuple):
-            if len(self._views) >= 1024:
-                self._views.clear()
-            self._views[(name, dtype, shape)] = view
+        if len(self._views) >= 1024:
+            self._views.clear()
+        self._views[(name, dtype, shape)] = view
         return view

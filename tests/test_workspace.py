@@ -1,0 +1,31 @@
+"""The workspace that parts take their scratch buffers from."""
+import pytest
+import torch
+
+from cpi_b200.parts import Workspace
+
+
+@pytest.mark.parametrize("shape", [(2, 3), [2, 3], torch.Size([2, 3]), range(2, 4)])
+def test_a_shape_is_any_sequence_of_sizes(shape):
+    ws = Workspace("cpu")
+    for _ in range(2):
+        assert ws.get("a", shape, torch.float32).shape == (2, 3)
+    assert ws.get("a", [4], torch.float32).data_ptr() == ws.get("a", (2, 2), torch.float32).data_ptr()
+
+
+def test_views_follow_a_buffer_that_grew():
+    ws = Workspace("cpu")
+    small, other = ws.get("a", (4,), torch.float32), ws.get("b", (4,), torch.float32)
+    assert ws.get("a", (4,), torch.float32) is small and ws.get("a", (4,), torch.int32) is not small
+    before = ws.generation
+    ws.get("a", (8, 2), torch.float32).fill_(1)
+    assert ws.generation == before + 1
+    again = ws.get("a", (4,), torch.float32)
+    assert again.data_ptr() == ws.get("a", (8, 2), torch.float32).data_ptr() != small.data_ptr() and bool((again == 1).all())
+    assert ws.get("b", (4,), torch.float32).data_ptr() == other.data_ptr()
+
+
+def test_views_of_many_shapes_stay_right():
+    ws = Workspace("cpu")
+    for i in range(3000):
+        assert ws.get("a", (1 + i % 1500, 2), torch.float32).shape == (1 + i % 1500, 2)
