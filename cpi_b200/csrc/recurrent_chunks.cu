@@ -719,14 +719,16 @@ __global__ void __launch_bounds__(64) chunk_out_kernel(Params p) {
     if (whole) product(std::false_type{});
     else product(std::true_type{});
   }
+  // (the skip adds v itself, also with the delta rule, whose products above take the corrected u)
   const float skip = p.skip ? load_any(p.skip, p.small_dtype, h) : 0.f;
+  const float* raw = p.v + (size_t)c.tok * p.v_stride + (size_t)h * Dv + c0;
 #pragma unroll
   for (int r = 0; r < 8; ++r) {
     const int i = i0 + r;
     if (i >= c.n) continue;
     if (p.skip) {
       float2 b[4];
-      load_cols(v + i * vstep + x0, b);
+      load_cols(raw + i * p.v_stride + x0, b);
 #pragma unroll
       for (int x = 0; x < 4; ++x) acc[r][x] = __ffma2_rn(two(skip), b[x], acc[r][x]);
     }

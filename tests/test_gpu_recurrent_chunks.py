@@ -116,3 +116,26 @@ def test_an_output_reads_nothing_of_later_tokens(kind):
                         n_cols=cols, **y, **fixed)
         got.append(out)
     assert torch.equal(got[0][:at], got[1][:at]) and bool(got[1][at:].isnan().all())
+
+
+@pytest.mark.parametrize("kind", ["rows", "delta"])
+def test_the_skip_adds_the_values_themselves(kind):
+    """With row decays and with the delta rule, whose sums take corrected values: the scan's outputs with a skip."""
+    from cpi_b200.csrc import lib as K
+    g = torch.Generator(device=DEV).manual_seed(9)
+    new, H, rows, cols = [70, 130], 2, 64, 128
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    T = sum(new)
+    k, q, v = torch.nn.functional.normalize(randn(T, H, rows), dim=-1).view(T, -1), randn(T, H * rows), randn(T, H * cols)
+    kw = dict(z=randn(T, H * rows), z_bias=randn(H * rows), skip=randn(H), n_heads=H, heads_per_group=1, n_rows=rows, n_cols=cols)
+    if kind == "delta":
+        kw.update(beta=randn(T, H), decay_kind=1, a_log=randn(H))
+    per = K.linear_chunks_scratch(H, 1, rows, cols, z=kw["z"], beta=kw.get("beta"))
+    outs, state = [], randn(2, H, rows, cols)
+    for fn, extra in ((K.linear_scan, {}), (K.linear_chunks, dict(scratch=torch.empty(5 * per, device=DEV)))):
+        S, out = state.clone(), torch.empty(T, H * cols, device=DEV)
+        fn(k, q, v, S, out, _batch(new, [0, 1]), **kw, **extra)
+        outs += [out, S]
+    # float32 sums of up to 64 + 64 terms and of the states' rows in two orders
+    for x, y in ((outs[0], outs[2]), (outs[1], outs[3])):
+        assert float((x - y).norm() / x.norm()) <= 2.0 ** -18
