@@ -160,23 +160,44 @@ __global__ void __launch_bounds__(NT) gemm_simt_kernel(GemmParams p) {
 // through registers while 16 are multiplied.
 // Bound: the FP32 pipe with enough warps (one warp per scheduler issues packed instructions at half rate, three at 0.95 of it);
 // 509 x 2,048 -> 3,072 and 2,048 in float32: 984 -> 343 us together (the kernel above with 64 rows a tile before).
-template <typename T>
-__device__ __forceinline__ void load4(const T* p, bool live, bool vec, int k, int K, float (&v)[4]) {
-  if (!live) { v[0] = v[1] = v[2] = v[3] = 0.f; return; }
-  if (vec && k + 4 <= K) {
-    if constexpr (sizeof(T) == 4) {
-      const float4 x = *reinterpret_cast<const float4*>(p + k);
-      v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
-    } else {
-      const uint2 x = *reinterpret_cast<const uint2*>(p + k);
-      const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x));
-      const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
-      v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
-    }
-    return;
+// Four neighbouring elements of a row as they lie in memory; they are widened on their way to shared memory, so that nothing
+// waits for a load while the 16 k before are multiplied.  64 rows, 2,048 x 2,048: bfloat16 weights widened at the load 205 us,
+// here 107 (float32 weights 117); with 4 x 4 outputs a thread and 64 rows a tile it was 169 (177).
+template <typename T> struct Four;
+template <> struct Four<float> {
+  float v[4];
+  __device__ __forceinline__ void clear() { v[0] = v[1] = v[2] = v[3] = 0.f; }
+  __device__ __forceinline__ void whole(const float* p) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
   }
+  __device__ __forceinline__ void some(const float* p, int k, int K) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) v[j] = k + j < K ? to_f32(p[k + j]) : 0.f;
+    for (int j = 0; j < 4; ++j) v[j] = k + j < K ? p[k + j] : 0.f;
+  }
+  __device__ __forceinline__ float at(int e) const { return v[e]; }
+};
+template <> struct Four<__nv_bfloat16> {
+  uint2 v;
+  __device__ __forceinline__ void clear() { v = make_uint2(0u, 0u); }
+  __device__ __forceinline__ void whole(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint2*>(p); }
+  __device__ __forceinline__ void some(const __nv_bfloat16* p, int k, int K) {
+    const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
+    uint32_t x[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = k + j < K ? u[k + j] : 0u;
+    v = make_uint2(x[0] | x[1] << 16, x[2] | x[3] << 16);
+  }
+  __device__ __forceinline__ float at(int e) const {                 // (a bfloat16 is the upper half of its float32)
+    const uint32_t w = e < 2 ? v.x : v.y;
+    return __uint_as_float(e & 1 ? w & 0xffff0000u : w << 16);
+  }
+};
+template <typename T>
+__device__ __forceinline__ void load4(const T* p, bool live, bool vec, int k, int K, Four<T>& v) {
+  if (!live) v.clear();
+  else if (vec && k + 4 <= K) v.whole(p + k);
+  else v.some(p, k, K);
 }
 
 constexpr int TILE_ROWS = 64, TILE_THREADS = 128;
@@ -229,7 +250,8 @@ __global__ void __launch_bounds__(TILE_THREADS) gemm_simt_tile_kernel(GemmParams
   }
   const int kq = (tid & 3) * 4;
   const bool va = p.vec_a, vw = p.vec_w;
-  float ra[LA][4], rw[LW][4];
+  Four<TA> ra[LA];
+  Four<TW> rw[LW];
   auto fetch = [&](int k0) {
 #pragma unroll
     for (int i = 0; i < LA; ++i) load4(a_ptr[i], a_live[i], va, k0 + kq, p.K, ra[i]);
@@ -240,9 +262,9 @@ __global__ void __launch_bounds__(TILE_THREADS) gemm_simt_tile_kernel(GemmParams
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
 #pragma unroll
-      for (int i = 0; i < LA; ++i) As[b][kq + e][(tid + i * TILE_THREADS) / 4] = ra[i][e];
+      for (int i = 0; i < LA; ++i) As[b][kq + e][(tid + i * TILE_THREADS) / 4] = ra[i].at(e);
 #pragma unroll
-      for (int i = 0; i < LW; ++i) Ws[b][kq + e][(tid + i * TILE_THREADS) / 4] = rw[i][e];
+      for (int i = 0; i < LW; ++i) Ws[b][kq + e][(tid + i * TILE_THREADS) / 4] = rw[i].at(e);
     }
   };
   float2 acc[RT][4];
@@ -307,7 +329,9 @@ __global__ void __launch_bounds__(TILE_THREADS) gemm_simt_tile_kernel(GemmParams
 
 template <typename TA, typename TW, typename TO, int MODE>
 int launch_simt(const GemmParams& p, int m_tiles_hint, cudaStream_t stream) {
-  // 16 rows per tile when few rows are expected per group, else 64
+  // 16 rows per tile when few rows are expected per group, else the register tiles of 64 (17 rows already, 2,048 x 2,048: 114 us,
+  // with 4 x 4 outputs a thread and 64 rows a tile 176; bfloat16 weights 104, 162; 17 rows in each of 16 experts of
+  // 2 x 2,048 x 2,048 471, 651)
   if (m_tiles_hint <= 16) {
     const int m_tiles = (p.M + 15) / 16 + (p.group_offsets ? p.n_groups : 0);
     const dim3 grid((p.N + BN - 1) / BN, m_tiles);
