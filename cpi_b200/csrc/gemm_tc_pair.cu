@@ -632,19 +632,9 @@ using namespace cpi;
 static int g_persistent = 1;
 extern "C" void cpi_gemm_tc_pair_persistent(int mode) { g_persistent = mode; }
 
-extern "C" int cpi_gemm_tc_pair_plan(int T, int N, int K, int swiglu, int n_groups) {
-  // Features that are no multiple of 256 leave part of the last pair's rows idle (their loads give zeros, their results are not
-  // stored): at most a fifth of the work from 1,024 on.  1,855 x 2,048 -> 10,304: 109 us on the
-  // single-CTA kernel, 85 here; 1,500 x 2,048 -> 3,144: 37, 24; 2,048 x 2,048 -> 1,344: 19, 17 (so 1,024 is near the line)
-  if ((N % 256 != 0 && (N < 1024 || n_groups > 0)) || K % 8 != 0) return 0;
-  if (n_groups > 0) {
-    // experts: one token tile per expert (its weights are then read once), sized for 1.5 x the mean rows
-    if (n_groups > 256 || T < 64 * n_groups) return 0;
-    const int want = (3 * ((T + n_groups - 1) / n_groups) + 1) / 2;
-    return want > 128 ? 256 : 128;
-  }
-  if (T < 512) return 0;
-  // one pair per two SMs at a time: time ~ waves x (weight rows + half the tile width) per SM
+// The token tile of a dense product, and what it costs: one pair per two SMs at a time, time ~ waves x (weight rows + half the
+// tile width) per SM.
+static int dense_tile(int T, int N, int swiglu, long* cost_out) {
   const long sm_pairs = cpi::sm_count() / 2 > 0 ? cpi::sm_count() / 2 : 1;
   long best_cost = -1;
   int bn = 0;
@@ -656,7 +646,48 @@ extern "C" int cpi_gemm_tc_pair_plan(int T, int N, int K, int swiglu, int n_grou
     const long cost = waves * (w_rows + cand / 2 + 16);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; bn = cand; }
   }
+  *cost_out = best_cost;
   return bn;
+}
+
+extern "C" int cpi_gemm_tc_pair_plan(int T, int N, int K, int swiglu, int n_groups) {
+  // Features that are no multiple of 256 leave part of the last pair's rows idle (their loads give zeros, their results are not
+  // stored): at most a fifth of the work from 1,024 on.  Where such a product is faster here, `cpi_gemm_tc_pair_pays` says.
+  if ((N % 256 != 0 && (N < 1024 || n_groups > 0)) || K % 8 != 0) return 0;
+  if (n_groups > 0) {
+    // experts: one token tile per expert (its weights are then read once), sized for 1.5 x the mean rows
+    if (n_groups > 256 || T < 64 * n_groups) return 0;
+    const int want = (3 * ((T + n_groups - 1) / n_groups) + 1) / 2;
+    return want > 128 ? 256 : 128;
+  }
+  if (T < 512) return 0;
+  long cost;
+  return dense_tile(T, N, swiglu, &cost);
+}
+
+// Whether a dense product of features that are no multiple of 256 is faster on the pairs than on single CTAs.  Measured over
+// 512 to 8,192 tokens, 1,025 to 32,008 features and K of 512 to 8,192 (single / pairs in us, float32 stored unless said):
+//   single CTAs in one wave without splits never lose: 2,048 x 2,048 -> 1,288 17 / 21, 1,024 x 2,048 -> 4,104 22 / 26;
+//   more than a wave loses what the last one leaves idle: 2,048 x 2,048 -> 3,144 35 / 24, 512 -> 10,304 1.5 times the pairs' time, but
+//     not below 1,152 features, where the pairs' idle rows weigh as much (8,192 x 8,192 -> 1,032: 0.93 times)
+//     (ADD 512 deep at 4,096 tokens and more is the exception: 0.87 to 1.2 times);
+//   two accumulators leave one CTA an SM on either side, so there the two costs decide: 2,048 x 2,048 -> 4,104 62 / 61 at a ratio of
+//     1.28, 3,000 -> 2,056 49 / 52 at 1.22, 4,096 -> 1,160 43 / 48 at 1.0;
+//   splits meet in a reduction that the pairs don't have, for a shorter loop: 1,024 x 2,048 -> 1,032 in two splits 27 / 17, 4,096 deep
+//     32 / 28, 8,192 deep 0.88 times; in three 2,048 deep 20 / 17, 4,096 deep 23 / 28.  Outputs whose rows do not start on 16 bytes
+//     cost the pairs more: half that depth.
+extern "C" int cpi_gemm_tc_plan(int T, int N, int K, int n_groups, int swiglu, int* bn_out, int* splits_out, int* live_y_out);
+extern "C" int cpi_gemm_tc_pair_pays(int T, int N, int K, int swiglu) {
+  int bn = 0, splits = 1, live = 0;
+  if (T < 512 || N < 1024 || cpi_gemm_tc_plan(T, N, K, 0, swiglu, &bn, &splits, &live)) return 0;
+  if (splits > 1) return (long)K * splits <= (N % 4 == 0 ? 9216 : 4608);
+  const long sms = cpi::sm_count();
+  const long waves = ((long)((N + 127) / 128) * ((T + bn - 1) / bn) + sms - 1) / sms;
+  if (waves < 2 || N < 1152) return 0;
+  if (!swiglu) return 1;
+  long pairs_cost;
+  dense_tile(T, N, swiglu, &pairs_cost);
+  return waves * (bn + 256) * 40 > pairs_cost * 49;
 }
 
 // x [T, K] bf16 (row stride ldx), w [N or 2N][K] bf16 contiguous, out [T, N]; bn from cpi_gemm_tc_pair_plan.

@@ -212,6 +212,8 @@ def _plan(kind: str, device: int, T: int, N: int, K: int, n_groups: int, swiglu:
     """What the library plans for a product of these sizes on this device (a function of the sizes alone)."""
     if kind == "pair":
         return load().cpi_gemm_tc_pair_plan(c_int(T), c_int(N), c_int(K), c_int(int(swiglu)), c_int(n_groups))
+    if kind == "pays":
+        return bool(load().cpi_gemm_tc_pair_pays(c_int(T), c_int(N), c_int(K), c_int(int(swiglu))))
     bn, splits, live_y = c_int(), c_int(), c_int()
     load().cpi_gemm_tc_plan(c_int(T), c_int(N), c_int(K), c_int(n_groups), c_int(int(swiglu)), ctypes.byref(bn),
                             ctypes.byref(splits), ctypes.byref(live_y))
@@ -235,6 +237,11 @@ def gemm_pair_persistent(mode) -> None:
     tiles (the epilogue of one tile under the MMAs of the next), 0 / False = always a launch slot per tile,
     1 = the library's choice by shape (the default)."""
     load().cpi_gemm_tc_pair_persistent(c_int(2 if mode is True else 0 if mode is False else int(mode)))
+
+
+def gemm_tc_pair_pays(T: int, N: int, K: int, swiglu: bool = False) -> bool:
+    """Whether a dense product of N features, no multiple of 256, is faster on the paired kernel (see gemm_tc_pair.cu)."""
+    return _plan("pays", torch._C._cuda_getDevice(), T, N, K, 0, bool(swiglu))
 
 
 def gemm_tc_pair(a, w, out, mode=MODE_STORE, *, m_rows=None, out_rows=None, row_scale=None, group_offsets=None,

@@ -34,10 +34,11 @@ class single_cta_products:
 def project(a, w, out, mode=MODE_STORE, **kw):
     """Dense or grouped projection; see csrc/lib.py: gemm_simt for the keyword arguments."""
     if use_tensor_cores and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
-        # products with many tokens go to the two-SM kernel, dense or grouped (it refuses, launching nothing,
-        # what it does not take: few tokens per group, few features that are no multiple of 256, a row gather)
-        if use_paired_kernel and not single_cta_products.depth and "a_rows" not in kw and kw.get("m_rows", a.shape[0]) >= 512 \
-                and K.gemm_tc_pair(a, w, out, mode, any_features=True, **kw):
+        # products with many tokens go to the two-SM kernel, dense or grouped (it refuses, launching nothing, what it
+        # does not take: few tokens per group, a row gather; features that are no multiple of 256 where they don't pay)
+        rows, n = kw.get("m_rows", a.shape[0]), out.shape[1]
+        if use_paired_kernel and not single_cta_products.depth and "a_rows" not in kw and rows >= 512 and K.gemm_tc_pair(
+                a, w, out, mode, any_features=bool(n % 256) and K.gemm_tc_pair_pays(rows, n, a.shape[1], mode in K.GATED_MODES), **kw):
             return
         if K.gemm_tc(a, w, out, mode, **kw):
             return

@@ -112,3 +112,29 @@ def test_two_sm_products_of_any_number_of_features(N, mode, out_dtype):
     tol = 2.0 ** -16 if out_dtype == torch.float32 else 2.0 ** -8 * 1.02
     assert bool(((out[:, :N].double() - ref).abs() <= tol * ref.abs() + 2.0 ** -14 * ref.abs().max() * 0.1).all())
     assert torch.equal(out[:, N:], before[:, N:]) and int(K.tc_error_flag(DEV)) == 0
+
+
+@pytest.mark.parametrize("T,N,Kd,mode,pays", [
+    (2048, 1288, 2048, 0, False), (2048, 3144, 2048, 0, True), (1024, 4104, 2048, 1, False), (1024, 1032, 2048, 0, True),
+    (1024, 1032, 8192, 0, False), (512, 1032, 4096, 0, False), (8192, 1032, 512, 0, False), (700, 1025, 264, 0, False),
+    (2048, 4104, 512, 2, True), (4096, 1160, 512, 2, False), (512, 1544, 512, 2, True), (511, 10304, 512, 0, False)])
+def test_features_that_are_no_multiple_take_the_faster_kernel(T, N, Kd, mode, pays, monkeypatch):
+    """Both sides of the rule on a GPU of 148 SMs, and that a product asks it."""
+    from cpi_b200.csrc import lib as K
+    from cpi_b200.parts import linear
+    if K.sm_count() != 148:
+        pytest.skip("the rule counts waves of 148 SMs")
+    assert K.gemm_tc_pair_pays(T, N, Kd, mode == 2) == pays
+    taken, pair = [], K.gemm_tc_pair
+    monkeypatch.setattr(K, "gemm_tc_pair", lambda *a, **kw: taken.append(pair(*a, **kw)) or taken[-1])
+    randn = _rand(N)
+    a, w = randn(T, Kd).bfloat16(), (randn((2 if mode == 2 else 1) * N, Kd) * 0.1).bfloat16()
+    out = torch.zeros(T, N, device=DEV, dtype=torch.bfloat16 if mode == 2 else torch.float32)
+    linear.project(a, w, out, mode)
+    assert taken == ([] if T < 512 else [pays])
+    rows = torch.tensor([0, T // 2, T - 1], device=DEV)
+    acc = a[rows].double() @ w.double().T
+    ref = torch.nn.functional.silu(acc[:, :N]) * acc[:, N:] if mode == 2 else acc
+    # float32 sums of Kd products in the tensor cores' order, and the output's rounding
+    tol = 2.0 ** -8 * 1.02 if mode == 2 else 2.0 ** -16
+    assert bool(((out[rows].double() - ref).abs() <= tol * ref.abs() + 2.0 ** -14 * ref.abs().max() * 0.1).all())
