@@ -45,6 +45,12 @@ use_chunked_kernel = True
 # heads, 128 x 64) 121 / 172, 104 / 114, 406 / 536, 818 / 1,048; delta rule (8 heads, 128 x 256) 134 / 128, 117 / 95, 357 / 414,
 # 709 / 789, a prompt of 500 178 / 231.
 CHUNKS_FROM, DELTA_CHUNKS_FROM = 192, 256
+# Decays of at most this rank take their first projection as the last rows of the gla mixer's input product, in float32, and the
+# second from the FP32 pipe; wider ones two products of their own on the tensor cores.  All projections of a width of 2,048, 8
+# heads of 128 x 256, one way / the other in us: rank 16 10 / 15, 26 / 39 and 60 / 75 at 1, 512 and 2,048 tokens, rank 64 13 / 15, 30 /
+# 38 and 68 / 74 (8,192 tokens 221 / 215), rank 128 17 / 16, 35 / 39 and 76 / 76 (8,192 tokens 253 / 216), rank 256 26 / 17, 46 / 46
+# and 91 / 78; of a width of 512 with 64 x 64 at 2,048 tokens rank 16 26 / 38, 64 29 / 38, 128 34 / 38, 256 31 / 25.
+RIDING_RANK = 64
 # bytes of scratch for a step's chunks; a longer step runs in segments (a segment's states stay in the L2 between its passes)
 CHUNK_BYTES = 96 << 20
 # a recurrence with constant decays is cut into runs of at least this many tokens, until its blocks fill the GPU this often
@@ -174,7 +180,8 @@ class GLAMixer(Mixer):
         tn.update(p.get("tensor_names") or {})
         self.tn = {k: prefix + v for k, v in tn.items()}
         self.ws = workspace
-        self.w_in = self.w_a2 = self.b_a2 = self.w_norm = self.w_o = None
+        self.w_in = self.w_a1 = self.w_a2 = self.b_a2 = self.w_norm = self.w_o = None
+        self.rides = False
 
     def requirements(self):
         t, H, nk, nv = self.tn, self.hidden, self.nh * self.dk, self.nh * self.dv
@@ -184,8 +191,13 @@ class GLAMixer(Mixer):
 
     def load(self, source, device):
         t = self.tn
-        # the decays' first projection rides on the same product: [q | k | v | g | a1]
-        self.w_in = _cat_rows([source.get(t[n], device) for n in ("q", "k", "v", "g", "a1")])
+        first = _cat_rows([source.get(t[n], device) for n in ("q", "k", "v", "g")])
+        self.w_a1 = source.get(t["a1"], device).contiguous()
+        # the decays' first projection rides on the same product, [q | k | v | g | a1], if it is narrow
+        self.rides = self.rank <= RIDING_RANK and self.w_a1.dtype == first.dtype
+        self.w_in = torch.cat([first, self.w_a1], dim=0) if self.rides else first
+        if self.rides:
+            self.w_a1 = None
         self.w_a2 = source.get(t["a2"], device).contiguous()
         self.b_a2 = source.get(t["a2_bias"], device).to(torch.float32).contiguous()
         self.w_norm = source.get(t["norm"], device).to(torch.float32).contiguous()
@@ -198,11 +210,15 @@ class GLAMixer(Mixer):
         T, f32 = h.shape[0], torch.float32
         nk, nv = self.nh * self.dk, self.nh * self.dv
         ng = 2 * nk + 2 * nv
-        proj = self.ws.get("gla_proj", (T, -(-(ng + self.rank) // 8) * 8), f32)[:, :ng + self.rank]      # rows on 16 bytes
+        n_in = ng + (self.rank if self.rides else 0)
+        proj = self.ws.get("gla_proj", (T, -(-n_in // 8) * 8), f32)[:, :n_in]      # rows on 16 bytes
+        low = proj[:, ng:] if self.rides else self.ws.get("gla_low", (T, self.rank), h.dtype)
         z = self.ws.get("gla_z", (T, nk), f32)
         with phase("qkv"):
             project(h, self.w_in, proj)
-            project(proj[:, ng:], self.w_a2, z)
+            if not self.rides:
+                project(h, self.w_a1, low)
+            project(low, self.w_a2, z)
         o = self.ws.get("gla_o", (T, nv), f32)
         with phase("scan"):
             recurrence(self.ws, h.dtype, proj[:, nk:2 * nk], proj[:, :nk], proj[:, 2 * nk:2 * nk + nv], cache.state("s"), o, batch,

@@ -1,0 +1,64 @@
+"""The recurrent mixers as a model runs them: the routes that their sizes and steps choose, against plain 64-bit mixers."""
+import pytest
+import torch
+
+import plain_veredra
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _mixer(kind, params, seed, dtype=torch.bfloat16):
+    """(mixer, its weights by the mixer's names)."""
+    from cpi_b200.config.spec import PartSpec
+    from cpi_b200.parts import Workspace, build_part
+    from cpi_b200.weights import DictSource
+    mixer = build_part("mixer", PartSpec(kind, params), "", workspace=Workspace(DEV))
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    w = {}
+    for r in mixer.requirements():
+        t = torch.randn(r.shape, generator=g, device=DEV) * (0.3 if "conv" in r.name else 0.05)
+        w[r.name] = (t + (1.0 if "ones" in r.init else 0.0)).to(dtype)
+    mixer.load(DictSource(w), DEV)
+    return mixer, {k: w[name].double().cpu() for k, name in mixer.tn.items()}
+
+
+def _cache(mixer, n, dtype=torch.bfloat16):
+    from cpi_b200.cache import CacheManager
+    cache = CacheManager({}, {0: mixer.state_requirements()}, max_tokens=4096, max_seqs=n, dtype=dtype, device=DEV)
+    return cache, [cache.acquire() for _ in range(n)]
+
+
+def _step(mixer, cache, slots, starts, h, new):
+    from cpi_b200.engine.batch import BatchStager
+    from cpi_b200.parts import CacheView
+    stager = BatchStager(DEV)
+    cache.prepare_step(slots, new)
+    batch = stager.stage(slots, starts, [[0] * n for n in new], [[] for _ in new], h.dtype)
+    out = torch.zeros(h.shape, device=DEV)
+    mixer.forward(h, out, batch, CacheView(cache, 0))
+    cache.commit_step(slots, new)
+    torch.cuda.synchronize()
+    return out
+
+
+GLA_NAMES = {"q": "q", "k": "k", "v": "v", "g": "g", "a1": "a1", "a2": "a2", "a2.b": "a2_bias", "norm": "norm", "o": "o"}
+
+
+# decays whose first projection is part of the input product, the widest such, one more, and one that is no multiple of 8
+@pytest.mark.parametrize("rank,rides", [(16, True), (64, True), (72, False), (128, False), (100, False)])
+@pytest.mark.parametrize("T", [1, 40, 530])
+def test_decays_of_a_wide_rank_take_the_tensor_cores(rank, rides, T, monkeypatch):
+    from cpi_b200.csrc import lib as K
+    m = {"heads": 2, "dim": 64, "vdim": 64, "tau": 16.0}
+    mixer, w = _mixer("gla", {"hidden_size": 256, "heads": 2, "key_dim": 64, "value_dim": 64, "tau": 16.0, "decay_rank": rank,
+                              "norm_eps": 1e-5}, rank)
+    cache, slots = _cache(mixer, 1)
+    h = torch.randn(T, 256, generator=torch.Generator(device=DEV).manual_seed(T), device=DEV).bfloat16()
+    calls, simt = [], K.gemm_simt
+    monkeypatch.setattr(K, "gemm_simt", lambda *a, **kw: calls.append(1) or simt(*a, **kw))
+    out = _step(mixer, cache, slots, [0], h, [T])
+    assert mixer.rides == rides and len(calls) == int(rides or rank % 8 != 0)      # (rows off 16 bytes are refused there)
+    want = plain_veredra.gla_mixer(h.double().cpu(), m, lambda n: w[GLA_NAMES[n]], 1e-5)
+    # bfloat16 rounds the gated heads before W_o (and a wide rank's rows): 2^-9 of each on average
+    assert float((out.double().cpu() - want).norm() / want.norm()) <= 2.0 ** -8
