@@ -40,8 +40,9 @@ from .linear import MODE_ADD, MODE_STORE, project
 
 # set to False to run every prompt over the cached rows themselves (tests compare the two forms)
 use_formed_keys = True
-# bytes of keys and values formed at a time; a step with more forms and attends a few heads after another
-FORMED_BYTES = 1 << 29
+# Bytes of keys and values formed at a time; a step with more forms and attends a few heads after another.  The mixer's us with
+# 64, 128 and 512 MB: 16 heads x 16,384 tokens 2,202, 2,157, 2,154; 64 x 4,096 934, 897, 897; 128 x 8,192 4,874, 4,777, 4,855.
+FORMED_BYTES = 128 << 20
 
 
 def use_tensor_core_kernels() -> bool:
@@ -115,8 +116,12 @@ class LatentAttentionMixer(Mixer):
         self.w_uv = source.get(t["uv"], device).view(self.nh, self.dv, self.kv_rank).contiguous()
         if uk.is_cuda and uk.dtype == self.w_uv.dtype == torch.bfloat16 \
                 and K.latent_prefill_supported(self.d, self.r, self.dv, self.kv_rank, 64):
-            # for prompts whose keys and values are formed: head after head its rows of W_uk, then of W_uv
-            self.w_kv = torch.cat([uk, self.w_uv], dim=1).view(self.nh * (self.d + self.dv), self.kv_rank).contiguous()
+            # for prompts whose keys and values are formed: head after head its rows of W_uk, then of W_uv (without the
+            # room for this copy prompts stay with the cached rows)
+            try:
+                self.w_kv = torch.cat([uk, self.w_uv], dim=1).view(self.nh * (self.d + self.dv), self.kv_rank)
+            except torch.OutOfMemoryError:
+                self.w_kv = None
         self.w_o = source.get(t["o"], device).contiguous()
         self.w_qnorm = f32("dq_norm")
         if self.has_kv:
@@ -158,9 +163,7 @@ class LatentAttentionMixer(Mixer):
         with phase("qkv"):
             project(cq, self.w_uq, q)
         out = self.ws.get("latent_values", (T, H * self.dv), dt)
-        if self._forms_keys(batch, dt, page_size):
-            self._attend_formed(q, out, pages, table, batch, inv_freq, inter, amp)
-        else:
+        if not (self._forms_keys(batch, dt, page_size) and self._attend_formed(q, out, pages, table, batch, inv_freq, inter, amp)):
             self._attend_latent(q, out, pages, table, page_size, batch, inv_freq, inter, amp)
         if self.gate_rows:
             with phase("head_post"):
@@ -188,24 +191,29 @@ class LatentAttentionMixer(Mixer):
             pairs += n * min(start + (n + 1) // 2, self.window or start + n)
         return pairs >= 32 * rows or rows * self.nh <= 128 * longest
 
-    def _attend_formed(self, q, out, pages, table, batch, inv_freq, inter, amp):
+    def _attend_formed(self, q, out, pages, table, batch, inv_freq, inter, amp) -> bool:
+        """False, with nothing done, if there is no room for the rows, keys and values."""
         H, D, R, rank, bf16 = self.nh, self.d, self.r, self.kv_rank, torch.bfloat16
         n_rows = sum(start + n - K.latent_first_row(start, self.window) for start, n in zip(batch.starts, batch.n_new))
-        rows = self.ws.get("latent_key_rows", (n_rows, self.row), bf16)
+        per = D + self.dv
+        group = max(1, min(H, FORMED_BYTES // (2 * n_rows * per)))
+        rows, formed = self.ws.scratch(n_rows * self.row, bf16), self.ws.scratch(n_rows * group * per, bf16)
+        if rows is None or formed is None:
+            return False
+        rows = rows.view(n_rows, self.row)
         heads = self.ws.get("latent_q_heads", (batch.n_tokens, H * (D + R)), bf16)
         with phase("kv_store"):
             K.latent_key_rows(pages, rows, table, batch, window=self.window)
             K.latent_q_rows(q, inv_freq, inter, heads, batch.token_pos, n_heads=H, dim=D, rot=R, amplitude=amp)
-        per = D + self.dv
-        group = max(1, min(H, FORMED_BYTES // (2 * n_rows * per)))
         for h0 in range(0, H, group):
             h1 = min(H, h0 + group)
-            kv = self.ws.get("latent_formed", (n_rows, (h1 - h0) * per), bf16)
+            kv = formed[:n_rows * (h1 - h0) * per].view(n_rows, (h1 - h0) * per)
             with phase("qkv"):
                 project(rows[:, :rank], self.w_kv[h0 * per:h1 * per], kv)
             with phase("latent_attention"):
                 K.latent_prefill(heads, kv, rows, out, batch, heads=(h0, h1), out_heads=H, rank=rank, scale=self.scale,
                                  sink=self.sink, window=self.window)
+        return True
 
     # ---- attention over the cached rows themselves
     def _attend_latent(self, q, out, pages, table, page_size, batch, inv_freq, inter, amp):

@@ -73,13 +73,14 @@ def recurrence(ws, dtype, k, q, v, state, out, batch, *, n_heads, heads_per_grou
     kw.update(n_heads=n_heads, heads_per_group=heads_per_group, n_rows=n_rows, n_cols=n_cols, z=z, a_log=a_log)
     least = CHUNKS_FROM if kw.get("beta") is None else DELTA_CHUNKS_FROM
     if (use_chunked_kernel and dtype == torch.bfloat16 and batch.max_new >= least and K.linear_chunks_supported(n_rows, n_cols)
-            and all(t is None or (t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0) for t in (k, q, v, z, out))):
+            and all(t is None or (t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0) for t in (k, q, v, z, out, state))):
         per = K.linear_chunks_scratch(n_heads, heads_per_group, n_rows, n_cols, z=z, beta=kw.get("beta"))
         total = sum(-(-n // 64) for n in batch.n_new)
         chunks = -(-total // -(-total // max(1, CHUNK_BYTES // (4 * per))))            # segments of about the same length
-        scratch = ws.get("recurrence_chunks", (chunks * per,), torch.float32)
-        K.linear_chunks(k, q, v, state, out, batch, scratch=scratch, z_bias=z_bias, tau=tau, decay_kind=decay_kind, **kw)
-        return
+        scratch = ws.scratch(chunks * per, torch.float32)
+        if scratch is not None:
+            K.linear_chunks(k, q, v, state, out, batch, scratch=scratch, z_bias=z_bias, tau=tau, decay_kind=decay_kind, **kw)
+            return
     if z is not None:
         ready = batch.max_new > DECAY_PREPASS_FROM
         if ready:

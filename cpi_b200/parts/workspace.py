@@ -9,6 +9,7 @@ class Workspace:
         self.device = device
         self._buffers: dict = {}
         self._views: dict = {}     # what `get` last returned for a name, type and shape (a view costs as much as a launch)
+        self._no_room, self._skip = 1 << 62, 0        # the bytes that `scratch` last could not have, and how often it does not ask again
         self.generation = 0        # grows whenever a buffer is (re)allocated: captured graphs then hold stale addresses
         # A block may leave the write-back of its last sublayer to whoever touches the residual next (the next
         # block fuses it with its first read): (streams x, y, write weights, mixing matrix) or None.  Whoever
@@ -59,3 +60,21 @@ class Workspace:
             self._views.clear()
         self._views[(name, dtype, shape)] = view
         return view
+
+    def scratch(self, n: int, dtype: torch.dtype):
+        """`n` elements of device memory for the time that the caller holds them, or None if there is no room: for what a
+        long prompt can do without (a part then takes its other route).  Not kept between steps: it grows with the
+        prompts and their contexts, and an engine whose cache fills the device needs the room for other things.  Sizes are
+        rounded up to 2^k or 3 2^k, so that the allocator's cached blocks serve again."""
+        size = 1 << max(n - 1, 1).bit_length()
+        if n <= size // 4 * 3:
+            size = size // 4 * 3
+        bytes_ = size * dtype.itemsize
+        if bytes_ >= self._no_room and self._skip > 0:
+            self._skip -= 1                # (an allocation that fails costs milliseconds: not in every layer of a prompt)
+            return None
+        try:
+            return torch.empty(size, dtype=dtype, device=self.device)[:n]
+        except torch.OutOfMemoryError:
+            self._no_room, self._skip = bytes_, 64
+            return None

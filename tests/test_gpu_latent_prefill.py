@@ -152,3 +152,53 @@ def test_many_short_continuations_stay_with_the_cached_rows():
         return latent.LatentAttentionMixer._forms_keys(m, b, torch.bfloat16, 64)
     assert forms([0], [2048]) and forms([0] * 40, [100] * 40) and forms([2000], [2]) and forms([100000], [512], 1024)
     assert not forms([1000] * 16, [2] * 16) and not forms([0] * 40, [20] * 40)
+
+
+def test_a_prompt_without_room_for_keys_and_values_stays_with_the_cached_rows(monkeypatch):
+    """The same bits as with the formed keys switched off, and nothing is written before the room is known."""
+    from cpi_b200.cache import CacheManager
+    from cpi_b200.config.spec import PartSpec
+    from cpi_b200.csrc import lib as K
+    from cpi_b200.parts import CacheView, Workspace, build_part, latent
+    from cpi_b200.weights import DictSource
+    from cpi_b200.engine.batch import BatchStager
+    rope = PartSpec("rope", {"head_dim": 64, "theta": 1e4, "pairing": "interleaved", "scaling": None})
+    spec = PartSpec("latent_attention", {"hidden_size": 256, "heads": 3, "head_dim": 128, "rot_dim": 64, "value_dim": 128, "q_rank": 96,
+                                         "kv_rank": 128, "softmax_scale": 192 ** -0.5, "norm_eps": 1e-6, "position": rope, "sink": False})
+    ws = Workspace(DEV)
+    mixer = build_part("mixer", spec, "", workspace=ws)
+    g = torch.Generator(device=DEV).manual_seed(11)
+    w = {r.name: ((0.05 * torch.randn(r.shape, generator=g, device=DEV)) + (1.0 if "ones" in r.init else 0.0)).bfloat16()
+         for r in mixer.requirements()}
+    mixer.load(DictSource(w), DEV)
+    cache = CacheManager({0: mixer.kv_requirement()}, {}, max_tokens=512, max_seqs=1, dtype=torch.bfloat16, device=DEV)
+    slots = [cache.acquire()]
+    cache.prepare_step(slots, [300])
+    stager = BatchStager(DEV)
+    batch = stager.stage(slots, [0], [[0] * 300], [[]], torch.bfloat16)
+    h = torch.randn(300, 256, generator=g, device=DEV).bfloat16()
+
+    def run():
+        out = torch.zeros(h.shape, device=DEV)
+        mixer.forward(h, out, batch, CacheView(cache, 0))
+        return out
+    run()
+    monkeypatch.setattr(latent, "use_formed_keys", False)
+    want = run()
+    grown = ws.generation
+    monkeypatch.setattr(latent, "use_formed_keys", True)
+    for which in (0, 1):                                     # no room for the rows, or for the keys and values
+        asked = []
+        scratch = Workspace.scratch
+        monkeypatch.setattr(Workspace, "scratch", lambda self, n, dt: asked.append(n) or (None if len(asked) == which + 1 else scratch(self, n, dt)))
+        monkeypatch.setattr(K, "latent_key_rows", None)
+        assert torch.equal(run(), want) and len(asked) == 2
+        monkeypatch.setattr(Workspace, "scratch", scratch)
+    # a longer context moves no buffer that a captured decode graph holds
+    cache.commit_step(slots, [300])
+    cache.prepare_step(slots, [200])
+    batch = stager.stage(slots, [300], [[0] * 200], [[]], torch.bfloat16)
+    h = h[:200]
+    monkeypatch.undo()
+    run()
+    assert ws.generation == grown

@@ -62,3 +62,20 @@ def test_decays_of_a_wide_rank_take_the_tensor_cores(rank, rides, T, monkeypatch
     want = plain_veredra.gla_mixer(h.double().cpu(), m, lambda n: w[GLA_NAMES[n]], 1e-5)
     # bfloat16 rounds the gated heads before W_o (and a wide rank's rows): 2^-9 of each on average
     assert float((out.double().cpu() - want).norm() / want.norm()) <= 2.0 ** -8
+
+
+def test_a_prompt_without_room_for_chunks_is_scanned(monkeypatch):
+    from cpi_b200.csrc import lib as K
+    from cpi_b200.parts import Workspace
+    params = {"hidden_size": 256, "heads": 2, "key_dim": 64, "value_dim": 64, "tau": 16.0, "decay_rank": 16, "norm_eps": 1e-5}
+    h = torch.randn(300, 256, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV).bfloat16()
+    outs = []
+    for room in (True, False):
+        mixer, _ = _mixer("gla", params, 5)
+        cache, slots = _cache(mixer, 1)
+        if not room:
+            monkeypatch.setattr(Workspace, "scratch", lambda *a: None)
+            monkeypatch.setattr(K, "linear_chunks", None)
+        outs.append((_step(mixer, cache, slots, [0], h, [300]), cache.state_view(0, "s").clone()))
+    for x, y in zip(*outs):                                  # two orders of float32 sums, bfloat16 rows into W_o
+        assert float((x - y).norm() / y.norm()) <= 2.0 ** -8

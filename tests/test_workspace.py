@@ -30,3 +30,30 @@ def test_views_of_many_shapes_stay_right():
     ws = Workspace("cpu")
     for i in range(3000):
         assert ws.get("a", (1 + i % 1500, 2), torch.float32).shape == (1 + i % 1500, 2)
+
+
+def test_scratch_is_not_kept_and_moves_no_buffer():
+    ws = Workspace("cpu")
+    ws.get("a", (4,), torch.float32)
+    before = ws.generation
+    for n in (1, 5, 97, 1000, 4097):
+        t = ws.scratch(n, torch.float32)
+        assert t.shape == (n,) and n * 4 <= t.untyped_storage().nbytes() <= max(8, 4 * (3 * n // 2 + 2))
+    assert ws.generation == before and len(ws._buffers) == 1
+
+
+def test_scratch_without_room_is_none(monkeypatch):
+    """Where the allocator has no room, nothing is raised, and for a while nothing of that size is asked for again."""
+    ws, asked, empty = Workspace("cpu"), [], torch.empty
+
+    def full(size, **kw):
+        asked.append(size)
+        if size > 1024:
+            raise torch.OutOfMemoryError("no room")
+        return empty(size, **kw)
+    monkeypatch.setattr(torch, "empty", full)
+    assert ws.scratch(2000, torch.float32) is None and ws.scratch(2000, torch.float32) is None and ws.scratch(9000, torch.float32) is None
+    assert asked == [2048] and ws.scratch(1000, torch.float32).numel() == 1000
+    monkeypatch.setattr(torch, "empty", empty)
+    got = [ws.scratch(2000, torch.float32) is not None for _ in range(80)]
+    assert not got[0] and got[-1]
