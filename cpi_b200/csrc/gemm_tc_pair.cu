@@ -33,6 +33,12 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr uint32_t kSpinLimit = 1u << 24;
 constexpr int kMaxSlots = 512;     // token tiles of a grouped product that the persistent kernel lists
+// Shared memory of a CTA of either kernel, at least: more than half of what an SM has, so that no second pair and no other CTA
+// with tensor memory shares an SM with it.  `tcgen05.alloc.cta_group::2` needs both SMs of the pair: of two pairs that start on
+// the same two SMs at one time, one may come first on the one SM and the other on the other, and each then waits for the other
+// without limit.  Two pairs did share an SM pair, with half the shared memory each, so that one's epilogue ran under the
+// other's products; now and then a prompt with one such product behind another did not return.
+constexpr int kAlone = 116 * 1024;
 enum Mode : int { kStore = 0, kAdd = 1, kSwiglu = 2 };
 
 struct Params {
@@ -548,6 +554,7 @@ static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const
   constexpr int S0 = (222 * 1024 - EPI) / STAGE;
   constexpr int STAGES = S0 > 8 ? 8 : S0;
   constexpr int SMEM = STAGES * STAGE + EPI;
+  static_assert(SMEM >= kAlone, "a pair has its SM pair to itself");
   auto kern = gemm_tc_pair_persistent_kernel<BN, MODE, TO, STAGES>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -583,13 +590,10 @@ template <int BN, int MODE, typename TO>
 static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, dim3 grid, cudaStream_t stream) {
   constexpr int ACC = MODE == kSwiglu ? 2 : 1;
   constexpr int STAGE = ACC * BM * BK * 2 + (BN / 2) * BK * 2;
-  // One accumulator: half the shared memory per pair, so that two pairs share an SM pair and the epilogue
-  // of one runs under the matrix product of the other (measured 1.4x).  Two accumulators fill the tensor
-  // memory: one pair per SM pair, with all the stages.
-  constexpr int SMEM_LIMIT = ACC == 1 ? 108 * 1024 : 196 * 1024;
-  constexpr int S0 = SMEM_LIMIT / STAGE;
+  constexpr int S0 = 196 * 1024 / STAGE;
   constexpr int STAGES = S0 > 8 ? 8 : S0;
   constexpr int SMEM = STAGES * STAGE + 1024;
+  static_assert(SMEM >= kAlone, "a pair has its SM pair to itself");
   auto kern = gemm_tc_pair_kernel<BN, MODE, TO, STAGES>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -626,9 +630,6 @@ using namespace cpi;
 // (0: always), or whichever measured faster (1, the default).  Both run at what the L2 can deliver to the
 // SMs (a 256 x 256 pair tile at the tensor pipe's full rate would pull 64 bytes per cycle and SM, ~15 TB/s
 // over the GPU; measured: the MMA thread of the persistent kernel waits for operands a third of the time).
-// Two pairs sharing an SM pair hide that latency better for one accumulator; the persistent kernel wins
-// where the epilogue is long or cannot overlap otherwise: SwiGLU (two accumulators fill the tensor memory,
-// no second pair fits) and the read-modify-write of ADD at many tokens.
 static int g_persistent = 1;
 extern "C" void cpi_gemm_tc_pair_persistent(int mode) { g_persistent = mode; }
 
@@ -715,12 +716,14 @@ extern "C" int cpi_gemm_tc_pair(const void* x, long ldx, const void* w, void* ou
   dim3 grid(2 * n_pairs, (T + bn - 1) / bn + (n_groups > 0 ? (T < n_groups ? T : n_groups) : 0), 1);
   CPI_REQUIRE(grid.y <= 65535, "gemm_tc_pair: too many token tiles (%u)", grid.y);
   const int cap = bn <= 128 ? 128 : 256;
-  // (ADD: the persistent kernel wins where the mainloop is short against the epilogue; measured at 8,192 tokens
-  // with the copy engine's add: K = 5120 314 against 321 us, K = 8192 513 against 495 us)
+  // More tiles than SM pairs: the persistent kernel, whose epilogues run under the next tile's products (list / slots in us: 2,048 x 2,048
+  // -> 5,120 48 / 56, 4,096 x 1,024 -> 3,072 33 / 44, 8,192 x 5,120 -> 7,168 460 / 504), but not for a few long ones (2,048 x 5,120 ->
+  // 3,072 71 / 67); a tile each: slots, which have nothing to list (1,024 x 2,048 -> 2,048 20 / 19).  SwiGLU: always the list.
   // (the persistent kernel stores whole 16-byte groups of a row only: rows that do not start on 16 bytes take the other one)
   const bool rows16 = (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % (out_dtype == kF32 ? 4 : 8) == 0;
+  const long sm_pairs = cpi::sm_count() / 2, tiles = (long)n_pairs * ((T + bn - 1) / bn);
   const bool persistent = g_persistent == 2 || (g_persistent == 1 && (mode == tc2::kSwiglu ||
-                                                (mode == tc2::kAdd && T >= 4096 && K <= 6144)));
+                                                (tiles > sm_pairs && (K <= 4096 || tiles > 4 * sm_pairs))));
   const int n_slots = (T + bn - 1) / bn + (n_groups > 0 ? (T < n_groups ? T : n_groups) : 0);
   const bool persistent_groups = (g_persistent == 2 || (g_persistent == 1 && mode == tc2::kSwiglu)) && n_groups > 0 &&
                                  n_slots <= tc2::kMaxSlots;      // (measured: 2 % faster for SwiGLU, slower for STORE)

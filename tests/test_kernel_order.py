@@ -39,3 +39,15 @@ def test_successors_start_after_the_tensor_memory_is_allocated(name):
     starts = [m.start() for m in re.finditer(r"pdl_launch_dependents\(\)", body)]
     allocated = ALLOCATES.search(body).end()
     assert all(s > allocated and "__syncthreads" in body[allocated:s] for s in starts)
+
+
+def test_a_pair_of_ctas_has_its_two_sms_to_itself():
+    """The kernels on CTA pairs allocate tensor memory on two SMs at once.  Two pairs that shared an SM pair could wait for each
+    other's half, so each of their launches takes more than half of an SM's 228 KB of shared memory."""
+    text = open(os.path.join(CSRC, "gemm_tc_pair.cu")).read()
+    alone = re.search(r"constexpr int kAlone = (\d+) \* 1024;", text)
+    assert alone and 2 * int(alone.group(1)) > 228
+    launches = re.findall(r"constexpr int SMEM = [^;]*;\s*(static_assert\(SMEM >= kAlone,)?", text)
+    assert len(launches) == 2 and all(launches)
+    pairs = [k for k, body in KERNELS.items() if "tcgen05.alloc.cta_group::2" in body]
+    assert sorted(pairs) == ["gemm_tc_pair.cu:gemm_tc_pair_" + k for k in ("kernel", "persistent_kernel")]
