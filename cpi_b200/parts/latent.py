@@ -17,12 +17,16 @@
                      runs on another run entry's cache has no dkv and dkv_norm: it reads that entry's latents and rotated
                      key parts with its own queries, W_uk and W_uv (their kv_rank, rot_dim and rotation are the same).
 
-How it runs.  Only [c | r] is cached, and the keys and values of the heads are never formed: since
-q_n . (W_uk,n c) = (W_uk,n^T q_n) . c, the plain part of a query is first taken through W_uk,n^T (a grouped product, one
-group per head, over rows laid out head by head), and attention then runs over the cached rows themselves as ONE
-key/value head of kv_rank + rot_dim elements that all query heads share, with the library's attention kernels.  Its
-output per head is a weighted sum of rows [c | r]; the first kv_rank elements go through W_uv,n (the second grouped
-product) and the result through W_o.  Norms, the rotation, scores and softmax are float32 in both precisions.
+How it runs.  Only [c | r] is cached.  Decode steps, float32, and prompts of few tokens behind many positions never form the
+heads' keys and values: since q_n . (W_uk,n c) = (W_uk,n^T q_n) . c, the plain part of a query is first taken through
+W_uk,n^T (a grouped product, one group per head, over rows laid out head by head), and attention then runs over the cached
+rows themselves as ONE key/value head of kv_rank + rot_dim elements that all query heads share, with the library's
+attention kernels.  Its output per head is a weighted sum of rows [c | r]; the first kv_rank elements go through W_uv,n (the
+second grouped product) and the result through W_o.  Other bfloat16 prompts with heads of 128 + 64 elements and values of
+128 form the keys and values of the rows that their queries see, for this step only, by one product, and attend over those
+(`_forms_keys` has the rule, csrc/latent_prefill.cu the kernel); that takes a copy of W_uk and W_uv side by side (heads * 256 *
+kv_rank elements) and scratch for the rows and for up to FORMED_BYTES of keys and values, and is left out where there is no room for
+them.  Norms, the rotation, scores and softmax are float32 in both precisions.
 """
 from __future__ import annotations
 
