@@ -190,7 +190,7 @@ def main() -> int:
     g.add_argument("--mode", choices=["store", "add", "swiglu"], default="store")
     g.add_argument("--groups", type=int, default=0)
     g.add_argument("--pair", action="store_true", help="use the paired (two-SM) kernel")
-    g.add_argument("--persistent", type=int, default=None, help="paired kernel: 2 a pair per SM pair works through the tiles, 0 a launch slot per tile, 1 by shape")
+    g.add_argument("--persistent", type=int, default=None, help="paired kernel: 2 a tile after another, 0 two at a time (with groups or two accumulators a launch slot per tile), 1 by shape")
     d = sub.add_parser("attention_decode")
     d.add_argument("--batch", type=int, default=8)
     d.add_argument("--context", type=int, default=4096)

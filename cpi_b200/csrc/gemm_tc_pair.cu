@@ -130,6 +130,62 @@ template <typename TO> __device__ __forceinline__ void store_out(TO* p, float v)
 template <> __device__ __forceinline__ void store_out<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void store_out<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
+// The epilogue of a thread (one output feature n, the tile's tokens in tensor memory from `acc` on, the second accumulator's from
+// `acc2` on) for rows that do not start on 16 bytes and for narrow tiles: straight from the registers.
+template <int MODE, typename TO>
+__device__ __forceinline__ void direct(const Params& p, uint32_t acc, uint32_t acc2, int n, int t0, int n_valid_t, int n_cols) {
+  const bool row_ok = n < p.N;
+  TO* out = reinterpret_cast<TO*>(p.out);
+  if (MODE == kAdd) {
+    float* outf = reinterpret_cast<float*>(p.out);
+    float old[2][16];
+    auto fetch = [&](int c, float* dst) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int col = c + j;
+        dst[j] = (row_ok && col < n_valid_t) ? outf[(size_t)(p.out_rows ? p.out_rows[t0 + col] : t0 + col) * p.ldo + n] : 0.f;
+      }
+    };
+    fetch(0, old[0]);
+#pragma unroll 1
+    for (int c = 0; c < n_cols; c += 32) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int cc = c + 16 * h;
+        if (cc >= n_cols) break;
+        if (cc + 16 < n_cols) fetch(cc + 16, old[h ^ 1]);
+        float v[16];
+        tmem_ld16(acc + cc, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int col = cc + j;
+          if (row_ok && col < n_valid_t) {
+            const float s = p.row_scale ? p.row_scale[t0 + col] : 1.0f;
+            outf[(size_t)(p.out_rows ? p.out_rows[t0 + col] : t0 + col) * p.ldo + n] = old[h][j] + v[j] * s;
+          }
+        }
+      }
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int c = 0; c < n_cols; c += 16) {
+    float v[16], u[16];
+    tmem_ld16(acc + c, v);
+    if (MODE == kSwiglu) tmem_ld16(acc2 + c, u);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int col = c + j;
+      if (!row_ok || col >= n_valid_t) continue;
+      const float s = p.row_scale ? p.row_scale[t0 + col] : 1.0f;
+      float x = v[j] * s;
+      if (MODE == kSwiglu) x = epi::gate_mul(x, u[j] * s, p.gate_act, p.gate_limit);
+      if (MODE == kStore) x = epi::store_act(x, p.gate_act);
+      store_out<TO>(out + (size_t)(p.out_rows ? p.out_rows[t0 + col] : t0 + col) * p.ldo + n, x);
+    }
+  }
+}
+
 template <int BN, int MODE, typename TO, int STAGES>
 __global__ void __launch_bounds__(128) gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w,
                                                            const __grid_constant__ CUtensorMap map_x, Params p) {
@@ -275,7 +331,6 @@ __global__ void __launch_bounds__(128) gemm_tc_pair_kernel(const __grid_constant
   const uint32_t lane_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
   const int n_cols = min(BN, (n_valid_t + 15) & ~15);
   TO* out = reinterpret_cast<TO*>(p.out);
-  const bool row_ok = n < p.N;
   if (ok && epi::staged_ok<TO>(p.out, p.ldo, n_valid_t)) {
     // the tile is turned in shared memory (the stages are idle: every MMA has completed) and leaves in
     // whole rows
@@ -284,53 +339,8 @@ __global__ void __launch_bounds__(128) gemm_tc_pair_kernel(const __grid_constant
       auto ld = [&](int c, float* d) { tmem_ld16(lane_addr + c, d); };
     auto ldu = [&](int c, float* d) { tmem_ld16(lane_addr + BN + c, d); };
     epi::staged<MODE, TO, kStageCols>(smem, ld, ldu, warp, lane, n0, p.N, t0, n_valid_t, n_cols, out, p.ldo, p.out_rows, p.row_scale, epi::CtaSync(), p.gate_act, p.gate_limit);
-  } else if (ok && MODE == kAdd) {
-    float* outf = reinterpret_cast<float*>(p.out);
-    float old[2][16];
-    auto fetch = [&](int c, float* dst) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int col = c + j;
-        dst[j] = (row_ok && col < n_valid_t) ? outf[(size_t)(p.out_rows ? p.out_rows[t0 + col] : t0 + col) * p.ldo + n] : 0.f;
-      }
-    };
-    fetch(0, old[0]);
-#pragma unroll 1
-    for (int c = 0; c < n_cols; c += 32) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int cc = c + 16 * h;
-        if (cc >= n_cols) break;
-        if (cc + 16 < n_cols) fetch(cc + 16, old[h ^ 1]);
-        float v[16];
-        tmem_ld16(lane_addr + cc, v);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int col = cc + j;
-          if (row_ok && col < n_valid_t) {
-            const float s = p.row_scale ? p.row_scale[t0 + col] : 1.0f;
-            outf[(size_t)(p.out_rows ? p.out_rows[t0 + col] : t0 + col) * p.ldo + n] = old[h][j] + v[j] * s;
-          }
-        }
-      }
-    }
   } else if (ok) {
-#pragma unroll 1
-    for (int c = 0; c < n_cols; c += 16) {
-      float v[16], u[16];
-      tmem_ld16(lane_addr + c, v);
-      if (ACC == 2) tmem_ld16(lane_addr + BN + c, u);
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int col = c + j;
-        if (!row_ok || col >= n_valid_t) continue;
-        const float s = p.row_scale ? p.row_scale[t0 + col] : 1.0f;
-        float x = v[j] * s;
-        if (MODE == kSwiglu) x = epi::gate_mul(x, u[j] * s, p.gate_act, p.gate_limit);
-        if (MODE == kStore) x = epi::store_act(x, p.gate_act);
-        store_out<TO>(out + (size_t)(p.out_rows ? p.out_rows[t0 + col] : t0 + col) * p.ldo + n, x);
-      }
-    }
+    direct<MODE, TO>(p, lane_addr, ACC == 2 ? lane_addr + BN : 0u, n, t0, n_valid_t, n_cols);
   }
   if (!ok) {
     if (tid == 0 && p.error_flag) atomicExch(p.error_flag, 3);
@@ -340,6 +350,140 @@ __global__ void __launch_bounds__(128) gemm_tc_pair_kernel(const __grid_constant
   __syncthreads();
   cluster_sync();                                                // neither CTA leaves while the other may still use it
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
+}
+
+// ---------------------------------------------------------------------------------------------- two tiles at a time
+// Dense products with one accumulator: a pair of CTAs per SM pair whose two halves of 128 threads work on a tile each, with
+// rings, barriers and 256 columns of tensor memory of their own, so that one's fill and epilogue run under the other's
+// products.  Tiles go round the halves: c, then c + clusters, .. for the halves of cluster c, so with fewer tiles than SM
+// pairs every tile has one to itself.  (Two pairs of CTAs that shared an SM pair did the same work; see kAlone for what was wrong.)
+struct HalfSync {
+  int id;
+  __device__ __forceinline__ void operator()() const { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
+};
+
+template <int BN, int MODE, typename TO, int STAGES>
+__global__ void __launch_bounds__(256) gemm_tc_pair_dual_kernel(const __grid_constant__ CUtensorMap map_w,
+                                                                const __grid_constant__ CUtensorMap map_x, Params p, int n_pairs,
+                                                                int n_tok) {
+  constexpr uint32_t A_BYTES = BM * BK * 2, STAGE_BYTES = A_BYTES + (BN / 2) * BK * 2, RING = STAGES * STAGE_BYTES;
+  constexpr int BOX_ROWS = 64;
+  constexpr uint32_t BOX_BYTES = BOX_ROWS * BK * 2;
+  constexpr uint32_t TMEM_COLS = 2 * BN;
+  static_assert(MODE != kSwiglu && TMEM_COLS <= 512, "two tiles with one accumulator each");
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ uint64_t full_all[2][STAGES], empty_all[2][STAGES], accum_all[2];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ int abort_s[2];
+
+  const int tid = threadIdx.x, half_no = tid >> 7, warp = (tid >> 5) & 3, lane = tid & 31;
+  const uint32_t rank = cluster_rank();                          // 0: leader (issues the MMAs), 1: peer
+  if (tid == 0) {
+    for (int h = 0; h < 2; ++h) {
+      for (int s = 0; s < STAGES; ++s) { mbar_init(&full_all[h][s], 1); mbar_init(&empty_all[h][s], 1); }
+      mbar_init(&accum_all[h], 1);
+      abort_s[h] = 0;
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (tid < 32) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  fence_before_sync();
+  __syncthreads();
+  cluster_sync();                                                // the peer's barriers exist before anyone signals them
+  fence_after_sync();
+  pdl_launch_dependents();                                       // (not before the tensor memory is ours: see common.cuh)
+  uint64_t *full_bar = full_all[half_no], *empty_bar = empty_all[half_no], *accum_bar = &accum_all[half_no];
+  uint8_t* ring = smem + half_no * RING;
+  const uint32_t tmem = tmem_base_s + half_no * BN;
+  volatile int* abort_flag = &abort_s[half_no];
+  const HalfSync sync{1 + half_no};
+  const int n_clusters = gridDim.x >> 1, n_tiles = n_pairs * n_tok, n_kt = p.k_tiles;
+  int it = 0, j = 0;                                             // k steps and tiles of this half before the present tile
+  for (int pid = (blockIdx.x >> 1) + half_no * n_clusters; pid < n_tiles; pid += 2 * n_clusters, ++j, it += n_kt) {
+    // bands of up to 8 token tiles times as many weight tiles as run at one time: see the kernel above
+    const int W = 8, band = pid / (W * n_pairs), rem = pid - band * W * n_pairs, w_eff = min(W, n_tok - band * W);
+    const int t0 = (band * W + rem % w_eff) * p.bn, n_valid_t = min(p.bn, p.T - t0);
+    const int n0 = ((rem / w_eff) * 2 + (int)rank) * BM;         // this CTA's output features
+    const int n_mma = min(BN, (n_valid_t + 31) & ~31), half = n_mma / 2;
+    const int n_boxes = (half + BOX_ROWS - 1) / BOX_ROWS;
+    const uint32_t cta_tx = A_BYTES + (uint32_t)n_boxes * BOX_BYTES;
+    auto load_w = [&](int i) {
+      const int s = (it + i) % STAGES;
+      if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * cta_tx);
+      tma2_load_3d(ring + (size_t)s * STAGE_BYTES, &map_w, map_to_cta(smem_u32(&full_bar[s]), 0), i * BK, n0, 0);
+    };
+    auto load_x = [&](int i) {
+      const int s = (it + i) % STAGES;
+      for (int b = 0; b < n_boxes; ++b)
+        tma2_load_2d(ring + (size_t)s * STAGE_BYTES + A_BYTES + b * BOX_BYTES, &map_x, map_to_cta(smem_u32(&full_bar[s]), 0), i * BK,
+                     t0 + (int)rank * half + b * BOX_ROWS);
+    };
+    if (warp == 0 && lane == 0) {
+      // ---- TMA producer (both CTAs): the first tile's weights before the wait on the preceding kernel, tokens after ----
+      const int n_early = j == 0 ? min(n_kt, STAGES) : 0;
+      for (int i = 0; i < n_early; ++i) load_w(i);
+      if (j == 0) pdl_wait();
+      for (int i = 0; i < n_early; ++i) load_x(i);
+      for (int i = n_early; i < n_kt; ++i) {
+        const int g = it + i;
+        if (g >= STAGES && !mbar_wait(&empty_bar[g % STAGES], ((g / STAGES) - 1) & 1, abort_flag)) break;
+        load_w(i);
+        load_x(i);
+      }
+    } else if (warp == 1 && lane == 0 && rank == 0) {
+      // ---- MMA issuer (leader only): one instruction spans both CTAs ----
+      const uint32_t idesc = instr_desc_pair(n_mma);
+      bool ok = true;
+      for (int i = 0; i < n_kt && ok; ++i) {
+        const int g = it + i, s = g % STAGES;
+        ok = mbar_wait(&full_bar[s], (g / STAGES) & 1, abort_flag);
+        if (!ok) break;
+        fence_after_sync();
+        const uint32_t a_addr = smem_u32(ring + (size_t)s * STAGE_BYTES);
+        const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + A_BYTES);
+#pragma unroll
+        for (int q = 0; q < BK / UMMA_K; ++q) umma2_bf16(tmem, da + 2 * q, db + 2 * q, idesc, (i > 0 || q > 0) ? 1u : 0u);
+        umma2_commit_both(&empty_bar[s]);
+      }
+      if (ok) umma2_commit_both(accum_bar);
+    }
+    __syncwarp();
+    // ---- epilogue: this half of each CTA stores its 128 features of the tile's tokens ----
+    if (j == 0) pdl_wait();
+    mbar_wait(accum_bar, j & 1, abort_flag);
+    sync();                                                      // one decision for the half: nobody sets its flag from here on
+    if (abort_s[half_no]) break;
+    fence_after_sync();
+    const uint32_t lane_addr = tmem + ((uint32_t)(warp * 32) << 16);
+    const int n_cols = min(BN, (n_valid_t + 15) & ~15);
+    TO* out = reinterpret_cast<TO*>(p.out);
+    if (epi::staged_ok<TO>(p.out, p.ldo, n_valid_t)) {
+      // turned in the half's stages, which are idle: every MMA has completed
+      constexpr int kFit = (int)((size_t)RING / (128 * sizeof(TO))) / 16 * 16, kStageCols = kFit < BN ? kFit : BN;
+      auto ld = [&](int c, float* d) { tmem_ld16(lane_addr + c, d); };
+      epi::staged<MODE, TO, kStageCols>(ring, ld, ld, warp, lane, n0, p.N, t0, n_valid_t, n_cols, out, p.ldo, p.out_rows, p.row_scale,
+                                        sync, p.gate_act, p.gate_limit);
+    } else {
+      direct<MODE, TO>(p, lane_addr, 0u, n0 + warp * 32 + lane, t0, n_valid_t, n_cols);
+    }
+    // The next tile's loads overwrite the stages (through the async proxy), its products the accumulator: they wait for this
+    // CTA's loads, the loads for all of this half.
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    fence_before_sync();
+    sync();
+  }
+  __syncwarp();
+  if (abort_s[half_no]) {
+    if ((tid & 127) == 0 && p.error_flag) atomicExch(p.error_flag, 3);
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+  }
+  fence_before_sync();
+  __syncthreads();
+  cluster_sync();                                                // neither CTA leaves while the other may still use it
+  if (tid < 32) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base_s), "r"(TMEM_COLS));
 }
 
 // ---------------------------------------------------------------------------------------------- persistent
@@ -545,21 +689,13 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_persistent_kernel(const __gr
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS));
 }
 
-template <int BN, int MODE, typename TO>
-static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int n_pairs, int n_tok,
-                             cudaStream_t stream) {
-  constexpr int ACC = MODE == kSwiglu ? 2 : 1;
-  constexpr int STAGE = ACC * BM * BK * 2 + (BN / 2) * BK * 2;
-  constexpr int EPI = 64 * 128 * (int)sizeof(TO);
-  constexpr int S0 = (222 * 1024 - EPI) / STAGE;
-  constexpr int STAGES = S0 > 8 ? 8 : S0;
-  constexpr int SMEM = STAGES * STAGE + EPI;
-  static_assert(SMEM >= kAlone, "a pair has its SM pair to itself");
-  auto kern = gemm_tc_pair_persistent_kernel<BN, MODE, TO, STAGES>;
-  static bool attr_set = false;
+// A launch of one pair of CTAs per SM pair, or per tile if there are fewer.
+template <typename Kernel>
+static int launch_clusters(Kernel kern, int smem, int threads, bool& attr_set, const char* name, const CUtensorMap& mw, const CUtensorMap& mx,
+                           const Params& p, int n_pairs, int n_tok, cudaStream_t stream) {
   if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) {
-      set_error("gemm_tc_pair: cannot reserve %d bytes of shared memory", SMEM);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+      set_error("%s: cannot reserve %d bytes of shared memory", name, smem);
       return 1;
     }
     attr_set = true;
@@ -571,8 +707,8 @@ static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const
   if (clusters > n_pairs * n_tok) clusters = n_pairs * n_tok;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * clusters);
-  cfg.blockDim = dim3(192);
-  cfg.dynamicSmemBytes = SMEM;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -583,7 +719,31 @@ static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const
   cfg.numAttrs = 2;
   count_launch();
   cudaLaunchKernelEx(&cfg, kern, mw, mx, p, n_pairs, n_tok);
-  return check_launch("gemm_tc_pair_persistent");
+  return check_launch(name);
+}
+
+template <int MODE, typename TO>
+static int launch_dual(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int n_pairs, int n_tok, cudaStream_t stream) {
+  constexpr int STAGES = 3;
+  constexpr int SMEM = 2 * STAGES * (BM + 128) * BK * 2;
+  static_assert(SMEM >= kAlone, "a pair has its SM pair to itself");
+  static bool attr_set = false;
+  return launch_clusters(gemm_tc_pair_dual_kernel<256, MODE, TO, STAGES>, SMEM, 256, attr_set, "gemm_tc_pair_dual", mw, mx, p, n_pairs, n_tok, stream);
+}
+
+template <int BN, int MODE, typename TO>
+static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p, int n_pairs, int n_tok,
+                             cudaStream_t stream) {
+  constexpr int ACC = MODE == kSwiglu ? 2 : 1;
+  constexpr int STAGE = ACC * BM * BK * 2 + (BN / 2) * BK * 2;
+  constexpr int EPI = 64 * 128 * (int)sizeof(TO);
+  constexpr int S0 = (222 * 1024 - EPI) / STAGE;
+  constexpr int STAGES = S0 > 8 ? 8 : S0;
+  constexpr int SMEM = STAGES * STAGE + EPI;
+  static_assert(SMEM >= kAlone, "a pair has its SM pair to itself");
+  static bool attr_set = false;
+  return launch_clusters(gemm_tc_pair_persistent_kernel<BN, MODE, TO, STAGES>, SMEM, 192, attr_set, "gemm_tc_pair_persistent", mw, mx, p, n_pairs,
+                         n_tok, stream);
 }
 
 template <int BN, int MODE, typename TO>
@@ -626,10 +786,13 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p,
 using namespace cpi;
 
 // Whether the paired kernel takes this product, and the token-tile width it would use (0: not taken).
-// Dense products: one pair per SM pair working through a tile list (2: always), one launch slot per tile
-// (0: always), or whichever measured faster (1, the default).  Both run at what the L2 can deliver to the
-// SMs (a 256 x 256 pair tile at the tensor pipe's full rate would pull 64 bytes per cycle and SM, ~15 TB/s
-// over the GPU; measured: the MMA thread of the persistent kernel waits for operands a third of the time).
+// Three kernels: a list of tiles one after another (persistent; 2: always), two tiles at a time or, with groups or two
+// accumulators, a launch slot per tile (0: always), or by shape (1, the default).  All run at what the L2 can deliver to the SMs (a
+// 256 x 256 pair tile at the tensor pipe's full rate would pull 64 bytes per cycle and SM, ~15 TB/s over the GPU; the MMA thread of
+// the list kernel waits for operands a third of the time), and two tiles at a time hide that latency better for one accumulator:
+// list / two at a time in us, bfloat16 stored: 2,048 x 2,048 -> 3,072 34 / 25, -> 5,120 47 / 42, 2,048 x 5,120 -> 7,168 148 / 115, 8,192 x
+// 5,120 -> 7,168 467 / 439 (two pairs of CTAs that shared an SM pair took 110 and 414 there).  The list wins where two
+// accumulators leave no room for a second tile, and where ADD's epilogue is long against the products.
 static int g_persistent = 1;
 extern "C" void cpi_gemm_tc_pair_persistent(int mode) { g_persistent = mode; }
 
@@ -668,15 +831,15 @@ extern "C" int cpi_gemm_tc_pair_plan(int T, int N, int K, int swiglu, int n_grou
 
 // Whether a dense product of features that are no multiple of 256 is faster on the pairs than on single CTAs.  Measured over
 // 512 to 8,192 tokens, 1,025 to 32,008 features and K of 512 to 8,192 (single / pairs in us, float32 stored unless said):
-//   single CTAs in one wave without splits never lose: 2,048 x 2,048 -> 1,288 17 / 21, 1,024 x 2,048 -> 4,104 22 / 26;
-//   more than a wave loses what the last one leaves idle: 2,048 x 2,048 -> 3,144 35 / 24, 512 -> 10,304 1.5 times the pairs' time, but
-//     not below 1,152 features, where the pairs' idle rows weigh as much (8,192 x 8,192 -> 1,032: 0.93 times)
+//   single CTAs in one wave without splits lose little or win: 2,048 x 2,048 -> 2,056 23 / 22, -> 1,288 17 / 21;
+//   more than a wave loses what the last one leaves idle: 2,048 x 2,048 -> 3,144 36 / 25, 512 -> 10,304 37 / 24, but
+//     not below 1,152 features, where the pairs' idle rows weigh as much (8,192 x 1,024 -> 1,032 32 / 31, 8,192 deep 0.93 times)
 //     (ADD 512 deep at 4,096 tokens and more is the exception: 0.87 to 1.2 times);
 //   two accumulators leave one CTA an SM on either side, so there the two costs decide: 2,048 x 2,048 -> 4,104 62 / 61 at a ratio of
 //     1.28, 3,000 -> 2,056 49 / 52 at 1.22, 4,096 -> 1,160 43 / 48 at 1.0;
-//   splits meet in a reduction that the pairs don't have, for a shorter loop: 1,024 x 2,048 -> 1,032 in two splits 27 / 17, 4,096 deep
-//     32 / 28, 8,192 deep 0.88 times; in three 2,048 deep 20 / 17, 4,096 deep 23 / 28.  Outputs whose rows do not start on 16 bytes
-//     cost the pairs more: half that depth.
+//   splits meet in a reduction that the pairs don't have, for a shorter loop: 1,024 x 2,048 -> 1,032 in two splits 36 / 23, 5,120 deep
+//     42 / 42; in three 1,024 deep 21 / 14, 5,120 deep 35 / 48.  Outputs whose rows do not start on 16 bytes cost the pairs more:
+//     half that depth.
 extern "C" int cpi_gemm_tc_plan(int T, int N, int K, int n_groups, int swiglu, int* bn_out, int* splits_out, int* live_y_out);
 extern "C" int cpi_gemm_tc_pair_pays(int T, int N, int K, int swiglu) {
   int bn = 0, splits = 1, live = 0;
@@ -716,23 +879,27 @@ extern "C" int cpi_gemm_tc_pair(const void* x, long ldx, const void* w, void* ou
   dim3 grid(2 * n_pairs, (T + bn - 1) / bn + (n_groups > 0 ? (T < n_groups ? T : n_groups) : 0), 1);
   CPI_REQUIRE(grid.y <= 65535, "gemm_tc_pair: too many token tiles (%u)", grid.y);
   const int cap = bn <= 128 ? 128 : 256;
-  // More tiles than SM pairs: the persistent kernel, whose epilogues run under the next tile's products (list / slots in us: 2,048 x 2,048
-  // -> 5,120 48 / 56, 4,096 x 1,024 -> 3,072 33 / 44, 8,192 x 5,120 -> 7,168 460 / 504), but not for a few long ones (2,048 x 5,120 ->
-  // 3,072 71 / 67); a tile each: slots, which have nothing to list (1,024 x 2,048 -> 2,048 20 / 19).  SwiGLU: always the list.
-  // (the persistent kernel stores whole 16-byte groups of a row only: rows that do not start on 16 bytes take the other one)
+  // (ADD, list / two at a time: 4,096 x 2,048 -> 5,120 76 / 86, 8,192 x 1,024 -> 5,120 88 / 111; 4,096 x 5,120 -> 7,168 253 / 242)
+  // (the list kernel stores whole 16-byte groups of a row only: rows that do not start on 16 bytes take another one)
   const bool rows16 = (reinterpret_cast<uintptr_t>(out) & 15) == 0 && ldo % (out_dtype == kF32 ? 4 : 8) == 0;
-  const long sm_pairs = cpi::sm_count() / 2, tiles = (long)n_pairs * ((T + bn - 1) / bn);
   const bool persistent = g_persistent == 2 || (g_persistent == 1 && (mode == tc2::kSwiglu ||
-                                                (tiles > sm_pairs && (K <= 4096 || tiles > 4 * sm_pairs))));
+                                                (mode == tc2::kAdd && T >= 4096 && K <= 3072)));
   const int n_slots = (T + bn - 1) / bn + (n_groups > 0 ? (T < n_groups ? T : n_groups) : 0);
-  const bool persistent_groups = (g_persistent == 2 || (g_persistent == 1 && mode == tc2::kSwiglu)) && n_groups > 0 &&
-                                 n_slots <= tc2::kMaxSlots;      // (measured: 2 % faster for SwiGLU, slower for STORE)
+  // (groups: one accumulator with at least 192 rows a group; 16 experts of 2,048 x 2,048, list / slots in us: 512 rows 82 / 101, 256
+  // 54 / 61, 128 41 / 45; 32 of 1,024 x 768: 512 rows 57 / 68, 256 39 / 41, 128 30 / 27)
+  const bool persistent_groups = (g_persistent == 2 || (g_persistent == 1 && (mode == tc2::kSwiglu || T >= 192 * n_groups))) &&
+                                 n_groups > 0 && n_slots <= tc2::kMaxSlots;
   if ((n_groups == 0 ? persistent : persistent_groups) && cap == 256 && rows16) {
     const int n_tok = n_slots;
     if (mode == tc2::kStore && out_dtype == kBF16) return tc2::launch_persistent<256, tc2::kStore, __nv_bfloat16>(mw, mx, p, n_pairs, n_tok, stream);
     if (mode == tc2::kStore && out_dtype == kF32) return tc2::launch_persistent<256, tc2::kStore, float>(mw, mx, p, n_pairs, n_tok, stream);
     if (mode == tc2::kAdd) return tc2::launch_persistent<256, tc2::kAdd, float>(mw, mx, p, n_pairs, n_tok, stream);
     if (mode == tc2::kSwiglu) return tc2::launch_persistent<256, tc2::kSwiglu, __nv_bfloat16>(mw, mx, p, n_pairs, n_tok, stream);
+  }
+  if (n_groups == 0 && cap == 256 && mode != tc2::kSwiglu) {
+    if (mode == tc2::kAdd) return tc2::launch_dual<tc2::kAdd, float>(mw, mx, p, n_pairs, n_slots, stream);
+    if (out_dtype == kBF16) return tc2::launch_dual<tc2::kStore, __nv_bfloat16>(mw, mx, p, n_pairs, n_slots, stream);
+    return tc2::launch_dual<tc2::kStore, float>(mw, mx, p, n_pairs, n_slots, stream);
   }
 #define CPI_PAIR(CAP)                                                                                         \
   if (mode == tc2::kStore && out_dtype == kBF16) return tc2::launch<CAP, tc2::kStore, __nv_bfloat16>(mw, mx, p, grid, stream); \

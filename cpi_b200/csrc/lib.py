@@ -233,9 +233,9 @@ def gemm_tc_wait_probe(spin_limit: int = 0, tx_extra: int = 0) -> None:
 
 
 def gemm_pair_persistent(mode) -> None:
-    """Dense products of `gemm_tc_pair`: 2 / True = always one pair of CTAs per SM pair working through the
-    tiles (the epilogue of one tile under the MMAs of the next), 0 / False = always a launch slot per tile,
-    1 = the library's choice by shape (the default)."""
+    """Products of `gemm_tc_pair`: 2 / True = always the kernel that takes one tile after another (the epilogue of one
+    under the MMAs of the next), 0 / False = always two tiles at a time (with groups or two accumulators a launch slot
+    per tile), 1 = the library's choice by shape (the default)."""
     load().cpi_gemm_tc_pair_persistent(c_int(2 if mode is True else 0 if mode is False else int(mode)))
 
 

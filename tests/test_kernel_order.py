@@ -48,6 +48,6 @@ def test_a_pair_of_ctas_has_its_two_sms_to_itself():
     alone = re.search(r"constexpr int kAlone = (\d+) \* 1024;", text)
     assert alone and 2 * int(alone.group(1)) > 228
     launches = re.findall(r"constexpr int SMEM = [^;]*;\s*(static_assert\(SMEM >= kAlone,)?", text)
-    assert len(launches) == 2 and all(launches)
+    assert len(launches) == 3 and all(launches)
     pairs = [k for k, body in KERNELS.items() if "tcgen05.alloc.cta_group::2" in body]
-    assert sorted(pairs) == ["gemm_tc_pair.cu:gemm_tc_pair_" + k for k in ("kernel", "persistent_kernel")]
+    assert sorted(pairs) == ["gemm_tc_pair.cu:gemm_tc_pair_" + k for k in ("dual_kernel", "kernel", "persistent_kernel")]
