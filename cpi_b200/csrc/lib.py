@@ -991,7 +991,7 @@ def attention_f32_tiles(q, out, k_cache, v_cache, page_table, page_size, batch, 
     assert q.is_contiguous() and out.is_contiguous() and k_cache.is_contiguous() and v_cache.is_contiguous()
     assert k_cache.shape == v_cache.shape and k_cache.shape[1:] == (n_kv_heads, page_size, head_dim)
     assert q.shape == out.shape == (batch.n_tokens, n_heads * head_dim)
-    assert sink is None or (sink.dtype == torch.float32 and sink.numel() == n_heads)
+    assert sink is None or (sink.dtype == torch.float32 and sink.is_contiguous() and sink.numel() == n_heads)
     _call("cpi_attention_f32_tiles", _p(q), _p(out), _p(k_cache), _p(v_cache), _p(page_table), c_int(page_table.shape[1]),
           c_int(page_size), _p(batch.token_seq), _p(batch.token_pos), _p(batch.seq_slot), _p(batch.tile_tok0), _p(batch.tile_rows),
           c_int(batch.n_q_tiles), c_int(min(PREFILL_TILE_ROWS, batch.max_new)), c_int(n_heads), c_int(n_kv_heads), c_int(head_dim),

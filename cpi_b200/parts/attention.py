@@ -448,7 +448,8 @@ def attend(q, att, k_cache, v_cache, table, page_size, batch, *, n_heads, n_kv_h
                             scale=scale, sink=sink, keep_first=keep_first, softcap=softcap)
         return
     if (use_tile_kernel and q.dtype == torch.float32 and not batch.is_decode and batch.n_q_tiles and d == dv and d in (64, 128)
-            and score_bias is None):
+            and score_bias is None and k_cache.shape == v_cache.shape == (k_cache.shape[0], nkv, page_size, d)
+            and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (q, att, k_cache, v_cache))):
         # a sliding window that reaches over every sequence so far is no window
         everything = window_kind == "full" or (window_kind == "sliding"
                                                and max(s + n for s, n in zip(batch.starts, batch.n_new)) <= window_size)

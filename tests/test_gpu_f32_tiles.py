@@ -71,3 +71,36 @@ def test_products_of_many_rows_give_the_bits_of_the_kernel_for_few(M, N, K, mode
                 L.gemm_simt(a, ww, out, mode, m_rows=M, rows_per_group_hint=hint, gate_limit=0.7, **kw)
                 outs.append(out)
             assert torch.equal(outs[0], outs[1]) and bool(outs[0].isfinite().all())
+
+
+# the choice between the two kernels: a sliding window as long as the longest context and one shorter, chunks, a score cap, kept first
+# positions, heads of another size; rows off 16 bytes, which only the general kernel takes
+@pytest.mark.parametrize("starts,new,window,size,keep,dim,off,tiles", [
+    ([0], [150], "full", 0, 0, 64, 0, True), ([70, 0], [60, 9], "sliding", 130, 0, 64, 0, True), ([70, 0], [60, 9], "sliding", 129, 0, 64, 0, False),
+    ([0, 30], [90, 70], "sliding", 64, 5, 128, 0, False), ([0, 30], [90, 70], "sliding", 100, 5, 128, 0, True),
+    ([20, 0], [90, 70], "chunk", 48, 0, 128, 0, True), ([0], [70], "full", 0, 0, 32, 0, False), ([0], [70], "full", 0, 0, 64, 1, False),
+    ([40, 9], [1, 1], "full", 0, 0, 64, 0, False)])
+def test_both_routes_of_float32_attention_give_the_same_bits(starts, new, window, size, keep, dim, off, tiles, monkeypatch):
+    from cpi_b200.csrc import lib as K
+    from cpi_b200.engine.batch import BatchStager
+    from cpi_b200.parts import attention
+    blocks = max(-(-(s + n) // 64) for s, n in zip(starts, new))
+    table = torch.arange(len(new) * blocks, dtype=torch.int32, device=DEV).flip(0).view(len(new), blocks)
+    stager = BatchStager(DEV)
+    batch = stager.stage(list(range(len(new))), starts, [[0] * n for n in new], [[] for _ in new], torch.float32)
+    g = torch.Generator(device=DEV).manual_seed(4)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    H, G, T = 4, 2, sum(new)
+    q = randn(T * H * dim + off)[off:].view(T, H * dim)
+    k, v = randn(len(new) * blocks, G, 64, dim), randn(len(new) * blocks, G, 64, dim)
+    calls, tile_kernel = [], K.attention_f32_tiles
+    monkeypatch.setattr(K, "attention_f32_tiles", lambda *a, **kw: calls.append(1) or tile_kernel(*a, **kw))
+    outs = []
+    for use in (True, False):
+        monkeypatch.setattr(attention, "use_tile_kernel", use)
+        out = torch.full((T, H * dim), float("nan"), device=DEV)
+        attention.attend(q, out, k, v, table, 64, batch, n_heads=H, n_kv_heads=G, head_dim=dim, value_dim=dim, window_kind=window,
+                         window_size=size, scale=dim ** -0.5, sink=randn(H) * 0 + 0.3, keep_first=keep, softcap=4.0)
+        outs.append(out)
+        assert len(calls) == int(tiles)
+    assert bool(outs[0].isfinite().all()) and torch.equal(outs[0], outs[1])
