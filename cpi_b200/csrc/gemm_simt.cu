@@ -53,11 +53,11 @@ __device__ __forceinline__ void put(const GemmParams& p, TO* o, float v, float u
   *o = from_f32<TO>(v);
 }
 
-template <typename TA, typename TW, typename TO, int MODE, int TM>
+template <typename TA, typename TW, typename TO, int MODE>
 __global__ void __launch_bounds__(NT) gemm_simt_kernel(GemmParams p) {
   pdl_launch_dependents();
   pdl_wait();
-  constexpr int BM = 16 * TM;
+  constexpr int BM = 16;
   constexpr bool GLU = MODE == kSwiglu;
   __shared__ float As[BK][BM + 4];
   __shared__ float Ws[GLU ? 2 : 1][BK][BN + 4];
@@ -82,11 +82,9 @@ __global__ void __launch_bounds__(NT) gemm_simt_kernel(GemmParams p) {
   const int n0 = blockIdx.x * BN;
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
 
-  float acc[TM][4], acc2[GLU ? TM : 1][4];
+  float acc[4], acc2[4];
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { acc[i][j] = 0.f; if (GLU) acc2[i][j] = 0.f; }
+  for (int j = 0; j < 4; ++j) acc[j] = acc2[j] = 0.f;
 
   const TA* a = reinterpret_cast<const TA*>(p.a);
   // loader mapping: A tile BM x BK, 4 consecutive k per thread
@@ -120,34 +118,25 @@ __global__ void __launch_bounds__(NT) gemm_simt_kernel(GemmParams p) {
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
-      float av[TM], wv[4], wv2[4];
+      const float av = As[k][ty];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) av[i] = As[k][ty * TM + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) { wv[j] = Ws[0][k][tx * 4 + j]; if (GLU) wv2[j] = Ws[1][k][tx * 4 + j]; }
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
-          if (GLU) acc2[i][j] = fmaf(av[i], wv2[j], acc2[i][j]);
-        }
+      for (int j = 0; j < 4; ++j) {
+        acc[j] = fmaf(av, Ws[0][k][tx * 4 + j], acc[j]);
+        if (GLU) acc2[j] = fmaf(av, Ws[1][k][tx * 4 + j], acc2[j]);
+      }
     }
     __syncthreads();
   }
 
   TO* out = reinterpret_cast<TO*>(p.out);
+  const int lr = m0 + ty;
+  if (lr >= m_end) return;
+  const float s = p.row_scale ? p.row_scale[lr] : 1.0f;
+  TO* o = out + (size_t)(p.out_rows ? p.out_rows[lr] : lr) * p.ldo;
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int lr = m0 + ty * TM + i;
-    if (lr >= m_end) continue;
-    const float s = p.row_scale ? p.row_scale[lr] : 1.0f;
-    TO* o = out + (size_t)(p.out_rows ? p.out_rows[lr] : lr) * p.ldo;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < p.N) put<MODE>(p, o + n, acc[i][j] * s, GLU ? acc2[i][j] * s : 0.f);
-    }
+  for (int j = 0; j < 4; ++j) {
+    const int n = n0 + tx * 4 + j;
+    if (n < p.N) put<MODE>(p, o + n, acc[j] * s, GLU ? acc2[j] * s : 0.f);
   }
 }
 
@@ -336,7 +325,7 @@ int launch_simt(const GemmParams& p, int m_tiles_hint, cudaStream_t stream) {
     const int m_tiles = (p.M + 15) / 16 + (p.group_offsets ? p.n_groups : 0);
     const dim3 grid((p.N + BN - 1) / BN, m_tiles);
     if (grid.y > 65535) { set_error("gemm: too many row tiles (%u)", grid.y); return 1; }
-    cpi::launch_pdl(gemm_simt_kernel<TA, TW, TO, MODE, 1>, grid, NT, 0, stream, p);
+    cpi::launch_pdl(gemm_simt_kernel<TA, TW, TO, MODE>, grid, NT, 0, stream, p);
     return check_launch("gemm_simt");
   }
   const int m_tiles = (p.M + TILE_ROWS - 1) / TILE_ROWS + (p.group_offsets ? p.n_groups : 0);

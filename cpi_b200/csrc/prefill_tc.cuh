@@ -48,15 +48,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem, const CUtensorMap* map, 
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(smem_u32(smem)), "l"(map), "r"(smem_u32(bar)), "r"(c0), "r"(c1) : "memory");
 }
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-               ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
-}
-// the same with the A operand (M x 16 bfloat16, two per 32-bit column) in tensor memory
-__device__ __forceinline__ void umma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-               ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc) : "memory");
-}
 // One lane of a converged warp.  The warp that issues the MMAs runs its loop with all 32 lanes (so that the
 // compiler sees uniform values and keeps descriptors and loop counters on the uniform datapath) and only
 // the tcgen05 instructions themselves sit under this predicate.
@@ -65,7 +56,7 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
   return pred != 0;
 }
-// accumulate known at compile time: no run-time predicate set-up per instruction
+// D (+)= A B; accumulating known at compile time: no run-time predicate set-up per instruction
 template <bool ACC>
 __device__ __forceinline__ void umma_bf16_c(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc) {
   if (ACC)
@@ -75,6 +66,7 @@ __device__ __forceinline__ void umma_bf16_c(uint32_t tmem_d, uint64_t da, uint64
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, 0, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc) : "memory");
 }
+// the same with the A operand (M x 16 bfloat16, two per 32-bit column) in tensor memory
 template <bool ACC>
 __device__ __forceinline__ void umma_bf16_a_tmem_c(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc) {
   if (ACC)
