@@ -33,11 +33,15 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr uint32_t kSpinLimit = 1u << 24;
 constexpr int kMaxSlots = 512;     // token tiles of a grouped product that the persistent kernel lists
-// Shared memory of a CTA of either kernel, at least: more than half of what an SM has, so that no second pair and no other CTA
-// with tensor memory shares an SM with it.  `tcgen05.alloc.cta_group::2` needs both SMs of the pair: of two pairs that start on
-// the same two SMs at one time, one may come first on the one SM and the other on the other, and each then waits for the other
-// without limit.  Two pairs did share an SM pair, with half the shared memory each, so that one's epilogue ran under the
-// other's products; now and then a prompt with one such product behind another did not return.
+// Two rules for every launch of a kernel on pairs.
+// No early start: these kernels are launched without programmatic dependence, after the kernel before them has ended (that one's
+// successors may start early as elsewhere).  Started early behind row kernels of many blocks, now and then such a product did
+// not return: prompts of 32,768 tokens (query product behind the norm and the page write, 32,768 blocks each) stopped within 11 to 50
+// passes, whether two pairs shared an SM pair or one had it alone; without the early start 525 passes ran through.  It costs a
+// product 2 to 4 us (a latent prompt's mixer of 2,048 tokens 167 -> 179 us with its four).
+// Alone: a CTA takes more than half of an SM's shared memory, so that no second pair and no other CTA with tensor memory shares
+// an SM with it.  `tcgen05.alloc.cta_group::2` has no limit and needs both SMs of the pair: of two pairs that start on the same two SMs
+// at one time, one may come first on the one SM and the other on the other.
 constexpr int kAlone = 116 * 1024;
 enum Mode : int { kStore = 0, kAdd = 1, kSwiglu = 2 };
 
@@ -710,13 +714,11 @@ static int launch_clusters(Kernel kern, int smem, int threads, bool& attr_set, c
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[1];                                   // (no early start: see above kAlone)
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = 1;
   count_launch();
   cudaLaunchKernelEx(&cfg, kern, mw, mx, p, n_pairs, n_tok);
   return check_launch(name);
@@ -768,13 +770,11 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const Params& p,
   cfg.blockDim = dim3(128);
   cfg.dynamicSmemBytes = SMEM;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[1];                                   // (no early start: see above kAlone)
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = 1;
   count_launch();
   cudaLaunchKernelEx(&cfg, kern, mw, mx, p);
   return check_launch("gemm_tc_pair");

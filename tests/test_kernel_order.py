@@ -51,3 +51,10 @@ def test_a_pair_of_ctas_has_its_two_sms_to_itself():
     assert len(launches) == 3 and all(launches)
     pairs = [k for k, body in KERNELS.items() if "tcgen05.alloc.cta_group::2" in body]
     assert sorted(pairs) == ["gemm_tc_pair.cu:gemm_tc_pair_" + k for k in ("dual_kernel", "kernel", "persistent_kernel")]
+
+
+def test_kernels_on_cta_pairs_are_not_started_early():
+    """Launched behind row kernels of many blocks before those had ended, they did not always return."""
+    text = open(os.path.join(CSRC, "gemm_tc_pair.cu")).read()
+    assert text.count("cudaLaunchKernelEx(") == 2 and "cudaLaunchAttributeProgrammaticStreamSerialization" not in text
+    assert "launch_pdl(" not in text
