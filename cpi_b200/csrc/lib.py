@@ -207,11 +207,38 @@ def gemm_tc(a, w, out, mode=MODE_STORE, *, n_out=None, m_rows=None, a_rows=None,
     return True
 
 
+def gemm_few(a, w, out, mode=MODE_STORE, *, m_rows=None, gate_limit=0.0, **kw) -> bool:
+    """The product of up to 32 tokens with a dense weight matrix in bfloat16, weights from memory into registers (see
+    gemm_few.cu).  Returns False, having launched nothing, when the product is outside what it takes (groups, row lists,
+    scales, unaligned operands) or `gemm_tc` is faster."""
+    T, K = m_rows if m_rows is not None else a.shape[0], a.shape[1]
+    if T > 32 or w.dim() != 2 or any(v is not None for v in kw.values()) or a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
+        return False
+    if a.stride(1) != 1 or not w.is_contiguous() or out.stride(-1) != 1:
+        return False
+    if K % 8 or a.stride(0) % 8 or a.data_ptr() % 16 or w.data_ptr() % 16 or w.shape[1] != K:
+        return False
+    N = w.shape[0] // 2 if mode in GATED_MODES else w.shape[0]
+    if out.shape[1] != N or out.dtype not in (torch.bfloat16, torch.float32) or T > a.shape[0]:
+        return False
+    if (mode in GATED_MODES and (out.dtype != torch.bfloat16 or w.shape[0] % 2)) or (mode == MODE_ADD and out.dtype != torch.float32):
+        return False
+    form = _plan("few", torch._C._cuda_getDevice(), T, N, 0, 0, False)
+    if not form:
+        return False
+    _need_cuda(a, w, out)
+    _call("cpi_gemm_few", _p(a), c_long(a.stride(0)), _p(w), _p(out), c_int(dtype_code(out.dtype)), c_long(out.stride(0)),
+          c_int(T), c_int(N), c_int(K), c_int(mode), c_int(form), c_float(gate_limit), _stream())
+    return True
+
+
 @functools.lru_cache(maxsize=4096)
 def _plan(kind: str, device: int, T: int, N: int, K: int, n_groups: int, swiglu: bool):
     """What the library plans for a product of these sizes on this device (a function of the sizes alone)."""
     if kind == "pair":
         return load().cpi_gemm_tc_pair_plan(c_int(T), c_int(N), c_int(K), c_int(int(swiglu)), c_int(n_groups))
+    if kind == "few":
+        return load().cpi_gemm_few_plan(c_int(T), c_int(N))
     if kind == "pays":
         return bool(load().cpi_gemm_tc_pair_pays(c_int(T), c_int(N), c_int(K), c_int(int(swiglu))))
     bn, splits, live_y = c_int(), c_int(), c_int()

@@ -1,7 +1,7 @@
 """Matrix products of the parts: picks the kernel for a contraction out[m, n] = sum_k a[m, k] w[n, k].
 
-bfloat16 activations and weights whose shapes the tensor-core kernel accepts go to the tcgen05
-kernel; everything else -- the whole float32 path, mixed dtypes, odd shapes -- goes to the FP32-pipe
+bfloat16 activations and weights whose shapes the tensor-core kernels accept go to the tcgen05
+kernels, or for a handful of tokens to one that is over when theirs have begun; everything else -- the whole float32 path, mixed dtypes, odd shapes -- goes to the FP32-pipe
 kernel, which accepts any size.  Either way accumulation is float32.
 """
 from __future__ import annotations
@@ -37,6 +37,9 @@ def project(a, w, out, mode=MODE_STORE, **kw):
         # products with many tokens go to the two-SM kernel, dense or grouped (it refuses, launching nothing, what it
         # does not take: few tokens per group, a row gather; features that are no multiple of 256 where they don't pay)
         rows, n = kw.get("m_rows", a.shape[0]), out.shape[1]
+        # a handful of tokens: weights straight into registers (refuses, launching nothing, where the tcgen05 kernel is faster)
+        if rows <= 32 and K.gemm_few(a, w, out, mode, **kw):
+            return
         if use_paired_kernel and not single_cta_products.depth and "a_rows" not in kw and rows >= 512 and K.gemm_tc_pair(
                 a, w, out, mode, any_features=bool(n % 256) and K.gemm_tc_pair_pays(rows, n, a.shape[1], mode in K.GATED_MODES), **kw):
             return

@@ -1,0 +1,91 @@
+"""The product for a handful of tokens (csrc/gemm_few.cu) against 64-bit products: edges of its 16 features, 8 tokens and 32 k."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def K():
+    from cpi_b200.csrc import lib
+    return lib
+
+
+def operands(T, N, Kd, rows, seed=0, ldx=0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    a = torch.randn(T, Kd + ldx, generator=g, device=DEV).bfloat16()[:, :Kd]
+    w = torch.randn(rows, Kd, generator=g, device=DEV).bfloat16()
+    return a, w
+
+
+def bound(a, w, out):
+    """Products of bfloat16 pairs are exact in float32; a sum of K of them in any order is off by at most K + 1 truncations."""
+    return (a.shape[1] + 1) * 2.0 ** -23 * (a.double().abs() @ w.double().abs().T) + 1e-30
+
+
+def launch(a, w, out, mode, form, limit=0.0):
+    from ctypes import c_float, c_int, c_long
+    k = K()
+    k._call("cpi_gemm_few", k._p(a), c_long(a.stride(0)), k._p(w), k._p(out), c_int(k.dtype_code(out.dtype)), c_long(out.stride(0)),
+            c_int(a.shape[0]), c_int(out.shape[1]), c_int(a.shape[1]), c_int(mode), c_int(form), c_float(limit), k._stream())
+
+
+@pytest.mark.parametrize("form", [1, 2, 3, 4])
+@pytest.mark.parametrize("T,N,Kd", [(1, 1, 8), (1, 17, 40), (3, 520, 264), (8, 16, 1032), (9, 33, 2048), (16, 200, 4104), (2, 48, 8200)])
+def test_forms_against_64_bit_products(form, T, N, Kd):
+    k = K()
+    a, w = operands(T, N, Kd, N, ldx=24)
+    ref = a.double() @ w.double().T
+    for dt in (torch.float32, torch.bfloat16):
+        buf = torch.full((T + 1, N + 5), 7.0, device=DEV, dtype=dt)
+        out = buf[:T, :N]
+        launch(a, w, out, k.MODE_STORE, form)
+        tol = bound(a, w, out) + (2.0 ** -8 * ref.abs() if dt == torch.bfloat16 else 0)
+        assert ((out.double() - ref).abs() <= tol).all()
+        assert (buf[T] == 7).all() and (buf[:, N:] == 7).all()                  # nothing beside the outputs
+    res = torch.randn(T, N, device=DEV)
+    out = res.clone()
+    launch(a, w, out, k.MODE_ADD, form)
+    assert ((out.double() - res.double() - ref).abs() <= bound(a, w, out) + 2.0 ** -23 * out.double().abs()).all()
+
+
+@pytest.mark.parametrize("T,N,Kd", [(17, 200, 264), (24, 2368, 520), (32, 16, 2048), (32, 33, 8)])
+def test_more_tokens(T, N, Kd):
+    k = K()
+    a, w = operands(T, N, Kd, N)
+    out = torch.zeros(T, N, device=DEV)
+    assert k.gemm_few(a, w, out) == (N <= 16 * k.sm_count())
+    if N <= 16 * k.sm_count():
+        assert ((out.double() - a.double() @ w.double().T).abs() <= bound(a, w, out)).all()
+
+
+@pytest.mark.parametrize("T", [1, 8, 11, 32])
+def test_gates_and_activations(T):
+    """Every mode against the tcgen05 kernel's epilogue: the same functions of sums that agree to the order of their terms."""
+    k = K()
+    N, Kd = 72, 512
+    a, w = operands(T, N, Kd, 2 * N, seed=3)
+    w *= 0.05
+    forms = [1] if T > 16 else [1, 2, 3, 4]
+    for mode in (k.MODE_SWIGLU, k.MODE_GEGLU, k.MODE_CLAMPED_GLU, k.MODE_STORE_RELU2, k.MODE_STORE_GELU):
+        gated = mode in k.GATED_MODES
+        wm = w if gated else w[:N].contiguous()
+        want, limit = torch.zeros(T, N, device=DEV, dtype=torch.bfloat16), 2.0 if mode == k.MODE_CLAMPED_GLU else 0.0
+        assert k.gemm_tc(a, wm, want, mode, gate_limit=limit)
+        for form in forms:
+            got = torch.zeros_like(want)
+            launch(a, wm, got, mode, form, limit)
+            # (a bfloat16 step, where a sum's last bits tip the rounding, and what sums near zero differ by)
+            assert ((got - want).float().abs() <= 2.0 ** -7 * want.float().abs() + 1e-4).all(), (mode, form)
+
+
+def test_what_it_leaves_to_other_kernels():
+    k = K()
+    a, w = operands(4, 64, 128, 64)
+    out = torch.zeros(4, 64, device=DEV)
+    assert k.gemm_few(a, w, out)
+    assert not k.gemm_few(a.float(), w, out) and not k.gemm_few(a, w.float(), out)
+    assert not k.gemm_few(a[:, 4:], w[:, 4:], out)                                # rows off 16 bytes
+    assert not k.gemm_few(a, w, out, k.MODE_SWIGLU) and not k.gemm_few(a, w, out.bfloat16(), k.MODE_ADD)
+    assert not k.gemm_few(a, w, out, row_scale=torch.ones(4, device=DEV))
+    assert not k.gemm_few(operands(33, 64, 128, 64)[0], w, torch.zeros(33, 64, device=DEV))
