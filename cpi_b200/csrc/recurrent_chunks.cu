@@ -15,28 +15,27 @@
 //
 // whose right-hand sides are solved for all chunks at once; the pass over the chunks then is u = U^ - W S, S' = D S + k~^T u.
 //
-// Everything is float32 on the FP32 pipe, as in the scan.  Products of decays are always taken forward, one factor after
-// another, never as a quotient or as the exponential of a sum of logarithms: they lose no digits however strong the decays
-// are and underflow to the zero that the scan reaches too.  A token's output reads nothing of later tokens.
+// Everything is float32, as in the scan; the two large products (U, and the outputs) run on the tensor cores with each operand
+// as three bfloat16 terms, which loses no more than the float32 sums (see there), the rest on the FP32 pipe.  Products of
+// decays are always taken forward, one factor after another, never as a quotient or as the exponential of a sum of logarithms:
+// they lose no digits however strong the decays are and underflow to the zero that the scan reaches too.  A token's output
+// reads nothing of later tokens.
 //
-// Why not the tensor cores: the operands are float32 (three bfloat16 terms each), which takes six products for one; at the
-// rate of mma.sync that is what the FP32 pipe does without any splitting.
-//
-// Measured (one prompt of 2,048 tokens, width 2,048): the recurrence of gated linear attention with 8 heads of 128 x 256
-// 480 -> 114 us (prepare_rows 34, chunk_state 24, chain 14, chunk_out 40; the FP32 pipe's floor is 36), the delta rule at
-// 1,500 tokens 435 -> 176 us (48, solve 21, delta_chain 76, 31), the state-space form with 64 heads of 128 x 64 at 1,855 tokens
-// 507 -> 183 us (prepare_step 15, 53, 35, 80; floor 64).
+// Measured (one prompt of 2,048 tokens, width 2,048), the scan, all on the FP32 pipe, here: the recurrence of gated linear
+// attention with 8 heads of 128 x 256 480, 114, 81 us (prepare_rows 32, chunk_state 25 -> 15, chain 15, chunk_out 41 -> 19; its bytes
+// through the L2 take about 20), the delta rule at 1,500 tokens 435, 176, 163 us (45, solve 21, delta_chain 77, 31 -> 19), the
+// state-space form with 64 heads of 128 x 64 at 1,855 tokens 507, 187, 149 us (prepare_step 18, 53 -> 26, 31, 80 -> 74).
 //
 //   prepare_rows   the decays per row (their transform too), and A, q~, k~, D (and M, K^) of a chunk and head
-//   prepare_step   C_i . B_j and C transposed, of a chunk and group of heads: one decay per head and token
+//   prepare_step   C_i . B_j of a chunk and group of heads, and the heads' decays: one per head and token
 //   solve          W and U^ of the delta rule: 128 right-hand sides a block, 16 x 16 blocks of the triangle in registers
-//   chunk_state    U = k~^T v, 128 x 64 (or 64 x 64) a block, 8 x 8 a thread
+//   chunk_state    U = k~^T v, tiles of 64 columns
 //   chain          the states between the chunks; `delta_chain` with the delta rule, 16 columns a block
-//   chunk_out      the outputs, 64 tokens x 64 columns a block, 8 x 8 a thread, the triangle's dead part left out
+//   chunk_out      the outputs, 64 tokens x 128 (or 64) columns a tile
 //
 // A long step runs in segments of chunks so that the scratch stays within what the caller gives.
 #include "decay.cuh"
-#include <type_traits>
+#include "prefill_tc.cuh"
 
 namespace cpi {
 namespace chunks {
@@ -55,8 +54,9 @@ struct Params {
   float* out; long out_stride;
   const int* seq_slot; const int* seq_tok0; const int* seq_new;
   int H, hpg, N, Dv, n_seqs;
+  int* error_flag;                               // raised by a tensor-core kernel whose wait ran out
   int seg0, seg_chunks;                          // this launch's chunks, counted over all sequences: seg0 .. seg0 + seg_chunks - 1
-  // scratch, per chunk of the segment and head (AT and QT of the step flavour: and group)
+  // scratch, per chunk of the segment and head (AT of the step flavour: and group; its MT: the heads' Decays)
   float *U, *KT, *QT, *AT, *DC, *MT, *KP, *WT, *UH;
 };
 
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
   copy_wait<0>();
   __syncthreads();
   {
-    float *AT = p.AT + c.item * (size_t)(C * C) + (size_t)j * C, *MT = DELTA ? p.MT + c.item * (size_t)(C * C) + (size_t)j * C : nullptr;
+    float *AT = p.AT + c.item * (size_t)(C * C) + j, *MT = DELTA ? p.MT + c.item * (size_t)(C * C) + (size_t)j * C : nullptr;
     auto decay = [&](int i) {
       const float* ai = as + i * N + 4 * kk;
 #pragma unroll
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
       }
       const float y = sum4(s, kk), z = DELTA ? sum4(m, kk) : 0.f;
       if (kk < 4) {
-        AT[i + kk] = y * p.q_scale;
+        AT[(i + kk) * C] = y * p.q_scale;
         if (DELTA) MT[i + kk] = z * bs[i + kk];
       }
     }
@@ -223,17 +223,12 @@ __global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
   if (tid >= 256 && tid < 256 + N) {
     const int n = tid - 256;
     float P = 1.f;
-    float *QT = p.QT + c.item * (size_t)(N * C) + (size_t)n * C, *KP = DELTA ? p.KP + c.item * (size_t)(N * C) + n : nullptr;
-#pragma unroll 4
-    for (int i = 0; i < C; i += 4) {
-      float y[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        P *= as[(i + e) * N + n];
-        y[e] = qs[(i + e) * N + n] * P * p.q_scale;
-        if (DELTA) KP[(size_t)(i + e) * N] = ks[(i + e) * N + n] * P;
-      }
-      st4(QT + i, y[0], y[1], y[2], y[3]);
+    float *QT = p.QT + c.item * (size_t)(N * C) + n, *KP = DELTA ? p.KP + c.item * (size_t)(N * C) + n : nullptr;
+#pragma unroll 16
+    for (int i = 0; i < C; ++i) {
+      P *= as[i * N + n];
+      QT[(size_t)i * N] = qs[i * N + n] * P * p.q_scale;
+      if (DELTA) KP[(size_t)i * N] = ks[i * N + n] * P;
     }
   } else if (tid >= 512 - N) {
     const int n = tid - (512 - N);
@@ -249,7 +244,56 @@ __global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
   }
 }
 
-// ---- one decay per head and token: C_i . B_j and C transposed, once per group of heads ---------------------------------
+// ---- one decay per head and token: C_i . B_j, once per group of heads, and the decays of its heads ------------------------
+// A chunk's decays, one per token: step sizes, decays, what the token's value is written with into the chunk's state (dt_j
+// prod_{t > j} a_t), products of decays from the chunk's begin and from the begin of the token's run of eight to the token, and
+// of the whole runs between two.  Formed here once and read by every block that needs them: the chain of loads, exponentials
+// and scans (5,000 cycles) would stand at the begin of each.
+struct Decays { float dt[C], a[C], w[C], upto[C], run[C], mid[8][8]; };
+constexpr int DECAYS = sizeof(Decays) / sizeof(float);
+__device__ __forceinline__ void decays_of(const Params& p, const Place& c, int h, int lane) {      // one warp; lane: tokens 2 lane, 2 lane + 1
+  const float rate = -expf(load_any(p.a_log, p.small_dtype, h)), bias = p.dt_bias ? load_any(p.dt_bias, p.small_dtype, h) : 0.f;
+  const size_t item = (size_t)blockIdx.x * p.H + h;
+  float dt[2], a[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int j = 2 * lane + e;
+    dt[e] = j < c.n ? softplus_f(p.dt[(size_t)(c.tok + j) * p.dt_stride + h] + bias) : 0.f;
+    a[e] = j < c.n ? expf(rate * dt[e]) : 1.f;
+  }
+  // over the lanes up to this one, from this one on, and within its run of eight tokens
+  float upto = a[0] * a[1], from = upto, run = upto;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float x = __shfl_up_sync(0xffffffffu, upto, o), y = __shfl_up_sync(0xffffffffu, run, o), z = __shfl_down_sync(0xffffffffu, from, o);
+    if (lane >= o) upto *= x;
+    if (lane + o < 32) from *= z;
+    if (o < 4 && (lane & 3) >= o) run *= y;
+  }
+  float before = __shfl_up_sync(0xffffffffu, upto, 1), run_before = __shfl_up_sync(0xffffffffu, run, 1), after = __shfl_down_sync(0xffffffffu, from, 1);
+  if (lane == 0) before = 1.f;
+  if ((lane & 3) == 0) run_before = 1.f;
+  if (lane == 31) after = 1.f;
+  Decays& D = reinterpret_cast<Decays*>(p.MT)[item];
+  auto put = [&](float* to, float x, float y) { reinterpret_cast<float2*>(to)[lane] = make_float2(x, y); };
+  put(D.dt, dt[0], dt[1]);
+  put(D.a, a[0], a[1]);
+  put(D.w, dt[0] * (a[1] * after), dt[1] * after);
+  put(D.upto, before * a[0], upto);
+  put(D.run, run_before * a[0], run);
+  float whole[8];                                              // of each run
+#pragma unroll
+  for (int r = 0; r < 8; ++r) whole[r] = __shfl_sync(0xffffffffu, run, 4 * r + 3);
+  const int x = lane / 4, y = lane % 4 * 2;                    // mid[x][y], mid[x][y + 1]: the runs x + 1 .. y - 1
+  float m0 = 1.f, m1 = 1.f;
+#pragma unroll
+  for (int r = 1; r < 8; ++r) {
+    if (r > x && r < y) m0 *= whole[r];
+    if (r > x && r < y + 1) m1 *= whole[r];
+  }
+  put(&D.mid[0][0], m0, m1);
+  if (lane == 0) p.DC[item] = from;
+}
 template <int N>
 __global__ void __launch_bounds__(256) prepare_step_kernel(Params p) {
   constexpr int LD = N + 4;
@@ -259,6 +303,7 @@ __global__ void __launch_bounds__(256) prepare_step_kernel(Params p) {
   const int g = blockIdx.y, G = p.H / p.hpg, tid = threadIdx.x;
   const Place c = place(p, blockIdx.x, g, G);
   if (c.n <= 0) return;
+  for (int h = g * p.hpg + (tid >> 5); h < (g + 1) * p.hpg; h += 8) decays_of(p, c, h, tid & 31);
   for (int e = tid; e < C * N / 4; e += 256) {
     const int j = e / (N / 4), n = e % (N / 4) * 4;
     const bool live = j < c.n;
@@ -268,7 +313,7 @@ __global__ void __launch_bounds__(256) prepare_step_kernel(Params p) {
   }
   __syncthreads();
   // thread: tokens i0, i0 + 16, .. of C against tokens j0, j0 + 16, .. of B
-  const int i0 = tid & 15, j0 = tid >> 4;
+  const int j0 = tid & 15, i0 = tid >> 4;
   float acc[4][4];
 #pragma unroll
   for (int x = 0; x < 4; ++x)
@@ -289,24 +334,7 @@ __global__ void __launch_bounds__(256) prepare_step_kernel(Params p) {
 #pragma unroll
   for (int x = 0; x < 4; ++x)
 #pragma unroll
-    for (int y = 0; y < 4; ++y) AT[(j0 + 16 * y) * C + i0 + 16 * x] = acc[x][y] * p.q_scale;
-  float* QT = p.QT + c.item * (size_t)(N * C);
-  for (int e = tid; e < N * C / 4; e += 256) {
-    const int n = e % N, i = e / N * 4;
-    st4(QT + (size_t)n * C + i, cs[i * LD + n] * p.q_scale, cs[(i + 1) * LD + n] * p.q_scale, cs[(i + 2) * LD + n] * p.q_scale,
-        cs[(i + 3) * LD + n] * p.q_scale);
-  }
-}
-
-// The step sizes and decays of a chunk's tokens: one warp, lane l holds the tokens 2 l and 2 l + 1 (a = 1, dt = 0 past them).
-__device__ __forceinline__ void step_of(const Params& p, const Place& c, int h, int lane, float (&dt)[2], float (&a)[2]) {
-  const float rate = -expf(load_any(p.a_log, p.small_dtype, h)), bias = p.dt_bias ? load_any(p.dt_bias, p.small_dtype, h) : 0.f;
-#pragma unroll
-  for (int e = 0; e < 2; ++e) {
-    const int j = 2 * lane + e;
-    dt[e] = j < c.n ? softplus_f(p.dt[(size_t)(c.tok + j) * p.dt_stride + h] + bias) : 0.f;
-    a[e] = j < c.n ? expf(rate * dt[e]) : 1.f;
-  }
+    for (int y = 0; y < 4; ++y) AT[(i0 + 16 * x) * C + j0 + 16 * y] = acc[x][y] * p.q_scale;
 }
 
 // ---- the delta rule's right-hand sides -----------------------------------------------------------------------------------
@@ -361,88 +389,261 @@ __global__ void __launch_bounds__(128) solve_kernel(Params p) {
   }
 }
 
-// A thread's eight columns of a 64-column row: x0 .. x0 + 3 and 32 further (eight lanes read 128 neighbouring bytes), as
-// pairs for the packed float32 instructions (each half rounds as the single instruction does; 122 against 92 FMA per clock
-// and SM measured at 16 warps).
-__device__ __forceinline__ void load_cols(const float* p, float2 (&b)[4]) {
-  const float4 u = ld4(p), v = ld4(p + 32);
-  b[0] = make_float2(u.x, u.y); b[1] = make_float2(u.z, u.w); b[2] = make_float2(v.x, v.y); b[3] = make_float2(v.z, v.w);
+// ---- products on the tensor cores -----------------------------------------------------------------------------------------
+// A float32 operand enters as three bfloat16 terms, x = h + m + l to 2^-25 of it (8 bits a term).  Of the nine products of
+// terms the six above 2^-24 are taken.  h h has an accumulator of its own and the small ones another: a product adds into its
+// accumulator with one truncation, so what counts is how many of them the large sum sees, K / 16 for the 64 to 192 terms
+// here, no more than a float32 sum of that length loses (against 64 bits, decays as layers are initialised: outputs 2.5e-7 and
+// states 2.4e-7 off with float32 sums, 1.9e-7 and 2.1e-7 with these; with one decay per token 1.5e-7 and 9.9e-7, 1.2e-7 and 9.7e-7).
+//
+// The operand with a row a lane (M) is loaded a lane's row a thread, its neighbours' beside it, split in registers and left in
+// tensor memory; the other goes to shared memory as it lies in memory, a tile of 64 rows of 64 columns per term, 128 bytes a
+// row in the 128-byte swizzle, read MN-major where its rows are k, else K-major.  With both in shared memory a product of 64
+// columns waits for its operands (83 cycles instead of 32), and writing and reading them fill that memory's pipe: blocks of 256
+// threads, three an SM, took 28 us for the outputs of 8 heads of 128 x 256 at 2,048 tokens, a stream of warps with a task each
+// (splitting, issuing, writing out) 33, the form here 19.  What bounds it now is latency: a slice of 64 k takes two blocks an SM
+// 4,000 cycles (splitting 700, loads' issue 900, 24 products 1,100, waits) of which the tensor pipe works 1,500.
+using pre::smem_u32;
+constexpr uint32_t TILE = 64 * 128;
+constexpr int TC_THREADS = 256;
+constexpr uint32_t TC_COLUMNS = 256;                           // tensor memory: h h, small products (64 each), three terms of M (96)
+constexpr uint32_t SMALL = 64, TERMS = 128;
+
+// h, m and l of a pair, packed
+__device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
+  h = pre::pack_bf16(a, b);
+  a -= __uint_as_float(h << 16);
+  b -= __uint_as_float(h & 0xffff0000u);
+  m = pre::pack_bf16(a, b);
+  a -= __uint_as_float(m << 16);
+  b -= __uint_as_float(m & 0xffff0000u);
+  l = pre::pack_bf16(a, b);
 }
-__device__ __forceinline__ void store_cols(float* p, const float2 (&a)[4]) {
-  st4(p, a[0].x, a[0].y, a[1].x, a[1].y);
-  st4(p + 32, a[2].x, a[2].y, a[3].x, a[3].y);
+// The M operand, 128 lanes x 64 k: a thread has 32 k of a lane's row (warps 0 to 3 the first ones).  Element k of a lane's row is
+// src[k * stride] with src at the lane's column.
+struct LaneOperand {
+  float x[32];
+  __device__ __forceinline__ void load(const float* src, size_t stride, int n) {     // n of the thread's k; the rest are zeros
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+      x[k] = k < n ? *src : 0.f;
+      src += stride;
+      asm volatile("" : "+l"(src));                            // (32 addresses at a time would not fit in registers)
+    }
+  }
+  __device__ __forceinline__ void split(uint32_t (&w)[3][16]) const {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) split2(x[2 * e], x[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+  }
+};
+__device__ __forceinline__ void put_lanes(uint32_t tmem, int warp, const uint32_t (&w)[3][16]) {
+  const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + TERMS + (warp >> 2) * 16;
+#pragma unroll
+  for (int t = 0; t < 3; ++t) pre::tmem_st16_nowait(at + t * 32, w[t]);
+  pre::tmem_wait_st();
+}
+// The other operand, 64 x 64: two groups of eight columns a thread.
+struct TileOperand {
+  float4 x[2][2];
+  // rows from src, `stride` floats apart, n of them; the rest are zeros
+  __device__ __forceinline__ void load(const float* src, size_t stride, int n, int tid) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int row = tid / 8 + u * 32, col = tid % 8 * 8;
+      x[u][0] = x[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (row < n) {
+        const float* at = src + row * stride + col;
+        x[u][0] = ld4(at);
+        x[u][1] = ld4(at + 4);
+      }
+    }
+  }
+  // fix(row, first column, the eight values)
+  template <typename Fix> __device__ __forceinline__ void put(uint8_t* tile, int tid, Fix fix) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int row = tid / 8 + u * 32, col = tid % 8 * 8;
+      float y[8] = {x[u][0].x, x[u][0].y, x[u][0].z, x[u][0].w, x[u][1].x, x[u][1].y, x[u][1].z, x[u][1].w};
+      fix(row, col, y);
+      uint32_t w[3][4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) split2(y[2 * e], y[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+      uint8_t* to = tile + row * 128 + (((col >> 3) ^ (row & 7)) << 4);
+#pragma unroll
+      for (int t = 0; t < 3; ++t) *reinterpret_cast<uint4*>(to + t * TILE) = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
+    }
+  }
+};
+// acc += A B over 64 k, one thread.  `fresh`: the accumulators hold nothing yet.
+template <bool B_MN>
+__device__ __forceinline__ void products(uint32_t tmem, uint32_t tile, bool fresh) {
+  constexpr uint32_t idesc = pre::instr_desc(128, 64, B_MN);
+  const uint64_t b = pre::smem_desc(tile, B_MN ? TILE : 16, 1024);
+  auto mma = [&](uint32_t d, uint32_t a, uint64_t bb, bool first) {
+    if (first) pre::umma_bf16_a_tmem_c<false>(d, a, bb, idesc);
+    else pre::umma_bf16_a_tmem_c<true>(d, a, bb, idesc);
+  };
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t h = tmem + TERMS + k * 8, m = h + 32, l = h + 64, s = tmem + SMALL;
+    const uint64_t bh = b + (uint64_t)(k * (B_MN ? 2048 >> 4 : 32 >> 4)), bm = bh + (TILE >> 4), bl = bm + (TILE >> 4);
+    mma(tmem, h, bh, fresh && k == 0);
+    mma(s, l, bh, fresh && k == 0);
+    mma(s, h, bl, false);
+    mma(s, m, bm, false);
+    mma(s, m, bh, false);
+    mma(s, h, bm, false);
+  }
+}
+// COLUMNS (16 or 32) of both accumulators, added.
+template <int COLUMNS>
+__device__ __forceinline__ void tmem_sum(uint32_t at, float (&v)[COLUMNS]) {
+  uint32_t a[COLUMNS], b[COLUMNS];
+  if constexpr (COLUMNS == 32) {
+    pre::tmem_ld32_issue(at, a);
+    pre::tmem_ld32_issue(at + SMALL, b);
+  } else {
+    pre::tmem_ld16_issue(at, a);
+    pre::tmem_ld16_issue(at + SMALL, b);
+  }
+  pre::tmem_wait_ld();
+#pragma unroll
+  for (int i = 0; i < COLUMNS; ++i) {
+    asm volatile("" : "+r"(a[i]), "+r"(b[i]));                 // (not before the wait)
+    v[i] = __uint_as_float(a[i]) + __uint_as_float(b[i]);
+  }
+}
+// What a block of the two kernels begins and ends with; two share an SM.
+struct Tensor { uint64_t bar; uint32_t base; int gave_up; };
+__device__ __forceinline__ void tensor_begin(Tensor& t, int tid) {
+  if (tid == 0) {
+    pre::mbar_init(&t.bar, 1);
+    t.gave_up = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (tid < 32) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&t.base)), "r"(TC_COLUMNS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  pre::fence_before_sync();
+  __syncthreads();
+  pre::fence_after_sync();
+}
+__device__ __forceinline__ void tensor_end(Tensor& t, int tid, bool ok, int* error_flag) {
+  if (!ok) {
+    if (tid == 0 && error_flag) atomicExch(error_flag, 1);
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);          // products in flight may still read shared memory
+  }
+  pre::fence_before_sync();
+  __syncthreads();
+  if (tid < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(t.base), "r"(TC_COLUMNS));
+}
+// All operands of a slice are in place: the products of a slice begin.
+template <bool B_MN>
+__device__ __forceinline__ bool tensor_issue(Tensor& t, int tid, uint8_t* tile, bool ok, bool fresh) {
+  pre::fence_async_proxy();
+  pre::fence_before_sync();
+  ok = __syncthreads_and(ok) != 0;
+  if (ok && tid < 32) {
+    pre::fence_after_sync();
+    if (pre::elect_one()) {
+      products<B_MN>(t.base, smem_u32(tile), fresh);
+      pre::umma_commit(&t.bar);
+    }
+    __syncwarp();
+  }
+  return ok;
 }
 
 // ---- U = k~^T v ------------------------------------------------------------------------------------------------------------
+// The state's rows are the product's lanes, so that what depends on the keys alone is split once for all columns that see
+// them: a block takes up to eight tiles of 64 columns, of one head or (one decay per head) of a group's heads.
+constexpr int MOST_TILES = 8;
+// The tiles of a block: of one unit (the heads whose keys are the same), `per_block` of them.
+template <int DT, bool STEP>
+struct Tiles {
+  int unit, heads, per_head, first, count;
+  __device__ __forceinline__ Tiles(const Params& p, int per_block)
+      : unit(blockIdx.y), heads(STEP ? p.hpg : 1), per_head(p.Dv / DT), first(blockIdx.z * per_block) {
+    count = min(per_block, heads * per_head - first);
+  }
+  __device__ __forceinline__ int head(int i) const { return unit * heads + (first + i) / per_head; }
+  __device__ __forceinline__ int column(int i) const { return (first + i) % per_head * DT; }
+};
+// Two buffers of the values' terms, and rows of U on their way out (a lane has a row of the state, a row of U goes out whole).
+template <int N> constexpr size_t STATE_BYTES = 6 * TILE + N * 64 * sizeof(float);
 template <int N, bool STEP>
-__global__ void __launch_bounds__(128) chunk_state_kernel(Params p) {
-  constexpr int RT = N / 16;                                  // rows of a thread: 8 or 4
-  extern __shared__ __align__(16) float sm[];
-  float *ks = sm, *vs = ks + C * N, *ws = vs + C * 64;
+__global__ void __launch_bounds__(TC_THREADS, 2) chunk_state_kernel(Params p, int per_block) {
+  extern __shared__ __align__(1024) uint8_t tile[];
+  __shared__ Tensor t;
+  __shared__ float ws[STEP ? MOST_TILES : 1][C];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, n = (warp & 3) * 32 + lane, half = warp >> 2;
+  tensor_begin(t, tid);
+  pdl_launch_dependents();                                    // (tensor memory is ours: see common.cuh)
   pdl_wait();
-  const int h = blockIdx.y, c0 = blockIdx.z * 64, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const Place c = place(p, blockIdx.x, h, p.H);
-  if (c.n <= 0) return;
-  const float* k = STEP ? p.k + (size_t)c.tok * p.k_stride + (size_t)(h / p.hpg) * N : p.KT + c.item * (size_t)(N * C);
-  const size_t kstep = STEP ? (size_t)p.k_stride : (size_t)N;
-  const float* v = p.v + (size_t)c.tok * p.v_stride + (size_t)h * p.Dv + c0;
-  for (int e = tid; e < C * N / 4; e += 128) {
-    const int j = e / (N / 4), n = e % (N / 4) * 4;
-    const bool live = j < c.n;
-    copy16(ks + j * N + n, live ? k + j * kstep + n : p.v, live);
-  }
-  for (int e = tid; e < C * 16; e += 128) {
-    const int j = e / 16, x = e % 16 * 4;
-    const bool live = j < c.n;
-    copy16(vs + j * 64 + x, live ? v + (size_t)j * p.v_stride + x : p.v, live);
-  }
-  copy_commit();
-  if (STEP && warp == 0) {
-    // v_j is written with dt_j prod_{t > j} a_t
-    float dt[2], a[2];
-    step_of(p, c, h, lane, dt, a);
-    float suf = a[0] * a[1];                                   // product over the lanes from this one on
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float x = __shfl_down_sync(0xffffffffu, suf, o);
-      if (lane + o < 32) suf *= x;
+  const Tiles<64, STEP> tiles(p, per_block);
+  const int count = tiles.count;
+  const Place c = place(p, blockIdx.x, tiles.unit * tiles.heads, p.H);
+  bool ok = true;
+  if (c.n > 0 && count > 0) {
+    auto item = [&](int h) { return (size_t)blockIdx.x * p.H + h; };
+    LaneOperand k;
+    TileOperand v;
+    if (n < N) {
+      const float* from = STEP ? p.k + (size_t)c.tok * p.k_stride + (size_t)tiles.unit * N : p.KT + c.item * (size_t)(N * C);
+      const size_t step = STEP ? (size_t)p.k_stride : (size_t)N;
+      k.load(from + half * 32 * step + n, step, c.n - half * 32);
     }
-    float after = __shfl_down_sync(0xffffffffu, suf, 1);
-    if (lane == 31) after = 1.f;
-    ws[2 * lane] = dt[0] * (a[1] * after);
-    ws[2 * lane + 1] = dt[1] * after;
-    if (lane == 0 && blockIdx.z == 0) p.DC[c.item] = suf;
-  }
-  copy_wait<0>();
-  __syncthreads();
-  const int r0 = warp * (4 * RT) + (lane >> 3) * RT, x0 = (lane & 7) * 4;
-  float2 acc[RT][4];
-#pragma unroll
-  for (int r = 0; r < RT; ++r)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) acc[r][x] = two(0.f);
-#pragma unroll 4
-  for (int j = 0; j < C; ++j) {
-    float a[RT];
-    float2 b[4];
-#pragma unroll
-    for (int r = 0; r < RT; r += 4) *reinterpret_cast<float4*>(a + r) = ld4(ks + j * N + r0 + r);
-    load_cols(vs + j * 64 + x0, b);
-    if (STEP) {
-      const float2 w = two(ws[j]);
-#pragma unroll
-      for (int x = 0; x < 4; ++x) b[x] = __fmul2_rn(b[x], w);
+    auto load = [&](int i) { v.load(p.v + (size_t)c.tok * p.v_stride + (size_t)tiles.head(i) * p.Dv + tiles.column(i), p.v_stride, c.n, tid); };
+    load(0);
+    if (STEP) {                                                // v_j is written with dt_j prod_{t > j} a_t
+      for (int e = tid; e < count * C; e += TC_THREADS) ws[e / C][e % C] = reinterpret_cast<const Decays*>(p.MT)[item(tiles.head(e / C))].w[e % C];
+      __syncthreads();
     }
+    auto put = [&](int i) {
+      v.put(tile + (i & 1) * 3 * TILE, tid, [&](int row, int, float* y) {
+        if (STEP) {
+          const float f = ws[STEP ? i : 0][row];
 #pragma unroll
-    for (int r = 0; r < RT; ++r) {
-      const float2 ar = two(a[r]);
-#pragma unroll
-      for (int x = 0; x < 4; ++x) acc[r][x] = __ffma2_rn(ar, b[x], acc[r][x]);
+          for (int e = 0; e < 8; ++e) y[e] *= f;
+        }
+      });
+    };
+    if (n < N) {
+      uint32_t w[3][16];
+      k.split(w);
+      put_lanes(t.base, warp, w);
     }
-  }
-  float* U = p.U + (c.item * N + r0) * (size_t)p.Dv + c0 + x0;
+    put(0);
+    if (count > 1) load(1);
+    ok = tensor_issue<true>(t, tid, tile, ok, true);
+    for (int i = 0; i < count && ok; ++i) {
+      if (i + 1 < count) put(i + 1);
+      if (i + 2 < count) load(i + 2);
+      ok = pre::mbar_wait(&t.bar, i & 1, &t.gave_up);
+      pre::fence_after_sync();
+      if (__all_sync(0xffffffffu, ok) && n < N) {
+        float y[32];
+        tmem_sum<32>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + half * 32, y);
+        // 16 bytes at a time, rows of 256 turned by their number; each warp reads what it wrote
+        uint8_t* rows = tile + 6 * TILE;
 #pragma unroll
-  for (int r = 0; r < RT; ++r) store_cols(U + (size_t)r * p.Dv, acc[r]);
+        for (int e = 0; e < 8; ++e)
+          st4(reinterpret_cast<float*>(rows + n * 256 + (((half * 8 + e) ^ (n & 15)) << 4)), y[4 * e], y[4 * e + 1], y[4 * e + 2], y[4 * e + 3]);
+        __syncwarp();
+        float* U = p.U + item(tiles.head(i)) * N * (size_t)p.Dv + tiles.column(i);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int r = (warp & 3) * 32 + e * 4 + lane / 8, x = half * 8 + lane % 8;
+          *reinterpret_cast<float4*>(U + (size_t)r * p.Dv + x * 4) = ld4(reinterpret_cast<const float*>(rows + r * 256 + ((x ^ (r & 15)) << 4)));
+        }
+        __syncwarp();
+      }
+      if (i + 1 < count) ok = tensor_issue<true>(t, tid, tile + ((i + 1) & 1) * 3 * TILE, ok, true);
+    }
+    ok = __syncthreads_and(ok) != 0;
+  }
+  tensor_end(t, tid, ok, p.error_flag);
 }
 
 // ---- the states between the chunks: U of a chunk becomes the state it starts from -----------------------------------------
@@ -597,143 +798,175 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(Params p) {
 }
 
 // ---- the outputs -----------------------------------------------------------------------------------------------------------
-// The contraction runs over the state's rows and then over the chunk's tokens, in slices of 16 that come through three
-// buffers.  A block is two warps of 8 x 8 outputs a thread (4 x 8 was bound by its shared-memory loads, 75 % of their
-// pipe), and eight blocks share an SM: a scheduler needs three or four warps to issue packed instructions back to back.
-constexpr int SLICE = 16, STAGES = 3;
-template <bool STEP>
-struct OutShape {
-  static constexpr int LDA = STEP ? C + 4 : C;
-  static constexpr size_t bytes = (STAGES * SLICE * (LDA + 64) + 3 * C) * sizeof(float);
-};
-template <int N, bool STEP, bool DELTA>
-__global__ void __launch_bounds__(64) chunk_out_kernel(Params p) {
-  constexpr int LDA = OutShape<STEP>::LDA, BUF = SLICE * (LDA + 64), NS = N / SLICE, SLICES = NS + C / SLICE;
-  extern __shared__ __align__(16) float sm[];
-  float *dts = sm + STAGES * BUF, *as = dts + C, *pre = as + C;
+// The contraction runs over the state's rows and then over the chunk's tokens, 64 at a time; a slice's loads are on the way
+// while the slice before is split and multiplied.  Columns are the product's lanes, tokens its columns.
+__device__ __forceinline__ bool finite_f(float x) { return fabsf(x) <= 3.402823466e38f; }
+
+// DT columns a tile: 128, or 64 (the upper lanes then do the same as the lower ones, and are not read).  A block takes up to
+// eight tiles; the queries and scores of one head are split for the first one only.
+template <int N> constexpr size_t OUT_BYTES = (N / 64 + 1) * 3 * TILE;
+template <int N, int DT, bool STEP, bool DELTA>
+__global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int per_block) {
+  constexpr int SLICES = N / 64 + 1;
+  extern __shared__ __align__(1024) uint8_t tile[];
+  __shared__ Tensor t;
+  __shared__ Decays decays[STEP ? 2 : 1];                      // this tile's, the next one's
+  __shared__ int bad[2][DT];                                   // per column the first token whose value is no finite number
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Dv = p.Dv;
+  const int x = ((warp & 3) * 32 + lane) % DT, half = warp >> 2;      // column of the tile
+  if (tid < DT) bad[0][tid] = bad[1][tid] = C;
+  tensor_begin(t, tid);
+  pdl_launch_dependents();                                    // (tensor memory is ours: see common.cuh)
   pdl_wait();
-  const int h = blockIdx.y, c0 = blockIdx.z * 64, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Dv = p.Dv;
-  const Place c = place(p, blockIdx.x, h, p.H);
-  if (c.n <= 0) return;
-  const size_t gi = STEP ? (size_t)blockIdx.x * (p.H / p.hpg) + h / p.hpg : c.item;
-  const float *QT = p.QT + gi * (size_t)(N * C), *AT = p.AT + gi * (size_t)(C * C);
-  const float* U = p.U + c.item * (size_t)N * Dv + c0;
-  const float* v = DELTA ? p.UH + c.item * (size_t)(C * Dv) + c0 : p.v + (size_t)c.tok * p.v_stride + (size_t)h * Dv + c0;
-  const size_t vstep = DELTA ? (size_t)Dv : (size_t)p.v_stride;
-  auto load = [&](int sl) {
-    float *a = sm + sl % STAGES * BUF, *b = a + SLICE * LDA;
-    if (sl < NS) {
-#pragma unroll
-      for (int e = tid; e < SLICE * 16; e += 64) {
-        const int n = e / 16, x = e % 16 * 4;
-        copy16(a + n * LDA + x, QT + (size_t)(sl * SLICE + n) * C + x, true);
-        copy16(b + n * 64 + x, U + (size_t)(sl * SLICE + n) * Dv + x, true);
-      }
-    } else if (sl < SLICES) {
-#pragma unroll
-      for (int e = tid; e < SLICE * 16; e += 64) {
-        const int j = e / 16, x = e % 16 * 4, t = (sl - NS) * SLICE + j;
-        const bool live = t < c.n;
-        copy16(a + j * LDA + x, AT + (size_t)t * C + x, true);
-        copy16(b + j * 64 + x, live ? v + t * vstep + x : p.v, live);
-      }
-    }
-    copy_commit();
-  };
-  load(0);
-  load(1);
-  if (STEP && warp == 0) {
-    float dt[2], a[2];
-    step_of(p, c, h, lane, dt, a);
-    float upto = a[0] * a[1];                                  // product over the lanes up to this one
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float x = __shfl_up_sync(0xffffffffu, upto, o);
-      if (lane >= o) upto *= x;
-    }
-    float before = __shfl_up_sync(0xffffffffu, upto, 1);
-    if (lane == 0) before = 1.f;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) { dts[2 * lane + e] = dt[e]; as[2 * lane + e] = a[e]; }
-    pre[2 * lane] = before * a[0];
-    pre[2 * lane + 1] = upto;
-  }
-  const int i0 = 32 * warp + 8 * (lane >> 3), x0 = 4 * (lane & 7);
-  float2 acc[8][4];
-#pragma unroll
-  for (int r = 0; r < 8; ++r)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) acc[r][x] = two(0.f);
-  for (int sl = 0; sl < SLICES; ++sl) {
-    copy_wait<1>();
-    __syncthreads();                                           // the slice is here; everybody is done with the one before
-    load(sl + 2);
-    float *a = sm + sl % STAGES * BUF, *b = a + SLICE * LDA;
-    const int t0 = (sl - NS) * SLICE;                          // the slice's first token, once the state's rows are done
-    if (STEP && sl >= NS) {
-      if (sl == NS) {
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          const float2 w = two(pre[i0 + r]);
-#pragma unroll
-          for (int x = 0; x < 4; ++x) acc[r][x] = __fmul2_rn(acc[r][x], w);
-        }
-      }
-      // (C_i . B_j) dt_j prod_{j < t <= i} a_t: a thread takes one j and a quarter of the tokens i, four at a time
-      const int j = t0 + tid % SLICE, from = tid / SLICE * 16;
-      float L = dts[j];
-      for (int t = j + 1; t < from; ++t) L *= as[t];
-#pragma unroll
-      for (int i = from; i < from + 16; i += 4) {
-        float* at = a + tid % SLICE * LDA + i;
-        const float4 f = ld4(at);
-        float y[4] = {f.x, f.y, f.z, f.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (i + e > j) L *= as[i + e];
-          y[e] *= L;
-        }
-        st4(at, y[0], y[1], y[2], y[3]);
-      }
+  const Tiles<DT, STEP> tiles(p, per_block);
+  const int count = tiles.count;
+  const Place c = place(p, blockIdx.x, tiles.unit * tiles.heads, p.H);
+  bool ok = true;
+  if (c.n > 0 && count > 0) {
+    auto item = [&](int h) { return (size_t)blockIdx.x * p.H + h; };
+    const float* AT = p.AT + (STEP ? (size_t)blockIdx.x * (p.H / p.hpg) + tiles.unit : c.item) * (size_t)(C * C);
+    const size_t vstep = DELTA ? (size_t)Dv : (size_t)p.v_stride;
+    auto values = [&](int i) {
+      return (DELTA ? p.UH + c.item * (size_t)(C * Dv) : p.v + (size_t)c.tok * p.v_stride + (size_t)tiles.head(i) * Dv) + tiles.column(i);
+    };
+    LaneOperand a;
+    TileOperand b;
+    auto load_a = [&](int i, int sl) {
+      if (sl < SLICES - 1) a.load(p.U + (item(tiles.head(i)) * N + sl * 64 + half * 32) * (size_t)Dv + tiles.column(i) + x, Dv, 32);
+      else a.load(values(i) + half * 32 * vstep + x, vstep, c.n - half * 32);
+    };
+    auto load_b = [&](int i, int sl) {
+      if (!STEP && i > 0) return;
+      if (sl == SLICES - 1) b.load(AT, C, c.n, tid);
+      else if (STEP) b.load(p.q + (size_t)c.tok * p.q_stride + (size_t)tiles.unit * N + sl * 64, p.q_stride, c.n, tid);
+      else b.load(p.QT + c.item * (size_t)(N * C) + sl * 64, N, c.n, tid);
+    };
+    auto ask_decays = [&](int i) {
+      if (STEP && tid < DECAYS / 4)
+        copy16(reinterpret_cast<float*>(&decays[STEP ? i & 1 : 0]) + tid * 4, p.MT + item(tiles.head(i)) * DECAYS + tid * 4, true);
+      copy_commit();
+    };
+    if (STEP) ask_decays(0);
+    load_a(0, 0);
+    load_b(0, 0);
+    if (STEP) {
+      copy_wait<0>();
       __syncthreads();
     }
-    // a warp's own 32 tokens under their diagonal (nothing of a later token is read), later ones not at all
-    if (sl >= NS && t0 >= 32 * warp + 32) continue;
-    const bool whole = sl < NS || t0 < 32 * warp;
-    auto product = [&](auto masked) {
-#pragma unroll 4
-      for (int k = 0; k < SLICE; ++k) {
-        float av[8];
-        float2 bv[4];
-        *reinterpret_cast<float4*>(av) = ld4(a + k * LDA + i0);
-        *reinterpret_cast<float4*>(av + 4) = ld4(a + k * LDA + i0 + 4);
-        load_cols(b + k * 64 + x0, bv);
+    int round = 0;                                             // products begun
+    for (int i = 0; i < count && ok; ++i) {
+      const Decays& D = decays[STEP ? i & 1 : 0];
+      // (the skip adds v itself, also with the delta rule, whose products take the corrected u)
+      const float skip = p.skip ? load_any(p.skip, p.small_dtype, tiles.head(i)) : 0.f;
 #pragma unroll
-        for (int r = 0; r < 8; ++r)
-          if (!masked || t0 + k <= i0 + r) {
+      for (int sl = 0; sl < SLICES; ++sl) {
+        const bool last = sl == SLICES - 1;
+        uint32_t w[3][16];
+        // A value that is no finite number is left out (its products with the zeros of earlier tokens would not be zeros)
+        // and added to the outputs that see it when they are written.
+        if (last) {
+          float zero = 0.f;                                    // no number, or no zero, if one of them is none
 #pragma unroll
-            for (int x = 0; x < 4; ++x) acc[r][x] = __ffma2_rn(two(av[r]), bv[x], acc[r][x]);
-          }
+          for (int e = 0; e < 32; ++e) zero = fmaf(a.x[e], 0.f, zero);
+          if (zero != 0.f)
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (!finite_f(a.x[e])) { atomicMin(&bad[i & 1][x], half * 32 + e); a.x[e] = 0.f; }
+        }
+        a.split(w);
+        if (sl > 0) {
+          ok = ok && pre::mbar_wait(&t.bar, (round - 1) & 1, &t.gave_up);
+          pre::fence_after_sync();
+        }
+        put_lanes(t.base, warp, w);
+        if (!last) load_a(i, sl + 1);
+        else if (i + 1 < count) load_a(i + 1, 0);
+        if (STEP || i == 0)
+          b.put(tile + sl * 3 * TILE, tid, [&](int r, int j0, float* y) {
+            if (!last) {
+              if (STEP) {
+                const float f = D.upto[r] * p.q_scale;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) y[e] *= f;
+              }
+              return;
+            }
+            if (STEP && r >= j0) {
+              // (C_i . B_j) dt_j prod_{j < t <= i} a_t, from the row's end of this run of eight backwards
+              const int from = j0 / 8, to = r / 8;
+              float L = to > from ? D.run[r] * D.mid[from][to] : 1.f, dt[8], d[8];
+#pragma unroll
+              for (int e = 0; e < 8; e += 4) {
+                *reinterpret_cast<float4*>(dt + e) = ld4(D.dt + j0 + e);
+                *reinterpret_cast<float4*>(d + e) = ld4(D.a + j0 + e);
+              }
+#pragma unroll
+              for (int e = 7; e >= 0; --e) {
+                y[e] *= dt[e] * L;
+                L = j0 + e > r ? 1.f : L * d[e];
+              }
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] = j0 + e > r ? 0.f : y[e];
+          });
+        if (!last) load_b(i, sl + 1);
+        else if (i + 1 < count) load_b(i + 1, 0);
+        if (STEP && last) copy_wait<0>();
+        ok = tensor_issue<false>(t, tid, tile + sl * 3 * TILE, ok, sl == 0);
+        ++round;
+        if (!ok) break;
+        if (STEP && sl == 0 && i + 1 < count) ask_decays(i + 1);      // (everybody is done with the tile before)
       }
-    };
-    if (whole) product(std::false_type{});
-    else product(std::true_type{});
-  }
-  // (the skip adds v itself, also with the delta rule, whose products above take the corrected u)
-  const float skip = p.skip ? load_any(p.skip, p.small_dtype, h) : 0.f;
-  const float* raw = p.v + (size_t)c.tok * p.v_stride + (size_t)h * Dv + c0;
+      // (with 64 columns two warps hold the same sums: each writes half of the tokens)
+      constexpr int ROWS = DT / 4;
+      const int i0 = half * 32 + (DT == 64 ? (warp >> 1 & 1) * 16 : 0);
+      float raw[ROWS];
+      if (p.skip) {
+        const float* from = p.v + (size_t)(c.tok + i0) * p.v_stride + (size_t)tiles.head(i) * Dv + tiles.column(i) + x;
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int i = i0 + r;
-    if (i >= c.n) continue;
-    if (p.skip) {
-      float2 b[4];
-      load_cols(raw + i * p.v_stride + x0, b);
+        for (int e = 0; e < ROWS; ++e) {
+          raw[e] = i0 + e < c.n ? *from : 0.f;
+          from += p.v_stride;
+          asm volatile("" : "+l"(from));
+        }
+      }
+      ok = ok && pre::mbar_wait(&t.bar, (round - 1) & 1, &t.gave_up);
+      pre::fence_after_sync();
+      if (__all_sync(0xffffffffu, ok) && i0 < c.n) {
+        const int first = bad[i & 1][x];
+        float y[ROWS];
+        tmem_sum<ROWS>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + i0, y);
+        float* out = p.out + (size_t)(c.tok + i0) * p.out_stride + (size_t)tiles.head(i) * Dv + tiles.column(i) + x;
+        float* to = out;
 #pragma unroll
-      for (int x = 0; x < 4; ++x) acc[r][x] = __ffma2_rn(two(skip), b[x], acc[r][x]);
+        for (int e = 0; e < ROWS; ++e) {
+          if (i0 + e < c.n) *to = p.skip ? fmaf(skip, raw[e], y[e]) : y[e];
+          to += p.out_stride;
+          asm volatile("" : "+l"(to));                         // (32 addresses at a time would not fit in registers)
+        }
+#pragma unroll 1
+        for (int r = max(first, i0); r < min(i0 + ROWS, c.n); ++r) {     // (runs for values that are no finite numbers)
+          float o = out[(r - i0) * p.out_stride];
+          for (int j = first; j <= r; ++j) {
+            const float val = values(i)[j * vstep + x];
+            if (finite_f(val)) continue;
+            float f = AT[r * C + j];
+            if (STEP) {
+              f *= D.dt[j];
+              for (int s = j + 1; s <= r; ++s) f *= D.a[s];
+            }
+            o = fmaf(f, val, o);
+          }
+          out[(r - i0) * p.out_stride] = o;
+        }
+      }
+      __syncthreads();                                         // everybody has read what the next tiles' values may change
+      if (half == 0) bad[i & 1][x] = C;
     }
-    store_cols(p.out + (size_t)(c.tok + i) * p.out_stride + (size_t)h * Dv + c0 + x0, acc[r]);
+    copy_wait<0>();
+    ok = __syncthreads_and(ok) != 0;
   }
+  tensor_end(t, tid, ok, p.error_flag);
 }
 
 // ---- launches --------------------------------------------------------------------------------------------------------------
@@ -756,26 +989,52 @@ static int allow(K kernel, size_t bytes, bool& done) {
     if (int rc = check_launch("linear_chunks")) return rc;                \
   } while (0)
 
+// A block's tiles: as many as leave two blocks an SM, up to eight.
+static int tiles_of_block(const Params& p, int units, int tiles) {
+  int n = 1;
+  while (n < MOST_TILES && n < tiles && (long)p.seg_chunks * units * ((tiles + n - 1) / n) > 2 * sm_count()) n *= 2;
+  return n;
+}
+#define CPI_TILES_LAUNCH(kernel, units, tiles, bytes)                                                       \
+  do {                                                                                                      \
+    static bool done = false;                                                                               \
+    if (allow(kernel, bytes, done)) return 1;                                                               \
+    const int n = tiles_of_block(p, units, tiles);                                                          \
+    cpi::launch_pdl(kernel, dim3(p.seg_chunks, units, ((tiles) + n - 1) / n), dim3(TC_THREADS), bytes, stream, p, n); \
+    return check_launch("linear_chunks");                                                                   \
+  } while (0)
+template <int N, bool STEP>
+static int state_products(const Params& p, cudaStream_t stream) {
+  const int units = STEP ? p.H / p.hpg : p.H;
+  CPI_TILES_LAUNCH((chunk_state_kernel<N, STEP>), units, p.H / units * (p.Dv / 64), STATE_BYTES<N>);
+}
+// column tiles of 128 where they come out even, else of 64
+template <int N, bool STEP, bool DELTA>
+static int output_products(const Params& p, cudaStream_t stream) {
+  const int units = STEP ? p.H / p.hpg : p.H;
+  if (p.Dv % 128 == 0) CPI_TILES_LAUNCH((chunk_out_kernel<N, 128, STEP, DELTA>), units, p.H / units * (p.Dv / 128), OUT_BYTES<N>);
+  else CPI_TILES_LAUNCH((chunk_out_kernel<N, 64, STEP, DELTA>), units, p.H / units * (p.Dv / 64), OUT_BYTES<N>);
+}
+
 template <int N>
 static int run(const Params& p, cudaStream_t stream) {
-  const dim3 items(p.seg_chunks, p.H), tiles(p.seg_chunks, p.H, p.Dv / 64);
+  const dim3 items(p.seg_chunks, p.H);
   const dim3 chain(p.n_seqs, p.H, (N * p.Dv / 4 + 255) / 256);
-  constexpr size_t state_bytes = (C * N + C * 64 + C) * sizeof(float);
   if (p.dt) {
     CPI_CHUNK_LAUNCH(prepare_step_kernel<N>, dim3(p.seg_chunks, p.H / p.hpg), 256, 2 * C * (N + 4) * sizeof(float));
-    CPI_CHUNK_LAUNCH((chunk_state_kernel<N, true>), tiles, 128, state_bytes);
+    if (int rc = state_products<N, true>(p, stream)) return rc;
     CPI_CHUNK_LAUNCH(chain_kernel<true>, chain, 256, (size_t)0);
-    CPI_CHUNK_LAUNCH((chunk_out_kernel<N, true, false>), tiles, 64, OutShape<true>::bytes);
+    if (int rc = output_products<N, true, false>(p, stream)) return rc;
   } else if (p.beta) {
     CPI_CHUNK_LAUNCH((prepare_rows_kernel<N / 8, true>), items, 512, (PrepShape<N / 8, true>::bytes));
     CPI_CHUNK_LAUNCH(solve_kernel, dim3(p.seg_chunks, p.H, (N + p.Dv + 127) / 128), 128, C * 128 * sizeof(float));
     CPI_CHUNK_LAUNCH(delta_chain_kernel<N>, dim3(p.n_seqs, p.H, p.Dv / 16), 256, ChainShape<N>::bytes);
-    CPI_CHUNK_LAUNCH((chunk_out_kernel<N, false, true>), tiles, 64, OutShape<false>::bytes);
+    if (int rc = output_products<N, false, true>(p, stream)) return rc;
   } else {
     CPI_CHUNK_LAUNCH((prepare_rows_kernel<N / 8, false>), items, 512, (PrepShape<N / 8, false>::bytes));
-    CPI_CHUNK_LAUNCH((chunk_state_kernel<N, false>), tiles, 128, state_bytes);
+    if (int rc = state_products<N, false>(p, stream)) return rc;
     CPI_CHUNK_LAUNCH(chain_kernel<false>, chain, 256, (size_t)0);
-    CPI_CHUNK_LAUNCH((chunk_out_kernel<N, false, false>), tiles, 64, OutShape<false>::bytes);
+    if (int rc = output_products<N, false, false>(p, stream)) return rc;
   }
   return 0;
 }
@@ -785,10 +1044,10 @@ static void sizes(int kind, int H, int groups, int N, int Dv, long (&n)[9]) {
   const long rows = (long)H * N * C, tri = (long)H * C * C;
   n[0] = (long)H * N * Dv;
   n[1] = kind == 0 ? 0 : rows;
-  n[2] = kind == 0 ? (long)groups * N * C : rows;
+  n[2] = kind == 0 ? 0 : rows;
   n[3] = kind == 0 ? (long)groups * C * C : tri;
   n[4] = kind == 0 ? (H + 3) / 4 * 4 : (long)H * N;
-  n[5] = kind == 2 ? tri : 0;
+  n[5] = kind == 2 ? tri : kind == 0 ? (long)H * DECAYS : 0;     // (the step flavour's decays)
   n[6] = n[7] = kind == 2 ? rows : 0;
   n[8] = kind == 2 ? (long)H * C * Dv : 0;
 }
@@ -818,7 +1077,7 @@ extern "C" int cpi_linear_chunks(const float* k, long k_stride, const float* q, 
                                  float q_scale, float* state, float* out, long out_stride, const int* seq_slot,
                                  const int* seq_tok0, const int* seq_new, int n_seqs, int total_chunks, int n_heads,
                                  int heads_per_group, int n_rows, int n_cols, float* scratch, int seg_chunks,
-                                 cudaStream_t stream) {
+                                 int* error_flag, cudaStream_t stream) {
   if (n_seqs == 0 || total_chunks <= 0) return 0;
   CPI_REQUIRE(cpi_linear_chunks_supported(n_rows, n_cols), "linear_chunks: a state of %d x %d is not supported", n_rows, n_cols);
   CPI_REQUIRE((z != nullptr) + (dt != nullptr) == 1 && (dt == nullptr || (a_log != nullptr && beta == nullptr)),
@@ -836,6 +1095,7 @@ extern "C" int cpi_linear_chunks(const float* k, long k_stride, const float* q, 
   p.small_dtype = small_dtype; p.beta = beta; p.beta_stride = beta_stride; p.q_scale = q_scale; p.state = state; p.out = out;
   p.out_stride = out_stride; p.seq_slot = seq_slot; p.seq_tok0 = seq_tok0; p.seq_new = seq_new;
   p.H = n_heads; p.hpg = heads_per_group; p.N = n_rows; p.Dv = n_cols; p.n_seqs = n_seqs;
+  p.error_flag = error_flag;
   const int kind = dt ? 0 : beta ? 2 : 1;
   long n[9];
   chunks::sizes(kind, n_heads, n_heads / heads_per_group, n_rows, n_cols, n);

@@ -139,3 +139,53 @@ def test_the_skip_adds_the_values_themselves(kind):
     # float32 sums of up to 64 + 64 terms and of the states' rows in two orders
     for x, y in ((outs[0], outs[2]), (outs[1], outs[3])):
         assert float((x - y).norm() / x.norm()) <= 2.0 ** -18
+
+
+# more tiles of columns than a block takes, counts that do not come out even, groups of an odd number of heads
+@pytest.mark.parametrize("kind,H,hpg,rows,cols", [("step", 10, 5, 128, 64), ("step", 24, 12, 64, 128), ("rows", 10, 1, 64, 192),
+                                                  ("rows", 3, 1, 128, 1024), ("delta", 6, 3, 128, 256), ("step", 9, 9, 128, 192)])
+def test_blocks_of_several_tiles(kind, H, hpg, rows, cols):
+    from cpi_b200.csrc import lib as K
+    g = torch.Generator(device=DEV).manual_seed(7)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    new, G = [1000, 37, 1300], H // hpg
+    T = sum(new)
+    k, q, v = torch.nn.functional.normalize(randn(T, G, rows), dim=-1).view(T, -1), randn(T, G * rows), randn(T, H * cols)
+    kw = dict(n_heads=H, heads_per_group=hpg, n_rows=rows, n_cols=cols, q_scale=0.1)
+    if kind == "step":
+        kw.update(dt=randn(T, H), dt_bias=randn(H) - 3, a_log=randn(H), skip=randn(H))
+    else:
+        kw.update(z=randn(T, H * rows), z_bias=randn(H * rows), tau=16.0)
+        if kind == "delta":
+            kw.update(beta=randn(T, H), decay_kind=1, a_log=randn(H) - 3)
+    per = K.linear_chunks_scratch(H, hpg, rows, cols, z=kw.get("z"), beta=kw.get("beta"))
+    outs, state = [], randn(4, H, rows, cols)
+    for fn, extra in ((K.linear_scan, {}), (K.linear_chunks, dict(scratch=torch.full((40 * per,), float("nan"), device=DEV)))):
+        S, out = state.clone(), torch.zeros(T, H * cols, device=DEV)
+        fn(k, q, v, S, out, _batch(new, [2, 0, 3]), **kw, **extra)
+        outs.append((out, S))
+    assert torch.equal(outs[1][1][1], state[1])
+    for a, b in zip(*outs):
+        # two float32 recurrences of 1,300 tokens, each some 2^-24 a token off (their errors against 64 bits are below 2e-6)
+        assert float((a - b).norm() / a.norm()) < 1e-5 and bool(b.isfinite().all())
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_values_that_are_no_numbers_reach_the_outputs_that_see_them(value):
+    """One value of one column: the outputs of that column from its token on are no finite numbers, all others keep their bits."""
+    from cpi_b200.csrc import lib as K
+    g = torch.Generator(device=DEV).manual_seed(4)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    T, H, rows, cols, at = 130, 2, 64, 128, 70
+    k, q, v, z = randn(T, H * rows), randn(T, H * rows), randn(T, H * cols), randn(T, H * rows)
+    got = []
+    for x in (0.5, value):
+        v[at, cols + 3] = x
+        per = K.linear_chunks_scratch(H, 1, rows, cols, z=z)
+        out = torch.zeros(T, H * cols, device=DEV)
+        K.linear_chunks(k, q, v, torch.zeros(1, H, rows, cols, device=DEV), out, _batch([T], [0]), scratch=torch.empty(3 * per, device=DEV),
+                        n_heads=H, heads_per_group=1, n_rows=rows, n_cols=cols, z=z, tau=4.0)
+        got.append(out)
+    same = torch.ones(T, H * cols, dtype=torch.bool, device=DEV)
+    same[at:, cols + 3] = False
+    assert torch.equal(got[0][same], got[1][same]) and not bool(got[1][~same].isfinite().any())

@@ -58,3 +58,14 @@ def test_kernels_on_cta_pairs_are_not_started_early():
     text = open(os.path.join(CSRC, "gemm_tc_pair.cu")).read()
     assert text.count("cudaLaunchKernelEx(") == 2 and "cudaLaunchAttributeProgrammaticStreamSerialization" not in text
     assert "launch_pdl(" not in text
+
+
+def test_kernels_that_allocate_through_a_helper_keep_the_order_too():
+    """`tensor_begin` (recurrent_chunks.cu) allocates and meets; what calls it lets successors start after it."""
+    text = open(os.path.join(CSRC, "recurrent_chunks.cu")).read()
+    helper = text[text.index("void tensor_begin("):]
+    helper = helper[:helper.index("\n}\n")]
+    assert helper.index("tcgen05.alloc") < helper.index("__syncthreads()")
+    users = {k: body for k, body in KERNELS.items() if "tensor_begin(" in body}
+    assert {k.split(":")[1] for k in users} == {"chunk_state_kernel", "chunk_out_kernel"}
+    assert all(body.index("tensor_begin(") < body.index("pdl_launch_dependents()") for body in users.values())
