@@ -142,13 +142,15 @@ __global__ void __launch_bounds__(NT) gemm_simt_kernel(GemmParams p) {
 
 // ---- many rows per group -------------------------------------------------------------------------------------------
 // The same sums in the same order (an output is one chain of fused multiply-adds over k, so its bits do not depend on
-// which of the two kernels made it), from register tiles of RT x 8 with the packed float32 instructions.  A CTA of four
-// warps takes 64 rows and COLS weight rows (in the gated mode half of them are gate rows, half up rows): a thread has RT
-// rows and four columns in either half, so that the eight distinct addresses of a warp's weight loads and the four of
-// its activation loads each take two cycles of the shared-memory pipe (32 distinct ones take eight).  The next 16 k come
-// through registers while 16 are multiplied.
-// Bound: the FP32 pipe with enough warps (one warp per scheduler issues packed instructions at half rate, three at 0.95 of it);
-// 509 x 2,048 -> 3,072 and 2,048 in float32: 984 -> 343 us together (the kernel above with 64 rows a tile before).
+// which of the two kernels made it), from register tiles of RT x 8 with the packed float32 instructions.  A CTA takes 64 rows
+// and COLS weight rows (in the gated mode half of them are gate rows, half up rows): a thread has RT rows and four columns in
+// either half, so that the eight distinct addresses of a warp's weight loads and the four of its activation loads each take
+// two cycles of the shared-memory pipe (32 distinct ones take eight).  DEPTH sixteens of k are on the way through registers
+// while 16 are multiplied, and a step's operands are read from shared memory one step ahead.  The k 8 to 15 of a sixteen lie
+// with their rows' eights exchanged: without it a warp's writes of four k at a time meet two and two in the same banks.
+// Bound: the issue of packed multiply-adds and of the moves that double an activation for them (3.0 cycles a multiply-add where
+// the pipe takes 2), and whole CTAs an SM; 509 x 2,048 -> 3,072 and 2,048 in float32: 335 -> 298 us together (floor 148), 2,048 x
+// 2,048 -> 6,144 1,092 -> 1,007 (716), 17 x 2,048 -> 2,048 108 -> 77.
 // Four neighbouring elements of a row as they lie in memory; they are widened on their way to shared memory, so that nothing
 // waits for a load while the 16 k before are multiplied.  64 rows, 2,048 x 2,048: bfloat16 weights widened at the load 205 us,
 // here 107 (float32 weights 117); with 4 x 4 outputs a thread and 64 rows a tile it was 169 (177).
@@ -189,12 +191,14 @@ __device__ __forceinline__ void load4(const T* p, bool live, bool vec, int k, in
   else v.some(p, k, K);
 }
 
-constexpr int TILE_ROWS = 64, TILE_THREADS = 128;
+constexpr int TILE_ROWS = 64;
+constexpr int tile_threads(int RT, int COLS) { return TILE_ROWS / (4 * RT) * (COLS / 64) * 32; }
 
-template <typename TA, typename TW, typename TO, int MODE, int RT>
-__global__ void __launch_bounds__(TILE_THREADS) gemm_simt_tile_kernel(GemmParams p) {
+template <typename TA, typename TW, typename TO, int MODE, int RT, int COLS, int DEPTH>
+__global__ void __launch_bounds__(tile_threads(RT, COLS)) gemm_simt_tile_kernel(GemmParams p) {
   constexpr bool GLU = MODE == kSwiglu;
-  constexpr int COLS = RT * 16, HALF = COLS / 2, OUT = GLU ? HALF : COLS;      // weight rows, their halves, output columns
+  constexpr int TILE_THREADS = tile_threads(RT, COLS);
+  constexpr int HALF = COLS / 2, OUT = GLU ? HALF : COLS;                      // halves of the weight rows, output columns
   constexpr int LDM = TILE_ROWS + 4, LDC = COLS + 4, LA = TILE_ROWS * BK / 4 / TILE_THREADS, LW = COLS * BK / 4 / TILE_THREADS;
   __shared__ __align__(16) float As[2][BK][LDM], Ws[2][BK][LDC];
   pdl_wait();
@@ -239,21 +243,20 @@ __global__ void __launch_bounds__(TILE_THREADS) gemm_simt_tile_kernel(GemmParams
   }
   const int kq = (tid & 3) * 4;
   const bool va = p.vec_a, vw = p.vec_w;
-  Four<TA> ra[LA];
-  Four<TW> rw[LW];
-  auto fetch = [&](int k0) {
+  struct Set { Four<TA> a[LA]; Four<TW> w[LW]; };
+  auto fetch = [&](int k0, Set& r) {
 #pragma unroll
-    for (int i = 0; i < LA; ++i) load4(a_ptr[i], a_live[i], va, k0 + kq, p.K, ra[i]);
+    for (int i = 0; i < LA; ++i) load4(a_ptr[i], a_live[i], va, k0 + kq, p.K, r.a[i]);
 #pragma unroll
-    for (int i = 0; i < LW; ++i) load4(w_ptr[i], w_live[i], vw, k0 + kq, p.K, rw[i]);
+    for (int i = 0; i < LW; ++i) load4(w_ptr[i], w_live[i], vw, k0 + kq, p.K, r.w[i]);
   };
-  auto stash = [&](int b) {
+  auto stash = [&](int b, const Set& r) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
 #pragma unroll
-      for (int i = 0; i < LA; ++i) As[b][kq + e][(tid + i * TILE_THREADS) / 4] = ra[i].at(e);
+      for (int i = 0; i < LA; ++i) As[b][kq + e][(tid + i * TILE_THREADS) / 4 ^ (kq & 8)] = r.a[i].at(e);
 #pragma unroll
-      for (int i = 0; i < LW; ++i) Ws[b][kq + e][(tid + i * TILE_THREADS) / 4] = rw[i].at(e);
+      for (int i = 0; i < LW; ++i) Ws[b][kq + e][(tid + i * TILE_THREADS) / 4 ^ (kq & 8)] = r.w[i].at(e);
     }
   };
   float2 acc[RT][4];
@@ -261,30 +264,41 @@ __global__ void __launch_bounds__(TILE_THREADS) gemm_simt_tile_kernel(GemmParams
   for (int r = 0; r < RT; ++r)
 #pragma unroll
     for (int x = 0; x < 4; ++x) acc[r][x] = make_float2(0.f, 0.f);
-  fetch(0);
-  stash(0);
+  // DEPTH sixteens of k on the way: slot i % DEPTH of the registers, buffer i % 2 of shared memory
+  constexpr int UNROLL = DEPTH % 2 ? 2 * DEPTH : DEPTH;
+  Set ring[DEPTH];
+#pragma unroll
+  for (int d = 0; d < DEPTH; ++d) fetch(d * BK, ring[d]);
+  stash(0, ring[0]);
   __syncthreads();
-  int b = 0;
-  for (int k0 = 0; k0 < p.K; k0 += BK, b ^= 1) {
-    const bool more = k0 + BK < p.K;
-    if (more) fetch(k0 + BK);
+  auto step = [&](int k0, int b, Set& next, Set& free) {
+    if (k0 + DEPTH * BK < p.K) fetch(k0 + DEPTH * BK, free);
+    // the operands of a step of k, one step ahead of its products
+    float av[2][RT], wv[2][8];
+    auto read = [&](int k, int to) {
+#pragma unroll
+      for (int r = 0; r < RT; r += 4) *reinterpret_cast<float4*>(av[to] + r) = *reinterpret_cast<const float4*>(&As[b][k][(r0 ^ (k & 8)) + r]);
+      *reinterpret_cast<float4*>(wv[to]) = *reinterpret_cast<const float4*>(&Ws[b][k][x0 ^ (k & 8)]);
+      *reinterpret_cast<float4*>(wv[to] + 4) = *reinterpret_cast<const float4*>(&Ws[b][k][HALF + (x0 ^ (k & 8))]);
+    };
+    read(0, 0);
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
-      float av[RT];
-#pragma unroll
-      for (int r = 0; r < RT; r += 4) *reinterpret_cast<float4*>(av + r) = *reinterpret_cast<const float4*>(&As[b][k][r0 + r]);
-      const float4 lo = *reinterpret_cast<const float4*>(&Ws[b][k][x0]), hi = *reinterpret_cast<const float4*>(&Ws[b][k][HALF + x0]);
-      const float2 wv[4] = {make_float2(lo.x, lo.y), make_float2(lo.z, lo.w), make_float2(hi.x, hi.y), make_float2(hi.z, hi.w)};
+      if (k + 1 < BK) read(k + 1, (k + 1) & 1);
 #pragma unroll
       for (int r = 0; r < RT; ++r) {
-        const float2 ar = make_float2(av[r], av[r]);
+        const float2 ar = make_float2(av[k & 1][r], av[k & 1][r]);
 #pragma unroll
-        for (int x = 0; x < 4; ++x) acc[r][x] = __ffma2_rn(ar, wv[x], acc[r][x]);
+        for (int x = 0; x < 4; ++x) acc[r][x] = __ffma2_rn(ar, make_float2(wv[k & 1][2 * x], wv[k & 1][2 * x + 1]), acc[r][x]);
       }
     }
-    if (more) stash(b ^ 1);
+    if (k0 + BK < p.K) stash(b ^ 1, next);
     __syncthreads();
-  }
+  };
+  for (int k0 = 0; k0 < p.K; k0 += UNROLL * BK)
+#pragma unroll
+    for (int i = 0; i < UNROLL; ++i)
+      if (k0 + i * BK < p.K) step(k0 + i * BK, i & 1, ring[(i + 1) % DEPTH], ring[i % DEPTH]);
   // (not earlier: blocks of the next kernel that wait beside the running ones slow them down, 343 us became 699 for the two
   // products of the figure above)
   pdl_launch_dependents();
@@ -330,12 +344,18 @@ int launch_simt(const GemmParams& p, int m_tiles_hint, cudaStream_t stream) {
   }
   const int m_tiles = (p.M + TILE_ROWS - 1) / TILE_ROWS + (p.group_offsets ? p.n_groups : 0);
   if (m_tiles > 65535) { set_error("gemm: too many row tiles (%d)", m_tiles); return 1; }
-  // 128 weight rows a CTA where that gives every SM three of them (twelve warps), else 64
   constexpr int per = MODE == kSwiglu ? 2 : 1;
-  if ((long)m_tiles * ((per * p.N + 127) / 128) >= 3l * sm_count())
-    cpi::launch_pdl(gemm_simt_tile_kernel<TA, TW, TO, MODE, 8>, dim3((per * p.N + 127) / 128, m_tiles), TILE_THREADS, 0, stream, p);
+  auto go = [&](auto kernel, int cols, int threads) { cpi::launch_pdl(kernel, dim3((per * p.N + cols - 1) / cols, m_tiles), threads, 0, stream, p); };
+  // 128 weight rows a CTA with 8 x 8 outputs a thread where that gives the SMs one and a half of them, else 64 with 4 x 8.  The
+  // wider tile / the narrower one, K = 2,048, CTAs of the wider one an SM: 0.9 150 / 123 us, 1.3 209 / 175, 1.7 209 / 234, 2.6
+  // 294 / 344, 10 1,007 / 1,180; a K of 16 and 1.7 4.8 / 3.9.  bfloat16 weights leave registers for three sixteens of k on the way
+  // (two / three: 509 x 2,048 -> 3,072 199 / 174 us, float32 175 / 180); more than one is in a short sum's way (K = 16: 2.5 / 3.0).
+  if (p.K >= 128 && 2l * m_tiles * ((per * p.N + 127) / 128) >= 3l * sm_count())
+    go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 8, 128, 1>, 128, tile_threads(8, 128));
+  else if (p.K <= 4 * BK)
+    go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 4, 64, 1>, 64, tile_threads(4, 64));
   else
-    cpi::launch_pdl(gemm_simt_tile_kernel<TA, TW, TO, MODE, 4>, dim3((per * p.N + 63) / 64, m_tiles), TILE_THREADS, 0, stream, p);
+    go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 4, 64, sizeof(TW) == 4 ? 2 : 3>, 64, tile_threads(4, 64));
   return check_launch("gemm_simt");
 }
 

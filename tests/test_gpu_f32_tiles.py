@@ -104,3 +104,20 @@ def test_both_routes_of_float32_attention_give_the_same_bits(starts, new, window
         outs.append(out)
         assert len(calls) == int(tiles)
     assert bool(outs[0].isfinite().all()) and torch.equal(outs[0], outs[1])
+
+
+# the wide tile (K of 128 and more, many rows and columns), and sums of up to and over four sixteens of k
+@pytest.mark.parametrize("M,N,K,mode", [(1500, 2056, 130, 0), (1500, 1028, 131, 2), (2000, 1500, 128, 1), (90, 200, 64, 0), (90, 200, 65, 2), (70, 300, 200, 0)])
+def test_more_products_of_many_rows_give_the_bits_of_the_kernel_for_few(M, N, K, mode):
+    from cpi_b200.csrc import lib as L
+    g = torch.Generator(device=DEV).manual_seed(M)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    for tw in (torch.float32, torch.bfloat16):
+        a, w = randn(M, K), randn(N * (2 if mode == 2 else 1), K).to(tw)
+        start = randn(M, N)
+        got = start.clone()
+        L.gemm_simt(a, w, got, mode)
+        for r in range(0, M, 16 * 37):                       # sixteen rows at a time take the kernel for few
+            want = start[r:r + 16].clone()
+            L.gemm_simt(a[r:r + 16], w, want, mode)
+            assert torch.equal(got[r:r + 16], want), (tw, r)
