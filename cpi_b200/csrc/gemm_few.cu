@@ -14,6 +14,9 @@
 // 1.3, 2,048 x 8,192 (N x K) 10.4 / 6.6 / 5.1, 3,072 x 2,048 6.2 / 2.9 / 1.9, 5,120 x 5,120 12.3 / 9.4 / 8.0, 8,192 pairs x 2,048
 // 14.3 / 11.1 / 10.2, 32,000 x 2,048 23.4 / 21.5 / 20.0; 16 tokens: 2,048 x 2,048 5.7 / 3.1, 5,120 x 5,120 13.1 / 12.3.
 //
+// Groups of equally many rows (the heads of latent attention: 16 of 8 rows, 512 x 128 and 128 x 512, 6.1 -> 2.0 us each) have their
+// weights side by side.
+//
 // Epilogues as in gemm_tc.cu: STORE (with its activations), ADD (float32 residual, one writer per element), gated pairs.
 #include "common.cuh"
 #include "gemm_epilogue.cuh"
@@ -26,7 +29,8 @@ struct Params {
   const __nv_bfloat16* x; long ldx;
   const __nv_bfloat16* w;
   void* out; long ldo;
-  int T, N, K;
+  const int* out_rows;           // where row r of all groups' goes; null: to r
+  int T, N, K;                   // T tokens a group: blockIdx.y takes rows from T blockIdx.y on and weights of its own
   int gate_act; float gate_limit;
 };
 
@@ -44,7 +48,8 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) gemm_few_kernel(Params p) 
   constexpr int CH = WARPS < 8 && ACC * NB < 4 ? 2 : 1;   // a warp's long share is summed in two chains (registers allow it)
   __shared__ float part[WARPS][ACC][NB * 8][17];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int n0 = blockIdx.x * 16;
+  const int n0 = blockIdx.x * 16, row0 = blockIdx.y * p.T;
+  const __nv_bfloat16 *px = p.x + (size_t)row0 * p.ldx, *pw = p.w + (size_t)blockIdx.y * ACC * p.N * p.K;
   const int steps = (p.K + 31) / 32, per = (steps + WARPS - 1) / WARPS;
   const int s0 = warp * per, s1 = min(steps, s0 + per);
   // rows past the last feature repeat it; their sums are not stored
@@ -52,10 +57,10 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) gemm_few_kernel(Params p) 
 #pragma unroll
   for (int a = 0; a < ACC; ++a)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) w[a][h] = p.w + (size_t)(a * p.N + min(n0 + g + 8 * h, p.N - 1)) * p.K + 8 * t;
+    for (int h = 0; h < 2; ++h) w[a][h] = pw + (size_t)(a * p.N + min(n0 + g + 8 * h, p.N - 1)) * p.K + 8 * t;
   const __nv_bfloat16* x[NB];
 #pragma unroll
-  for (int b = 0; b < NB; ++b) x[b] = p.x + (size_t)(b * 8 + g) * p.ldx + 8 * t;
+  for (int b = 0; b < NB; ++b) x[b] = px + (size_t)(b * 8 + g) * p.ldx + 8 * t;
 
   uint4 wr[D][ACC][2], xr[DX][NB];
   float acc[CH][ACC][NB][4];
@@ -88,11 +93,13 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) gemm_few_kernel(Params p) 
   // the residual's old values, while the weights are on the way: thread tid adds to feature tid % 16 of token tid / 16
   constexpr int OUT = NB * 8 * 16, PER = (OUT + WARPS * 32 - 1) / (WARPS * 32);
   float old[PER];
-  TO* out = reinterpret_cast<TO*>(p.out);
+  TO *out = reinterpret_cast<TO*>(p.out), *at[PER];
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     const int e = tid + i * WARPS * 32, tok = e / 16, n = n0 + e % 16;
-    old[i] = MODE == epi::kAdd && e < OUT && tok < p.T && n < p.N ? to_f32(out[(size_t)tok * p.ldo + n]) : 0.f;
+    const bool live = e < OUT && tok < p.T && n < p.N;
+    at[i] = !live ? nullptr : out + (size_t)(p.out_rows ? p.out_rows[row0 + tok] : row0 + tok) * p.ldo + n;
+    old[i] = MODE == epi::kAdd && live ? to_f32(*at[i]) : 0.f;
   }
   for (int s = s0; s < s1; s += D) {
 #pragma unroll
@@ -120,8 +127,8 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) gemm_few_kernel(Params p) 
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
-    const int e = tid + i * WARPS * 32, tok = e / 16, f = e % 16, n = n0 + f;
-    if (e >= OUT || tok >= p.T || n >= p.N) continue;
+    const int e = tid + i * WARPS * 32, tok = e / 16, f = e % 16;
+    if (at[i] == nullptr) continue;
     float v = part[0][0][tok][f], u = ACC == 2 ? part[0][ACC - 1][tok][f] : 0.f;
 #pragma unroll
     for (int q = 1; q < WARPS; ++q) {
@@ -131,7 +138,7 @@ __global__ void __launch_bounds__(WARPS * 32, PER_SM) gemm_few_kernel(Params p) 
     if (MODE == epi::kSwiglu) v = epi::gate_mul(v, u, p.gate_act, p.gate_limit);
     else if (MODE == epi::kAdd) v = old[i] + v;
     else v = epi::store_act(v, p.gate_act);
-    out[(size_t)tok * p.ldo + n] = from_f32<TO>(v);
+    *at[i] = from_f32<TO>(v);
   }
 }
 
@@ -175,8 +182,8 @@ static void go(dim3 grid, cudaStream_t stream, const Params& p) {
 }
 
 template <int MODE, typename TO, int NB>
-static int launch(const Params& p, int form, cudaStream_t stream) {
-  const dim3 grid((p.N + 15) / 16);
+static int launch(const Params& p, int groups, int form, cudaStream_t stream) {
+  const dim3 grid((p.N + 15) / 16, groups);
   constexpr int A = MODE == epi::kSwiglu ? 2 : 1;              // (a pair's weights take twice the registers a step)
   constexpr int X = NB > 1 ? 2 : 4 / A;
   if constexpr (NB < 4) {
@@ -196,25 +203,33 @@ static int launch(const Params& p, int form, cudaStream_t stream) {
 
 using namespace cpi;
 
-// The form that a product of T tokens and N features takes (0: it is left to gemm_tc).
-extern "C" int cpi_gemm_few_plan(int T, int N) { return T > 0 && N > 0 ? few::plan(T, N, sm_count()) : few::kNone; }
+// The form that a product of T tokens (a group) and N features takes (0: it is left to gemm_tc).  Of groups it takes those of up
+// to 16 rows whose blocks are all resident; short sums (up to eight steps of 32 k) need no more than four warps a block.
+extern "C" int cpi_gemm_few_plan(int T, int N, int K, int groups) {
+  if (T <= 0 || N <= 0) return few::kNone;
+  if (groups <= 1) return few::plan(T, N, sm_count());
+  const long blocks = (long)((N + 15) / 16) * groups;
+  return T > 16 || groups > 65535 || blocks > 4l * sm_count() ? few::kNone : K > 256 && blocks <= sm_count() ? few::kOne : few::kFour;
+}
 
-// x [T, K] bf16 (row stride ldx), w [N or 2N][K] bf16 contiguous, out [T, N]; modes as in cpi_gemm_tc; form as cpi_gemm_few_plan gives it.
-extern "C" int cpi_gemm_few(const void* x, long ldx, const void* w, void* out, int out_dtype, long ldo, int T, int N, int K, int mode,
-                            int form, float gate_limit, cudaStream_t stream) {
+// x [groups T, K] bf16 (row stride ldx), w [groups][N or 2N][K] bf16 contiguous, out [groups T, N] or its rows out_rows; modes as in
+// cpi_gemm_tc; form as cpi_gemm_few_plan gives it.
+extern "C" int cpi_gemm_few(const void* x, long ldx, const void* w, void* out, int out_dtype, long ldo, const int* out_rows, int groups, int T,
+                            int N, int K, int mode, int form, float gate_limit, cudaStream_t stream) {
   if (T == 0 || N == 0) return 0;
   const int gate_act = mode == 3 ? 1 : mode == 4 ? 2 : mode == 5 ? 3 : mode == 6 ? 4 : 0;
   if (mode == 3 || mode == 4) mode = 2;
   if (mode == 5 || mode == 6) mode = 0;
   CPI_REQUIRE(T > 0 && T <= 32 && N > 0 && K > 0, "gemm_few: bad sizes T=%d N=%d K=%d", T, N, K);
+  CPI_REQUIRE(groups >= 1 && groups <= 65535, "gemm_few: %d groups", groups);
   CPI_REQUIRE(form == few::kOne || (form > few::kOne && form <= few::kFour && T <= 16), "gemm_few: no form %d for %d tokens", form, T);
   CPI_REQUIRE(K % 8 == 0 && ldx % 8 == 0, "gemm_few: K (%d) and the activation row stride (%ld) must be multiples of 8", K, ldx);
   CPI_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0,
               "gemm_few: operands must be 16-byte aligned");
   CPI_REQUIRE(mode != epi::kAdd || out_dtype == kF32, "gemm_few: ADD mode needs a float32 output");
   CPI_REQUIRE(mode != epi::kSwiglu || out_dtype == kBF16, "gemm_few: gated modes write bfloat16");
-  few::Params p{reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(w), out, ldo, T, N, K, gate_act, gate_limit};
-#define CPI_FEW(MODE, TO) return T <= 8 ? few::launch<MODE, TO, 1>(p, form, stream) : T <= 16 ? few::launch<MODE, TO, 2>(p, form, stream) : few::launch<MODE, TO, 4>(p, form, stream)
+  few::Params p{reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(w), out, ldo, out_rows, T, N, K, gate_act, gate_limit};
+#define CPI_FEW(MODE, TO) return T <= 8 ? few::launch<MODE, TO, 1>(p, groups, form, stream) : T <= 16 ? few::launch<MODE, TO, 2>(p, groups, form, stream) : few::launch<MODE, TO, 4>(p, groups, form, stream)
   if (mode == epi::kStore && out_dtype == kBF16) CPI_FEW(epi::kStore, __nv_bfloat16);
   if (mode == epi::kStore && out_dtype == kF32) CPI_FEW(epi::kStore, float);
   if (mode == epi::kAdd) CPI_FEW(epi::kAdd, float);

@@ -207,28 +207,35 @@ def gemm_tc(a, w, out, mode=MODE_STORE, *, n_out=None, m_rows=None, a_rows=None,
     return True
 
 
-def gemm_few(a, w, out, mode=MODE_STORE, *, m_rows=None, gate_limit=0.0, **kw) -> bool:
+def gemm_few(a, w, out, mode=MODE_STORE, *, m_rows=None, gate_limit=0.0, even_groups=0, out_rows=None, **kw) -> bool:
     """The product of up to 32 tokens with a dense weight matrix in bfloat16, weights from memory into registers (see
-    gemm_few.cu).  Returns False, having launched nothing, when the product is outside what it takes (groups, row lists,
-    scales, unaligned operands) or `gemm_tc` is faster."""
+    gemm_few.cu).  Returns False, having launched nothing, when the product is outside what it takes (row lists, scales,
+    unaligned operands) or `gemm_tc` is faster.  `even_groups`: that many groups of equally many rows, one after another,
+    each with its own weights w[g], and with `out_rows` the rows that the results go to."""
     T, K = m_rows if m_rows is not None else a.shape[0], a.shape[1]
-    if T > 32 or w.dim() != 2 or any(v is not None for v in kw.values()) or a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
+    if even_groups:
+        if T % even_groups or w.dim() != 3 or w.shape[0] != even_groups:
+            return False
+    elif w.dim() != 2 or out_rows is not None or any(v is not None for v in kw.values()):
+        return False
+    rows, w_rows = T // max(1, even_groups), w.shape[-2]
+    if rows > 32 or T > a.shape[0] or a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         return False
     if a.stride(1) != 1 or not w.is_contiguous() or out.stride(-1) != 1:
         return False
-    if K % 8 or a.stride(0) % 8 or a.data_ptr() % 16 or w.data_ptr() % 16 or w.shape[1] != K:
+    if K % 8 or a.stride(0) % 8 or a.data_ptr() % 16 or w.data_ptr() % 16 or w.shape[-1] != K:
         return False
-    N = w.shape[0] // 2 if mode in GATED_MODES else w.shape[0]
-    if out.shape[1] != N or out.dtype not in (torch.bfloat16, torch.float32) or T > a.shape[0]:
+    N = w_rows // 2 if mode in GATED_MODES else w_rows
+    if out.shape[1] != N or out.dtype not in (torch.bfloat16, torch.float32):
         return False
-    if (mode in GATED_MODES and (out.dtype != torch.bfloat16 or w.shape[0] % 2)) or (mode == MODE_ADD and out.dtype != torch.float32):
+    if (mode in GATED_MODES and (out.dtype != torch.bfloat16 or w_rows % 2)) or (mode == MODE_ADD and out.dtype != torch.float32):
         return False
-    form = _plan("few", torch._C._cuda_getDevice(), T, N, 0, 0, False)
+    form = _plan("few", torch._C._cuda_getDevice(), rows, N, K, even_groups, False)
     if not form:
         return False
-    _need_cuda(a, w, out)
-    _call("cpi_gemm_few", _p(a), c_long(a.stride(0)), _p(w), _p(out), c_int(dtype_code(out.dtype)), c_long(out.stride(0)),
-          c_int(T), c_int(N), c_int(K), c_int(mode), c_int(form), c_float(gate_limit), _stream())
+    _need_cuda(a, w, out, out_rows)
+    _call("cpi_gemm_few", _p(a), c_long(a.stride(0)), _p(w), _p(out), c_int(dtype_code(out.dtype)), c_long(out.stride(0)), _p(out_rows),
+          c_int(max(1, even_groups)), c_int(rows), c_int(N), c_int(K), c_int(mode), c_int(form), c_float(gate_limit), _stream())
     return True
 
 
@@ -238,7 +245,7 @@ def _plan(kind: str, device: int, T: int, N: int, K: int, n_groups: int, swiglu:
     if kind == "pair":
         return load().cpi_gemm_tc_pair_plan(c_int(T), c_int(N), c_int(K), c_int(int(swiglu)), c_int(n_groups))
     if kind == "few":
-        return load().cpi_gemm_few_plan(c_int(T), c_int(N))
+        return load().cpi_gemm_few_plan(c_int(T), c_int(N), c_int(K), c_int(n_groups))
     if kind == "pays":
         return bool(load().cpi_gemm_tc_pair_pays(c_int(T), c_int(N), c_int(K), c_int(int(swiglu))))
     bn, splits, live_y = c_int(), c_int(), c_int()
@@ -635,20 +642,27 @@ def rglru_scan(gates, u, y, state, out, batch, *, block, lam, r_bias=None, i_bia
 
 
 def latent_kv_write(x, norm_weight, eps, inv_freq, interleaved, cache, page_table, page_size, token_seq, token_pos,
-                    seq_slot, *, rank, rot, amplitude=1.0):
+                    seq_slot, *, rank, rot, amplitude=1.0, queries=None):
     """Per token, from float32 rows x [T, rank + rot] (a column slice allowed): the first `rank` elements RMS-normed
     (times `norm_weight`), the last `rot` rotated by the token's position (sines and cosines times `amplitude`); the row goes into the page of its position
-    in `cache` [pages, 1, page_size, rank + rot]."""
+    in `cache` [pages, 1, page_size, rank + rot].  `queries` (x2, weight, out): out = x2 RMS-normed times the weight in the
+    same launch, in the cache's dtype."""
     _need_cuda(x, norm_weight, inv_freq, cache, page_table, token_seq, token_pos, seq_slot)
     assert x.dtype == torch.float32 and x.dim() == 2 and x.stride(1) == 1 and x.shape[1] == rank + rot
     assert cache.is_contiguous() and cache.shape[-1] == rank + rot and cache.shape[-3] == 1
     assert inv_freq is None or (inv_freq.dtype == torch.float32 and inv_freq.numel() == rot // 2)
     assert norm_weight is None or (norm_weight.is_contiguous() and norm_weight.numel() == rank)
+    x2, w2, out2 = queries if queries is not None else (None, None, None)
+    if x2 is not None:
+        _need_cuda(x2, w2, out2)
+        assert x2.dtype == torch.float32 and x2.dim() == 2 and x2.stride(1) == 1 and out2.dtype == cache.dtype and out2.shape == x2.shape
+        assert out2.stride(1) == 1 and x2.shape[0] == x.shape[0] and (w2 is None or (w2.is_contiguous() and w2.numel() == x2.shape[1]))
     _call("cpi_latent_kv_write", _p(x), c_long(x.stride(0)), _p(norm_weight),
           c_int(F32 if norm_weight is None else dtype_code(norm_weight.dtype)), c_float(eps), _p(inv_freq),
           c_int(int(interleaved)), c_float(float(amplitude)), _p(cache), c_int(dtype_code(cache.dtype)), _p(page_table), c_int(page_table.shape[1]),
           c_int(page_size), _p(token_seq), _p(token_pos), _p(seq_slot), c_int(x.shape[0]), c_int(rank), c_int(rot),
-          _stream())
+          _p(x2), c_long(0 if x2 is None else x2.stride(0)), _p(w2), c_int(F32 if w2 is None else dtype_code(w2.dtype)), _p(out2),
+          c_long(0 if out2 is None else out2.stride(0)), c_int(0 if x2 is None else x2.shape[1]), _stream())
 
 
 def latent_prefill_supported(dim, rot, value_dim, kv_rank, page_size) -> bool:

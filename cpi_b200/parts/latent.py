@@ -156,13 +156,19 @@ class LatentAttentionMixer(Mixer):
         gate, low = down[:, :self.gate_rows], down[:, self.gate_rows:]
         with phase("qkv"):
             project(h, self.w_down, down)
-        if self.has_kv and cache.owns:
-            with phase("kv_store"):      # the normed latent and the rotated key part of every token go into its page
-                K.latent_kv_write(low[:, self.q_rank:], self.w_cnorm, self.eps, inv_freq, inter, pages, table, page_size,
-                                  batch.token_seq, batch.token_pos, batch.seq_slot, rank=rank, rot=R, amplitude=amp)
         cq = self.ws.get("latent_cq", (T, self.q_rank), dt)
-        with phase("rmsnorm"):
-            K.rmsnorm(low[:, :self.q_rank], self.w_qnorm, self.eps, cq)
+        if self.has_kv and cache.owns:
+            # the normed latent and the rotated key part of every token go into its page; the queries' latent is normed beside
+            beside = pages.dtype == dt
+            with phase("kv_store"):
+                K.latent_kv_write(low[:, self.q_rank:], self.w_cnorm, self.eps, inv_freq, inter, pages, table, page_size,
+                                  batch.token_seq, batch.token_pos, batch.seq_slot, rank=rank, rot=R, amplitude=amp,
+                                  queries=(low[:, :self.q_rank], self.w_qnorm, cq) if beside else None)
+        else:
+            beside = False
+        if not beside:
+            with phase("rmsnorm"):
+                K.rmsnorm(low[:, :self.q_rank], self.w_qnorm, self.eps, cq)
         q = self.ws.get("latent_q", (T, H * (D + R)), f32)
         with phase("qkv"):
             project(cq, self.w_uq, q)
@@ -232,7 +238,7 @@ class LatentAttentionMixer(Mixer):
                              rank=rank, amplitude=amp)
         with phase("qkv"):               # the plain part of every query through its head's W_uk^T, into full[t, head, :rank]
             project(plain, self.w_ukT, full.view(T * H, row)[:, :rank], MODE_STORE, out_rows=rows, group_offsets=offsets,
-                    n_groups=H, rows_per_group_hint=T)
+                    n_groups=H, rows_per_group_hint=T, even_groups=H)
         lat = self.ws.get("latent_att_heads", (H * T, rank), dt)            # head-major, the latent part only
         if use_tensor_core_kernels() and dt == torch.bfloat16 and K.latent_attention_supported(row, rank):
             with phase("latent_attention"):
@@ -259,4 +265,4 @@ class LatentAttentionMixer(Mixer):
                 K.head_major_rows(att, lat, n_heads=H, n=rank)
         with phase("wo"):
             project(lat, self.w_uv, out.view(T * H, self.dv), MODE_STORE, out_rows=rows, group_offsets=offsets,
-                    n_groups=H, rows_per_group_hint=T)
+                    n_groups=H, rows_per_group_hint=T, even_groups=H)

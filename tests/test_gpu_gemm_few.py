@@ -27,7 +27,7 @@ def launch(a, w, out, mode, form, limit=0.0):
     from ctypes import c_float, c_int, c_long
     k = K()
     k._call("cpi_gemm_few", k._p(a), c_long(a.stride(0)), k._p(w), k._p(out), c_int(k.dtype_code(out.dtype)), c_long(out.stride(0)),
-            c_int(a.shape[0]), c_int(out.shape[1]), c_int(a.shape[1]), c_int(mode), c_int(form), c_float(limit), k._stream())
+            k._p(None), c_int(1), c_int(a.shape[0]), c_int(out.shape[1]), c_int(a.shape[1]), c_int(mode), c_int(form), c_float(limit), k._stream())
 
 
 @pytest.mark.parametrize("form", [1, 2, 3, 4])
@@ -89,3 +89,20 @@ def test_what_it_leaves_to_other_kernels():
     assert not k.gemm_few(a, w, out, k.MODE_SWIGLU) and not k.gemm_few(a, w, out.bfloat16(), k.MODE_ADD)
     assert not k.gemm_few(a, w, out, row_scale=torch.ones(4, device=DEV))
     assert not k.gemm_few(operands(33, 64, 128, 64)[0], w, torch.zeros(33, 64, device=DEV))
+
+
+@pytest.mark.parametrize("groups,T,N,Kd", [(3, 1, 17, 40), (16, 8, 512, 128), (16, 8, 128, 512), (5, 16, 64, 264), (2, 9, 33, 8)])
+def test_even_groups(groups, T, N, Kd):
+    """Every group's rows by its own weights, sent where the row list says."""
+    k = K()
+    a, _ = operands(groups * T, N, Kd, 1, ldx=8)
+    w = torch.randn(groups, N, Kd, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV).bfloat16()
+    rows = torch.randperm(groups * T, generator=torch.Generator().manual_seed(2)).int().to(DEV)
+    ref = torch.einsum("gtk,gnk->gtn", a.double().view(groups, T, Kd), w.double()).reshape(groups * T, N)
+    tol = torch.einsum("gtk,gnk->gtn", a.double().abs().view(groups, T, Kd), w.double().abs()).reshape(groups * T, N) * (Kd + 1) * 2.0 ** -23 + 1e-30
+    for to in (None, rows):
+        buf = torch.full((groups * T, N + 3), 7.0, device=DEV)
+        assert k.gemm_few(a, w, buf[:, :N], even_groups=groups, out_rows=to)
+        got = buf[:, :N] if to is None else buf[rows.long()][:, :N]
+        assert ((got.double() - ref).abs() <= tol).all() and (buf[:, N:] == 7).all()
+    assert not k.gemm_few(a, w, buf[:, :N], even_groups=groups + 1)
