@@ -22,8 +22,8 @@
 // reads nothing of later tokens.
 //
 // Measured (one prompt of 2,048 tokens, width 2,048), the scan, all on the FP32 pipe, here: the recurrence of gated linear
-// attention with 8 heads of 128 x 256 480, 114, 81 us (prepare_rows 32, chunk_state 25 -> 15, chain 15, chunk_out 41 -> 19; its bytes
-// through the L2 take about 20), the delta rule at 1,500 tokens 435, 176, 163 us (45, solve 21, delta_chain 77, 31 -> 19), the
+// attention with 8 heads of 128 x 256 480, 114, 72 us (prepare_rows 34 -> 23, chunk_state 25 -> 15, chain 15, chunk_out 41 -> 19; its bytes
+// through the L2 take about 20), the delta rule at 1,500 tokens 435, 176, 153 us (48 -> 35, solve 21, delta_chain 77, 31 -> 19), the
 // state-space form with 64 heads of 128 x 64 at 1,855 tokens 507, 187, 149 us (prepare_step 18, 53 -> 26, 31, 80 -> 74).
 //
 //   prepare_rows   the decays per row (their transform too), and A, q~, k~, D (and M, K^) of a chunk and head
@@ -109,15 +109,18 @@ __device__ __forceinline__ float2 two(float x) { return make_float2(x, x); }
 __device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) { *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d); }
 
 // ---- row decays: A, q~, k~, D (and M, K^) --------------------------------------------------------------------------
-// Thread (j, kk) of the scores carries k_j[n] prod a_t[n] for its eighth of the rows (n / 4 mod 8 = kk: eight lanes read
-// 128 neighbouring bytes) forward over the tokens i; the warps
-// with the late j, which are done first, then take q~ and k~ while the others go on.  What is waited for is the longest
-// warp's chain (an instruction every 13 cycles), hence sixteen warps of four j; with eight of eight j 42 us instead of
-// 34 for 2,048 tokens of 8 heads, 128 rows.
+// Over the whole chunk, carrying each key forward past every later token costs a multiplication and a multiply-add per pair
+// of tokens and row, and a load of decay and query for both (34 us for 2,048 tokens of 8 heads of 128 rows; delta rule 45).  So
+// the chunk is taken in four runs of 16.  Within a run the keys are carried forward token by token: thread (j, kk) has k_j[n]
+// prod a_t[n] for its eighth of the rows (n / 4 mod 8 = kk: eight lanes read 128 neighbouring bytes).  Then every thread takes
+// a row and a run: q_i and k_i times the decays from the run's begin to i, k_j times those from j to the run's end, and the
+// run's whole product, still one factor after another.  A pair in different runs is the plain product of two such rows, with
+// the whole runs between them: 4 x 4 pairs a thread over a quarter of the rows.  Here 23 (delta rule 35) us, of 14 a block 5 the decays (delta rule 8: their exponentials and logarithms), 5 the pairs within runs, 3 those between.
+constexpr int RUN = 16, RUNS = C / RUN;
 template <int NPT, bool DELTA>
 struct PrepShape {
-  static constexpr int N = 8 * NPT;
-  static constexpr size_t bytes = ((DELTA ? 3 : 2) * C * N + C + N) * sizeof(float);
+  static constexpr int N = 8 * NPT, LD = N + 4;
+  static constexpr size_t bytes = (3 * C * LD + C + N + RUNS * N) * sizeof(float);
 };
 
 // Of four numbers per lane: their sums over eight neighbouring lanes, the (kk mod 4)-th of them for lane kk.
@@ -131,11 +134,11 @@ __device__ __forceinline__ float sum4(const float (&s)[4], int kk) {
 }
 
 template <int NPT, bool DELTA>
-__global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
+__global__ void __launch_bounds__(512, 2) prepare_rows_kernel(Params p) {
   using Sh = PrepShape<NPT, DELTA>;
-  constexpr int N = Sh::N, PIECES = C * N / 4 / 512;
+  constexpr int N = Sh::N, LD = Sh::LD, PIECES = C * N / 4 / 512;
   extern __shared__ __align__(16) float sm[];
-  float *qs = sm, *as = qs + C * N, *ks = as + C * N, *bs = DELTA ? ks + C * N : ks, *zb = bs + C;
+  float *qs = sm, *as = qs + C * LD, *ks = as + C * LD, *bs = ks + C * LD, *zb = bs + C, *whole = zb + N;
   const int h = blockIdx.y, g = h / p.hpg, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const float rate = p.decay_kind == 1 ? expf(load_any(p.a_log, p.small_dtype, h)) : 0.f;
   if (tid < N) zb[tid] = p.z_bias ? load_any(p.z_bias, p.small_dtype, (size_t)h * N + tid) : 0.f;
@@ -148,18 +151,18 @@ __global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
   float4 d[PIECES];
 #pragma unroll
   for (int i = 0; i < PIECES; ++i) {
-    const int e = tid + i * 512, j = e / (N / 4), n = e % (N / 4) * 4, to = j * N + n;
+    const int e = tid + i * 512, j = e / (N / 4), n = e % (N / 4) * 4, to = j * LD + n;
     const bool live = j < c.n;
     if (live) d[i] = ld4(a + (size_t)j * p.z_stride + n);
     copy16(qs + to, live ? q + (size_t)j * p.q_stride + n : p.q, live);
-    if (DELTA) copy16(ks + to, live ? k + (size_t)j * p.k_stride + n : p.k, live);
+    copy16(ks + to, live ? k + (size_t)j * p.k_stride + n : p.k, live);
   }
   copy_commit();
   if (DELTA && tid < C) bs[tid] = tid < c.n ? 1.0f / (1.0f + expf(-p.beta[(size_t)(c.tok + tid) * p.beta_stride + h])) : 0.f;
   __syncthreads();                                             // the biases are in place
 #pragma unroll
   for (int i = 0; i < PIECES; ++i) {
-    const int e = tid + i * 512, j = e / (N / 4), n = e % (N / 4) * 4, to = j * N + n;
+    const int e = tid + i * 512, j = e / (N / 4), n = e % (N / 4) * 4, to = j * LD + n;
     float4 y = make_float4(1.f, 1.f, 1.f, 1.f);
     if (j < c.n) {
       const float* b = zb + n;
@@ -168,20 +171,17 @@ __global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
     }
     *reinterpret_cast<float4*>(as + to) = y;
   }
-  const int j = 4 * warp + (lane >> 3), kk = lane & 7;
-  float w[NPT];
-#pragma unroll
-  for (int r = 0; r < NPT; r += 4) {
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (j < c.n) x = ld4(k + (size_t)j * p.k_stride + 8 * r + 4 * kk);
-    w[r] = x.x; w[r + 1] = x.y; w[r + 2] = x.z; w[r + 3] = x.w;
-  }
   copy_wait<0>();
   __syncthreads();
+  float *AT = p.AT + c.item * (size_t)(C * C), *MT = DELTA ? p.MT + c.item * (size_t)(C * C) : nullptr;      // A by rows i, M by rows j
+  // ---- pairs within a run
   {
-    float *AT = p.AT + c.item * (size_t)(C * C) + j, *MT = DELTA ? p.MT + c.item * (size_t)(C * C) + (size_t)j * C : nullptr;
+    const int j = 4 * warp + (lane >> 3), kk = lane & 7, end = warp / 4 * RUN + RUN;
+    float w[NPT];
+#pragma unroll
+    for (int r = 0; r < NPT; r += 4) *reinterpret_cast<float4*>(w + r) = ld4(ks + j * LD + 8 * r + 4 * kk);
     auto decay = [&](int i) {
-      const float* ai = as + i * N + 4 * kk;
+      const float* ai = as + i * LD + 4 * kk;
 #pragma unroll
       for (int r = 0; r < NPT; r += 4) {
         const float4 y = ld4(ai + 8 * r);
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
       }
     };
     auto dot = [&](const float* rows, int i) -> float {        // this thread's eighth of row i . w
-      const float* y = rows + i * N + 4 * kk;
+      const float* y = rows + i * LD + 4 * kk;
       float2 s2[2] = {two(0.f), two(0.f)};
 #pragma unroll
       for (int r = 0; r < NPT; r += 4) {
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
     // Four tokens at a time, their sums over the eight lanes side by side, after which lane kk holds token kk's.  A j's own
     // tokens begin at i = j: before that the decays are left out (what is stored above the diagonal is not read).  The rows
     // past the chunk's tokens are zeros, which the delta rule's right-hand sides rely on.
-    for (int i = 4 * warp; i < C; i += 4) {
+    for (int i = 4 * warp; i < end; i += 4) {
       float s[4], m[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -214,33 +214,97 @@ __global__ void __launch_bounds__(512) prepare_rows_kernel(Params p) {
       }
       const float y = sum4(s, kk), z = DELTA ? sum4(m, kk) : 0.f;
       if (kk < 4) {
-        AT[(i + kk) * C] = y * p.q_scale;
-        if (DELTA) MT[i + kk] = z * bs[i + kk];
+        AT[(i + kk) * C + j] = y * p.q_scale;
+        if (DELTA) MT[j * C + i + kk] = z * bs[i + kk];
       }
     }
   }
-  // forward over the tokens: q~, K^; backward: k~, D
-  if (tid >= 256 && tid < 256 + N) {
-    const int n = tid - 256;
-    float P = 1.f;
-    float *QT = p.QT + c.item * (size_t)(N * C) + n, *KP = DELTA ? p.KP + c.item * (size_t)(N * C) + n : nullptr;
-#pragma unroll 16
-    for (int i = 0; i < C; ++i) {
-      P *= as[i * N + n];
-      QT[(size_t)i * N] = qs[i * N + n] * P * p.q_scale;
-      if (DELTA) KP[(size_t)i * N] = ks[i * N + n] * P;
+  __syncthreads();
+  // ---- a row n and a run b: queries (and keys, for the delta rule) from the run's begin, keys to its end in place of the decays
+  const int n = tid % N, b = tid / N;
+  if (b < RUNS) {
+    float *qc = qs + b * RUN * LD + n, *ac = as + b * RUN * LD + n, *kc = ks + b * RUN * LD + n, key[RUN], P = 1.f, R = 1.f;
+#pragma unroll
+    for (int t = 0; t < RUN; ++t) {
+      P *= ac[t * LD];
+      key[t] = kc[t * LD];
+      qc[t * LD] *= P;
+      if (DELTA) kc[t * LD] = key[t] * P;
     }
-  } else if (tid >= 512 - N) {
-    const int n = tid - (512 - N);
-    float R = 1.f;
-    float* KT = p.KT + c.item * (size_t)(N * C) + n;
-#pragma unroll 16
-    for (int t = C - 1; t >= 0; --t) {
-      const float x = DELTA ? ks[t * N + n] : t < c.n ? k[(size_t)t * p.k_stride + n] : 0.f;
-      KT[(size_t)t * N] = x * R;
-      R *= as[t * N + n];
+    whole[b * N + n] = P;
+#pragma unroll
+    for (int t = RUN - 1; t >= 0; --t) {
+      const float x = ac[t * LD];
+      ac[t * LD] = key[t] * R;
+      R *= x;
     }
-    p.DC[c.item * N + n] = R;
+  }
+  __syncthreads();
+  // ---- what the other kernels read: the same from the chunk's begin, to its end
+  if (b < RUNS) {
+    const float *qc = qs + b * RUN * LD + n, *ac = as + b * RUN * LD + n, *kc = ks + b * RUN * LD + n;
+    float before = 1.f, after = 1.f;
+#pragma unroll
+    for (int r = 0; r < RUNS; ++r) {
+      const float x = whole[r * N + n];
+      if (r < b) before *= x;
+      if (r > b) after *= x;
+    }
+    const size_t at = c.item * (size_t)(N * C) + (size_t)b * RUN * N + n;
+#pragma unroll 8
+    for (int t = 0; t < RUN; ++t) {
+      p.QT[at + t * N] = qc[t * LD] * before * p.q_scale;
+      p.KT[at + t * N] = ac[t * LD] * after;
+      if (DELTA) p.KP[at + t * N] = kc[t * LD] * before;
+    }
+    if (b == 0) p.DC[c.item * N + n] = whole[n] * after;
+  }
+  // ---- pairs in different runs I > J: four lanes have 4 x 4 of them, a quarter of the rows each
+  if (tid < 6 * 16 * 4) {
+    const int pair = tid / 64, l = tid % 4, I = pair < 3 ? pair + 1 : pair < 5 ? pair - 1 : 3, J = pair < 3 ? pair : pair < 5 ? pair - 3 : 0;
+    const int i0 = I * RUN + tid / 16 % 4 * 4, j0 = J * RUN + tid / 4 % 4 * 4;
+    auto cross = [&](const float* rows, float (&sum)[4]) {     // lane l: rows[i0 + l] . the four keys
+      float acc[4][4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[r][x] = 0.f;
+#pragma unroll 2
+      for (int m = 4 * l; m < N; m += 16) {
+        float4 f = make_float4(1.f, 1.f, 1.f, 1.f), y[4];
+        for (int r = J + 1; r < I; ++r) {                      // the whole runs between
+          const float4 x = ld4(whole + r * N + m);
+          f = make_float4(f.x * x.x, f.y * x.y, f.z * x.z, f.w * x.w);
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const float4 u = ld4(as + (j0 + x) * LD + m);
+          y[x] = make_float4(u.x * f.x, u.y * f.y, u.z * f.z, u.w * f.w);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float4 u = ld4(rows + (i0 + r) * LD + m);
+#pragma unroll
+          for (int x = 0; x < 4; ++x) acc[r][x] = fmaf(u.w, y[x].w, fmaf(u.z, y[x].z, fmaf(u.y, y[x].y, fmaf(u.x, y[x].x, acc[r][x]))));
+        }
+      }
+      const bool hi = l & 2, odd = l & 1;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        float u = hi ? acc[2][x] : acc[0][x], v = hi ? acc[3][x] : acc[1][x];
+        u += __shfl_xor_sync(0xffffffffu, hi ? acc[0][x] : acc[2][x], 2);
+        v += __shfl_xor_sync(0xffffffffu, hi ? acc[1][x] : acc[3][x], 2);
+        sum[x] = (odd ? v : u) + __shfl_xor_sync(0xffffffffu, odd ? u : v, 1);
+      }
+    };
+    float sum[4];
+    cross(qs, sum);
+    st4(AT + (i0 + l) * C + j0, sum[0] * p.q_scale, sum[1] * p.q_scale, sum[2] * p.q_scale, sum[3] * p.q_scale);
+    if (DELTA) {
+      cross(ks, sum);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) MT[(j0 + x) * C + i0 + l] = sum[x] * bs[i0 + l];
+    }
   }
 }
 
