@@ -24,14 +24,14 @@
 // Measured (one prompt of 2,048 tokens, width 2,048), the scan, all on the FP32 pipe, here: the recurrence of gated linear
 // attention with 8 heads of 128 x 256 480, 114, 72 us (prepare_rows 34 -> 23, chunk_state 25 -> 15, chain 15, chunk_out 41 -> 19; its bytes
 // through the L2 take about 20), the delta rule at 1,500 tokens 435, 176, 153 us (48 -> 35, solve 21, delta_chain 77, 31 -> 19), the
-// state-space form with 64 heads of 128 x 64 at 1,855 tokens 507, 187, 149 us (prepare_step 18, 53 -> 26, 31, 80 -> 74).
+// state-space form with 64 heads of 128 x 64 at 1,855 tokens 507, 187, 134 us (prepare_step 18, 53 -> 26, 31, 80 -> 57).
 //
 //   prepare_rows   the decays per row (their transform too), and A, q~, k~, D (and M, K^) of a chunk and head
 //   prepare_step   C_i . B_j of a chunk and group of heads, and the heads' decays: one per head and token
 //   solve          W and U^ of the delta rule: 128 right-hand sides a block, 16 x 16 blocks of the triangle in registers
 //   chunk_state    U = k~^T v, tiles of 64 columns
 //   chain          the states between the chunks; `delta_chain` with the delta rule, 16 columns a block
-//   chunk_out      the outputs, 64 tokens x 128 (or 64) columns a tile
+//   chunk_out      the outputs, 64 tokens x 128 (or 64) columns a tile; `chunk_out_step` with one decay per head and token
 //
 // A long step runs in segments of chunks so that the scratch stays within what the caller gives.
 #include "decay.cuh"
@@ -559,6 +559,28 @@ __device__ __forceinline__ void products(uint32_t tmem, uint32_t tile, bool fres
     mma(s, h, bm, false);
   }
 }
+// The same for sums of which the large part holds something already, in a half of the 128 lanes or in all of them.
+enum Lanes : int { kAllLanes, kLowerLanes, kUpperLanes };
+__device__ __forceinline__ void products_onto(uint32_t tmem, uint32_t tile, Lanes lanes) {
+  constexpr uint32_t idesc = pre::instr_desc(128, 64, false);
+  const uint64_t b = pre::smem_desc(tile, 16, 1024);
+  const uint32_t lo = lanes == kUpperLanes ? ~0u : 0u, hi = lanes == kLowerLanes ? ~0u : 0u;      // lanes that stay as they are
+  auto mma = [&](uint32_t d, uint32_t a, uint64_t bb, uint32_t onto) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %6, %6}, p;\n\t}"
+                 ::"r"(d), "r"(a), "l"(bb), "r"(idesc), "r"(onto), "r"(lo), "r"(hi) : "memory");
+  };
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t h = tmem + TERMS + k * 8, m = h + 32, l = h + 64, s = tmem + SMALL;
+    const uint64_t bh = b + (uint64_t)(k * (32 >> 4)), bm = bh + (TILE >> 4), bl = bm + (TILE >> 4);
+    mma(tmem, h, bh, 1);
+    mma(s, l, bh, k > 0);
+    mma(s, h, bl, 1);
+    mma(s, m, bm, 1);
+    mma(s, m, bh, 1);
+    mma(s, h, bm, 1);
+  }
+}
 // COLUMNS (16 or 32) of both accumulators, added.
 template <int COLUMNS>
 __device__ __forceinline__ void tmem_sum(uint32_t at, float (&v)[COLUMNS]) {
@@ -612,6 +634,22 @@ __device__ __forceinline__ bool tensor_issue(Tensor& t, int tid, uint8_t* tile, 
     pre::fence_after_sync();
     if (pre::elect_one()) {
       products<B_MN>(t.base, smem_u32(tile), fresh);
+      pre::umma_commit(&t.bar);
+    }
+    __syncwarp();
+  }
+  return ok;
+}
+// Scores times values onto the state's products: one head's for all lanes, or those of two heads for a half of the lanes each.
+__device__ __forceinline__ bool tensor_issue_heads(Tensor& t, int tid, uint8_t* tile, bool ok, bool two_heads) {
+  pre::fence_async_proxy();
+  pre::fence_before_sync();
+  ok = __syncthreads_and(ok) != 0;
+  if (ok && tid < 32) {
+    pre::fence_after_sync();
+    if (pre::elect_one()) {
+      products_onto(t.base, smem_u32(tile), two_heads ? kLowerLanes : kAllLanes);
+      if (two_heads) products_onto(t.base, smem_u32(tile + 3 * TILE), kUpperLanes);
       pre::umma_commit(&t.bar);
     }
     __syncwarp();
@@ -869,12 +907,11 @@ __device__ __forceinline__ bool finite_f(float x) { return fabsf(x) <= 3.4028234
 // DT columns a tile: 128, or 64 (the upper lanes then do the same as the lower ones, and are not read).  A block takes up to
 // eight tiles; the queries and scores of one head are split for the first one only.
 template <int N> constexpr size_t OUT_BYTES = (N / 64 + 1) * 3 * TILE;
-template <int N, int DT, bool STEP, bool DELTA>
+template <int N, int DT, bool DELTA>
 __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int per_block) {
   constexpr int SLICES = N / 64 + 1;
   extern __shared__ __align__(1024) uint8_t tile[];
   __shared__ Tensor t;
-  __shared__ Decays decays[STEP ? 2 : 1];                      // this tile's, the next one's
   __shared__ int bad[2][DT];                                   // per column the first token whose value is no finite number
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Dv = p.Dv;
   const int x = ((warp & 3) * 32 + lane) % DT, half = warp >> 2;      // column of the tile
@@ -882,13 +919,12 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
   tensor_begin(t, tid);
   pdl_launch_dependents();                                    // (tensor memory is ours: see common.cuh)
   pdl_wait();
-  const Tiles<DT, STEP> tiles(p, per_block);
+  const Tiles<DT, false> tiles(p, per_block);
   const int count = tiles.count;
   const Place c = place(p, blockIdx.x, tiles.unit * tiles.heads, p.H);
   bool ok = true;
   if (c.n > 0 && count > 0) {
-    auto item = [&](int h) { return (size_t)blockIdx.x * p.H + h; };
-    const float* AT = p.AT + (STEP ? (size_t)blockIdx.x * (p.H / p.hpg) + tiles.unit : c.item) * (size_t)(C * C);
+    const float* AT = p.AT + c.item * (size_t)(C * C);
     const size_t vstep = DELTA ? (size_t)Dv : (size_t)p.v_stride;
     auto values = [&](int i) {
       return (DELTA ? p.UH + c.item * (size_t)(C * Dv) : p.v + (size_t)c.tok * p.v_stride + (size_t)tiles.head(i) * Dv) + tiles.column(i);
@@ -896,30 +932,18 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
     LaneOperand a;
     TileOperand b;
     auto load_a = [&](int i, int sl) {
-      if (sl < SLICES - 1) a.load(p.U + (item(tiles.head(i)) * N + sl * 64 + half * 32) * (size_t)Dv + tiles.column(i) + x, Dv, 32);
+      if (sl < SLICES - 1) a.load(p.U + (c.item * N + sl * 64 + half * 32) * (size_t)Dv + tiles.column(i) + x, Dv, 32);
       else a.load(values(i) + half * 32 * vstep + x, vstep, c.n - half * 32);
     };
     auto load_b = [&](int i, int sl) {
-      if (!STEP && i > 0) return;
+      if (i > 0) return;
       if (sl == SLICES - 1) b.load(AT, C, c.n, tid);
-      else if (STEP) b.load(p.q + (size_t)c.tok * p.q_stride + (size_t)tiles.unit * N + sl * 64, p.q_stride, c.n, tid);
       else b.load(p.QT + c.item * (size_t)(N * C) + sl * 64, N, c.n, tid);
     };
-    auto ask_decays = [&](int i) {
-      if (STEP && tid < DECAYS / 4)
-        copy16(reinterpret_cast<float*>(&decays[STEP ? i & 1 : 0]) + tid * 4, p.MT + item(tiles.head(i)) * DECAYS + tid * 4, true);
-      copy_commit();
-    };
-    if (STEP) ask_decays(0);
     load_a(0, 0);
     load_b(0, 0);
-    if (STEP) {
-      copy_wait<0>();
-      __syncthreads();
-    }
     int round = 0;                                             // products begun
     for (int i = 0; i < count && ok; ++i) {
-      const Decays& D = decays[STEP ? i & 1 : 0];
       // (the skip adds v itself, also with the delta rule, whose products take the corrected u)
       const float skip = p.skip ? load_any(p.skip, p.small_dtype, tiles.head(i)) : 0.f;
 #pragma unroll
@@ -945,41 +969,17 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
         put_lanes(t.base, warp, w);
         if (!last) load_a(i, sl + 1);
         else if (i + 1 < count) load_a(i + 1, 0);
-        if (STEP || i == 0)
+        if (i == 0)
           b.put(tile + sl * 3 * TILE, tid, [&](int r, int j0, float* y) {
-            if (!last) {
-              if (STEP) {
-                const float f = D.upto[r] * p.q_scale;
-#pragma unroll
-                for (int e = 0; e < 8; ++e) y[e] *= f;
-              }
-              return;
-            }
-            if (STEP && r >= j0) {
-              // (C_i . B_j) dt_j prod_{j < t <= i} a_t, from the row's end of this run of eight backwards
-              const int from = j0 / 8, to = r / 8;
-              float L = to > from ? D.run[r] * D.mid[from][to] : 1.f, dt[8], d[8];
-#pragma unroll
-              for (int e = 0; e < 8; e += 4) {
-                *reinterpret_cast<float4*>(dt + e) = ld4(D.dt + j0 + e);
-                *reinterpret_cast<float4*>(d + e) = ld4(D.a + j0 + e);
-              }
-#pragma unroll
-              for (int e = 7; e >= 0; --e) {
-                y[e] *= dt[e] * L;
-                L = j0 + e > r ? 1.f : L * d[e];
-              }
-            }
+            if (!last) return;
 #pragma unroll
             for (int e = 0; e < 8; ++e) y[e] = j0 + e > r ? 0.f : y[e];
           });
         if (!last) load_b(i, sl + 1);
         else if (i + 1 < count) load_b(i + 1, 0);
-        if (STEP && last) copy_wait<0>();
         ok = tensor_issue<false>(t, tid, tile + sl * 3 * TILE, ok, sl == 0);
         ++round;
         if (!ok) break;
-        if (STEP && sl == 0 && i + 1 < count) ask_decays(i + 1);      // (everybody is done with the tile before)
       }
       // (with 64 columns two warps hold the same sums: each writes half of the tokens)
       constexpr int ROWS = DT / 4;
@@ -1014,11 +1014,193 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
           for (int j = first; j <= r; ++j) {
             const float val = values(i)[j * vstep + x];
             if (finite_f(val)) continue;
-            float f = AT[r * C + j];
-            if (STEP) {
-              f *= D.dt[j];
-              for (int s = j + 1; s <= r; ++s) f *= D.a[s];
+            o = fmaf(AT[r * C + j], val, o);
+          }
+          out[(r - i0) * p.out_stride] = o;
+        }
+      }
+      __syncthreads();                                         // everybody has read what the next tiles' values may change
+      if (half == 0) bad[i & 1][x] = C;
+    }
+    ok = __syncthreads_and(ok) != 0;
+  }
+  tensor_end(t, tid, ok, p.error_flag);
+}
+
+// The same with one decay per head and token, for 128 neighbouring columns of a group's heads a tile, each half of 64 of one
+// head.  The queries are the group's, so their terms are formed once for a block's tiles and the decays up to each token are put
+// on the sums of the state's products in tensor memory.  The scores are a head's own: of a tile with two heads either's products
+// leave the other's lanes alone (the instruction's lane mask: nothing of one head reaches the other, whatever its values).
+// A tile per 64 columns, with every lane's work done twice and the queries' terms formed for each head, took 72 us for 64 heads
+// of 128 x 64 at 1,855 tokens, this form 57 (a block's tiles: four there; two or one take 60).
+template <int N> constexpr size_t STEP_OUT_BYTES = (N / 64 + 2) * 3 * TILE;
+template <int N>
+__global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_step_kernel(Params p, int per_block) {
+  constexpr int SLICES = N / 64;
+  extern __shared__ __align__(1024) uint8_t tile[];
+  __shared__ Tensor t;
+  __shared__ __align__(16) Decays decays[2][2];                // this tile's, the next one's: of either half's head
+  __shared__ int bad[2][128];                                  // per column the first token whose value is no finite number
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Dv = p.Dv;
+  const int x = (warp & 3) * 32 + lane, half = warp >> 2, side = x >> 6;      // column of the tile, tokens' half, the column's half
+  if (tid < 128) bad[0][tid] = bad[1][tid] = C;
+  tensor_begin(t, tid);
+  pdl_launch_dependents();                                    // (tensor memory is ours: see common.cuh)
+  pdl_wait();
+  const int unit = blockIdx.y, columns = p.hpg * Dv, first = blockIdx.z * per_block;
+  const int count = min(per_block, (columns + 127) / 128 - first);
+  const Place c = place(p, blockIdx.x, unit * p.hpg, p.H);
+  bool ok = true;
+  if (c.n > 0 && count > 0) {
+    // the last tile may hold one half; its other lanes work on zeros and are not stored
+    auto column = [&](int i) { return (first + i) * 128 + x; };
+    auto live = [&](int i) { return column(i) < columns; };
+    auto head = [&](int i, int s) { return unit * p.hpg + min((first + i) * 128 + s * 64, columns - 64) / Dv; };
+    auto item = [&](int h) { return (size_t)blockIdx.x * p.H + h; };
+    const float* AT = p.AT + ((size_t)blockIdx.x * (p.H / p.hpg) + unit) * (size_t)(C * C);
+    auto values = [&](int i) { return p.v + (size_t)c.tok * p.v_stride + (size_t)unit * columns + column(i); };
+    LaneOperand a;
+    TileOperand b;                                             // the queries' slices (for the first tile), the scores
+    auto load_a = [&](int i, int sl) {
+      if (sl < SLICES) a.load(p.U + (item(head(i, side)) * N + sl * 64 + half * 32) * (size_t)Dv + column(i) % Dv, Dv, live(i) ? 32 : 0);
+      else a.load(values(i) + half * 32 * p.v_stride, p.v_stride, live(i) ? c.n - half * 32 : 0);
+    };
+    auto load_b = [&](int sl) {
+      if (sl < SLICES) b.load(p.q + (size_t)c.tok * p.q_stride + (size_t)unit * N + sl * 64, p.q_stride, c.n, tid);
+      else b.load(AT, C, c.n, tid);
+    };
+    auto ask_decays = [&](int i) {
+      for (int e = tid; e < DECAYS / 2; e += TC_THREADS) {
+        const int s = e / (DECAYS / 4), at = e % (DECAYS / 4) * 4;
+        copy16(reinterpret_cast<float*>(&decays[i & 1][s]) + at, p.MT + item(head(i, s)) * DECAYS + at, true);
+      }
+      copy_commit();
+    };
+    ask_decays(0);
+    load_a(0, 0);
+    load_b(0);
+    int round = 0;                                             // products begun
+    const uint32_t sums = t.base + ((uint32_t)((warp & 3) * 32) << 16) + half * 32;
+    for (int i = 0; i < count && ok; ++i) {
+      const int h = head(i, side);
+      const Decays& D = decays[i & 1][side];
+      const float skip = p.skip ? load_any(p.skip, p.small_dtype, h) : 0.f;
+#pragma unroll
+      for (int sl = 0; sl < SLICES; ++sl) {
+        uint32_t w[3][16];
+        a.split(w);
+        if (sl > 0) {
+          ok = ok && pre::mbar_wait(&t.bar, (round - 1) & 1, &t.gave_up);
+          pre::fence_after_sync();
+        }
+        put_lanes(t.base, warp, w);
+        load_a(i, sl + 1);
+        if (i == 0) {
+          b.put(tile + sl * 3 * TILE, tid, [&](int, int, float* y) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) y[e] *= p.q_scale;
+          });
+        }
+        if (i == 0 || sl == SLICES - 1) load_b(sl + 1);
+        if (sl == SLICES - 1) copy_wait<0>();                  // this tile's decays
+        ok = tensor_issue<false>(t, tid, tile + sl * 3 * TILE, ok, sl == 0);
+        ++round;
+        if (!ok) break;
+      }
+      if (!ok) break;
+      if (i + 1 < count) ask_decays(i + 1);                    // (everybody is done with the tile before)
+      // A value that is no finite number is left out and added to the outputs that see it: see the kernel above.
+      float zero = 0.f;
+#pragma unroll
+      for (int e = 0; e < 32; ++e) zero = fmaf(a.x[e], 0.f, zero);
+      if (zero != 0.f)
+#pragma unroll
+        for (int e = 0; e < 32; ++e)
+          if (!finite_f(a.x[e])) { atomicMin(&bad[i & 1][x], half * 32 + e); a.x[e] = 0.f; }
+      const bool two_heads = head(i, 0) != head(i, 1);
+      for (int s = 0; s <= (two_heads ? 1 : 0); ++s) {
+        const Decays& E = decays[i & 1][s];
+        b.put(tile + (SLICES + s) * 3 * TILE, tid, [&](int r, int j0, float* y) {
+          if (r >= j0) {
+            // (C_i . B_j) dt_j prod_{j < t <= i} a_t, from the row's end of this run of eight backwards
+            const int from = j0 / 8, to = r / 8;
+            float L = to > from ? E.run[r] * E.mid[from][to] : 1.f, dt[8], d[8];
+#pragma unroll
+            for (int e = 0; e < 8; e += 4) {
+              *reinterpret_cast<float4*>(dt + e) = ld4(E.dt + j0 + e);
+              *reinterpret_cast<float4*>(d + e) = ld4(E.a + j0 + e);
             }
+#pragma unroll
+            for (int e = 7; e >= 0; --e) {
+              y[e] *= dt[e] * L;
+              L = j0 + e > r ? 1.f : L * d[e];
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) y[e] = j0 + e > r ? 0.f : y[e];
+        });
+      }
+      ok = pre::mbar_wait(&t.bar, (round - 1) & 1, &t.gave_up);
+      pre::fence_after_sync();
+#pragma unroll
+      for (int e = 0; e < 32; e += 16) {                       // the decays up to each token, on the state's products
+        float y[16];
+        uint32_t u[16];
+        tmem_sum<16>(sums + e, y);
+#pragma unroll
+        for (int r = 0; r < 16; r += 4) {
+          const float4 f = ld4(D.upto + half * 32 + e + r);
+          u[r] = __float_as_uint(y[r] * f.x); u[r + 1] = __float_as_uint(y[r + 1] * f.y);
+          u[r + 2] = __float_as_uint(y[r + 2] * f.z); u[r + 3] = __float_as_uint(y[r + 3] * f.w);
+        }
+        pre::tmem_st16_nowait(sums + e, u);
+      }
+      {
+        uint32_t w[3][16];
+        a.split(w);
+        put_lanes(t.base, warp, w);
+      }
+      if (i + 1 < count) load_a(i + 1, 0);
+      ok = tensor_issue_heads(t, tid, tile + SLICES * 3 * TILE, ok, two_heads);
+      ++round;
+      const int i0 = half * 32;
+      float raw[16];
+      const float* from = values(i) + i0 * p.v_stride;
+      auto load_raw = [&](int first_token) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          raw[e] = live(i) && first_token + e < c.n ? *from : 0.f;
+          from += p.v_stride;
+          asm volatile("" : "+l"(from));                       // (16 addresses at a time would not fit in registers)
+        }
+      };
+      if (p.skip) load_raw(i0);
+      ok = ok && pre::mbar_wait(&t.bar, (round - 1) & 1, &t.gave_up);
+      pre::fence_after_sync();
+      if (__all_sync(0xffffffffu, ok) && live(i) && i0 < c.n) {      // (a warp's columns are of one half)
+        const int wrong = bad[i & 1][x];
+        float* out = p.out + (size_t)(c.tok + i0) * p.out_stride + (size_t)unit * columns + column(i);
+        float* to = out;
+#pragma unroll
+        for (int q = 0; q < 32; q += 16) {
+          float y[16];
+          tmem_sum<16>(sums + q, y);
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            if (i0 + q + e < c.n) *to = p.skip ? fmaf(skip, raw[e], y[e]) : y[e];
+            to += p.out_stride;
+            asm volatile("" : "+l"(to));
+          }
+          if (q == 0 && p.skip) load_raw(i0 + 16);
+        }
+#pragma unroll 1
+        for (int r = max(wrong, i0); r < min(i0 + 32, c.n); ++r) {     // (runs for values that are no finite numbers)
+          float o = out[(r - i0) * p.out_stride];
+          for (int j = wrong; j <= r; ++j) {
+            const float val = values(i)[j * p.v_stride];
+            if (finite_f(val)) continue;
+            float f = AT[r * C + j] * D.dt[j];
+            for (int s = j + 1; s <= r; ++s) f *= D.a[s];
             o = fmaf(f, val, o);
           }
           out[(r - i0) * p.out_stride] = o;
@@ -1073,11 +1255,14 @@ static int state_products(const Params& p, cudaStream_t stream) {
   CPI_TILES_LAUNCH((chunk_state_kernel<N, STEP>), units, p.H / units * (p.Dv / 64), STATE_BYTES<N>);
 }
 // column tiles of 128 where they come out even, else of 64
-template <int N, bool STEP, bool DELTA>
+template <int N, bool DELTA>
 static int output_products(const Params& p, cudaStream_t stream) {
-  const int units = STEP ? p.H / p.hpg : p.H;
-  if (p.Dv % 128 == 0) CPI_TILES_LAUNCH((chunk_out_kernel<N, 128, STEP, DELTA>), units, p.H / units * (p.Dv / 128), OUT_BYTES<N>);
-  else CPI_TILES_LAUNCH((chunk_out_kernel<N, 64, STEP, DELTA>), units, p.H / units * (p.Dv / 64), OUT_BYTES<N>);
+  if (p.Dv % 128 == 0) CPI_TILES_LAUNCH((chunk_out_kernel<N, 128, DELTA>), p.H, p.Dv / 128, OUT_BYTES<N>);
+  else CPI_TILES_LAUNCH((chunk_out_kernel<N, 64, DELTA>), p.H, p.Dv / 64, OUT_BYTES<N>);
+}
+template <int N>
+static int output_products_step(const Params& p, cudaStream_t stream) {
+  CPI_TILES_LAUNCH(chunk_out_step_kernel<N>, p.H / p.hpg, (p.hpg * p.Dv + 127) / 128, STEP_OUT_BYTES<N>);
 }
 
 template <int N>
@@ -1088,17 +1273,17 @@ static int run(const Params& p, cudaStream_t stream) {
     CPI_CHUNK_LAUNCH(prepare_step_kernel<N>, dim3(p.seg_chunks, p.H / p.hpg), 256, 2 * C * (N + 4) * sizeof(float));
     if (int rc = state_products<N, true>(p, stream)) return rc;
     CPI_CHUNK_LAUNCH(chain_kernel<true>, chain, 256, (size_t)0);
-    if (int rc = output_products<N, true, false>(p, stream)) return rc;
+    if (int rc = output_products_step<N>(p, stream)) return rc;
   } else if (p.beta) {
     CPI_CHUNK_LAUNCH((prepare_rows_kernel<N / 8, true>), items, 512, (PrepShape<N / 8, true>::bytes));
     CPI_CHUNK_LAUNCH(solve_kernel, dim3(p.seg_chunks, p.H, (N + p.Dv + 127) / 128), 128, C * 128 * sizeof(float));
     CPI_CHUNK_LAUNCH(delta_chain_kernel<N>, dim3(p.n_seqs, p.H, p.Dv / 16), 256, ChainShape<N>::bytes);
-    if (int rc = output_products<N, false, true>(p, stream)) return rc;
+    if (int rc = output_products<N, true>(p, stream)) return rc;
   } else {
     CPI_CHUNK_LAUNCH((prepare_rows_kernel<N / 8, false>), items, 512, (PrepShape<N / 8, false>::bytes));
     if (int rc = state_products<N, false>(p, stream)) return rc;
     CPI_CHUNK_LAUNCH(chain_kernel<false>, chain, 256, (size_t)0);
-    if (int rc = output_products<N, false, false>(p, stream)) return rc;
+    if (int rc = output_products<N, false>(p, stream)) return rc;
   }
   return 0;
 }

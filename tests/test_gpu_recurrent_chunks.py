@@ -189,3 +189,43 @@ def test_values_that_are_no_numbers_reach_the_outputs_that_see_them(value):
     same = torch.ones(T, H * cols, dtype=torch.bool, device=DEV)
     same[at:, cols + 3] = False
     assert torch.equal(got[0][same], got[1][same]) and not bool(got[1][~same].isfinite().any())
+
+
+# tiles of 128 columns over a group's heads: two heads side by side, a half tile at the end, heads of one and a half tiles
+@pytest.mark.parametrize("hpg,cols,rows", [(1, 64, 64), (3, 64, 128), (3, 192, 64), (8, 64, 128), (2, 128, 64)])
+def test_heads_that_share_a_tile_stay_apart(hpg, cols, rows):
+    """One decay per head: against the scan in 64 bits, and with a head whose step sizes and values are no numbers the other
+    heads' outputs and states keep their bits."""
+    from cpi_b200.csrc import lib as K
+    g = torch.Generator(device=DEV).manual_seed(11)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    T, G = 150, 2
+    H = G * hpg
+    k, q, v, raw, bias, a_log, skip = randn(T, G * rows), randn(T, G * rows), randn(T, H * cols), randn(T, H), randn(H), randn(H), randn(H)
+    state = randn(1, H, rows, cols)
+    size = dict(n_heads=H, heads_per_group=hpg, n_rows=rows, n_cols=cols)
+    got = []
+    for broken in (False, True):
+        r, w = raw.clone(), v.clone()
+        if broken:
+            r[40:, hpg - 1], w[70, (hpg - 1) * cols:hpg * cols] = float("nan"), float("inf")
+        S, out = state.clone(), torch.full((T, H * cols), float("nan"), device=DEV)
+        per = K.linear_chunks_scratch(H, hpg, rows, cols)
+        K.linear_chunks(k, q, w, S, out, _batch([T], [0]), scratch=torch.empty(2 * per, device=DEV), q_scale=0.25, dt=r, dt_bias=bias,
+                        a_log=a_log, skip=skip, **size)
+        got.append((out.view(T, H, cols), S[0]))
+    others = [h for h in range(H) if h != hpg - 1]
+    assert torch.equal(got[0][0][:, others], got[1][0][:, others]) and torch.equal(got[0][1][others], got[1][1][others])
+    assert torch.equal(got[0][0][:40], got[1][0][:40]) and bool(got[1][0][40:, hpg - 1].isnan().all())
+    S2, out2 = state.clone(), torch.empty(T, H * cols, device=DEV)
+    K.linear_scan(k, q, v, S2, out2, _batch([T], [0]), q_scale=0.25, dt=raw, dt_bias=bias, a_log=a_log, skip=skip, **size)
+    dt = torch.nn.functional.softplus(raw.double() + bias.double())
+    a = torch.exp(-torch.exp(a_log.double()) * dt)[:, :, None].expand(T, H, rows)
+    kd, qd = (x.double().view(T, G, rows).repeat_interleave(hpg, 1) for x in (k, q))
+    vd = v.double().view(T, H, cols)
+    o, ref = _plain(a, kd, qd * 0.25, vd * dt[:, :, None], state[0].double())
+    o = o + skip.double()[:, None] * vd
+    err = lambda x, y: float((x.double() - y).norm() / y.norm())
+    # the scan's own error, and 2^-22 for sums of 64 terms taken in another order
+    assert err(got[0][0], o) <= 1.5 * err(out2.view(T, H, cols), o) + 2.0 ** -22
+    assert err(got[0][1], ref) <= 1.5 * err(S2[0], ref) + 2.0 ** -22
