@@ -116,6 +116,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, float* v) {      // complete after tcgen05.wait::ld
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+      : "r"(taddr));
+}
 __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
@@ -496,17 +503,90 @@ __global__ void __launch_bounds__(256) gemm_tc_pair_dual_kernel(const __grid_con
 // warp 5 (of the leading CTA) the MMAs.  The stage ring runs on across tiles, and with one accumulator per
 // tile there are two accumulator buffers in tensor memory: the MMAs of tile j+1 run while tile j is turned
 // in shared memory and written out, so an SM pair's tiles follow each other at the tensor pipe's rate
-// instead of each paying fill, drain and epilogue.  (With two accumulators, SwiGLU, the tensor memory
-// holds one tile: its MMAs wait for the epilogue, but its loads do not.)
+// instead of each paying fill, drain and epilogue.  With two accumulators, SwiGLU, the tensor memory
+// holds one tile, whose successor's MMAs wait until it has been read (its loads do not): two groups of four warps take half of
+// the tokens each, keep their gated products as packed bfloat16 in registers (64 a thread), give the accumulators
+// back and turn and store the tile under the next one's MMAs.  By four warps that gave them back with the last token stored,
+// gate/up of 16 experts of 2,048 x 2,048 took 147 us at 512 rows each, so 141.
 //   full[s] / empty[s]            stage ring, as above
 //   acc_full[b]                   MMA -> epilogue warps of both CTAs (commit with multicast)
-//   acc_empty[b] (in the leader)  epilogue warps of both CTAs -> MMA: one arrival per warp, 8 in all
+//   acc_empty[b] (in the leader)  epilogue warps of both CTAs -> MMA: one arrival per warp, 8 in all (16 with two groups)
+// The gated products of a group's tokens (up to 128 of the tile, from `acc` on), packed two tokens a register.
+__device__ __forceinline__ void gated_read(uint32_t acc, uint32_t acc2, int n_cols, int n_valid_t, const float* scale, int act, float limit,
+                                           uint32_t (&packed)[64]) {
+#pragma unroll
+  for (int c = 0; c < 128; c += 16) {
+    if (c >= n_cols) continue;
+    float v[16], u[16];
+    tmem_ld16_issue(acc + c, v);
+    tmem_ld16_issue(acc2 + c, u);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j = 0; j < 16; ++j) asm volatile("" : "+f"(v[j]), "+f"(u[j]));      // (not before the wait)
+    if (scale) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float f = scale[min(c + j, n_valid_t - 1)];
+        v[j] *= f;
+        u[j] *= f;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = epi::gate_mul(v[j], u[j], act, limit);
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+      const __nv_bfloat162 two = __floats2bfloat162_rn(v[j], v[j + 1]);
+      packed[(c + j) / 2] = *reinterpret_cast<const uint32_t*>(&two);
+    }
+  }
+}
+// Turned in shared memory 32 tokens at a time (a thread has a feature's), and out in rows; 128 threads, `sync` their barrier.
+template <typename Sync>
+__device__ __forceinline__ void gated_store(const uint32_t (&packed)[64], __nv_bfloat16* stage, int warp, int lane, int n0, int N, int t0,
+                                            int n_valid_t, __nv_bfloat16* out, long ldo, const int* out_rows, Sync sync) {
+  const int n = n0 + 4 * lane;
+#pragma unroll
+  for (int p0 = 0; p0 < 128; p0 += 32) {
+    if (p0 >= n_valid_t) continue;
+    if (p0 > 0) sync();                                          // the pass before has been copied out
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const uint32_t w = packed[(p0 + j) / 2];
+      const __nv_bfloat162 two = *reinterpret_cast<const __nv_bfloat162*>(&w);
+      stage[j * 128 + warp * 32 + lane] = two.x;
+      stage[(j + 1) * 128 + warp * 32 + lane] = two.y;
+    }
+    sync();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int col = p0 + warp + 4 * q;
+      if (col >= n_valid_t) break;
+      const uint2 x = *reinterpret_cast<const uint2*>(stage + (col - p0) * 128 + 4 * lane);
+      __nv_bfloat16* to = out + (size_t)(out_rows ? out_rows[t0 + col] : t0 + col) * ldo + n;
+      if (n + 4 <= N) {
+        *reinterpret_cast<uint2*>(to) = x;
+      } else {
+        const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&x);
+        for (int i = 0; i < 4 && n + i < N; ++i) to[i] = e[i];
+      }
+    }
+  }
+}
+// One decision of 128 threads that meet at barrier `id`: whether any of them says so.
+__device__ __forceinline__ bool any_of_group(int id, bool x) {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, %2, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(r) : "r"((uint32_t)x), "r"(id) : "memory");
+  return r != 0;
+}
+
 template <int BN, int MODE, typename TO, int STAGES>
-__global__ void __launch_bounds__(192) gemm_tc_pair_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
+__global__ void __launch_bounds__(MODE == kSwiglu ? 384 : 192) gemm_tc_pair_persistent_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                       const __grid_constant__ CUtensorMap map_x,
                                                                       Params p, int n_pairs, int n_tok) {
   constexpr int ACC = MODE == kSwiglu ? 2 : 1;
   constexpr int NB = ACC == 1 ? 2 : 1;                           // accumulator buffers in tensor memory
+  constexpr int GROUPS = ACC;                                    // groups of four epilogue warps: 0 to 3, and 8 to 11
   constexpr int HALF = BN / 2;
   constexpr uint32_t A_BYTES = BM * BK * 2, B_BYTES = HALF * BK * 2;
   constexpr uint32_t STAGE_BYTES = ACC * A_BYTES + B_BYTES;
@@ -574,7 +654,7 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_persistent_kernel(const __gr
 
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int b = 0; b < NB; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+    for (int b = 0; b < NB; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8 * GROUPS); }
     abort_s = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -651,9 +731,10 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_persistent_kernel(const __gr
         if (ok) umma2_commit_both(&acc_full[b]);
       }
     }
-  } else {
-    // ---- epilogue: warps 0-3 of both CTAs; each CTA stores its 128 features of the tile's tokens ----
+  } else if (warp < 4 || warp >= 8) {
+    // ---- epilogue: each CTA stores its 128 features of the tile's tokens ----
     pdl_wait();
+    const int group_no = warp >> 3, wq = warp & 3;               // (a warp reads the lanes of its number mod 4)
     const uint32_t leader_empty0 = map_to_cta(smem_u32(&acc_empty[0]), 0);
     int j = 0;
     for (int pid = cluster_id; pid < n_tiles; pid += n_clusters, ++j) {
@@ -665,21 +746,32 @@ __global__ void __launch_bounds__(192) gemm_tc_pair_persistent_kernel(const __gr
       mbar_wait(&acc_full[b], (j / NB) & 1, abort_flag);
       // one decision for the four warps (a named barrier has no time limit: nobody may leave alone); it also
       // keeps the turning buffer of the tile before from being overwritten while a warp still copies it out
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (abort_s) break;
+      if (any_of_group(1 + group_no, abort_s != 0)) break;
       fence_after_sync();
-      const uint32_t lane_addr = tmem_base + b * (ACC * BN) + ((uint32_t)(warp * 32) << 16);
-      auto ld = [&](int c, float* d) { tmem_ld16(lane_addr + c, d); };
-      auto ldu = [&](int c, float* d) { tmem_ld16(lane_addr + BN + c, d); };
+      const uint32_t lane_addr = tmem_base + b * (ACC * BN) + ((uint32_t)(wq * 32) << 16);
+      // the accumulator has been read: one arrival per warp
+      auto give_back = [&] {
+        fence_before_sync();
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];"
+                       ::"r"(leader_empty0 + (uint32_t)(b * sizeof(uint64_t))) : "memory");
+      };
       TO* out = reinterpret_cast<TO*>(p.out);
-      epi::staged<MODE, TO, EPI_COLS>(epi, ld, ldu, warp, lane, n0, p.N, t0, n_valid_t, n_cols, out, p.ldo, p.out_rows,
-                                      p.row_scale, epi::NamedSync<1, 128>(), p.gate_act, p.gate_limit);
-      // the accumulator has been read (the last tensor-memory load of the tile precedes the last barrier above)
-      fence_before_sync();
-      __syncwarp();
-      if (lane == 0)
-        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];"
-                     ::"r"(leader_empty0 + (uint32_t)(b * sizeof(uint64_t))) : "memory");
+      if constexpr (MODE == kSwiglu) {
+        const int mid = min((n_cols / 2 + 15) & ~15, n_valid_t), from = group_no ? mid : 0, valid = group_no ? n_valid_t - mid : mid;
+        uint32_t packed[64];
+        gated_read(lane_addr + from, lane_addr + BN + from, valid, valid, p.row_scale ? p.row_scale + t0 + from : nullptr, p.gate_act,
+                   p.gate_limit, packed);
+        give_back();
+        gated_store(packed, reinterpret_cast<__nv_bfloat16*>(epi) + group_no * (EPI_COLS / GROUPS * 128), wq, lane, n0, p.N, t0 + from, valid,
+                    out, p.ldo, p.out_rows, HalfSync{1 + group_no});
+      } else {
+        auto ld = [&](int c, float* d) { tmem_ld16(lane_addr + c, d); };
+        epi::staged<MODE, TO, EPI_COLS>(epi, ld, ld, warp, lane, n0, p.N, t0, n_valid_t, n_cols, out, p.ldo, p.out_rows,
+                                        p.row_scale, epi::NamedSync<1, 128>(), p.gate_act, p.gate_limit);
+        give_back();                                             // (its last load precedes the last barrier above)
+      }
     }
   }
   __syncwarp();
@@ -744,7 +836,7 @@ static int launch_persistent(const CUtensorMap& mw, const CUtensorMap& mx, const
   constexpr int SMEM = STAGES * STAGE + EPI;
   static_assert(SMEM >= kAlone, "a pair has its SM pair to itself");
   static bool attr_set = false;
-  return launch_clusters(gemm_tc_pair_persistent_kernel<BN, MODE, TO, STAGES>, SMEM, 192, attr_set, "gemm_tc_pair_persistent", mw, mx, p, n_pairs,
+  return launch_clusters(gemm_tc_pair_persistent_kernel<BN, MODE, TO, STAGES>, SMEM, MODE == kSwiglu ? 384 : 192, attr_set, "gemm_tc_pair_persistent", mw, mx, p, n_pairs,
                          n_tok, stream);
 }
 
