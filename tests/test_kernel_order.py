@@ -67,5 +67,5 @@ def test_kernels_that_allocate_through_a_helper_keep_the_order_too():
     helper = helper[:helper.index("\n}\n")]
     assert helper.index("tcgen05.alloc") < helper.index("__syncthreads()")
     users = {k: body for k, body in KERNELS.items() if "tensor_begin(" in body}
-    assert {k.split(":")[1] for k in users} == {"chunk_state_kernel", "chunk_out_kernel"}
+    assert {k.split(":")[1] for k in users} == {"chunk_state_kernel", "chunk_out_kernel", "chunk_out_step_kernel"}
     assert all(body.index("tensor_begin(") < body.index("pdl_launch_dependents()") for body in users.values())
