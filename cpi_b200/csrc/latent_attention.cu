@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(256, 1) latent_decode_kernel(Params p, int buf
   float* Ss = reinterpret_cast<float*>(KVs + (size_t)TEAMS * buffers * BN * LD);
   int* qpos_s = reinterpret_cast<int*>(Ss + 4 * 16 * SLD);
   const int tok = blockIdx.x, split = blockIdx.y;
-  // (the step's index arrays are in place before its first kernel, and of the rows only the newest position's is this step's)
+  pdl_wait();                                                    // (the rows of earlier positions too may be on their way: see common.cuh)
   const int* table = p.page_table + (size_t)p.seq_slot[p.token_seq[tok]] * p.max_blocks;
   const int last_pos = p.token_pos[tok], first_pos = p.window > 0 ? max(0, last_pos - p.window + 1) : 0;
   const int first_tile = first_pos / BN, n_kv_tiles = last_pos / BN + 1 - first_tile;
@@ -347,9 +347,6 @@ __global__ void __launch_bounds__(256, 1) latent_decode_kernel(Params p, int buf
     }
   };
   const int t0 = t_begin + team;
-  const bool early = t0 < t_end && t0 * BN + BN <= last_pos;
-  if (early) load_kv(t0, 0);
-  pdl_wait();
   for (int m = warp; m < BM; m += 8) {
     __nv_bfloat16* dst = Qs + (size_t)m * LD;
     const __nv_bfloat16* src = p.q + ((size_t)tok * H + m) * row;
@@ -359,7 +356,7 @@ __global__ void __launch_bounds__(256, 1) latent_decode_kernel(Params p, int buf
     }
     if (lane == 0) qpos_s[m] = m < H ? last_pos : -1;
   }
-  if (t0 < t_end && !early) load_kv(t0, 0);
+  if (t0 < t_end) load_kv(t0, 0);
   cp_async_commit();
   if (buffers > 1 && t0 + TEAMS < t_end) load_kv(t0 + TEAMS, 1);
   cp_async_commit();

@@ -69,3 +69,18 @@ def test_kernels_that_allocate_through_a_helper_keep_the_order_too():
     users = {k: body for k, body in KERNELS.items() if "tensor_begin(" in body}
     assert {k.split(":")[1] for k in users} == {"chunk_state_kernel", "chunk_out_kernel", "chunk_out_step_kernel"}
     assert all(body.index("tensor_begin(") < body.index("pdl_launch_dependents()") for body in users.values())
+
+
+def _before_the_wait(body):
+    return body[:body.index("pdl_wait()")]
+
+
+def test_index_arrays_are_read_before_the_wait_by_the_named_kernels_only():
+    """They come from copies that end before a step's first kernel.  Anything else, cached rows above all, is written by kernels
+    that may still be running when a kernel starts; `attention_decode` alone reads older pages early."""
+    arrays = re.compile(r"\b(token_pos|token_seq|seq_slot|seq_tok0|seq_new|seq_start|page_table|tile_tok0|tile_rows)\s*\[")
+    waiting = {k.split(":")[1]: _before_the_wait(body) for k, body in KERNELS.items() if "pdl_wait()" in body}
+    assert {k for k, text in waiting.items() if arrays.search(text)} == {
+        "attention_decode_kernel", "qkv_post_d128_kernel", "qkv_conv_rotate_kernel", "head_turn_kernel"}
+    cached = re.compile(r"\bp\.(cache|k_cache|v_cache|q|state)\b|load_kv\(|load_tile\(")
+    assert {k for k, text in waiting.items() if cached.search(text)} == {"attention_decode_kernel"}
