@@ -71,6 +71,13 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
 // pdl_launch_dependents() lets its own successor be scheduled; a kernel that does not call it does so by ending.  What
 // precedes the wait (barrier set-up, tensor-memory allocation, loads of weights, which no kernel writes) overlaps the
 // predecessor's tail.
+// Two things besides weights are read before the wait, by few kernels and under a condition each.  A step's index arrays
+// (positions, slots, page tables, runs of tokens) come from copies that end before the step's first kernel starts: read by
+// attention_decode, qkv_post_d128, qkv_conv_rotate and head_turn.  Cached pages, all but the one that holds the newest position:
+// read by attention_decode.  Rows of earlier positions come from kernels before the one that stores the newest, and a kernel
+// that stores rows for attention_decode lets its successors start only after its own wait, when all kernels before it have
+// ended.  So steps may follow one another without anything between them; a launch that stores several positions of a
+// sequence is not to be followed by attention_decode over that sequence.
 // A kernel that allocates tensor memory lets its successors start only when it has it.  Before, a successor's block that
 // fits the same SM could take the columns first and keep them until this kernel ends, which waits for those columns.  With
 // that order whoever holds columns belongs to a kernel that is wholly resident, has all it needs and waits for earlier

@@ -84,3 +84,14 @@ def test_index_arrays_are_read_before_the_wait_by_the_named_kernels_only():
         "attention_decode_kernel", "qkv_post_d128_kernel", "qkv_conv_rotate_kernel", "head_turn_kernel"}
     cached = re.compile(r"\bp\.(cache|k_cache|v_cache|q|state)\b|load_kv\(|load_tile\(")
     assert {k for k, text in waiting.items() if cached.search(text)} == {"attention_decode_kernel"}
+
+
+@pytest.mark.parametrize("name", ["attention_simt.cu:qkv_post_kernel", "attention_simt.cu:qkv_post_d128_kernel",
+                                  "attention_simt.cu:qkv_prepare_kernel", "attention_simt.cu:qkv_prepare_heads_kernel",
+                                  "rotate.cu:qkv_conv_rotate_kernel"])
+def test_kernels_that_store_cached_rows_wait_before_their_successors_start(name):
+    """`attention_decode` behind them reads rows of earlier positions before its own wait: those are complete once the storing
+    kernel has waited."""
+    body = KERNELS[name]
+    assert "k_cache" in body and body.count("pdl_launch_dependents()") == 1
+    assert body.index("pdl_wait()") < body.index("pdl_launch_dependents()")
