@@ -473,6 +473,12 @@ constexpr int TC_THREADS = 256;
 constexpr uint32_t TC_COLUMNS = 256;                           // tensor memory: h h, small products (64 each), three terms of M (96)
 constexpr uint32_t SMALL = 64, TERMS = 128;
 
+// A float32 that is no finite number, or so large that its first term is none (from 2^128 - 2^119 on), has no such terms: its last
+// one is NaN, and so are the sums that it enters, whatever it meets there.  A sum that comes out as NaN is formed again in
+// float32, as one chain of multiply-adds, by the thread that writes it: it is then the infinity or NaN of float32 sums.
+// Values, which would also reach the sums of earlier tokens through the zeros above the diagonal, are taken as zero
+// instead, and the sums that they belong to are formed again.
+__device__ __forceinline__ bool has_terms(float x) { return fabsf(x) < 3.3961775292304601e38f; }      // 2^128 - 2^119
 // h, m and l of a pair, packed
 __device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
   h = pre::pack_bf16(a, b);
@@ -498,6 +504,18 @@ struct LaneOperand {
   __device__ __forceinline__ void split(uint32_t (&w)[3][16]) const {
 #pragma unroll
     for (int e = 0; e < 16; ++e) split2(x[2 * e], x[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+  }
+  // The same for values of the tokens from `token` on: those without terms become zeros, and `first` the first such token.
+  __device__ __forceinline__ void split_values(uint32_t (&w)[3][16], int token, int* first) {
+    split(w);
+    __nv_bfloat162 none = __floats2bfloat162_rn(0.f, 0.f);      // not zero if any last term is NaN
+#pragma unroll
+    for (int e = 0; e < 16; ++e) none = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&w[2][e]), __floats2bfloat162_rn(0.f, 0.f), none);
+    if ((*reinterpret_cast<const uint32_t*>(&none) & 0x7fff7fffu) == 0) return;
+#pragma unroll
+    for (int e = 0; e < 32; ++e)
+      if (!has_terms(x[e])) { atomicMin(first, token + e); x[e] = 0.f; }
+    split(w);
   }
 };
 __device__ __forceinline__ void put_lanes(uint32_t tmem, int warp, const uint32_t (&w)[3][16]) {
@@ -581,9 +599,9 @@ __device__ __forceinline__ void products_onto(uint32_t tmem, uint32_t tile, Lane
     mma(s, h, bm, 1);
   }
 }
-// COLUMNS (16 or 32) of both accumulators, added.
+// COLUMNS (16 or 32) of both accumulators, added; whether any sum is no finite number.
 template <int COLUMNS>
-__device__ __forceinline__ void tmem_sum(uint32_t at, float (&v)[COLUMNS]) {
+__device__ __forceinline__ bool tmem_sum(uint32_t at, float (&v)[COLUMNS]) {
   uint32_t a[COLUMNS], b[COLUMNS];
   if constexpr (COLUMNS == 32) {
     pre::tmem_ld32_issue(at, a);
@@ -598,6 +616,10 @@ __device__ __forceinline__ void tmem_sum(uint32_t at, float (&v)[COLUMNS]) {
     asm volatile("" : "+r"(a[i]), "+r"(b[i]));                 // (not before the wait)
     v[i] = __uint_as_float(a[i]) + __uint_as_float(b[i]);
   }
+  float zero = 0.f;
+#pragma unroll
+  for (int i = 0; i < COLUMNS; ++i) zero = fmaf(v[i], 0.f, zero);
+  return zero != 0.f;
 }
 // What a block of the two kernels begins and ends with; two share an SM.
 struct Tensor { uint64_t bar; uint32_t base; int gave_up; };
@@ -691,12 +713,11 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_state_kernel(Params p, in
     auto item = [&](int h) { return (size_t)blockIdx.x * p.H + h; };
     LaneOperand k;
     TileOperand v;
-    if (n < N) {
-      const float* from = STEP ? p.k + (size_t)c.tok * p.k_stride + (size_t)tiles.unit * N : p.KT + c.item * (size_t)(N * C);
-      const size_t step = STEP ? (size_t)p.k_stride : (size_t)N;
-      k.load(from + half * 32 * step + n, step, c.n - half * 32);
-    }
-    auto load = [&](int i) { v.load(p.v + (size_t)c.tok * p.v_stride + (size_t)tiles.head(i) * p.Dv + tiles.column(i), p.v_stride, c.n, tid); };
+    const float* keys = STEP ? p.k + (size_t)c.tok * p.k_stride + (size_t)tiles.unit * N : p.KT + c.item * (size_t)(N * C);
+    const size_t step = STEP ? (size_t)p.k_stride : (size_t)N;
+    if (n < N) k.load(keys + half * 32 * step + n, step, c.n - half * 32);
+    auto values = [&](int i) { return p.v + (size_t)c.tok * p.v_stride + (size_t)tiles.head(i) * p.Dv + tiles.column(i); };
+    auto load = [&](int i) { v.load(values(i), p.v_stride, c.n, tid); };
     load(0);
     if (STEP) {                                                // v_j is written with dt_j prod_{t > j} a_t
       for (int e = tid; e < count * C; e += TC_THREADS) ws[e / C][e % C] = reinterpret_cast<const Decays*>(p.MT)[item(tiles.head(e / C))].w[e % C];
@@ -726,7 +747,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_state_kernel(Params p, in
       pre::fence_after_sync();
       if (__all_sync(0xffffffffu, ok) && n < N) {
         float y[32];
-        tmem_sum<32>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + half * 32, y);
+        const bool again = tmem_sum<32>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + half * 32, y);
         // 16 bytes at a time, rows of 256 turned by their number; each warp reads what it wrote
         uint8_t* rows = tile + 6 * TILE;
 #pragma unroll
@@ -740,6 +761,17 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_state_kernel(Params p, in
           *reinterpret_cast<float4*>(U + (size_t)r * p.Dv + x * 4) = ld4(reinterpret_cast<const float*>(rows + r * 256 + ((x ^ (r & 15)) << 4)));
         }
         __syncwarp();
+#pragma unroll 1
+        for (int x = half * 32; again && x < half * 32 + 32; ++x) {      // (sums of numbers without terms)
+          float* at = U + (size_t)n * p.Dv + x;
+          if (*at == *at) continue;
+          float sum = 0.f;
+          for (int j = 0; j < c.n; ++j) {
+            const float y = values(i)[j * p.v_stride + x];
+            sum = fmaf(keys[j * step + n], STEP ? y * ws[STEP ? i : 0][j] : y, sum);
+          }
+          *at = sum;
+        }
       }
       if (i + 1 < count) ok = tensor_issue<true>(t, tid, tile + ((i + 1) & 1) * 3 * TILE, ok, true);
     }
@@ -902,8 +934,6 @@ __global__ void __launch_bounds__(256) delta_chain_kernel(Params p) {
 // ---- the outputs -----------------------------------------------------------------------------------------------------------
 // The contraction runs over the state's rows and then over the chunk's tokens, 64 at a time; a slice's loads are on the way
 // while the slice before is split and multiplied.  Columns are the product's lanes, tokens its columns.
-__device__ __forceinline__ bool finite_f(float x) { return fabsf(x) <= 3.402823466e38f; }
-
 // DT columns a tile: 128, or 64 (the upper lanes then do the same as the lower ones, and are not read).  A block takes up to
 // eight tiles; the queries and scores of one head are split for the first one only.
 template <int N> constexpr size_t OUT_BYTES = (N / 64 + 1) * 3 * TILE;
@@ -912,7 +942,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
   constexpr int SLICES = N / 64 + 1;
   extern __shared__ __align__(1024) uint8_t tile[];
   __shared__ Tensor t;
-  __shared__ int bad[2][DT];                                   // per column the first token whose value is no finite number
+  __shared__ int bad[2][DT];                                   // per column the first token whose value has no terms
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Dv = p.Dv;
   const int x = ((warp & 3) * 32 + lane) % DT, half = warp >> 2;      // column of the tile
   if (tid < DT) bad[0][tid] = bad[1][tid] = C;
@@ -950,18 +980,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
       for (int sl = 0; sl < SLICES; ++sl) {
         const bool last = sl == SLICES - 1;
         uint32_t w[3][16];
-        // A value that is no finite number is left out (its products with the zeros of earlier tokens would not be zeros)
-        // and added to the outputs that see it when they are written.
-        if (last) {
-          float zero = 0.f;                                    // no number, or no zero, if one of them is none
-#pragma unroll
-          for (int e = 0; e < 32; ++e) zero = fmaf(a.x[e], 0.f, zero);
-          if (zero != 0.f)
-#pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (!finite_f(a.x[e])) { atomicMin(&bad[i & 1][x], half * 32 + e); a.x[e] = 0.f; }
-        }
-        a.split(w);
+        if (last) a.split_values(w, half * 32, &bad[i & 1][x]);
+        else a.split(w);
         if (sl > 0) {
           ok = ok && pre::mbar_wait(&t.bar, (round - 1) & 1, &t.gave_up);
           pre::fence_after_sync();
@@ -999,7 +1019,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
       if (__all_sync(0xffffffffu, ok) && i0 < c.n) {
         const int first = bad[i & 1][x];
         float y[ROWS];
-        tmem_sum<ROWS>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + i0, y);
+        const bool again = tmem_sum<ROWS>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + i0, y) || first < C;
         float* out = p.out + (size_t)(c.tok + i0) * p.out_stride + (size_t)tiles.head(i) * Dv + tiles.column(i) + x;
         float* to = out;
 #pragma unroll
@@ -1009,14 +1029,15 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
           asm volatile("" : "+l"(to));                         // (32 addresses at a time would not fit in registers)
         }
 #pragma unroll 1
-        for (int r = max(first, i0); r < min(i0 + ROWS, c.n); ++r) {     // (runs for values that are no finite numbers)
-          float o = out[(r - i0) * p.out_stride];
-          for (int j = first; j <= r; ++j) {
-            const float val = values(i)[j * vstep + x];
-            if (finite_f(val)) continue;
-            o = fmaf(AT[r * C + j], val, o);
-          }
-          out[(r - i0) * p.out_stride] = o;
+        for (int r = i0; again && r < min(i0 + ROWS, c.n); ++r) {      // (sums of numbers without terms)
+          float* at = out + (r - i0) * p.out_stride;
+          if (r < first && *at == *at) continue;
+          const float *query = p.QT + (c.item * C + r) * (size_t)N, *states = p.U + c.item * N * (size_t)Dv + tiles.column(i) + x;
+          float o = 0.f;
+          for (int n = 0; n < N; ++n) o = fmaf(query[n], states[(size_t)n * Dv], o);
+          for (int j = 0; j <= r; ++j) o = fmaf(AT[r * C + j], values(i)[j * vstep + x], o);
+          if (p.skip) o = fmaf(skip, p.v[(size_t)(c.tok + r) * p.v_stride + (size_t)tiles.head(i) * Dv + tiles.column(i) + x], o);
+          *at = o;
         }
       }
       __syncthreads();                                         // everybody has read what the next tiles' values may change
@@ -1040,7 +1061,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_step_kernel(Params p,
   extern __shared__ __align__(1024) uint8_t tile[];
   __shared__ Tensor t;
   __shared__ __align__(16) Decays decays[2][2];                // this tile's, the next one's: of either half's head
-  __shared__ int bad[2][128];                                  // per column the first token whose value is no finite number
+  __shared__ int bad[2][128];                                  // as above
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, Dv = p.Dv;
   const int x = (warp & 3) * 32 + lane, half = warp >> 2, side = x >> 6;      // column of the tile, tokens' half, the column's half
   if (tid < 128) bad[0][tid] = bad[1][tid] = C;
@@ -1109,14 +1130,6 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_step_kernel(Params p,
       }
       if (!ok) break;
       if (i + 1 < count) ask_decays(i + 1);                    // (everybody is done with the tile before)
-      // A value that is no finite number is left out and added to the outputs that see it: see the kernel above.
-      float zero = 0.f;
-#pragma unroll
-      for (int e = 0; e < 32; ++e) zero = fmaf(a.x[e], 0.f, zero);
-      if (zero != 0.f)
-#pragma unroll
-        for (int e = 0; e < 32; ++e)
-          if (!finite_f(a.x[e])) { atomicMin(&bad[i & 1][x], half * 32 + e); a.x[e] = 0.f; }
       const bool two_heads = head(i, 0) != head(i, 1);
       for (int s = 0; s <= (two_heads ? 1 : 0); ++s) {
         const Decays& E = decays[i & 1][s];
@@ -1157,7 +1170,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_step_kernel(Params p,
       }
       {
         uint32_t w[3][16];
-        a.split(w);
+        a.split_values(w, half * 32, &bad[i & 1][x]);
         put_lanes(t.base, warp, w);
       }
       if (i + 1 < count) load_a(i + 1, 0);
@@ -1179,12 +1192,13 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_step_kernel(Params p,
       pre::fence_after_sync();
       if (__all_sync(0xffffffffu, ok) && live(i) && i0 < c.n) {      // (a warp's columns are of one half)
         const int wrong = bad[i & 1][x];
+        bool again = wrong < C;
         float* out = p.out + (size_t)(c.tok + i0) * p.out_stride + (size_t)unit * columns + column(i);
         float* to = out;
 #pragma unroll
         for (int q = 0; q < 32; q += 16) {
           float y[16];
-          tmem_sum<16>(sums + q, y);
+          again |= tmem_sum<16>(sums + q, y);
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             if (i0 + q + e < c.n) *to = p.skip ? fmaf(skip, raw[e], y[e]) : y[e];
@@ -1194,16 +1208,21 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_step_kernel(Params p,
           if (q == 0 && p.skip) load_raw(i0 + 16);
         }
 #pragma unroll 1
-        for (int r = max(wrong, i0); r < min(i0 + 32, c.n); ++r) {     // (runs for values that are no finite numbers)
-          float o = out[(r - i0) * p.out_stride];
-          for (int j = wrong; j <= r; ++j) {
-            const float val = values(i)[j * p.v_stride];
-            if (finite_f(val)) continue;
-            float f = AT[r * C + j] * D.dt[j];
+        for (int r = i0; again && r < min(i0 + 32, c.n); ++r) {      // (sums of numbers without terms)
+          float* at = out + (r - i0) * p.out_stride;
+          if (r < wrong && *at == *at) continue;
+          const float* query = p.q + (size_t)(c.tok + r) * p.q_stride + (size_t)unit * N;
+          const float* states = p.U + item(h) * N * (size_t)Dv + column(i) % Dv;
+          float o = 0.f;
+          for (int n = 0; n < N; ++n) o = fmaf(query[n] * p.q_scale, states[(size_t)n * Dv], o);
+          o *= D.upto[r];
+          for (int j = 0; j <= r; ++j) {
+            float f = D.dt[j];
             for (int s = j + 1; s <= r; ++s) f *= D.a[s];
-            o = fmaf(f, val, o);
+            o = fmaf(AT[r * C + j] * f, values(i)[j * p.v_stride], o);
           }
-          out[(r - i0) * p.out_stride] = o;
+          if (p.skip) o = fmaf(skip, values(i)[r * p.v_stride], o);
+          *at = o;
         }
       }
       __syncthreads();                                         // everybody has read what the next tiles' values may change

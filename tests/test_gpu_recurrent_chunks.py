@@ -191,6 +191,70 @@ def test_values_that_are_no_numbers_reach_the_outputs_that_see_them(value):
     assert torch.equal(got[0][same], got[1][same]) and not bool(got[1][~same].isfinite().any())
 
 
+# what no three bfloat16 terms hold: infinities, and numbers that bfloat16 rounds to one; tiles of 64 and of 128 columns, a tile
+# that two heads share, and (with 16 groups) blocks of several tiles
+@pytest.mark.parametrize("kind,groups,hpg,cols,segs", [
+    ("rows", 2, 1, 64, 1), ("rows", 2, 1, 128, 1), ("rows", 2, 1, 192, 3), ("rows", 16, 1, 1024, 4), ("step", 2, 3, 64, 3), ("step", 2, 1, 128, 1),
+    ("step", 2, 2, 192, 3), ("step", 16, 12, 64, 4), ("delta", 2, 1, 64, 3), ("delta", 2, 1, 128, 1), ("delta", 16, 1, 1024, 4)])
+@pytest.mark.parametrize("what,value", [("v", float("inf")), ("v", float("-inf")), ("v", 3.4e38), ("v", -3.39e38), ("k", float("inf")),
+                                        ("q", float("inf")), ("state", float("-inf")), ("state", 3.4e38)])
+def test_numbers_without_bfloat16_terms(kind, groups, hpg, cols, segs, what, value):
+    """One such number: outputs and states that do not see it keep their bits, the others are the scan's, infinities with its
+    signs (but where an infinity meets one of its own column, as in all later tokens of the delta rule, and a query's, whose
+    product with a state is taken in two parts: there no finite numbers)."""
+    from cpi_b200.csrc import lib as K
+    g = torch.Generator(device=DEV).manual_seed(6)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    G, rows, T, at, n = groups, 64, 200, 70, 5
+    H = G * hpg
+    h, col = hpg - 1 if hpg > 1 else 1, 3 if cols < 1024 else 700
+    grp = h // hpg
+    x = {"k": randn(T, G * rows).abs() * 0.05 + 0.01, "q": randn(T, G * rows).abs() * 0.05 + 0.01, "v": randn(T, H * cols)}
+    state = randn(1, H, rows, cols)
+    size = dict(n_heads=H, heads_per_group=hpg, n_rows=rows, n_cols=cols)
+    if kind == "step":
+        kw = dict(dt=randn(T, H), dt_bias=0.3 * randn(H) - 6, a_log=randn(H) - 2)      # (step sizes below one)
+    else:
+        kw = dict(z=randn(T, H * rows) + 2, z_bias=randn(H * rows), tau=4.0)
+        if kind == "delta":
+            kw.update(beta=randn(T, H), decay_kind=1, a_log=randn(H) - 3)
+    per = K.linear_chunks_scratch(H, hpg, rows, cols, z=kw.get("z"), beta=kw.get("beta"))
+    got = []
+    for fn, broken in ((K.linear_chunks, False), (K.linear_chunks, True), (K.linear_scan, True)):
+        y, S, out = {m: t.clone() for m, t in x.items()}, state.clone(), torch.zeros(T, H * cols, device=DEV)
+        if broken:
+            if what == "state":
+                S[0, h, n, col] = value
+            else:
+                y[what][at, {"v": h * cols + col, "k": grp * rows + n, "q": grp * rows + n}[what]] = value
+        extra = dict(scratch=torch.full((segs * per,), float("nan"), device=DEV)) if fn is K.linear_chunks else {}
+        fn(y["k"], y["q"], y["v"], S, out, _batch([T], [0]), **size, **kw, **extra)
+        got.append((out.view(T, H, cols), S[0]))
+    sees, holds = torch.zeros(T, H, cols, dtype=torch.bool, device=DEV), torch.zeros(H, rows, cols, dtype=torch.bool, device=DEV)
+    if what in ("v", "state"):
+        sees[at if what == "v" else 0:, h, col] = holds[h, :, col] = True
+    elif what == "k":
+        sees[at:, grp * hpg:(grp + 1) * hpg] = holds[grp * hpg:(grp + 1) * hpg] = True
+    else:
+        sees[at, grp * hpg:(grp + 1) * hpg] = True
+    (o0, s0), (o1, s1), (o2, s2) = got
+    assert torch.equal(o0[~sees], o1[~sees]) and torch.equal(s0[~holds], s1[~holds])
+    if value in (3.4e38, -3.39e38):
+        assert bool(o1.isfinite().all()) and bool(s1.isfinite().all())
+        # float32 sums of up to 128 terms and products of 200 decays, of numbers with no cancellation to speak of
+        for a, b, m in ((o1, o2, sees), (s1, s2, holds)):
+            assert float((a[m] / 3e38 - b[m] / 3e38).norm()) <= 2.0 ** -16 * float((b[m] / 3e38).norm())
+        return
+    if what == "q" or kind == "delta":
+        assert not bool(o1[at][sees[at]].isfinite().any()) and torch.equal(o1.isfinite(), o2.isfinite())
+        return
+    if what == "v":
+        o2[at, h, col] = o1[at, h, col]                      # (the scan adds the value times a skip of zero: NaN)
+    for a, b in ((o1, o2), (s1, s2)):
+        assert torch.equal(a.isposinf(), b.isposinf()) and torch.equal(a.isneginf(), b.isneginf()) and torch.equal(a.isnan(), b.isnan())
+    assert bool(o1[sees].isinf().all())
+
+
 # tiles of 128 columns over a group's heads: two heads side by side, a half tile at the end, heads of one and a half tiles
 @pytest.mark.parametrize("hpg,cols,rows", [(1, 64, 64), (3, 64, 128), (3, 192, 64), (8, 64, 128), (2, 128, 64)])
 def test_heads_that_share_a_tile_stay_apart(hpg, cols, rows):
