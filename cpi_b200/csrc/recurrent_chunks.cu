@@ -1040,7 +1040,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
           *at = o;
         }
       }
-      __syncthreads();                                         // everybody has read what the next tiles' values may change
+      ok = __syncthreads_and(ok) != 0;                         // (one decision; everybody has read what the next tiles' values may change)
       if (half == 0) bad[i & 1][x] = C;
     }
     ok = __syncthreads_and(ok) != 0;
@@ -1225,7 +1225,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_step_kernel(Params p,
           *at = o;
         }
       }
-      __syncthreads();                                         // everybody has read what the next tiles' values may change
+      ok = __syncthreads_and(ok) != 0;                         // (one decision; everybody has read what the next tiles' values may change)
       if (half == 0) bad[i & 1][x] = C;
     }
     copy_wait<0>();

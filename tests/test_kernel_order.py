@@ -95,3 +95,18 @@ def test_kernels_that_store_cached_rows_wait_before_their_successors_start(name)
     body = KERNELS[name]
     assert "k_cache" in body and body.count("pdl_launch_dependents()") == 1
     assert body.index("pdl_wait()") < body.index("pdl_launch_dependents()")
+
+
+@pytest.mark.parametrize("name", ["chunk_state_kernel", "chunk_out_kernel", "chunk_out_step_kernel"])
+def test_tiles_of_the_chunked_recurrences_end_with_one_decision(name):
+    """A wait runs out for some threads and not for others.  In the loop over a block's tiles, which ends when one has, every
+    barrier of the block is one that decides for all of them, so none meets another barrier than its neighbours."""
+    body = KERNELS["recurrent_chunks.cu:" + name]
+    start = body.index("for (int i = 0; i < count && ok; ++i) {")
+    depth, end = 0, start
+    while depth or "{" not in body[start:end]:
+        depth += {"{": 1, "}": -1}.get(body[end], 0)
+        end += 1
+    loop = body[start:end]
+    assert "mbar_wait(" in loop and "__syncthreads()" not in loop
+    assert name == "chunk_state_kernel" or loop.rindex("ok = __syncthreads_and(ok) != 0;") > loop.rindex("mbar_wait(")
