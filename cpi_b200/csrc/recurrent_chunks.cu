@@ -457,8 +457,10 @@ __global__ void __launch_bounds__(128) solve_kernel(Params p) {
 // A float32 operand enters as three bfloat16 terms, x = h + m + l to 2^-25 of it (8 bits a term).  Of the nine products of
 // terms the six above 2^-24 are taken.  h h has an accumulator of its own and the small ones another: a product adds into its
 // accumulator with one truncation, so what counts is how many of them the large sum sees, K / 16 for the 64 to 192 terms
-// here, no more than a float32 sum of that length loses (against 64 bits, decays as layers are initialised: outputs 2.5e-7 and
-// states 2.4e-7 off with float32 sums, 1.9e-7 and 2.1e-7 with these; with one decay per token 1.5e-7 and 9.9e-7, 1.2e-7 and 9.7e-7).
+// here, no more than a float32 sum of that length loses, and what truncation takes on average is given back (OUT_LOST).  Against
+// 64 bits, four heads of 128 x 256 at 1,500 tokens, decays as layers are initialised: outputs 2.05e-7 and states 1.74e-7 off with
+// float32 sums, 1.71e-7 and 1.66e-7 with these; with one decay per token 2.98e-7 and 2.37e-7, 2.74e-7 and 2.33e-7; outputs of the
+// delta rule 2.03e-7, 1.99e-7.
 //
 // The operand with a row a lane (M) is loaded a lane's row a thread, its neighbours' beside it, split in registers and left in
 // tensor memory; the other goes to shared memory as it lies in memory, a tile of 64 rows of 64 columns per term, 128 bytes a
@@ -466,12 +468,16 @@ __global__ void __launch_bounds__(128) solve_kernel(Params p) {
 // columns waits for its operands (83 cycles instead of 32), and writing and reading them fill that memory's pipe: blocks of 256
 // threads, three an SM, took 28 us for the outputs of 8 heads of 128 x 256 at 2,048 tokens, a stream of warps with a task each
 // (splitting, issuing, writing out) 33, the form here 19.  What bounds it now is latency: a slice of 64 k takes two blocks an SM
-// 4,000 cycles (splitting 700, loads' issue 900, 24 products 1,100, waits) of which the tensor pipe works 1,500.
+// 4,000 cycles (splitting 700, loads' issue 900, 24 products 1,100, waits) of which the tensor pipe works 1,500.  Two blocks an SM leave
+// 128 registers a thread: the outputs of 128 columns keep 29 to 31 of their numbers in memory, the step flavour's 9 to 12.
 using pre::smem_u32;
 constexpr uint32_t TILE = 64 * 128;
 constexpr int TC_THREADS = 256;
 constexpr uint32_t TC_COLUMNS = 256;                           // tensor memory: h h, small products (64 each), three terms of M (96)
 constexpr uint32_t SMALL = 64, TERMS = 128;
+// The share of a sum that the truncation of its K / 16 additions takes from it on average (2 to 4e-8 measured, by the mean of (result - exact)
+// sign(exact) against that of float32 sums), given back where the two accumulators are added, before that rounding.
+constexpr float STATE_LOST = 1.5f / (1 << 25), OUT_LOST = 1.f / (1 << 25);
 
 // A float32 that is no finite number, or so large that its first term is none (from 2^128 - 2^119 on), has no such terms: its last
 // one is NaN, and so are the sums that it enters, whatever it meets there.  A sum that comes out as NaN is formed again in
@@ -599,9 +605,9 @@ __device__ __forceinline__ void products_onto(uint32_t tmem, uint32_t tile, Lane
     mma(s, h, bm, 1);
   }
 }
-// COLUMNS (16 or 32) of both accumulators, added; whether any sum is no finite number.
+// COLUMNS (16 or 32) of both accumulators, added; whether any sum is no finite number.  `lost`: see OUT_LOST, or 0.
 template <int COLUMNS>
-__device__ __forceinline__ bool tmem_sum(uint32_t at, float (&v)[COLUMNS]) {
+__device__ __forceinline__ bool tmem_sum(uint32_t at, float lost, float (&v)[COLUMNS]) {
   uint32_t a[COLUMNS], b[COLUMNS];
   if constexpr (COLUMNS == 32) {
     pre::tmem_ld32_issue(at, a);
@@ -614,7 +620,8 @@ __device__ __forceinline__ bool tmem_sum(uint32_t at, float (&v)[COLUMNS]) {
 #pragma unroll
   for (int i = 0; i < COLUMNS; ++i) {
     asm volatile("" : "+r"(a[i]), "+r"(b[i]));                 // (not before the wait)
-    v[i] = __uint_as_float(a[i]) + __uint_as_float(b[i]);
+    const float large = __uint_as_float(a[i]), small = __uint_as_float(b[i]);
+    v[i] = large + (lost == 0.f ? small : fmaf(large, lost, small));
   }
   float zero = 0.f;
 #pragma unroll
@@ -747,7 +754,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_state_kernel(Params p, in
       pre::fence_after_sync();
       if (__all_sync(0xffffffffu, ok) && n < N) {
         float y[32];
-        const bool again = tmem_sum<32>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + half * 32, y);
+        const bool again = tmem_sum<32>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + half * 32, STATE_LOST, y);
         // 16 bytes at a time, rows of 256 turned by their number; each warp reads what it wrote
         uint8_t* rows = tile + 6 * TILE;
 #pragma unroll
@@ -1019,7 +1026,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_kernel(Params p, int 
       if (__all_sync(0xffffffffu, ok) && i0 < c.n) {
         const int first = bad[i & 1][x];
         float y[ROWS];
-        const bool again = tmem_sum<ROWS>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + i0, y) || first < C;
+        const bool again = tmem_sum<ROWS>(t.base + ((uint32_t)((warp & 3) * 32) << 16) + i0, OUT_LOST, y) || first < C;
         float* out = p.out + (size_t)(c.tok + i0) * p.out_stride + (size_t)tiles.head(i) * Dv + tiles.column(i) + x;
         float* to = out;
 #pragma unroll
@@ -1159,7 +1166,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_step_kernel(Params p,
       for (int e = 0; e < 32; e += 16) {                       // the decays up to each token, on the state's products
         float y[16];
         uint32_t u[16];
-        tmem_sum<16>(sums + e, y);
+        tmem_sum<16>(sums + e, 0.f, y);
 #pragma unroll
         for (int r = 0; r < 16; r += 4) {
           const float4 f = ld4(D.upto + half * 32 + e + r);
@@ -1198,7 +1205,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) chunk_out_step_kernel(Params p,
 #pragma unroll
         for (int q = 0; q < 32; q += 16) {
           float y[16];
-          again |= tmem_sum<16>(sums + q, y);
+          again |= tmem_sum<16>(sums + q, OUT_LOST, y);
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
             if (i0 + q + e < c.n) *to = p.skip ? fmaf(skip, raw[e], y[e]) : y[e];

@@ -293,3 +293,27 @@ def test_heads_that_share_a_tile_stay_apart(hpg, cols, rows):
     # the scan's own error, and 2^-22 for sums of 64 terms taken in another order
     assert err(got[0][0], o) <= 1.5 * err(out2.view(T, H, cols), o) + 2.0 ** -22
     assert err(got[0][1], ref) <= 1.5 * err(S2[0], ref) + 2.0 ** -22
+
+
+@pytest.mark.parametrize("kind", ["rows", "step"])
+def test_sums_lean_to_neither_side(kind):
+    """States and outputs of one chunk without decays are plain sums of products.  Against 64 bits their mean error in the direction
+    of the sum stays below 2^-26 of the mean sum: the tensor core truncates, 2^-25 of a sum and more if nothing is given back,
+    float32 rounding to nearest none.  (65,536 sums and more, each some 2^-24 off: their mean is known to 2^-32.)"""
+    from cpi_b200.csrc import lib as K
+    g = torch.Generator(device=DEV).manual_seed(8)
+    randn = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    T, H, rows, cols = 64, 8, 128, 128
+    k, q, v = randn(T, H * rows), randn(T, H * rows), randn(T, H * cols)
+    kw = dict(dt=torch.zeros(T, H, device=DEV), dt_bias=torch.zeros(H, device=DEV), a_log=torch.full((H,), -60.0, device=DEV)) if kind == "step" \
+        else dict(z=torch.full((T, H * rows), float("inf"), device=DEV))
+    per = K.linear_chunks_scratch(H, 1, rows, cols, z=kw.get("z"))
+    S, out = torch.zeros(1, H, rows, cols, device=DEV), torch.zeros(T, H * cols, device=DEV)
+    K.linear_chunks(k, q, v, S, out, _batch([T], [0]), scratch=torch.zeros(per, device=DEV), n_heads=H, heads_per_group=1, n_rows=rows,
+                    n_cols=cols, **kw)
+    kd, qd, vd = (x.double().view(T, H, -1) for x in (k, q, v))
+    if kind == "step":
+        vd = vd * float(torch.nn.functional.softplus(torch.zeros(1, device=DEV)))            # (the step size as float32 has it)
+    o, ref = _plain(torch.ones(T, H, rows, device=DEV, dtype=torch.float64), kd, qd, vd, S[0].double() * 0)
+    lean = lambda x, y: abs(float(((x.double() - y) * y.sign()).mean() / y.abs().mean()))
+    assert lean(S[0], ref) <= 2.0 ** -26 and lean(out.view(T, H, cols), o) <= 2.0 ** -26
