@@ -211,10 +211,14 @@ def gemm_few(a, w, out, mode=MODE_STORE, *, m_rows=None, gate_limit=0.0, even_gr
     """The product of up to 32 tokens with a dense weight matrix in bfloat16, weights from memory into registers (see
     gemm_few.cu).  Returns False, having launched nothing, when the product is outside what it takes (row lists, scales,
     unaligned operands) or `gemm_tc` is faster.  `even_groups`: that many groups of equally many rows, one after another,
-    each with its own weights w[g], and with `out_rows` the rows that the results go to."""
+    each with its own weights w[g], and with `out_rows` the rows that the results go to; what describes the same groups to the
+    other kernels may be given beside it."""
     T, K = m_rows if m_rows is not None else a.shape[0], a.shape[1]
     if even_groups:
-        if T % even_groups or w.dim() != 3 or w.shape[0] != even_groups:
+        same = ("group_offsets", "n_groups", "rows_per_group_hint")
+        if T % even_groups or w.dim() != 3 or w.shape[0] != even_groups or kw.get("n_groups", even_groups) != even_groups:
+            return False
+        if any(v is not None for name, v in kw.items() if name not in same):
             return False
     elif w.dim() != 2 or out_rows is not None or any(v is not None for v in kw.values()):
         return False

@@ -39,10 +39,7 @@ def project(a, w, out, mode=MODE_STORE, *, even_groups=0, **kw):
         # does not take: few tokens per group, a row gather; features that are no multiple of 256 where they don't pay)
         rows, n = kw.get("m_rows", a.shape[0]), out.shape[1]
         # a handful of tokens: weights straight into registers (refuses, launching nothing, where the tcgen05 kernel is faster)
-        if even_groups:
-            if K.gemm_few(a, w, out, mode, even_groups=even_groups, out_rows=kw.get("out_rows")):
-                return
-        elif rows <= 32 and K.gemm_few(a, w, out, mode, **kw):
+        if (even_groups or rows <= 32) and K.gemm_few(a, w, out, mode, even_groups=even_groups, **kw):
             return
         if use_paired_kernel and not single_cta_products.depth and "a_rows" not in kw and rows >= 512 and K.gemm_tc_pair(
                 a, w, out, mode, any_features=bool(n % 256) and K.gemm_tc_pair_pays(rows, n, a.shape[1], mode in K.GATED_MODES), **kw):
