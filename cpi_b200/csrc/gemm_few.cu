@@ -9,7 +9,8 @@
 // weights are asked for before the wait on the preceding kernel (no kernel writes weights), and nothing here is held that a
 // successor waits for, so a decode step's next product has its weights on the way while this one ends.
 //
-// What bounds it is bytes in flight: D steps of 32 k a warp, and all blocks of a launch resident at once (see plan()).
+// What bounds it is bytes in flight: D steps of 32 k a warp, and up to a block an SM, or up to three or four of the smaller forms,
+// resident at once (see plan(); with more the launch takes rounds).
 // Measured on a chain of products over different weights, one token, gemm_tc.cu / here / floor in us: 2,048 x 2,048 4.9 / 2.4 /
 // 1.3, 2,048 x 8,192 (N x K) 10.4 / 6.6 / 5.1, 3,072 x 2,048 6.2 / 2.9 / 1.9, 5,120 x 5,120 12.3 / 9.4 / 8.0, 8,192 pairs x 2,048
 // 14.3 / 11.1 / 10.2, 32,000 x 2,048 23.4 / 21.5 / 20.0; 16 tokens: 2,048 x 2,048 5.7 / 3.1, 5,120 x 5,120 13.1 / 12.3.
@@ -150,14 +151,25 @@ enum Form : int { kNone = 0, kOne = 1, kTwo = 2, kThree = 3, kFour = 4 };
 // blocks, so the form whose rounds hold the fewest blocks per SM is taken, of equals the one with more blocks in flight.  One
 // token, forms two / three / four in us: 192 blocks (3,072 x 2,048) 2.9 / 3.9 / 3.9, 320 (5,120 x 5,120) 14.2 / 9.4 / 10.8, 448
 // (7,168 x 5,120) 15.5 / 14.7 / 12.8, 2,000 (32,000 x 2,048) 22.9 / 21.5 / 21.8: beyond six a place the last round no longer
-// counts.  More than 8 tokens take more registers and loads for them: 16 tokens, gemm_tc.cu / here: 320 blocks 13.5 / 12.3, 448
-// 16.8 / 17.0, 512 of pairs 15.8 / 16.8, 2,000 25.4 / 30; 32 tokens 128 blocks (2,048 x 8,192) 11.6 / 11.3, 192 blocks 7.1 / 7.8.
-static int plan(int T, int N, int sms) {
+// counts.
+// The lines, as this kernel's time over gemm_tc.cu's at one to eight, nine to 16 and 17 to 32 tokens (K of 64 to 16,384; gated
+// products, twice the weights a block, in brackets):
+//   up to 8 tokens, up to six blocks an SM: 0.3 to 1.0 (1.02).  More blocks: a block's begin and end count again and again, 1,024
+//     blocks K 256 1.16 (1.12), 512 0.83 (0.77), 4,096 0.96 (1.02), 12,288 1.04; 2,000 blocks K 512 1.23 (1.02), 1,024 0.93 (1.11);
+//   up to 16, up to a block an SM: 0.3 to 0.9.  To two: K 8,192 0.96 (0.94), 12,288 1.05 (1.01).  To three: K 2,048 0.73 (0.90),
+//     4,096 0.91 (1.06), 8,192 1.04 (1.15).  More: 512 blocks K 2,048 0.80 (0.88), 8,192 1.02 (1.01), not taken;
+//   up to 32, up to a block an SM: registers for the tokens leave fewer weights in flight.  K 4,096 0.82 to 0.91 (0.87 to 1.07, but
+//     0.95 from half of the SMs on), 8,192 1.0 to 1.1 (1.0 to 1.4; up to 24 tokens 0.9 to 1.04).  More blocks: 1.0 to 1.8.
+static int plan(int T, int N, int K, bool gated, int sms) {
   const int blocks = (N + 15) / 16;
   if (T > 32) return kNone;
-  if (blocks <= sms) return kOne;
-  if (T > 16 || (T > 8 && blocks > 3 * sms)) return kNone;
-  if (blocks > 6 * sms) return kThree;
+  if (blocks <= sms) {
+    const int deepest = gated ? (2 * blocks > sms ? 4096 : 2048) : T > 24 ? 4096 : 8192;
+    return T > 16 && K > deepest ? kNone : kOne;
+  }
+  if (T > 16) return kNone;
+  if (T > 8 && (blocks > 3 * sms || K > (blocks <= 2 * sms ? 8192 : gated ? 2048 : 4096))) return kNone;
+  if (blocks > 6 * sms) return K < 512 || K > (gated ? 2048 : 4096) || (blocks > 8 * sms && (K < 1024 || gated)) ? kNone : kThree;
   int best = kNone, least = 0;
   for (int f = kFour; f >= kTwo; --f) {
     const int load = (blocks + f * sms - 1) / (f * sms) * f;
@@ -205,9 +217,9 @@ using namespace cpi;
 
 // The form that a product of T tokens (a group) and N features takes (0: it is left to gemm_tc).  Of groups it takes those of up
 // to 16 rows whose blocks are all resident; short sums (up to eight steps of 32 k) need no more than four warps a block.
-extern "C" int cpi_gemm_few_plan(int T, int N, int K, int groups) {
+extern "C" int cpi_gemm_few_plan(int T, int N, int K, int gated, int groups) {
   if (T <= 0 || N <= 0) return few::kNone;
-  if (groups <= 1) return few::plan(T, N, sm_count());
+  if (groups <= 1) return few::plan(T, N, K, gated != 0, sm_count());
   const long blocks = (long)((N + 15) / 16) * groups;
   return T > 16 || groups > 65535 || blocks > 4l * sm_count() ? few::kNone : K > 256 && blocks <= sm_count() ? few::kOne : few::kFour;
 }

@@ -234,7 +234,7 @@ def gemm_few(a, w, out, mode=MODE_STORE, *, m_rows=None, gate_limit=0.0, even_gr
         return False
     if (mode in GATED_MODES and (out.dtype != torch.bfloat16 or w_rows % 2)) or (mode == MODE_ADD and out.dtype != torch.float32):
         return False
-    form = _plan("few", torch._C._cuda_getDevice(), rows, N, K, even_groups, False)
+    form = _plan("few", torch._C._cuda_getDevice(), rows, N, K, even_groups, mode in GATED_MODES)
     if not form:
         return False
     _need_cuda(a, w, out, out_rows)
@@ -249,7 +249,7 @@ def _plan(kind: str, device: int, T: int, N: int, K: int, n_groups: int, swiglu:
     if kind == "pair":
         return load().cpi_gemm_tc_pair_plan(c_int(T), c_int(N), c_int(K), c_int(int(swiglu)), c_int(n_groups))
     if kind == "few":
-        return load().cpi_gemm_few_plan(c_int(T), c_int(N), c_int(K), c_int(n_groups))
+        return load().cpi_gemm_few_plan(c_int(T), c_int(N), c_int(K), c_int(int(swiglu)), c_int(n_groups))
     if kind == "pays":
         return bool(load().cpi_gemm_tc_pair_pays(c_int(T), c_int(N), c_int(K), c_int(int(swiglu))))
     bn, splits, live_y = c_int(), c_int(), c_int()

@@ -106,3 +106,19 @@ def test_even_groups(groups, T, N, Kd):
         got = buf[:, :N] if to is None else buf[rows.long()][:, :N]
         assert ((got.double() - ref).abs() <= tol).all() and (buf[:, N:] == 7).all()
     assert not k.gemm_few(a, w, buf[:, :N], even_groups=groups + 1)
+
+
+@pytest.mark.parametrize("T,per_sm,Kd,gated,takes", [
+    (1, 13.5, 256, False, False), (1, 13.5, 2048, False, True), (8, 7, 128, False, False), (1, 13.5, 1024, True, False), (4, 3.9, 16384, False, True),
+    (16, 2.1, 8192, False, False), (16, 2.1, 2048, False, True), (16, 2.1, 4096, True, False), (9, 1.5, 8192, False, True), (9, 1.5, 12288, False, False),
+    (32, 0.4, 8192, False, False), (17, 0.4, 8192, False, True), (17, 0.1, 8192, True, False), (17, 0.9, 4096, True, True), (16, 0.9, 16384, True, True)])
+def test_products_that_gemm_tc_finishes_sooner_are_left_to_it(T, per_sm, Kd, gated, takes):
+    """Blocks of 16 features per SM, the depth and the tokens decide (the times of both sides stand at the rule)."""
+    k = K()
+    N = 16 * int(per_sm * k.sm_count())
+    assert bool(k._plan("few", torch.cuda.current_device(), T, N, Kd, 0, gated)) == takes
+    if not takes:                                                             # (asked with operands as well: refused before they are read)
+        a = torch.zeros(T, Kd, device=DEV, dtype=torch.bfloat16)
+        out = torch.empty(T, N, device=DEV, dtype=torch.bfloat16)
+        w = torch.empty(2 * N if gated else N, Kd, device=DEV, dtype=torch.bfloat16)
+        assert not k.gemm_few(a, w, out, k.MODE_SWIGLU if gated else k.MODE_STORE)
