@@ -184,11 +184,12 @@ constexpr int kSharedPercent = 28;
 template <int MODE, typename TO, int NB, int WARPS, int D, int DX, int PER_SM>
 static void go(dim3 grid, cudaStream_t stream, const Params& p) {
   auto kernel = gemm_few_kernel<MODE, TO, NB, WARPS, D, DX, PER_SM>;
-  static bool done = false;
-  if (!done) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kSharedPercent);
-    cudaGetLastError();                                        // (a preference: the kernel runs without it)
-    done = true;
+  static bool done[64] = {false};                              // per device, as the attribute is
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && !done[dev]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, kSharedPercent) != cudaSuccess)
+      cudaGetLastError();                                      // (a preference: the kernel runs without it)
+    done[dev] = true;
   }
   cpi::launch_pdl(kernel, grid, WARPS * 32, 0, stream, p);
 }
