@@ -194,7 +194,7 @@ __device__ __forceinline__ void load4(const T* p, bool live, bool vec, int k, in
 constexpr int TILE_ROWS = 64;
 constexpr int tile_threads(int RT, int COLS) { return TILE_ROWS / (4 * RT) * (COLS / 64) * 32; }
 
-template <typename TA, typename TW, typename TO, int MODE, int RT, int COLS, int DEPTH>
+template <typename TA, typename TW, typename TO, int MODE, int RT, int COLS, int DEPTH, bool SHORT>
 __global__ void __launch_bounds__(tile_threads(RT, COLS)) gemm_simt_tile_kernel(GemmParams p) {
   constexpr bool GLU = MODE == kSwiglu;
   constexpr int TILE_THREADS = tile_threads(RT, COLS);
@@ -265,7 +265,9 @@ __global__ void __launch_bounds__(tile_threads(RT, COLS)) gemm_simt_tile_kernel(
 #pragma unroll
     for (int x = 0; x < 4; ++x) acc[r][x] = make_float2(0.f, 0.f);
   // DEPTH sixteens of k on the way: slot i % DEPTH of the registers, buffer i % 2 of shared memory
-  constexpr int UNROLL = DEPTH % 2 ? 2 * DEPTH : DEPTH;
+  // (SHORT: see launch_simt)
+  static_assert(!SHORT || DEPTH == 1, "a loop of one step has one set of registers");
+  constexpr int UNROLL = SHORT ? 1 : DEPTH % 2 ? 2 * DEPTH : DEPTH;
   Set ring[DEPTH];
 #pragma unroll
   for (int d = 0; d < DEPTH; ++d) fetch(d * BK, ring[d]);
@@ -298,9 +300,9 @@ __global__ void __launch_bounds__(tile_threads(RT, COLS)) gemm_simt_tile_kernel(
   for (int k0 = 0; k0 < p.K; k0 += UNROLL * BK)
 #pragma unroll
     for (int i = 0; i < UNROLL; ++i)
-      if (k0 + i * BK < p.K) step(k0 + i * BK, i & 1, ring[(i + 1) % DEPTH], ring[i % DEPTH]);
-  // (not earlier: blocks of the next kernel that wait beside the running ones slow them down, 343 us became 699 for the two
-  // products of the figure above)
+      if (k0 + i * BK < p.K) step(k0 + i * BK, SHORT ? (k0 / BK) & 1 : i & 1, ring[(i + 1) % DEPTH], ring[i % DEPTH]);
+  // (not earlier: blocks of the next kernel that wait beside the running ones slow them down, 343 us became 699 when the two
+  // products of the figure above took 343)
   pdl_launch_dependents();
 
   TO* out = reinterpret_cast<TO*>(p.out);
@@ -346,16 +348,27 @@ int launch_simt(const GemmParams& p, int m_tiles_hint, cudaStream_t stream) {
   if (m_tiles > 65535) { set_error("gemm: too many row tiles (%d)", m_tiles); return 1; }
   constexpr int per = MODE == kSwiglu ? 2 : 1;
   auto go = [&](auto kernel, int cols, int threads) { cpi::launch_pdl(kernel, dim3((per * p.N + cols - 1) / cols, m_tiles), threads, 0, stream, p); };
-  // 128 weight rows a CTA with 8 x 8 outputs a thread where that gives the SMs one and a half of them, else 64 with 4 x 8.  The
-  // wider tile / the narrower one, K = 2,048, CTAs of the wider one an SM: 0.9 150 / 123 us, 1.3 209 / 175, 1.7 209 / 234, 2.6
-  // 294 / 344, 10 1,007 / 1,180; a K of 16 and 1.7 4.8 / 3.9.  bfloat16 weights leave registers for three sixteens of k on the way
-  // (two / three: 509 x 2,048 -> 3,072 199 / 174 us, float32 175 / 180); more than one is in a short sum's way (K = 16: 2.5 / 3.0).
-  if (p.K >= 128 && 2l * m_tiles * ((per * p.N + 127) / 128) >= 3l * sm_count())
-    go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 8, 128, 1>, 128, tile_threads(8, 128));
-  else if (p.K <= 4 * BK)
-    go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 4, 64, 1>, 64, tile_threads(4, 64));
-  else
-    go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 4, 64, sizeof(TW) == 4 ? 2 : 3>, 64, tile_threads(4, 64));
+  // Two tiles: 128 weight rows a CTA with 8 x 8 outputs a thread, 64 with 4 x 8.  The wide one needs CTAs enough for the SMs and,
+  // up to two and a half an SM, a sum long enough for its longer begin and end; with bfloat16 weights it gains less.  Wide /
+  // narrow in us, wide CTAs an SM: float32 weights, K = 2,048, 0.9 167 / 123, 1.3 209 / 175, 1.7 212 / 234, 2.2 294 / 297, 2.6 289 / 345,
+  // K = 128, 1.7 16.5 / 16.7, K = 96, 1.7 12.8 / 12.9; bfloat16 weights, K = 2,048, 1.7 239 / 232, 2.2 313 / 352, K = 4,096, 1.7 440 / 460.
+  // Sums over soon, and the wide tile's with bfloat16 weights, take the loop of one step, the first since its code is there sooner:
+  // wide, one step / two, 10 an SM, K = 64 39.6 / 42.9, K = 128 71.7 / 70.7; bfloat16 38.5 / 44.3, 70.5 / 76.6, K = 4,096, 2.6 an SM 598 / 622.
+  // The narrow tile has two sixteens of k on the way (one / two: 509 x 16 -> 64 2.9 / 2.6, 2,048 ->
+  // 3,072 187 / 175); bfloat16 weights one, which widening four at a time leaves no room to do better (K = 256, 1.3 an SM 24.4, two
+  // 29.1, three 26.4), or three where the sum is long (K = 2,048 179, 199, 174; half an SM's CTA, K = 256 15.4, 16.6, 14.7).
+  const long sms = sm_count(), ctas = (long)m_tiles * ((per * p.N + 127) / 128);
+  constexpr bool f32 = sizeof(TW) == 4;
+  if (2 * ctas >= 5 * sms || (p.K >= 128 && 2 * ctas >= (f32 || p.K >= 4096 ? 3 : 4) * sms)) {
+    if (p.K <= 64) go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 8, 128, 1, true>, 128, tile_threads(8, 128));
+    else go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 8, 128, 1, !f32>, 128, tile_threads(8, 128));
+  } else if constexpr (f32) {
+    go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 4, 64, 2, false>, 64, tile_threads(4, 64));
+  } else {
+    if (p.K <= 64) go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 4, 64, 1, true>, 64, tile_threads(4, 64));
+    else if (p.K <= (2 * ctas <= sms ? 192 : 384)) go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 4, 64, 1, false>, 64, tile_threads(4, 64));
+    else go(gemm_simt_tile_kernel<TA, TW, TO, MODE, 4, 64, 3, false>, 64, tile_threads(4, 64));
+  }
   return check_launch("gemm_simt");
 }
 

@@ -106,8 +106,11 @@ def test_both_routes_of_float32_attention_give_the_same_bits(starts, new, window
     assert bool(outs[0].isfinite().all()) and torch.equal(outs[0], outs[1])
 
 
-# the wide tile (K of 128 and more, many rows and columns), and sums of up to and over four sixteens of k
-@pytest.mark.parametrize("M,N,K,mode", [(1500, 2056, 130, 0), (1500, 1028, 131, 2), (2000, 1500, 128, 1), (90, 200, 64, 0), (90, 200, 65, 2), (70, 300, 200, 0)])
+# the wide tile (many rows and columns; from one and a half CTAs an SM for longer sums, bfloat16 weights from two), either loop of it
+# and of the narrow one, and its depths for bfloat16 weights
+@pytest.mark.parametrize("M,N,K,mode", [(1500, 2056, 130, 0), (1500, 1028, 131, 2), (2000, 1500, 128, 1), (90, 200, 64, 0), (90, 200, 65, 2), (70, 300, 200, 0),
+                                        (1500, 6200, 63, 0), (1500, 3100, 65, 2), (1500, 6200, 129, 1), (2000, 900, 4100, 0), (2000, 900, 2000, 1),
+                                        (70, 300, 192, 2), (70, 300, 193, 1), (900, 1000, 385, 0), (900, 1000, 384, 0)])
 def test_more_products_of_many_rows_give_the_bits_of_the_kernel_for_few(M, N, K, mode):
     from cpi_b200.csrc import lib as L
     g = torch.Generator(device=DEV).manual_seed(M)
