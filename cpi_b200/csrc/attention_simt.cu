@@ -957,7 +957,12 @@ extern "C" int cpi_qkv_prepare(const void* qkv, int in_dtype, long qkv_stride, c
   CPI_REQUIRE(head_norm >= 0 && head_norm <= 2, "qkv_prepare: unknown kind of head norm %d", head_norm);
   CPI_REQUIRE(v_mix_mode == 0 || (v_first != nullptr && write_kv && (v_mix_mode == 1 || (v_mix_mode == 2 && v_mix))),
               "qkv_prepare: value mixing needs the buffer of the first values (and, to mix, the mixing weight)");
-  // The kernel with a warp per head, where it applies: one map, values as projected and of the keys' size, a rotation that ends between lanes and whose halves are whole lanes, and rows that start on 16 bytes.
+  const size_t row = (size_t)maps * (n_heads + (write_kv ? n_kv_heads : 0)) * head_dim;
+  const size_t n_norms = (size_t)maps * (n_heads + n_kv_heads);
+  const size_t smem = (head_norm == 1 ? 2 * row + n_norms : head_norm == 2 ? row + n_norms : row) * sizeof(float);
+  CPI_REQUIRE(smem <= 200 * 1024, "qkv_prepare: a q and k row of %zu bytes does not fit in shared memory", smem);
+  // The kernel with a warp per head, where it applies: one map, values as projected and of the keys' size, a rotation that ends
+  // between lanes and whose halves are whole lanes, and rows that start on 16 bytes.
   const int per_lane = head_dim / 32;
   auto aligned16 = [](const void* x) { return (reinterpret_cast<uintptr_t>(x) & 15) == 0; };
   const bool by_heads = (head_dim == 64 || head_dim == 128) && v_dim == head_dim && maps == 1 && v_mix_mode == 0 && !v_from_k &&
@@ -971,7 +976,6 @@ extern "C" int cpi_qkv_prepare(const void* qkv, int in_dtype, long qkv_stride, c
     const bool few = n_tokens < 2 * sm_count();
     const int per_block = few && !norm_whole ? 8 : heads, threads = few && norm_whole ? 32 * (heads < 8 ? 8 : heads > 32 ? 32 : heads) : 256;
     const dim3 grid(n_tokens, (heads + per_block - 1) / per_block);
-    CPI_REQUIRE(grid.y <= 65535, "qkv_prepare: %d heads", heads);
 #define CPI_PREP_HEADS(TI, TO)                                                                                  \
   do {                                                                                                          \
     if (head_dim == 128) cpi::launch_pdl(qkv_prepare_heads_kernel<TI, TO, 4>, grid, dim3(threads), 0, stream, p, per_block); \
@@ -983,10 +987,6 @@ extern "C" int cpi_qkv_prepare(const void* qkv, int in_dtype, long qkv_stride, c
     if (in_dtype == kBF16 && out_dtype == kBF16) CPI_PREP_HEADS(__nv_bfloat16, __nv_bfloat16);
 #undef CPI_PREP_HEADS
   }
-  const size_t row = (size_t)maps * (n_heads + (write_kv ? n_kv_heads : 0)) * head_dim;
-  const size_t n_norms = (size_t)maps * (n_heads + n_kv_heads);
-  const size_t smem = (head_norm == 1 ? 2 * row + n_norms : head_norm == 2 ? row + n_norms : row) * sizeof(float);
-  CPI_REQUIRE(smem <= 200 * 1024, "qkv_prepare: a q and k row of %zu bytes does not fit in shared memory", smem);
   // with few tokens a row is cut along its heads into slices, enough blocks for two per SM (a norm over the whole
   // projection keeps a row in one block, which is then large); a prompt has blocks enough
   const int heads_all = maps * (n_heads + (write_kv ? n_kv_heads : 0));

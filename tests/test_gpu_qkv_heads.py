@@ -52,3 +52,19 @@ def test_heads_equal_the_general_form(T, nh, nkv, d, rot, interleaved, norm, bia
         assert bool(((a - b).abs() <= unit * b.abs() + 2.0 ** -21 * b.abs().max()).all())
         assert dst == "f32" or float((a != b).double().mean()) <= 2.0 ** -8
     assert write or bool((got[0][1] == 7.0).all() and (got[0][2] == 7.0).all())
+
+
+@pytest.mark.parametrize("norm", [0, 1])
+def test_rows_beyond_shared_memory_are_refused_by_either_form(norm):
+    """410 heads of 128 are 205 KB of q and k rows, 200 heads with the rotated rows beside them too: neither form takes them."""
+    from cpi_b200.csrc import lib as K
+    nh, nkv, d = (200, 5, 128) if norm else (400, 10, 128)
+    n = (nh + 2 * nkv) * d
+    i32 = lambda *x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    for off in (0, 1):
+        x = torch.zeros(1, n + 8, device=DEV)[:, off:off + n]
+        q = torch.zeros(1, nh * d, device=DEV)
+        kc, vc = (torch.zeros(1, nkv, 16, d, device=DEV) for _ in range(2))
+        with pytest.raises(K.KernelError, match="does not fit in shared memory"):
+            K.qkv_prepare(x, q, kc, vc, i32(0).view(1, 1), 16, i32(0), i32(0), i32(0), n_heads=nh, n_kv_heads=nkv, head_dim=d,
+                          value_dim=d, head_norm=norm, norm_eps=1e-6)
