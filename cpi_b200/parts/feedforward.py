@@ -103,7 +103,7 @@ class DenseSwiGLU(FeedForward):
 
     can_store = True          # forward(..., add=False) stores the output (float32) instead of adding it
 
-    def forward(self, h, residual, batch, add=True):
+    def forward(self, h, residual, batch, add=True, few=True):
         T = h.shape[0]
         a = self.ws.get("ffn_act", (T, self.inter), h.dtype)
         with phase("mlp"):
@@ -114,10 +114,10 @@ class DenseSwiGLU(FeedForward):
                 K.row_gates(h, self.w_token_gate, scale)
             # the gate's activation (its clamps too) and the product with `up` happen in the epilogue of the first product
             if self.activation == "swish_clamped":
-                project(h, self.w_gate_up, a, MODE_CLAMPED_GLU, gate_limit=self.limit)
+                project(h, self.w_gate_up, a, MODE_CLAMPED_GLU, gate_limit=self.limit, few=few)
             else:
-                project(h, self.w_gate_up, a, MODE_SWIGLU if self.activation == "silu" else MODE_GEGLU)
-            project(a, self.w_down, residual, MODE_ADD if add else MODE_STORE, row_scale=scale)
+                project(h, self.w_gate_up, a, MODE_SWIGLU if self.activation == "silu" else MODE_GEGLU, few=few)
+            project(a, self.w_down, residual, MODE_ADD if add else MODE_STORE, row_scale=scale, few=few)
 
 
 UNGATED_ACTIVATIONS = {"relu_squared": MODE_STORE_RELU2, "gelu_tanh": MODE_STORE_GELU}
@@ -293,6 +293,12 @@ class MoESwiGLU(FeedForward):
         T, E, R, Kk = h.shape[0], self.n_experts, self.n_routed, self.top_k
         ws, i32, f32 = self.ws, torch.int32, torch.float32
         forked = None
+        # Beside one or two routed rows a small shared expert stays on the kernel that the routed ones run on.  The layer
+        # with it / with the kernel for a handful of tokens in us, one expert of 16 a token: 6 MB of shared weights 20.8 / 23.7
+        # at one token and 21.6 / 23.8 at two, 12 MB 24.4 / 25.1 and 25.1 / 25.7, but 18 MB 28.4 / 28.8 and 37.7 / 33.4, 48 MB
+        # 29.0 / 29.8 and 35.5 / 33.2; four rows, 6 MB: 24.7 / 24.6 (four tokens), 33.1 / 33.6 (four experts), 12 MB 30.4 / 28.3.
+        # (One after the other, as for the phase timer, they take the same kernels: the results stay the same.)
+        few = T * Kk > 2 or 3 * self.hidden * self.shared_inter * h.element_size() > 16 << 20
         if self.shared is not None and self.overlap_shared and h.is_cuda and phases_active() is None:
             if self._side_stream is None:
                 self._side_stream = torch.cuda.Stream(device=h.device)
@@ -300,7 +306,7 @@ class MoESwiGLU(FeedForward):
             fork.record(torch.cuda.current_stream())
             self._side_stream.wait_event(fork)
             with torch.cuda.stream(self._side_stream):
-                self.shared.forward(h, residual, batch)
+                self.shared.forward(h, residual, batch, few=few)
                 forked = torch.cuda.Event()
                 forked.record(self._side_stream)
         idx = ws.get("moe_topk_idx", (T, Kk), i32)
@@ -367,7 +373,7 @@ class MoESwiGLU(FeedForward):
         if forked is not None:
             return
         if self.shared is not None:
-            self.shared.forward(h, residual, batch)
+            self.shared.forward(h, residual, batch, few=few)
 
 
 @register_feed_forward("moe_mlp")

@@ -31,15 +31,16 @@ class single_cta_products:
         single_cta_products.depth -= 1
 
 
-def project(a, w, out, mode=MODE_STORE, *, even_groups=0, **kw):
+def project(a, w, out, mode=MODE_STORE, *, even_groups=0, few=True, **kw):
     """Dense or grouped projection; see csrc/lib.py: gemm_simt for the keyword arguments.  `even_groups`: the groups' number,
-    where all of them have equally many rows whatever the step (what `group_offsets` says too)."""
+    where all of them have equally many rows whatever the step (what `group_offsets` says too).  `few` False: a handful of tokens
+    goes to the tcgen05 kernel all the same."""
     if use_tensor_cores and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16:
         # products with many tokens go to the two-SM kernel, dense or grouped (it refuses, launching nothing, what it
         # does not take: few tokens per group, a row gather; features that are no multiple of 256 where they don't pay)
         rows, n = kw.get("m_rows", a.shape[0]), out.shape[1]
         # a handful of tokens: weights straight into registers (refuses, launching nothing, where the tcgen05 kernel is faster)
-        if (even_groups or rows <= 32) and K.gemm_few(a, w, out, mode, even_groups=even_groups, **kw):
+        if few and (even_groups or rows <= 32) and K.gemm_few(a, w, out, mode, even_groups=even_groups, **kw):
             return
         if use_paired_kernel and not single_cta_products.depth and "a_rows" not in kw and rows >= 512 and K.gemm_tc_pair(
                 a, w, out, mode, any_features=bool(n % 256) and K.gemm_tc_pair_pays(rows, n, a.shape[1], mode in K.GATED_MODES), **kw):

@@ -122,3 +122,26 @@ def test_products_that_gemm_tc_finishes_sooner_are_left_to_it(T, per_sm, Kd, gat
         out = torch.empty(T, N, device=DEV, dtype=torch.bfloat16)
         w = torch.empty(2 * N if gated else N, Kd, device=DEV, dtype=torch.bfloat16)
         assert not k.gemm_few(a, w, out, k.MODE_SWIGLU if gated else k.MODE_STORE)
+
+
+@pytest.mark.parametrize("T,top,taken", [(1, 1, 0), (2, 1, 0), (1, 2, 0), (4, 1, 2), (2, 2, 2)])
+@pytest.mark.parametrize("overlap", [True, False])
+def test_a_small_shared_expert_beside_one_or_two_routed_rows(monkeypatch, T, top, taken, overlap):
+    """Its two products stay on the tcgen05 kernel then, beside the routed ones and after them alike."""
+    from cpi_b200.config.spec import PartSpec
+    from cpi_b200.engine.batch import BatchStager
+    from cpi_b200.parts import Workspace, build_part
+    from cpi_b200.weights import DictSource
+    k = K()
+    part = build_part("feed_forward", PartSpec("moe_swiglu", {"hidden_size": 256, "num_experts": 8, "top_k": top, "expert_size": 128,
+                                                             "shared_size": 128, "router_gate": "softmax_chosen"}), "", workspace=Workspace(DEV))
+    g = torch.Generator(device=DEV).manual_seed(1)
+    part.load(DictSource({r.name: (torch.randn(*r.shape, generator=g, device=DEV) * 0.05).bfloat16() for r in part.requirements()}), DEV)
+    part.overlap_shared = overlap
+    calls, real = [], k.gemm_few
+    monkeypatch.setattr(k, "gemm_few", lambda *a, **kw: calls.append(real(*a, **kw)) or calls[-1])
+    stager = BatchStager(DEV)
+    batch = stager.stage(list(range(T)), [0] * T, [[0]] * T, [[]] * T, torch.bfloat16)
+    out = torch.zeros(T, 256, device=DEV)
+    part.forward(torch.randn(T, 256, generator=g, device=DEV).bfloat16(), out, batch)
+    assert sum(calls) == taken and bool(out.isfinite().all()) and bool(out.any())

@@ -27,3 +27,13 @@ def test_products_of_even_groups_lose_no_argument(monkeypatch, extra):
 def test_what_products_of_even_groups_leave_to_other_kernels(extra):
     a, w, out, groups = _operands()
     assert not K.gemm_few(a, w, out, even_groups=2, **{**groups, **extra})
+
+
+def test_a_product_may_be_kept_from_the_kernel_for_a_handful_of_tokens(monkeypatch):
+    a, w, out = torch.zeros(4, 16, dtype=torch.bfloat16), torch.zeros(8, 16, dtype=torch.bfloat16), torch.zeros(4, 8)
+    asked = []
+    monkeypatch.setattr(K, "gemm_few", lambda *args, **kw: asked.append("few") or True)
+    monkeypatch.setattr(K, "gemm_tc", lambda *args, **kw: asked.append("tc") or "few" not in kw)
+    linear.project(a, w, out)
+    linear.project(a, w, out, few=False)
+    assert asked == ["few", "tc"]
