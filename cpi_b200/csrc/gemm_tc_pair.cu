@@ -499,15 +499,18 @@ __global__ void __launch_bounds__(256) gemm_tc_pair_dual_kernel(const __grid_con
 
 // ---------------------------------------------------------------------------------------------- persistent
 // The same product with one pair per SM pair that works through a list of tiles (dense products only).
-// Six warps per CTA: 0-3 own the accumulator's lanes and run the epilogue, warp 4 issues the TMA loads,
-// warp 5 (of the leading CTA) the MMAs.  The stage ring runs on across tiles, and with one accumulator per
+// Warps 0-3 own the accumulator's lanes and run the epilogue, warp 4 issues the TMA loads, warp 5 (of the leading CTA) the
+// MMAs; the gated form has twelve warps, 8-11 a second group of the epilogue.  The stage ring runs on across tiles, and with one accumulator per
 // tile there are two accumulator buffers in tensor memory: the MMAs of tile j+1 run while tile j is turned
 // in shared memory and written out, so an SM pair's tiles follow each other at the tensor pipe's rate
 // instead of each paying fill, drain and epilogue.  With two accumulators, SwiGLU, the tensor memory
 // holds one tile, whose successor's MMAs wait until it has been read (its loads do not): two groups of four warps take half of
 // the tokens each, keep their gated products as packed bfloat16 in registers (64 a thread), give the accumulators
-// back and turn and store the tile under the next one's MMAs.  By four warps that gave them back with the last token stored,
-// gate/up of 16 experts of 2,048 x 2,048 took 147 us at 512 rows each, so 141.
+// back and turn and store the tile under the next one's MMAs.  A pair with one tile takes the loop over 16 tokens at a time that
+// the other forms take: all of that unrolled code, run once, costs more than it saves.  By four warps that gave the accumulators
+// back with the last token stored / by two groups / by two groups with the loop, in us: gate/up of 16 experts of 2,048 x 2,048
+// at 512 rows each 141 / 132 / 134; one tile a pair, 512 x 2,048 -> 8,192 pairs 34.0 / 36.0 / 32.9, 2,048 x 1,024 -> 2,048 24.2 / 25.6 /
+// 22.7, 8 experts of 2,048 x 1,024 at 192 rows 36.0 / 39.1 / 33.9.
 //   full[s] / empty[s]            stage ring, as above
 //   acc_full[b]                   MMA -> epilogue warps of both CTAs (commit with multicast)
 //   acc_empty[b] (in the leader)  epilogue warps of both CTAs -> MMA: one arrival per warp, 8 in all (16 with two groups)
@@ -760,12 +763,20 @@ __global__ void __launch_bounds__(MODE == kSwiglu ? 384 : 192) gemm_tc_pair_pers
       TO* out = reinterpret_cast<TO*>(p.out);
       if constexpr (MODE == kSwiglu) {
         const int mid = min((n_cols / 2 + 15) & ~15, n_valid_t), from = group_no ? mid : 0, valid = group_no ? n_valid_t - mid : mid;
-        uint32_t packed[64];
-        gated_read(lane_addr + from, lane_addr + BN + from, valid, valid, p.row_scale ? p.row_scale + t0 + from : nullptr, p.gate_act,
-                   p.gate_limit, packed);
-        give_back();
-        gated_store(packed, reinterpret_cast<__nv_bfloat16*>(epi) + group_no * (EPI_COLS / GROUPS * 128), wq, lane, n0, p.N, t0 + from, valid,
-                    out, p.ldo, p.out_rows, HalfSync{1 + group_no});
+        uint8_t* stage = epi + group_no * (EPI_COLS / GROUPS * 128 * sizeof(TO));
+        if (j > 0 || pid + n_clusters < n_tiles) {
+          uint32_t packed[64];
+          gated_read(lane_addr + from, lane_addr + BN + from, valid, valid, p.row_scale ? p.row_scale + t0 + from : nullptr, p.gate_act,
+                     p.gate_limit, packed);
+          give_back();
+          gated_store(packed, reinterpret_cast<__nv_bfloat16*>(stage), wq, lane, n0, p.N, t0 + from, valid, out, p.ldo, p.out_rows,
+                      HalfSync{1 + group_no});
+        } else {                                                 // the pair's only tile: nothing waits for the accumulators
+          auto ld = [&](int c, float* d) { tmem_ld16(lane_addr + from + c, d); };
+          auto ldu = [&](int c, float* d) { tmem_ld16(lane_addr + BN + from + c, d); };
+          epi::staged<MODE, TO, EPI_COLS / GROUPS>(stage, ld, ldu, wq, lane, n0, p.N, t0 + from, valid, (valid + 15) & ~15, out, p.ldo,
+                                                   p.out_rows, p.row_scale, HalfSync{1 + group_no}, p.gate_act, p.gate_limit);
+        }
       } else {
         auto ld = [&](int c, float* d) { tmem_ld16(lane_addr + c, d); };
         epi::staged<MODE, TO, EPI_COLS>(epi, ld, ld, warp, lane, n0, p.N, t0, n_valid_t, n_cols, out, p.ldo, p.out_rows,

@@ -164,8 +164,15 @@ def test_gemm_tensor_core_pair_kernel_grouped(counts, mode, persistent):
         K().gemm_pair_persistent(1)
 
 
-def _pair_kernel_grouped_case(counts, mode):
-    G, N, Kd = len(counts), 512, 320
+# several tiles a pair, whose accumulators the gated form gives back before it stores them; tiles whose tokens the first group of its
+# warps takes alone (5, 16), and that end within the second group's
+@pytest.mark.parametrize("counts", [[300, 5, 129, 83, 16, 256, 64, 700], [600, 0, 17, 31]])
+def test_gated_products_of_several_tiles_a_pair(counts):
+    _pair_kernel_grouped_case(counts, 2, N=8192, Kd=72)
+
+
+def _pair_kernel_grouped_case(counts, mode, N=512, Kd=320):
+    G = len(counts)
     M = sum(counts)
     w = rnd(G, 2 * N if mode == 2 else N, Kd, dtype=torch.bfloat16, seed=1, scale=Kd ** -0.5)
     a = rnd(M, Kd, dtype=torch.bfloat16)
