@@ -408,7 +408,7 @@ def qkv_prepare(qkv, q_out, k_cache, v_cache, page_table, page_size, token_seq, 
                 inv_freq=None, rotary_dims=0, write_kv=True, head_norm=False, interleaved=False, v_first=None,
                 v_mix=None, v_mix_mode=0, q2_out=None, k2_cache=None, values_from_keys=False, temperature=None,
                 rotary_amplitude=1.0, v_inv_freq=None):
-    """The general form of `qkv_post`, a block per token: rows [q | k | v] (float32 or the cache's dtype) get
+    """The general form of `qkv_post` (a warp per head for heads of 64 or 128, else a block per token): rows [q | k | v] (float32 or the cache's dtype) get
     their bias, q and k an RMS norm over the whole projection (`norm_whole`, weights `q_norm` / `k_norm`), the
     first `rotary_dims` elements of each head their rotation, and then (`head_norm` True or 1) every q and k head a
     weightless RMS norm with `norm_eps`; q goes to q_out, k and v into the cache pages.  `head_norm` 2: every q and k

@@ -40,16 +40,17 @@ DECAY_PREPASS_FROM = 16
 # set to False to run every recurrence token by token (tests compare the two)
 use_chunked_kernel = True
 # A bfloat16 prompt's recurrence runs in chunks when its longest portion has this many tokens: the scan's time goes with the
-# longest portion, the chunks' with all tokens.  Mixers of width 2,048, chunks / scan in us, a prompt of 200, of 130, 8 of 200
-# and 32 of 100 tokens: gated linear attention (8 heads, 128 x 256) 113 / 124, 98 / 92, 213 / 322, 402 / 681; state space (64
-# heads, 128 x 64) 121 / 172, 104 / 114, 406 / 536, 818 / 1,048; delta rule (8 heads, 128 x 256) 134 / 128, 117 / 95, 357 / 414,
-# 709 / 789, a prompt of 500 178 / 231.
+# longest portion, the chunks' with all tokens.  Mixers of width 2,048, chunks / scan in us, a prompt of 100, of 130, of 200, 8 of
+# 200 and 32 of 100 tokens: gated linear attention (8 heads, 128 x 256) 70 / 66, 69 / 71, 75 / 96, 148 / 297, 284 / 629; state space
+# (64 heads, 128 x 64) 74 / 90, 90 / 119, 108 / 163, 263 / 439, 539 / 850; delta rule (8 heads, 128 x 256) 104 / 75, 115 / 92, 130 / 123,
+# 275 / 360, 559 / 694, a prompt of 256 135 / 144, of 500 153 / 215.  The lines were drawn when the chunks of 200
+# tokens took 113, 121 and 134 us; where they win now lies below them, for the state space near 80 tokens.
 CHUNKS_FROM, DELTA_CHUNKS_FROM = 192, 256
 # Decays of at most this rank take their first projection as the last rows of the gla mixer's input product, in float32, and the
-# second from the FP32 pipe; wider ones two products of their own on the tensor cores.  All projections of a width of 2,048, 8
-# heads of 128 x 256, one way / the other in us: rank 16 10 / 15, 26 / 39 and 60 / 75 at 1, 512 and 2,048 tokens, rank 64 13 / 15, 30 /
-# 38 and 68 / 74 (8,192 tokens 221 / 215), rank 128 17 / 16, 35 / 39 and 76 / 76 (8,192 tokens 253 / 216), rank 256 26 / 17, 46 / 46
-# and 91 / 78; of a width of 512 with 64 x 64 at 2,048 tokens rank 16 26 / 38, 64 29 / 38, 128 34 / 38, 256 31 / 25.
+# second from the FP32 pipe; wider ones two products of their own on the tensor cores.  The mixer with a width of 2,048 and 8
+# heads of 128 x 256, one way / the other in us, at 1, 8, 512 and 2,048 tokens: rank 16 14 / 13, 16 / 16.5, 83 / 99 and 163 / 179, rank 64
+# 16.5 / 13, 18.5 / 17, 87 / 100 and 167 / 179, rank 128 20 / 13, 22 / 17, 95 / 99 and 182 / 179, rank 256 28 / 13, 32 / 17, 106 / 107 and 200 / 184.
+# (Up to rank 64 a prompt gains more than single tokens lose.)
 RIDING_RANK = 64
 # bytes of scratch for a step's chunks; a longer step runs in segments (a segment's states stay in the L2 between its passes)
 CHUNK_BYTES = 96 << 20
