@@ -209,7 +209,6 @@ __global__ void __launch_bounds__(NT) attention_decode_kernel(const __grid_const
 
   const int split = blockIdx.x, kvh = blockIdx.y, t = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  pdl_launch_dependents();
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) mbar_init(&full_bar[s], 1);
     abort_s = 0;
@@ -252,6 +251,7 @@ __global__ void __launch_bounds__(NT) attention_decode_kernel(const __grid_const
   if (tid == 0)
     for (; asked < STAGES && b_begin + asked < b_end && block_of(b_begin + asked) != b_hi; ++asked) load_tile(b_begin + asked, asked);
   pdl_wait();
+  pdl_launch_dependents();                                           // (in this order: it reads cached rows, see common.cuh)
   if (tid == 0)
     for (; asked < STAGES && b_begin + asked < b_end; ++asked) load_tile(b_begin + asked, asked);
 

@@ -91,8 +91,8 @@ __global__ void __launch_bounds__(kThreads) attention_prefill_kernel(const __gri
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
-  pdl_launch_dependents();                              // (not before the tensor memory is ours: see common.cuh)
   pdl_wait();
+  pdl_launch_dependents();                              // (in this order, and not before the tensor memory is ours: see common.cuh)
   const int tile = blockIdx.y, head = blockIdx.x;       // heads are the fast axis: all heads of the longest tile start first
   const int kvh = head / (p.n_heads / p.n_kv_heads);
   const int tok0 = p.tile_tok0[tile], rows = p.tile_rows[tile];

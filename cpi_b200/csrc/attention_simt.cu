@@ -44,8 +44,8 @@ struct QkvPostParams {
 
 template <typename T>
 __global__ void qkv_post_kernel(QkvPostParams p) {
+  pdl_launch_dependents();
   pdl_wait();
-  pdl_launch_dependents();                               // (in this order: it writes cached rows, see common.cuh)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int heads_total = p.n_heads + (p.write_kv ? 2 * p.n_kv_heads : 0);
   const int hs = blockIdx.y * (blockDim.x >> 5) + warp;       // head slot
@@ -130,6 +130,7 @@ __global__ void qkv_post_kernel(QkvPostParams p) {
 // sines and cosines once.  Same formulas as qkv_post_kernel; sums of squares in another order.
 __global__ void __launch_bounds__(256) qkv_post_d128_kernel(QkvPostParams p, int heads_per_block) {
   __shared__ float cos_s[64], sin_s[64];
+  pdl_launch_dependents();
   // positions and page tables are copied to the device before the step's first kernel and the frequencies
   // are constants: the angles do not wait for the kernel that writes q, k and v
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -140,7 +141,6 @@ __global__ void __launch_bounds__(256) qkv_post_d128_kernel(QkvPostParams p, int
     cos_s[tid] = c; sin_s[tid] = s;
   }
   pdl_wait();
-  pdl_launch_dependents();                               // (in this order: it writes cached rows, see common.cuh)
   __syncthreads();
   const int heads_total = p.n_heads + (p.write_kv ? 2 * p.n_kv_heads : 0);
   const int h_begin = blockIdx.y * heads_per_block, h_end = min(heads_total, h_begin + heads_per_block);
@@ -266,10 +266,10 @@ __device__ __forceinline__ void rot_pair(int d, int half, int interleaved, bool&
 
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(1024) qkv_prepare_kernel(QkvPrepParams p) {
+  pdl_launch_dependents();
   extern __shared__ float row_s[];                       // q then k of this token, float32
   __shared__ float scratch[32];
   pdl_wait();
-  pdl_launch_dependents();                               // (in this order: it writes cached rows, see common.cuh)
   const int t = blockIdx.x, tid = threadIdx.x;
   const int D = p.head_dim, DV = p.v_dim;
   const int nq = p.maps * p.n_heads * D, nk = p.write_kv ? p.maps * p.n_kv_heads * D : 0, nv = p.write_kv ? p.n_kv_heads * DV : 0;
@@ -471,8 +471,8 @@ __global__ void __launch_bounds__(1024) qkv_prepare_heads_kernel(QkvPrepParams p
   constexpr int D = 32 * E;
   __shared__ float scratch[32];
   __shared__ float2 turn[D / 2];                         // cosine, sine
+  pdl_launch_dependents();
   pdl_wait();
-  pdl_launch_dependents();                               // (in this order: it writes cached rows, see common.cuh)
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, warps = blockDim.x >> 5, lane = tid & 31;
   const TI* src = reinterpret_cast<const TI*>(p.qkv) + (size_t)t * p.qkv_stride + lane * E;
   const int nh = p.n_heads, nkv = p.write_kv ? p.n_kv_heads : 0;
@@ -602,8 +602,8 @@ constexpr int ATT_ACC = ATT_MAX_DIM / ATT_NT;
 
 template <typename T>
 __global__ void __launch_bounds__(ATT_NT) attention_general_kernel(AttnParams p) {
-  pdl_launch_dependents();
   pdl_wait();
+  pdl_launch_dependents();                       // (in this order: it reads cached rows, see common.cuh)
   __shared__ float q_s[ATT_MAX_DIM];
   __shared__ float p_s[ATT_NT];
   __shared__ size_t off_s[ATT_NT];

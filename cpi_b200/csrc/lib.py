@@ -1057,8 +1057,9 @@ def attention_decode(q, out, k_cache, v_cache, page_table, page_size, token_seq,
                      softcap=0.0):
     """bfloat16 attention of independent tokens against the paged cache, keys split over `n_splits` blocks.
     `sink`: float32 [heads] whose exponentials join the softmax denominators.  `keep_first`: with a sliding window,
-    a sequence's first positions that every later query still sees.  Of the rows it reads, the kernel launched before it on
-    the stream may store each token's own position and no other (older pages are read before that kernel ends)."""
+    a sequence's first positions that every later query still sees.  Of the rows it reads, what was launched since the
+    stream's last attention over this cache (or a copy, or any kernel that is not this library's) may have stored each token's own
+    position and no other: older pages are read before the kernels in front of this one end."""
     _need_cuda(q, out, k_cache, v_cache, page_table, token_seq, token_pos, seq_slot, sink)
     assert sink is None or (sink.dtype == torch.float32 and sink.is_contiguous() and sink.numel() == n_heads)
     assert q.is_contiguous() and out.is_contiguous() and q.dtype == out.dtype == k_cache.dtype == torch.bfloat16

@@ -81,6 +81,7 @@ __device__ __forceinline__ void group_columns(int g, int rot, int interleaved, i
 
 template <typename TO, int TAPS>
 __global__ void __launch_bounds__(QR_THREADS, TAPS > 4 ? 2 : QR_BLOCKS_PER_SM) qkv_conv_rotate_kernel(ConvRotParams p) {
+  pdl_launch_dependents();
   extern __shared__ float table_s[];               // [tb][pairs] cosines then sines: of q and k, then of v
   __shared__ size_t kv_row_s[QR_MAX_TB];
   const int tid = threadIdx.x, TB = p.tb;
@@ -149,7 +150,6 @@ __global__ void __launch_bounds__(QR_THREADS, TAPS > 4 ? 2 : QR_BLOCKS_PER_SM) q
     }
   }
   pdl_wait();
-  pdl_launch_dependents();                         // (in this order: it writes cached rows, see common.cuh)
   if (!live) return;
   // hist[j]: the input TAPS - 1 - j tokens before the current one
   float hist[TAPS > 1 ? TAPS - 1 : 1][8];

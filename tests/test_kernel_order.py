@@ -86,15 +86,14 @@ def test_index_arrays_are_read_before_the_wait_by_the_named_kernels_only():
     assert {k for k, text in waiting.items() if cached.search(text)} == {"attention_decode_kernel"}
 
 
-@pytest.mark.parametrize("name", ["attention_simt.cu:qkv_post_kernel", "attention_simt.cu:qkv_post_d128_kernel",
-                                  "attention_simt.cu:qkv_prepare_kernel", "attention_simt.cu:qkv_prepare_heads_kernel",
-                                  "rotate.cu:qkv_conv_rotate_kernel"])
-def test_kernels_that_store_cached_rows_wait_before_their_successors_start(name):
-    """`attention_decode` behind them reads rows of earlier positions before its own wait: those are complete once the storing
-    kernel has waited."""
+@pytest.mark.parametrize("name", ["attention_decode.cu:attention_decode_kernel", "attention_prefill.cu:attention_prefill_kernel",
+                                  "attention_simt.cu:attention_general_kernel", "attention_simt.cu:attention_f32_tile_kernel"])
+def test_attention_over_cached_keys_waits_before_its_successors_start(name):
+    """`attention_decode` of a later step reads rows of earlier positions before its own wait: they have been stored once the
+    attention kernel behind their launch has waited, and whatever starts after it finds them."""
     body = KERNELS[name]
-    assert "k_cache" in body and body.count("pdl_launch_dependents()") == 1
-    assert body.index("pdl_wait()") < body.index("pdl_launch_dependents()")
+    starts = [m.start() for m in re.finditer(r"pdl_launch_dependents\(\)", body)]
+    assert all(body.index("pdl_wait()") < s for s in starts)
 
 
 @pytest.mark.parametrize("name", ["chunk_state_kernel", "chunk_out_kernel", "chunk_out_step_kernel"])
