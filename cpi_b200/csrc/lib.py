@@ -910,7 +910,7 @@ def linear_chunks(k, q, v, state, out, batch, *, n_heads, heads_per_group, n_row
           _p(skip), c_int(dtype_code(sd)), _p(beta), c_long(0 if beta is None else beta.stride(0)), c_float(q_scale), _p(state),
           _p(out), c_long(out.stride(0)), _p(batch.seq_slot), _p(batch.seq_tok0), _p(batch.seq_new), c_int(batch.n_seqs),
           c_int(total), c_int(n_heads), c_int(heads_per_group), c_int(n_rows), c_int(n_cols), _p(scratch), c_int(seg),
-          _p(tc_error_flag(k.device)), _stream())
+          _p(device_error_flags(k.device)), _stream())      # (its first number is tc_error_flag; a slice costs 1 us of host)
     launch_count += 4 * -(-total // seg) - 1
 
 
